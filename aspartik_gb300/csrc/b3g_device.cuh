@@ -16,6 +16,7 @@
 #include <stdint.h>
 
 #include "index_width.hpp"
+#include "soft64.cuh"
 
 namespace b3g {
 
@@ -58,6 +59,7 @@ struct PtabParams {
 	uint32_t n;
 	uint32_t C;
 	void *ptab; // R [n][2][C][S+1][S]
+	SoftTab4 *soft; // [n][2][C] beside the four-state FP64 tables, or null
 };
 
 struct PruneParams {
@@ -66,6 +68,8 @@ struct PruneParams {
 	int32_t *scales;
 	const NodeOp *ops;
 	const void *ptab;
+	const SoftTab4 *soft; // four-state FP64 form: the tables as integers, or
+			      // null (the caller's own tables: plain walk)
 	const double *pi;
 	const uint32_t *weights;
 	double *site_lnl;   // [ldp]

@@ -224,6 +224,9 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		dev_alloc(d_model_, sizeof(ModelDev), "model");
 		dev_alloc(d_ptab_, (size_t)I_ * 2 * C_ * (S_ + 1) * S_ * rsz,
 			  "transition tables");
+		if (!f32_ && S_ == 4)
+			dev_alloc(d_soft_, (size_t)I_ * 2 * C_ * sizeof(SoftTab4),
+				  "integer transition tables");
 
 		off_pi_ = align_up((size_t)I_ * sizeof(NodeOp), 256);
 		off_runs_ = align_up(off_pi_ + S_ * sizeof(double), 256);
@@ -328,6 +331,8 @@ void Calculator::release()
 	cudaFree(d_lnl_);
 	cudaFree(d_model_);
 	cudaFree(d_ptab_);
+	cudaFree(d_soft_);
+	d_soft_ = nullptr;
 	cudaFree(own_d_stage_ ? own_d_stage_ : d_stage_);
 	cudaFreeHost(own_h_stage_ ? own_h_stage_ : h_stage_);
 	own_d_stage_ = nullptr;
@@ -621,6 +626,7 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 	pt.n = n;
 	pt.C = C_;
 	pt.ptab = d_ptab_;
+	pt.soft = d_soft_;
 	if (pp.tables_inline) {
 		pp.model = d_model_;
 		pp.lengths = pt.lengths;
@@ -638,6 +644,7 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 	pp.scales = d_scales_;
 	pp.ops = reinterpret_cast<const NodeOp *>(d_stage_);
 	pp.ptab = d_ptab_;
+	pp.soft = d_soft_;
 	pp.pi = reinterpret_cast<const double *>(d_stage_ + off_pi_);
 	pp.weights = d_weights_;
 	pp.site_lnl = d_site_;

@@ -208,6 +208,7 @@ class Calculator {
 	double *d_lnl_ = nullptr;
 	ModelDev *d_model_ = nullptr;
 	void *d_ptab_ = nullptr;
+	SoftTab4 *d_soft_ = nullptr; // four-state FP64 form: d_ptab_ as integers
 	unsigned char *d_stage_ = nullptr;
 
 	// pinned host staging

@@ -145,39 +145,6 @@ __device__ __forceinline__ int32_t rescale_pow2(float4 &y)
 // ---------------------------------------------------------------------------
 // transition matrices
 
-__device__ void transition4(const ModelDev *__restrict__ m, double d,
-			    double P[16])
-{
-	if (m->shortcuts && d > 20.0) {
-		// transition_freqs (substitution.rs:245-252)
-		for (int i = 0; i < 4; i++)
-			for (int j = 0; j < 4; j++)
-				P[i * 4 + j] = m->pi[j];
-		return;
-	}
-	if (m->shortcuts && d < 1e-10) {
-		// transition_q (substitution.rs:258-268): I + Q d, unit diagonal
-		for (int i = 0; i < 4; i++)
-			for (int j = 0; j < 4; j++)
-				P[i * 4 + j] = i == j ? 1.0 : m->Q[i * 4 + j] * d;
-		return;
-	}
-	double e[4];
-	for (int k = 0; k < 4; k++)
-		e[k] = exp(m->lambda[k] * d);
-	for (int i = 0; i < 4; i++) {
-		double t0 = m->V[i * 4 + 0] * e[0], t1 = m->V[i * 4 + 1] * e[1];
-		double t2 = m->V[i * 4 + 2] * e[2], t3 = m->V[i * 4 + 3] * e[3];
-		for (int j = 0; j < 4; j++) {
-			double s = t0 * m->Vinv[0 * 4 + j];
-			s = fma(t1, m->Vinv[1 * 4 + j], s);
-			s = fma(t2, m->Vinv[2 * 4 + j], s);
-			s = fma(t3, m->Vinv[3 * 4 + j], s);
-			P[i * 4 + j] = s;
-		}
-	}
-}
-
 // FP32 chosen form: P(t) in single precision from the FP64 eigensystem
 // (the decomposition of Q is the only FP64 work of this step; on GB300 FP64
 // issues at 1/64 of the FP32 rate).  The shortcut tests stay in FP64.
@@ -234,7 +201,80 @@ __device__ void transition4f(const ModelDev *__restrict__ m, double d,
 	transition4f_eig(m, eig, d, P);
 }
 
-template <typename R>
+// FP64 tables, four lanes a table: lane k takes exp(lambda_k d) (the other
+// three come by shuffles), then row i = k of P; the warp issues the
+// exponential once instead of four times and the products of a row instead
+// of the matrix (an FP64 instruction occupies the scheduler's pipe for 64
+// cycles whatever its active lanes).  The same operations in the same order
+// as the matrix form V diag(e) V^-1 row by row.  With `soft` the integer form of the table is written too.
+__global__ void __launch_bounds__(32) ptab4_f64_kernel(PtabParams prm)
+{
+	const uint32_t t = blockIdx.x * 32u + threadIdx.x;
+	const uint32_t id = t >> 2, i = t & 3u;
+	const bool live = id < prm.n * 2u * prm.C;
+	const uint32_t c = id % prm.C;
+	const uint32_t es = id / prm.C;
+	const ModelDev *m = prm.model;
+	double P[4] = {1.0, 1.0, 1.0, 1.0};
+	if (prm.matrices) {
+		if (live)
+			for (int j = 0; j < 4; j++)
+				P[j] = prm.matrices[(size_t)id * 16 + i * 4 + j];
+	} else {
+		const double d = live ? prm.lengths[es] * (prm.clock_rate * m->cat_rates[c])
+				      : 0.0;
+		const double mine = exp(m->lambda[i] * d);
+		double e[4];
+#pragma unroll
+		for (int k = 0; k < 4; k++)
+			e[k] = __shfl_sync(0xffffffffu, mine, k, 4);
+		if (m->shortcuts && d > 20.0) {
+			for (int j = 0; j < 4; j++)
+				P[j] = m->pi[j];
+		} else if (m->shortcuts && d < 1e-10) {
+			for (int j = 0; j < 4; j++)
+				P[j] = (int)i == j ? 1.0 : m->Q[i * 4 + j] * d;
+		} else {
+			const double t0 = m->V[i * 4 + 0] * e[0], t1 = m->V[i * 4 + 1] * e[1];
+			const double t2 = m->V[i * 4 + 2] * e[2], t3 = m->V[i * 4 + 3] * e[3];
+			for (int j = 0; j < 4; j++) {
+				double s = t0 * m->Vinv[0 * 4 + j];
+				s = fma(t1, m->Vinv[1 * 4 + j], s);
+				s = fma(t2, m->Vinv[2 * 4 + j], s);
+				s = fma(t3, m->Vinv[3 * 4 + j], s);
+				P[j] = s;
+			}
+		}
+	}
+	if (live) {
+		double *out = (double *)prm.ptab + (size_t)id * 20;
+		for (int j = 0; j < 4; j++)
+			out[j * 4 + i] = P[j];
+		out[16 + i] = 1.0;
+	}
+	if (!prm.soft)
+		return;
+	uint32_t plain = 0;
+	SoftTab4 *st = prm.soft + id;
+#pragma unroll
+	for (int k = 0; k < 5; k++) {
+		const double v = k < 4 ? P[k] : 1.0;
+		const uint32_t dh = (uint32_t)__double2hiint(v);
+		plain |= soft_normal(dh) ? 0u : 1u;
+		const SoftNum n = soft_split(dh, (uint32_t)__double2loint(v));
+		if (live) {
+			st->hi[k][i] = n.hi;
+			st->lo[k][i] = n.lo;
+			reinterpret_cast<uint16_t *>(st->e[k])[i] = (uint16_t)n.e;
+		}
+	}
+	plain |= __shfl_xor_sync(0xffffffffu, plain, 1);
+	plain |= __shfl_xor_sync(0xffffffffu, plain, 2);
+	if (live && i == 0)
+		st->plain = plain;
+}
+
+// FP32 tables, one thread a table
 __global__ void __launch_bounds__(32) ptab4_kernel(PtabParams prm)
 {
 	const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
@@ -242,38 +282,22 @@ __global__ void __launch_bounds__(32) ptab4_kernel(PtabParams prm)
 		return;
 	const uint32_t c = id % prm.C;
 	const uint32_t es = id / prm.C; // dirty index * 2 + side
-	R *out = (R *)prm.ptab + (size_t)id * 20;
-	if constexpr (sizeof(R) == 4) {
-		float P[16];
-		if (prm.matrices) {
-			const double *src = prm.matrices + (size_t)id * 16;
-			for (int k = 0; k < 16; k++)
-				P[k] = (float)src[k];
-		} else {
-			const double d = prm.lengths[es] *
-					 (prm.clock_rate * prm.model->cat_rates[c]);
-			transition4f(prm.model, d, P);
-		}
-		for (int k = 0; k < 4; k++)
-			for (int j = 0; j < 4; j++)
-				out[k * 4 + j] = P[j * 4 + k];
+	float *out = (float *)prm.ptab + (size_t)id * 20;
+	float P[16];
+	if (prm.matrices) {
+		const double *src = prm.matrices + (size_t)id * 16;
+		for (int k = 0; k < 16; k++)
+			P[k] = (float)src[k];
 	} else {
-		double P[16];
-		if (prm.matrices) {
-			const double *src = prm.matrices + (size_t)id * 16;
-			for (int k = 0; k < 16; k++)
-				P[k] = src[k];
-		} else {
-			const double d = prm.lengths[es] *
-					 (prm.clock_rate * prm.model->cat_rates[c]);
-			transition4(prm.model, d, P);
-		}
-		for (int k = 0; k < 4; k++)
-			for (int j = 0; j < 4; j++)
-				out[k * 4 + j] = (R)P[j * 4 + k];
+		const double d = prm.lengths[es] *
+				 (prm.clock_rate * prm.model->cat_rates[c]);
+		transition4f(prm.model, d, P);
 	}
+	for (int k = 0; k < 4; k++)
+		for (int j = 0; j < 4; j++)
+			out[k * 4 + j] = P[j * 4 + k];
 	for (int j = 0; j < 4; j++)
-		out[16 + j] = (R)1.0;
+		out[16 + j] = 1.0f;
 }
 
 // ---------------------------------------------------------------------------
@@ -685,6 +709,7 @@ __global__ void __launch_bounds__(512) prune4_plain_kernel(PruneParams prm)
 }
 
 // ---------------------------------------------------------------------------
+#include "prune4f64.cuh"
 #include "runs4.cuh"
 
 // ---------------------------------------------------------------------------
@@ -699,11 +724,10 @@ cudaError_t launch_ptab4(const PtabParams &p, bool f32, cudaStream_t s)
 	if (total == 0)
 		return cudaSuccess;
 	// one warp per block spreads the (mostly FP64/exp) work over many SMs
-	const uint32_t blocks = (total + 31u) / 32u;
 	if (f32)
-		ptab4_kernel<float><<<blocks, 32, 0, s>>>(p);
+		ptab4_kernel<<<(total + 31u) / 32u, 32, 0, s>>>(p);
 	else
-		ptab4_kernel<double><<<blocks, 32, 0, s>>>(p);
+		ptab4_f64_kernel<<<(4u * total + 31u) / 32u, 32, 0, s>>>(p);
 	return cudaGetLastError();
 }
 
@@ -738,6 +762,11 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 		return launch_prune4_t<V4f, true>(p, tile, s);
 	const dim3 grid(p.ldp / tile), block(tile, p.C);
 	const size_t smem = sizeof(double) * (2 * (size_t)p.C * tile + 32);
+	if (p.soft) {
+		const size_t ring = (size_t)(p.C * tile / 32u) * kF64Ring * sizeof(F64Entry);
+		prune4_f64_kernel<<<grid, block, smem + ring, s>>>(p);
+		return cudaGetLastError();
+	}
 	prune4_plain_kernel<<<grid, block, smem, s>>>(p);
 	return cudaGetLastError();
 }
