@@ -70,6 +70,8 @@ struct PruneParams {
 	const void *ptab;
 	const SoftTab4 *soft; // four-state FP64 form: the tables as integers, or
 			      // null (the caller's own tables: plain walk)
+	uint32_t f64_groups;  // with soft: groups a block of the run form (needs
+			      // runs, C * groups <= 16), 1: the serial form
 	const double *pi;
 	const uint32_t *weights;
 	double *site_lnl;   // [ldp]

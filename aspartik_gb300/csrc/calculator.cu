@@ -144,6 +144,13 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 			tc20_groups_fixed_ = true;
 		}
 	}
+	// groups of the FP64 run form (B3G_F64_GROUPS: 1, 2, 4, 8 or 16 where
+	// they fit a block; default: chosen per list)
+	if (const char *env = std::getenv("B3G_F64_GROUPS")) {
+		const int gr = std::atoi(env);
+		if (gr == 1 || gr == 2 || gr == 4 || gr == 8 || gr == 16)
+			f64_groups_ = static_cast<uint32_t>(gr);
+	}
 	use_direct_ = f32_ && S_ == 4 && (C_ == 1 || C_ == 2 || C_ == 4);
 	if (const char *env = std::getenv("B3G_DIRECT"))
 		use_direct_ = use_direct_ && std::atoi(env) != 0;
@@ -246,7 +253,7 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 			   "pinned lnl");
 		check_cuda(cudaHostGetDevicePointer((void **)&d_lnl_host_, h_lnl_, 0),
 			   "mapped lnl");
-		if (f32_ && S_ == 4) {
+		if (S_ == 4) {
 			check_cuda(cudaHostAlloc((void **)&h_bsums_,
 						 block_sums_cap_ * sizeof(double),
 						 cudaHostAllocMapped),
@@ -540,6 +547,24 @@ uint32_t Calculator::assign_slots(uint32_t n, uint32_t capacity)
 	return used;
 }
 
+// Groups a block of the FP64 walk's run form, 1 for the serial form.
+uint32_t Calculator::pick_f64_groups(uint32_t n) const
+{
+	if (f64_groups_)
+		return C_ * f64_groups_ <= 16 && n_runs_ <= 2048 ? f64_groups_ : 1u;
+	// doubled while a group's share of a run stays at two thirds of an
+	// entry or more, and every block still runs at once (16 warps an SM at
+	// this kernel's registers): us per whole tree with 1 / 2 / 4 / 8 / 16
+	// groups, 37 taxa x 1,147 patterns: 49 / 41 / 34 / 32 / 32; 64 x 7,855,
+	// one category: 71 / 57 / 47 / 45 / 62, four: 88 / 78 / 94; 128 x 17,764,
+	// one category: 137 / 102 / 81 / 92 / 120.  A path's runs have one entry.
+	const uint32_t warps = ldp_ / 32u * C_;
+	uint32_t G = 1;
+	while (2 * G * C_ <= 16 && 4 * G * n_runs_ <= 3 * n && 2 * G * warps <= 16 * num_sms_)
+		G *= 2;
+	return n_runs_ <= 2048 ? G : 1u;
+}
+
 void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 			bool want_cat)
 {
@@ -688,13 +713,20 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 		check_cuda(launch_prune4_runs(pp, ctas, block, stream_), "pruning kernel");
 	} else {
 		poll_result_ = false;
+		if (pp.soft) { // the blocks' sums go to mapped host memory here too
+			pp.f64_groups = pick_f64_groups(n);
+			pp.runs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
+			pp.n_runs = n_runs_;
+			pp.sums_host = d_bsums_;
+			arm_host_fold(ldp_ / (pp.f64_groups > 1 ? 32u : tile_));
+		}
 		check_cuda(launch_prune4(pp, f32_, tile_, stream_), "pruning kernel");
 	}
 	++in_flight_;
 	record(slot.k1);
 	slot.pending = timing_;
 	ring_next_ += timing_ ? 1 : 0;
-	if (!runs)
+	if (!pp.sums_host && !pp.lnl_host)
 		check_cuda(cudaMemcpyAsync(h_lnl_, d_lnl_, sizeof(double),
 					   cudaMemcpyDeviceToHost, stream_),
 			   "read lnl");
@@ -1072,7 +1104,8 @@ bool Calculator::wait_host_sums()
 
 double Calculator::fold_host_sums() const
 {
-	return fold_block_sums(h_bsums_, host_fold_blocks_);
+	return f32_ ? fold_block_sums(h_bsums_, host_fold_blocks_)
+		    : fold_block_sums_compensated(h_bsums_, host_fold_blocks_);
 }
 
 // Waits for the mapped result word to leave the sentinel; every 64 polls

@@ -208,6 +208,8 @@ class Calculator {
 	double *d_lnl_ = nullptr;
 	ModelDev *d_model_ = nullptr;
 	void *d_ptab_ = nullptr;
+	uint32_t f64_groups_ = 0; // 0: chosen per list
+	uint32_t pick_f64_groups(uint32_t n) const;
 	SoftTab4 *d_soft_ = nullptr; // four-state FP64 form: d_ptab_ as integers
 	unsigned char *d_stage_ = nullptr;
 

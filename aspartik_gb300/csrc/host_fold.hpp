@@ -6,9 +6,25 @@
 // offsets 16, 8, 4, 2, 1 leaves the total in lane 0.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 namespace b3g {
+
+// The plain FP64 form's fold: the sums in order with Neumaier compensation.
+// An impossible pattern (-inf) makes the sum -inf; the compensation of
+// infinities would be NaN, so it only tracks finite sums.
+inline double fold_block_sums_compensated(const double *sums, uint32_t count)
+{
+	double sum = 0.0, comp = 0.0;
+	for (uint32_t k = 0; k < count; ++k) {
+		const double x = sums[k], t = sum + x;
+		if (std::isfinite(t))
+			comp += std::fabs(sum) >= std::fabs(x) ? (sum - t) + x : (x - t) + sum;
+		sum = t;
+	}
+	return std::isfinite(sum) ? sum + comp : sum;
+}
 
 inline double fold_block_sums(const double *sums, uint32_t count)
 {

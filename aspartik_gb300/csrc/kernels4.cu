@@ -261,12 +261,19 @@ __global__ void __launch_bounds__(32) ptab4_f64_kernel(PtabParams prm)
 		const double v = k < 4 ? P[k] : 1.0;
 		const uint32_t dh = (uint32_t)__double2hiint(v);
 		plain |= soft_normal(dh) ? 0u : 1u;
-		const SoftNum n = soft_split(dh, (uint32_t)__double2loint(v));
-		if (live) {
-			st->hi[k][i] = n.hi;
-			st->lo[k][i] = n.lo;
-			reinterpret_cast<uint16_t *>(st->e[k])[i] = (uint16_t)n.e;
+		if (!live)
+			continue;
+		if (i == 0) {
+			st->row[k].d0 = v;
+			continue;
 		}
+		const SoftNum n = soft_split(dh, (uint32_t)__double2loint(v));
+		st->row[k].hi[i - 1] = n.hi;
+		(i == 1 ? st->row[k].lo1 : i == 2 ? st->row[k].lo2 : st->row[k].lo3) = n.lo;
+		if (i == 3)
+			st->e[k][1] = n.e;
+		else
+			reinterpret_cast<uint16_t *>(st->e[k])[i - 1] = (uint16_t)n.e;
 	}
 	plain |= __shfl_xor_sync(0xffffffffu, plain, 1);
 	plain |= __shfl_xor_sync(0xffffffffu, plain, 2);
@@ -417,99 +424,129 @@ __device__ __forceinline__ void neumaier_merge(double &sum, double &comp,
 }
 
 // Root of the schedule: category mixing, pattern weights, block sum and the
-// fold of all block sums by the last block to finish.  One `lead` thread per
-// (pattern, category) column reports its root dot product pi . x and count;
-// `pl` is the column's pattern inside the block.  Shared memory: 2 * nthr +
-// 32 doubles, nthr = threads per block.
+// fold of all block sums by the last block to finish (or by the host).  One
+// `lead` thread per (pattern, category) column reports its root dot product
+// pi . x and count; `pl` is the column's pattern inside the block, whose
+// patterns start at p0.  Shared memory: 2 * nthr + 32 doubles, nthr =
+// threads per block >= tp * C.
+//
+// The categories are mixed as sums scaled to the smallest (FP64 form:
+// e^-scale_ln a step) or largest (power-of-two form) count, then one
+// logarithm a pattern: an FP64 logarithm or exponential is 30 to 40
+// instructions of 64 cycles each here, and a logarithm a category, an
+// exponential a category and a logarithm on top (the log-sum-exp this
+// equals) took 15,000 to 20,000 cycles of a launch against 4,000.
 template <bool kPow2>
 __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem,
-					    uint32_t tp, uint32_t pl, uint32_t p,
+					    uint32_t tp, uint32_t pl, uint32_t p0,
 					    uint32_t c, bool lead, double root_dot,
 					    int32_t cnt)
 {
 	const uint32_t C = prm.C, ldp = prm.ldp;
-	const uint32_t nthr = blockDim.x * blockDim.y;
+	const uint32_t nthr = blockDim.x * blockDim.y * blockDim.z;
 	double *s_val = smem;                         // [tp * C]
 	int32_t *s_exp = (int32_t *)(smem + nthr);    // [tp * C]
 	double *s_warp = smem + 2 * nthr;             // [32]
 	__shared__ unsigned s_last;
 
 	if (lead) {
-		if constexpr (kPow2) {
-			s_val[c * tp + pl] = root_dot;
-			s_exp[c * tp + pl] = cnt;
-			if (prm.cat_lnl)
-				prm.cat_lnl[(size_t)c * ldp + p] =
-					log(root_dot) +
-					(double)cnt * 0.69314718055994530942;
-		} else {
+		s_val[c * tp + pl] = root_dot;
+		s_exp[c * tp + pl] = cnt;
+		if (prm.cat_lnl) {
 			// cpu4.rs:277-284 and :63-68; the count times scale_ln
 			// is an unsigned 32-bit product as in the reference
-			const double lcat = log(root_dot) -
-					    (double)((uint32_t)cnt * prm.scale_ln);
-			s_val[c * tp + pl] = lcat;
-			if (prm.cat_lnl)
-				prm.cat_lnl[(size_t)c * ldp + p] = lcat;
+			const double off =
+				kPow2 ? (double)cnt * 0.69314718055994530942
+				      : -(double)((uint32_t)cnt * prm.scale_ln);
+			prm.cat_lnl[(size_t)c * ldp + p0 + pl] = log(root_dot) + off;
 		}
 	}
 	__syncthreads();
 
+	const uint32_t tid =
+		(threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+	const uint32_t lane = tid & 31u, warp = tid >> 5;
 	double contrib = 0.0;
-	if (c == 0 && lead) {
+	if (tid < tp) {
 		double site;
 		if constexpr (kPow2) {
 			// sum_c s_c 2^E_c = 2^Emax sum_c s_c 2^(E_c - Emax)
 			int32_t emax = INT32_MIN;
 			for (uint32_t k = 0; k < C; k++)
-				if (s_val[k * tp + pl] > 0.0)
-					emax = max(emax, s_exp[k * tp + pl]);
+				if (s_val[k * tp + tid] > 0.0)
+					emax = max(emax, s_exp[k * tp + tid]);
 			if (emax == INT32_MIN) {
 				site = -INFINITY;
 			} else {
 				double acc = 0.0;
 				for (uint32_t k = 0; k < C; k++)
-					acc += scalbn(s_val[k * tp + pl],
-						      s_exp[k * tp + pl] - emax);
+					acc += scalbn(s_val[k * tp + tid],
+						      s_exp[k * tp + tid] - emax);
 				site = log(acc) +
 				       (double)emax * 0.69314718055994530942 +
 				       prm.log_inv_c;
 			}
 		} else {
 			// log_sum_exp (likelihood/mod.rs:141-151) + ln(1/C)
-			// (gamma.rs:155-165); exact identity for C = 1
-			double mx = -INFINITY;
-			for (uint32_t k = 0; k < C; k++)
-				mx = fmax(mx, s_val[k * tp + pl]);
-			if (mx == -INFINITY) {
-				site = -INFINITY;
-			} else {
-				double se = 0.0;
-				for (uint32_t k = 0; k < C; k++)
-					se += exp(s_val[k * tp + pl] - mx);
-				site = mx + log(se) + prm.log_inv_c;
+			// (gamma.rs:155-165), scaled to the smallest count (as
+			// unsigned products with scale_ln) of the categories above
+			// zero; classes by bit pattern, as the largest-term form
+			// treats them: no category above zero -> -inf, else a
+			// negative, NaN or infinite one -> NaN
+			constexpr long long kInf = 0x7FF0000000000000ll;
+			uint32_t least = 0xFFFFFFFFu;
+			bool any = false, bad = false;
+			for (uint32_t k = 0; k < C; k++) {
+				const long long u = __double_as_longlong(s_val[k * tp + tid]);
+				if (u > 0 && u <= kInf) {
+					any = true;
+					least = min(least, (uint32_t)s_exp[k * tp + tid] *
+								   prm.scale_ln);
+				}
+				bad = bad || u >= kInf || (u < 0 && (u << 1) != 0);
 			}
+			double acc = s_val[tid];
+			if (C > 1) {
+				acc = 0.0;
+				for (uint32_t k = 0; k < C; k++) {
+					double v = s_val[k * tp + tid];
+					const uint32_t steps =
+						(uint32_t)s_exp[k * tp + tid] * prm.scale_ln;
+					if (steps > least) // zero or scaled further
+						v *= exp((double)least - (double)steps);
+					acc += v;
+				}
+			}
+			site = !any ? -INFINITY
+			       : bad ? NAN
+				     : log(acc) - (double)least + prm.log_inv_c;
 		}
-		prm.site_lnl[p] = site;
-		const uint32_t w = prm.weights[p];
+		prm.site_lnl[p0 + tid] = site;
+		const uint32_t w = prm.weights[p0 + tid];
 		contrib = w ? site * (double)w : 0.0;
 	}
 
-	// block sum over the category-0 warps, in a fixed order
-	const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
-	const uint32_t lane = tid & 31u, warp = tid >> 5;
-	for (int off = 16; off > 0; off >>= 1)
-		contrib += __shfl_down_sync(0xffffffffu, contrib, off);
-	if (c == 0 && lane == 0)
-		s_warp[warp] = contrib;
+	// block sum over the warps that hold patterns, in a fixed order
+	if (warp * 32u < tp) {
+		for (int off = 16; off > 0; off >>= 1)
+			contrib += __shfl_down_sync(0xffffffffu, contrib, off);
+		if (lane == 0)
+			s_warp[warp] = contrib;
+	}
 	__syncthreads();
 	if (tid == 0) {
 		double bsum = 0.0;
-		for (uint32_t w = 0; w < blockDim.x / 32u; w++)
+		for (uint32_t w = 0; w < (tp + 31u) / 32u; w++)
 			bsum += s_warp[w];
-		prm.block_sums[blockIdx.x] = bsum;
-		__threadfence();
-		const unsigned t = atomicAdd(prm.ticket, 1u);
-		s_last = (t == gridDim.x - 1u);
+		if (prm.sums_host) { // the host folds the blocks' sums
+			prm.sums_host[blockIdx.x] = bsum;
+			s_last = 0u;
+		} else {
+			prm.block_sums[blockIdx.x] = bsum;
+			__threadfence();
+			const unsigned t = atomicAdd(prm.ticket, 1u);
+			s_last = (t == gridDim.x - 1u);
+		}
 	}
 	__syncthreads();
 	if (!s_last)
@@ -615,11 +652,12 @@ __global__ void __launch_bounds__(512) prune4_kernel(PruneParams prm)
 				(double)prm.pi[1] * (double)y.y +
 				(double)prm.pi[2] * (double)y.z +
 				(double)prm.pi[3] * (double)y.w;
-	finish_root<kPow2>(prm, smem, tp, threadIdx.x, p, c, true, root_dot, cnt);
+	finish_root<kPow2>(prm, smem, tp, threadIdx.x, p0, c, true, root_dot, cnt);
 }
 
 // ---------------------------------------------------------------------------
-// Plain FP64 form: the same walk with every child read straight from
+// Plain FP64 form on the caller's own tables (the allocation-free entry
+// point; calculators walk with prune4_f64_kernel): every child read straight from
 // global memory (tip codes included) and 64-bit indices formed per access.
 // On this part the FP64 arithmetic dominates; the shared-memory tip tile and
 // hoisted indexing of prune4_kernel, which help the FP32 walk, measured 19 %
@@ -705,7 +743,8 @@ __global__ void __launch_bounds__(512) prune4_plain_kernel(PruneParams prm)
 	}
 	const double root_dot = prm.pi[0] * y.x + prm.pi[1] * y.y + prm.pi[2] * y.z +
 				prm.pi[3] * y.w;
-	finish_root<false>(prm, smem, tp, threadIdx.x, p, c, true, root_dot, cnt);
+	finish_root<false>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, true, root_dot,
+			   cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -763,8 +802,21 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 	const dim3 grid(p.ldp / tile), block(tile, p.C);
 	const size_t smem = sizeof(double) * (2 * (size_t)p.C * tile + 32);
 	if (p.soft) {
-		const size_t ring = (size_t)(p.C * tile / 32u) * kF64Ring * sizeof(F64Entry);
-		prune4_f64_kernel<<<grid, block, smem + ring, s>>>(p);
+		const bool narrow = narrow_index((uint64_t)p.num_leaves * 2, p.C, p.ldp);
+		const uint32_t warps = p.f64_groups > 1 ? p.C * p.f64_groups : p.C * tile / 32u;
+		const size_t bytes = sizeof(double) * (64 * (size_t)warps + 32) +
+				     (size_t)warps * kF64Ring * sizeof(F64Entry);
+		if (p.f64_groups > 1) {
+			if (warps > 16 || !p.runs || p.n_runs > 2048)
+				return cudaErrorInvalidValue;
+			auto kern = narrow ? prune4_f64_runs_kernel<uint32_t>
+					   : prune4_f64_runs_kernel<size_t>;
+			kern<<<p.ldp / 32u, dim3(32, p.C, p.f64_groups),
+			       bytes + (p.n_runs + 1) * sizeof(uint32_t), s>>>(p);
+			return cudaGetLastError();
+		}
+		auto kern = narrow ? prune4_f64_kernel<uint32_t> : prune4_f64_kernel<size_t>;
+		kern<<<grid, block, bytes, s>>>(p);
 		return cudaGetLastError();
 	}
 	prune4_plain_kernel<<<grid, block, smem, s>>>(p);

@@ -225,5 +225,6 @@ __global__ void __launch_bounds__(256) prune20_kernel(PruneParams prm)
 #pragma unroll
 	for (int i = 0; i < S; i++)
 		root_dot = fma(prm.pi[i], (double)y[i], root_dot);
-	finish_root<kPow2>(prm, smem, tp, threadIdx.x, p, c, true, root_dot, cnt);
+	finish_root<kPow2>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, true, root_dot,
+			   cnt);
 }

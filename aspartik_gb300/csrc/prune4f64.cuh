@@ -12,9 +12,16 @@
 //   - Children: the partials of entry i + 1 are loaded before entry i is
 //     computed; a child that is entry i's output is taken from registers (no
 //     other output can be missing: this thread stored it earlier).
-//   - Arithmetic: soft_dot4 and soft_mul_round.  A lane whose inputs or
+//   - Arithmetic: soft_dot4, soft_mul_round and soft_scale.  A lane whose inputs or
 //     result are not positive normal numbers, and a warp whose table is
 //     not, take the FP64 instructions of the plain walk for that entry.
+//
+// Whole tree, 256 taxa x 17,764 patterns, four categories: 1,290 us as the
+// plain walk (bound by the FP64 pipe), 400 us here (about 430 instructions a
+// column and entry at 3.65 warps a scheduler: issue and dependent latency).
+// Tried and slower: four lanes a column, one state each (1,027 against 480
+// us, and 50 against 34 us on a 64-taxon path: the inputs are split and the
+// table words read four times over).
 
 constexpr uint32_t kF64Ring = 4;
 struct __align__(16) F64Entry {
@@ -39,65 +46,80 @@ template <int kPending> __device__ __forceinline__ void cp_async_wait()
 	asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-// A child's contribution: four significands, their exponents and whether
-// the soft arithmetic holds for it.
+// A child's contribution: state 0 as a double, states 1..3 as significands
+// with their exponents (value = m 2^e).
 struct SoftVec {
-	uint64_t m[4];
-	int32_t e[4]; // value = m 2^e
+	double d0;
+	uint64_t m[3];
+	int32_t e[3];
 };
+
+__device__ __forceinline__ uint64_t soft_pair(uint32_t hi, uint32_t lo)
+{
+	return ((uint64_t)hi << 32) | lo;
+}
+
+__device__ __forceinline__ SoftRow4 soft_row(const SoftRow4 &r)
+{
+	const uint4 a = *reinterpret_cast<const uint4 *>(&r);
+	const uint4 b = *(reinterpret_cast<const uint4 *>(&r) + 1);
+	SoftRow4 v;
+	v.hi[0] = a.x;
+	v.hi[1] = a.y;
+	v.hi[2] = a.z;
+	v.lo1 = a.w;
+	v.lo2 = b.x;
+	v.lo3 = b.y;
+	v.d0 = __hiloint2double((int)b.w, (int)b.z);
+	return v;
+}
 
 __device__ __forceinline__ void soft_tip(const SoftTab4 &t, uint32_t code, SoftVec &v)
 {
-	const uint4 hi = *reinterpret_cast<const uint4 *>(t.hi[code]);
-	const uint4 lo = *reinterpret_cast<const uint4 *>(t.lo[code]);
+	const SoftRow4 r = soft_row(t.row[code]);
 	const uint2 e = *reinterpret_cast<const uint2 *>(t.e[code]);
-	v.m[0] = ((uint64_t)hi.x << 32) | lo.x;
-	v.m[1] = ((uint64_t)hi.y << 32) | lo.y;
-	v.m[2] = ((uint64_t)hi.z << 32) | lo.z;
-	v.m[3] = ((uint64_t)hi.w << 32) | lo.w;
+	v.d0 = r.d0;
+	v.m[0] = soft_pair(r.hi[0], r.lo1);
+	v.m[1] = soft_pair(r.hi[1], r.lo2);
+	v.m[2] = soft_pair(r.hi[2], r.lo3);
 	v.e[0] = (int32_t)(e.x & 0xFFFFu) - kSoftBias;
 	v.e[1] = (int32_t)(e.x >> 16) - kSoftBias;
-	v.e[2] = (int32_t)(e.y & 0xFFFFu) - kSoftBias;
-	v.e[3] = (int32_t)(e.y >> 16) - kSoftBias;
+	v.e[2] = (int32_t)e.y - kSoftBias;
 }
 
-// Sums sum_k P[i][k] x[k], i = 0..3; false: some x[k] is not a positive
-// normal number (the sums are then meaningless).
+// Sums sum_k P[i][k] x[k]; false: some x[k] is not a positive normal number
+// (the integer sums are then meaningless).
 __device__ __forceinline__ bool soft_dot4(const SoftTab4 &t, const double4_32a &x, SoftVec &v)
 {
 	const double xs[4] = {x.x, x.y, x.z, x.w};
 	SoftNum n[4];
 	bool ok = true;
-	uint32_t s01[4], s23[4];
+	uint32_t s12[4], s3[4];
 #pragma unroll
 	for (int k = 0; k < 4; ++k) {
 		const uint32_t dh = (uint32_t)__double2hiint(xs[k]);
 		ok = ok && soft_normal(dh);
 		n[k] = soft_split(dh, (uint32_t)__double2loint(xs[k]));
-		const uint32_t e2 = __byte_perm(n[k].e, 0, 0x1010);
 		const uint2 te = *reinterpret_cast<const uint2 *>(t.e[k]);
-		s01[k] = te.x + e2; // both halves stay below 4096
-		s23[k] = te.y + e2;
+		s12[k] = te.x + __byte_perm(n[k].e, 0, 0x1010); // halves below 4096
+		s3[k] = te.y + n[k].e;
 	}
-	const uint32_t m01 = soft_max2(soft_max2(s01[0], s01[1]), soft_max2(s01[2], s01[3]));
-	const uint32_t m23 = soft_max2(soft_max2(s23[0], s23[1]), soft_max2(s23[2], s23[3]));
-#pragma unroll
-	for (int i = 0; i < 4; ++i)
-		v.m[i] = 0;
+	const uint32_t m12 =
+		soft_max2(soft_max2(s12[0], s12[1]), soft_max2(s12[2], s12[3]));
+	const uint32_t m3 = max(max(s3[0], s3[1]), max(s3[2], s3[3]));
+	v.m[0] = v.m[1] = v.m[2] = 0;
 #pragma unroll
 	for (int k = 0; k < 4; ++k) {
-		const uint4 hi = *reinterpret_cast<const uint4 *>(t.hi[k]);
-		const uint4 lo = *reinterpret_cast<const uint4 *>(t.lo[k]);
-		const uint32_t d01 = m01 - s01[k], d23 = m23 - s23[k]; // no borrow
-		v.m[0] += soft_shr(soft_prod(n[k].hi, n[k].lo, hi.x, lo.x), d01 & 0xFFFFu);
-		v.m[1] += soft_shr(soft_prod(n[k].hi, n[k].lo, hi.y, lo.y), d01 >> 16);
-		v.m[2] += soft_shr(soft_prod(n[k].hi, n[k].lo, hi.z, lo.z), d23 & 0xFFFFu);
-		v.m[3] += soft_shr(soft_prod(n[k].hi, n[k].lo, hi.w, lo.w), d23 >> 16);
+		const SoftRow4 r = soft_row(t.row[k]);
+		v.d0 = k == 0 ? r.d0 * xs[0] : fma(r.d0, xs[k], v.d0);
+		const uint32_t d12 = m12 - s12[k], d3 = m3 - s3[k]; // no borrow
+		v.m[0] += soft_shr(soft_prod(n[k].hi, n[k].lo, r.hi[0], r.lo1), d12 & 0xFFFFu);
+		v.m[1] += soft_shr(soft_prod(n[k].hi, n[k].lo, r.hi[1], r.lo2), d12 >> 16);
+		v.m[2] += soft_shr(soft_prod(n[k].hi, n[k].lo, r.hi[2], r.lo3), d3);
 	}
-	v.e[0] = (int32_t)(m01 & 0xFFFFu) - kSoftDotBias;
-	v.e[1] = (int32_t)(m01 >> 16) - kSoftDotBias;
-	v.e[2] = (int32_t)(m23 & 0xFFFFu) - kSoftDotBias;
-	v.e[3] = (int32_t)(m23 >> 16) - kSoftDotBias;
+	v.e[0] = (int32_t)(m12 & 0xFFFFu) - kSoftDotBias;
+	v.e[1] = (int32_t)(m12 >> 16) - kSoftDotBias;
+	v.e[2] = (int32_t)m3 - kSoftDotBias;
 	return ok;
 }
 
@@ -107,25 +129,72 @@ struct F64Child {
 	uint32_t code;
 };
 
-// The same entry in FP64 instructions (plain_batch's arithmetic), from the
-// double tables in global memory.
-__device__ __noinline__ double4_32a f64_plain_entry(const double4_32a *tl,
-						    const double4_32a *tr, uint32_t left,
-						    uint32_t right, F64Child l, F64Child r)
+// Four doubles of a partial, 32-byte aligned.  Volatile, so that the load
+// stays where it is written, ahead of the previous entry's arithmetic (left
+// to the compiler it sinks below it, and every entry then waits a memory
+// round trip: 400 of 3,080 cycles an entry).
+__device__ __forceinline__ double4_32a ld_partial(const double4_32a *p)
 {
-	const double4_32a a = (left & kTipBit) ? tl[l.code] : v4_apply(tl, l.x);
-	const double4_32a b = (right & kTipBit) ? tr[r.code] : v4_apply(tr, r.x);
-	return v4_mul(a, b);
+	double4_32a v;
+	asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+		     : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+		     : "l"(p)
+		     : "memory");
+	return v;
 }
 
-// One entry for one column: its value before rescaling.
-__device__ __forceinline__ double4_32a f64_entry(const F64Entry &en, const double4_32a *ptab,
-						 uint32_t i, uint32_t C, uint32_t c,
-						 const F64Child &l, const F64Child &r)
+template <typename Idx>
+__device__ __forceinline__ void f64_load(const PruneParams &prm, uint32_t id,
+					 uint32_t forward, uint32_t p, Idx stride, Idx col,
+					 F64Child &in)
 {
-	const NodeOp op = en.op;
-	SoftVec a, b;
+	if (id & kTipBit) {
+		in.code = prm.tips[(size_t)(id & ~kTipBit) * prm.ldp + p];
+		in.s = 0;
+	} else if (id != forward) {
+		const Idx ix = (Idx)id * stride + col;
+		in.x = ld_partial((const double4_32a *)prm.partials + ix);
+		in.s = prm.scales[ix];
+	}
+}
+
+// Entry i in FP64 instructions (plain_batch's arithmetic), from the double
+// tables and the inputs in global memory (a forwarded one was stored by
+// this thread), so that nothing of it stays in registers while the integer
+// form runs.
+__device__ __forceinline__ double4_32a f64_apply_plain(const PruneParams &prm,
+							const double4_32a *tab, uint32_t id,
+							uint32_t p, uint32_t c)
+{
+	if (id & kTipBit)
+		return tab[prm.tips[(size_t)(id & ~kTipBit) * prm.ldp + p]];
+	const double4_32a *partials = (const double4_32a *)prm.partials;
+	return v4_apply(tab, partials[((size_t)id * prm.C + c) * prm.ldp + p]);
+}
+__device__ __noinline__ double4_32a f64_plain_entry(const PruneParams &prm, uint32_t left,
+						    uint32_t right, uint32_t i, uint32_t p,
+						    uint32_t c)
+{
+	const double4_32a *tl =
+		(const double4_32a *)prm.ptab + ((size_t)(2 * i) * prm.C + c) * 5;
+	return v4_mul(f64_apply_plain(prm, tl, left, p, c),
+		      f64_apply_plain(prm, tl + (size_t)prm.C * 5, right, p, c));
+}
+
+// One entry for one column.  Returns the number of rescalings (0 or 1) by
+// cpu4.rs:403-433's rule: all four entries below the threshold, and none at
+// tip-tip nodes (cpu4.rs:288-318).  The threshold is positive, so comparing
+// the bits of non-negative numbers as integers decides as comparing the
+// doubles does.
+__device__ __forceinline__ int32_t f64_entry(const PruneParams &prm, const F64Entry &en,
+					     const NodeOp &op, uint32_t i, uint32_t p,
+					     uint32_t c, const F64Child &l, const F64Child &r,
+					     const SoftNum &mult, double4_32a &y)
+{
+	const bool cherry = ((op.left & op.right) & kTipBit) != 0;
+	const uint64_t thr = (uint64_t)__double_as_longlong(prm.scale_threshold);
 	bool ok = (en.tab[0].plain | en.tab[1].plain) == 0u;
+	SoftVec a, b;
 	if (op.left & kTipBit)
 		soft_tip(en.tab[0], l.code, a);
 	else
@@ -134,128 +203,190 @@ __device__ __forceinline__ double4_32a f64_entry(const F64Entry &en, const doubl
 		soft_tip(en.tab[1], r.code, b);
 	else
 		ok = soft_dot4(en.tab[1], r.x, b) && ok;
-	uint64_t bits[4];
+	y.x = a.d0 * b.d0;
+	uint64_t bits[3];
 #pragma unroll
-	for (int q = 0; q < 4; ++q) {
+	for (int k = 0; k < 3; ++k) {
 		bool in;
-		bits[q] = soft_mul_round(a.m[q], a.e[q], b.m[q], b.e[q], in);
+		bits[k] = soft_mul_round(a.m[k], a.e[k], b.m[k], b.e[k], in);
 		ok = ok && in;
 	}
-	double4_32a y;
-	y.x = __longlong_as_double((long long)bits[0]);
-	y.y = __longlong_as_double((long long)bits[1]);
-	y.z = __longlong_as_double((long long)bits[2]);
-	y.w = __longlong_as_double((long long)bits[3]);
 	if (!ok) {
-		const double4_32a *tl = ptab + ((size_t)(2 * i) * C + c) * 5;
-		y = f64_plain_entry(tl, tl + (size_t)C * 5, op.left, op.right, l, r);
+		y = f64_plain_entry(prm, op.left, op.right, i, p, c);
+		return cherry ? 0
+			      : rescale_threshold(y, prm.scale_threshold, prm.scale_mult);
 	}
-	return y;
+	int32_t own = 0;
+	if (!cherry && bits[0] < thr && bits[1] < thr && bits[2] < thr &&
+	    (uint64_t)__double_as_longlong(y.x) < thr) {
+		own = 1;
+		y.x *= prm.scale_mult;
+#pragma unroll
+		for (int k = 0; k < 3; ++k)
+			bits[k] = soft_scale(bits[k], mult);
+	}
+	y.y = __longlong_as_double((long long)bits[0]);
+	y.z = __longlong_as_double((long long)bits[1]);
+	y.w = __longlong_as_double((long long)bits[2]);
+	return own;
 }
 
-// rescale_threshold with the comparisons on the bit patterns: thr > 0, so a
-// double is below it exactly when its bits, as a signed integer, are (all
-// negative numbers included; a NaN made here is positive and is not).
-__device__ __forceinline__ int32_t f64_rescale(double4_32a &y, double thr, double mult)
+// The warp's copy of entry e (schedule word and the two tables of category
+// c) into `dst`, a 16-byte piece a lane; commits a group in any case.
+__device__ __forceinline__ void f64_fill(const PruneParams &prm, F64Entry *dst, uint32_t e,
+					 uint32_t c, uint32_t lane)
 {
-	const long long t = __double_as_longlong(thr);
-	if (__double_as_longlong(y.x) < t && __double_as_longlong(y.y) < t &&
-	    __double_as_longlong(y.z) < t && __double_as_longlong(y.w) < t) {
-		y.x *= mult;
-		y.y *= mult;
-		y.z *= mult;
-		y.w *= mult;
-		return 1;
+	if (e < prm.n && lane < 27) {
+		const uint32_t side = lane < 14 ? 0u : 1u, k = lane - 1 - 13 * side;
+		const void *src =
+			lane == 0 ? (const void *)(prm.ops + e)
+				  : (const void *)((const uint4 *)(prm.soft +
+								   ((size_t)(2 * e + side) * prm.C + c)) +
+						   k);
+		cp_async16((uint4 *)dst + lane, src);
 	}
-	return 0;
+	cp_async_commit();
 }
 
-__device__ __forceinline__ void f64_load(const PruneParams &prm,
-					 const double4_32a *__restrict__ partials, uint32_t id,
-					 uint32_t forward, uint32_t p, uint32_t c, F64Child &in)
+__device__ __forceinline__ double f64_root_dot(const PruneParams &prm, const double4_32a &y)
 {
-	if (id & kTipBit) {
-		in.code = prm.tips[(size_t)(id & ~kTipBit) * prm.ldp + p];
-		in.s = 0;
-	} else if (id != forward) {
-		const size_t ix = ((size_t)id * prm.C + c) * prm.ldp + p;
-		in.x = partials[ix];
-		in.s = prm.scales[ix];
-	}
+	return prm.pi[0] * y.x + prm.pi[1] * y.y + prm.pi[2] * y.z + prm.pi[3] * y.w;
 }
 
+// Serial form: a thread walks its column's whole list.
+template <typename Idx>
 __global__ void __launch_bounds__(512) prune4_f64_kernel(PruneParams prm)
 {
 	const uint32_t tp = blockDim.x, c = threadIdx.y, C = prm.C;
 	const uint32_t p = blockIdx.x * tp + threadIdx.x;
-	double4_32a *partials = (double4_32a *)prm.partials;
+	const Idx stride = (Idx)C * prm.ldp, col = (Idx)c * prm.ldp + p;
 	extern __shared__ __align__(16) double smem[];
 	const uint32_t tid = threadIdx.y * tp + threadIdx.x, lane = tid & 31u;
 	F64Entry *ring = reinterpret_cast<F64Entry *>(smem + 2 * tp * C + 32) +
 			 (tid >> 5) * kF64Ring;
-	auto fill = [&](uint32_t e) {
-		if (e < prm.n && lane < 27) {
-			F64Entry *dst = ring + (e & (kF64Ring - 1));
-			const uint32_t side = lane < 14 ? 0u : 1u, q = lane - 1 - 13 * side;
-			const void *src =
-				lane == 0 ? (const void *)(prm.ops + e)
-					  : (const void *)((const uint4 *)(prm.soft +
-									   ((size_t)(2 * e + side) * C + c)) +
-							   q);
-			cp_async16((uint4 *)dst + lane, src);
+#pragma unroll
+	for (uint32_t e = 0; e < kF64Ring; ++e)
+		f64_fill(prm, ring + e, e, c, lane);
+	cp_async_wait<kF64Ring - 2>(); // entries 0 and 1 have landed
+	__syncwarp();
+	const NodeOp none{kTipBit, kTipBit, kTipBit, 0};
+	NodeOp op = ring[0].op, nop = prm.n > 1 ? ring[1].op : none;
+	F64Child l, r;
+	f64_load<Idx>(prm, op.left, kTipBit, p, stride, col, l);
+	f64_load<Idx>(prm, op.right, kTipBit, p, stride, col, r);
+	const SoftNum mult = soft_split((uint32_t)__double2hiint(prm.scale_mult),
+					(uint32_t)__double2loint(prm.scale_mult));
+	double4_32a y = v4_make<double4_32a, double>(0, 0, 0, 0);
+	int32_t cnt = 0;
+	for (uint32_t i = 0; i < prm.n; ++i) {
+		F64Child nl, nr;
+		if (i + 1 < prm.n) {
+			f64_load<Idx>(prm, nop.left, op.out, p, stride, col, nl);
+			f64_load<Idx>(prm, nop.right, op.out, p, stride, col, nr);
 		}
-		cp_async_commit();
+		cp_async_wait<kF64Ring - 3>(); // entry i + 2 has landed
+		__syncwarp();
+		const NodeOp nnop = i + 2 < prm.n ? ring[(i + 2) & (kF64Ring - 1)].op : none;
+		const int32_t own = f64_entry(prm, ring[i & (kF64Ring - 1)], op, i, p, c, l, r,
+					      mult, y);
+		cnt = l.s + r.s + own;
+		const Idx ox = (Idx)op.out * stride + col;
+		((double4_32a *)prm.partials)[ox] = y;
+		prm.scales[ox] = cnt;
+		__syncwarp(); // every lane has read the slot that is filled next
+		f64_fill(prm, ring + (i & (kF64Ring - 1)), i + kF64Ring, c, lane);
+		l = nl;
+		r = nr;
+		if (nop.left == op.out) {
+			l.x = y;
+			l.s = cnt;
+		}
+		if (nop.right == op.out) {
+			r.x = y;
+			r.s = cnt;
+		}
+		op = nop;
+		nop = nnop;
+	}
+	finish_root<false>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, true,
+			   f64_root_dot(prm, y), cnt);
+}
+
+// Run form, for problems whose columns leave the schedulers short of warps:
+// a block of (32 patterns, C categories, G groups) walks the list run by run
+// (prm.runs: entries of a run are mutually independent), group g taking
+// entries g, g + G, ... of each run; a barrier ends a run.  A child may be
+// another group's output, so all of them come from memory.
+template <typename Idx>
+__global__ void __launch_bounds__(512) prune4_f64_runs_kernel(PruneParams prm)
+{
+	const uint32_t tp = 32, c = threadIdx.y, C = prm.C;
+	const uint32_t g = threadIdx.z, G = blockDim.z;
+	const uint32_t p = blockIdx.x * tp + threadIdx.x;
+	const Idx stride = (Idx)C * prm.ldp, col = (Idx)c * prm.ldp + p;
+	extern __shared__ __align__(16) double smem[];
+	const uint32_t lane = threadIdx.x, warp = threadIdx.z * C + threadIdx.y;
+	const uint32_t warps = C * G;
+	F64Entry *ring = reinterpret_cast<F64Entry *>(smem + 64 * warps + 32) + warp * kF64Ring;
+	uint32_t *s_runs = reinterpret_cast<uint32_t *>(
+		reinterpret_cast<F64Entry *>(smem + 64 * warps + 32) + warps * kF64Ring);
+	for (uint32_t k = warp * 32u + lane; k <= prm.n_runs; k += warps * 32u)
+		s_runs[k] = prm.runs[k];
+	__syncthreads();
+	// the next entry of this group to copy: entry fe of run fr
+	uint32_t fr = 0, fe = s_runs[0] + g;
+	auto settle = [&] {
+		while (fr < prm.n_runs && fe >= s_runs[fr + 1]) {
+			++fr;
+			fe = s_runs[fr] + g;
+		}
+	};
+	auto fill = [&](uint32_t slot) {
+		settle();
+		f64_fill(prm, ring + (slot & (kF64Ring - 1)), fr < prm.n_runs ? fe : prm.n, c,
+			 lane);
+		fe += G;
 	};
 #pragma unroll
 	for (uint32_t e = 0; e < kF64Ring; ++e)
 		fill(e);
-	cp_async_wait<kF64Ring - 1>();
-	__syncwarp();
-	F64Child l, r;
-	uint32_t prev = kTipBit; // the previous entry's output: none yet
-	f64_load(prm, partials, ring[0].op.left, prev, p, c, l);
-	f64_load(prm, partials, ring[0].op.right, prev, p, c, r);
+	const SoftNum mult = soft_split((uint32_t)__double2hiint(prm.scale_mult),
+					(uint32_t)__double2loint(prm.scale_mult));
 	double4_32a y = v4_make<double4_32a, double>(0, 0, 0, 0);
 	int32_t cnt = 0;
-	for (uint32_t i = 0; i < prm.n; ++i) {
-		// entries i and i + 1 have landed
-		cp_async_wait<kF64Ring - 2>();
-		__syncwarp();
-		const F64Entry &en = ring[i & (kF64Ring - 1)];
-		const uint32_t left = en.op.left, right = en.op.right, out = en.op.out;
-		F64Child nl, nr;
-		uint32_t next_l = kTipBit, next_r = kTipBit;
-		if (i + 1 < prm.n) {
-			const F64Entry &nx = ring[(i + 1) & (kF64Ring - 1)];
-			next_l = nx.op.left;
-			next_r = nx.op.right;
-			f64_load(prm, partials, next_l, out, p, c, nl);
-			f64_load(prm, partials, next_r, out, p, c, nr);
+	uint32_t j = 0; // entries this group has walked
+	for (uint32_t run = 0; run < prm.n_runs; ++run) {
+		const uint32_t lo = s_runs[run], hi = s_runs[run + 1];
+		F64Child l, r;
+		for (uint32_t i = lo + g; i < hi; i += G, ++j) {
+			// this group's entries j and j + 1 have landed
+			cp_async_wait<kF64Ring - 2>();
+			__syncwarp();
+			const F64Entry &en = ring[j & (kF64Ring - 1)];
+			const NodeOp op = en.op;
+			if (i == lo + g) {
+				f64_load<Idx>(prm, op.left, kTipBit, p, stride, col, l);
+				f64_load<Idx>(prm, op.right, kTipBit, p, stride, col, r);
+			}
+			F64Child nl, nr;
+			if (i + G < hi) {
+				const NodeOp &nop = ring[(j + 1) & (kF64Ring - 1)].op;
+				f64_load<Idx>(prm, nop.left, kTipBit, p, stride, col, nl);
+				f64_load<Idx>(prm, nop.right, kTipBit, p, stride, col, nr);
+			}
+			const int32_t own = f64_entry(prm, en, op, i, p, c, l, r, mult, y);
+			cnt = l.s + r.s + own;
+			const Idx ox = (Idx)op.out * stride + col;
+			((double4_32a *)prm.partials)[ox] = y;
+			prm.scales[ox] = cnt;
+			__syncwarp(); // every lane has read the slot that is filled next
+			fill(j);
+			l = nl;
+			r = nr;
 		}
-		y = f64_entry(en, (const double4_32a *)prm.ptab, i, C, c, l, r);
-		// tip-tip nodes are never rescaled (cpu4.rs:288-318)
-		const int32_t own =
-			((left & right) & kTipBit)
-				? 0
-				: f64_rescale(y, prm.scale_threshold, prm.scale_mult);
-		cnt = l.s + r.s + own;
-		const size_t ox = ((size_t)out * C + c) * prm.ldp + p;
-		partials[ox] = y;
-		prm.scales[ox] = cnt;
-		__syncwarp(); // every lane has read the slot that is filled next
-		fill(i + kF64Ring);
-		l = nl;
-		r = nr;
-		if (next_l == out) {
-			l.x = y;
-			l.s = cnt;
-		}
-		if (next_r == out) {
-			r.x = y;
-			r.s = cnt;
-		}
+		__syncthreads(); // the run's outputs are visible to every group
 	}
-	const double root_dot = prm.pi[0] * y.x + prm.pi[1] * y.y + prm.pi[2] * y.z +
-				prm.pi[3] * y.w;
-	finish_root<false>(prm, smem, tp, threadIdx.x, p, c, true, root_dot, cnt);
+	// the last entry (the root) is alone in its run: group 0 walked it
+	finish_root<false>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, g == 0,
+			   f64_root_dot(prm, y), cnt);
 }

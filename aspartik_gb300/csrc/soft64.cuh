@@ -17,6 +17,9 @@
 //   - the sum S (2^60 <= S < 2^64) keeps its exponent, so the two children's
 //     sums multiply and round to a double once.
 //
+// (Of a node's four states the walk leaves one to the FP64 pipe, which would
+// otherwise idle.)
+//
 // A term keeps at least 60 significant bits relative to the row's largest
 // term and nothing rounds in between, so a node's value is within 0.6 units
 // in the last place of the exact product of sums (four chained FMAs, then a
@@ -38,15 +41,20 @@
 
 namespace b3g {
 
-// Transition table of one (entry, side, category): row k holds the
-// significands and biased exponents of P[i][k], i = 0..3; row 4 is the
-// unknown state (all ones).  Exponents of i = 0, 1 and i = 2, 3 share a
-// word (low and high half).
+// Transition table of one (entry, side, category): row k holds P[0][k] as a
+// double and the significands and biased exponents of P[i][k], i = 1..3; row
+// 4 is the unknown state (all ones).  State 0 stays with the FP64 pipe, which
+// works beside the integer pipes: a quarter of the products costs it 256
+// cycles a sum, less than the integer pipes take for the other three.
+struct SoftRow4 {
+	uint32_t hi[3], lo1; // hi of i = 1, 2, 3; lo of i = 1
+	uint32_t lo2, lo3;
+	double d0;
+};
 struct SoftTab4 {
-	uint32_t hi[5][4];
-	uint32_t lo[5][4];
-	uint32_t e[5][2];
-	uint32_t plain; // some entry is not a positive normal number
+	SoftRow4 row[5];
+	uint32_t e[5][2]; // exponents of i = 1 (low half) and 2 (high), of i = 3
+	uint32_t plain;   // some entry is not a positive normal number
 	uint32_t pad;
 };
 static_assert(sizeof(SoftTab4) == 208, "13 copies of 16 bytes");
@@ -134,6 +142,19 @@ B3G_HD uint64_t soft_mul_round(uint64_t a, int32_t ea, uint64_t b, int32_t eb, b
 	// the significand's leading one adds the missing 1 to the exponent; a
 	// rounding carry adds another
 	return mant + ((uint64_t)(uint32_t)(eb2 - 1) << 52);
+}
+
+// The product of a positive normal double's bits and the positive normal
+// number `f`, rounded; the exponent of the result must lie in the normal
+// range (a caller that scales a small number up to at most 1 knows it does).
+B3G_HD uint64_t soft_scale(uint64_t bits, const SoftNum &f)
+{
+	const SoftNum n = soft_split((uint32_t)(bits >> 32), (uint32_t)bits);
+	const uint64_t p = soft_prod(n.hi, n.lo, f.hi, f.lo); // 2^60 <= p < 2^62
+	const uint32_t s = (uint32_t)(p >> 61);
+	const uint64_t q = p >> s; // 2^60 <= q < 2^61
+	const uint64_t mant = (q >> 8) + ((q >> 7) & 1u);
+	return mant + ((uint64_t)(n.e + f.e - 1024u + s) << 52);
 }
 
 } // namespace b3g

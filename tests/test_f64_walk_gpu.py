@@ -1,0 +1,71 @@
+"""The four-state FP64 walk in its forms: a thread a column walking the whole
+list, and 2 to 16 groups a block walking it run by run; integer products
+(soft64.cuh) wherever values are positive normal numbers, FP64 instructions
+elsewhere.  Every form against the restated GammaLikelihood at 1e-10 (the FP64
+bar of the other parity tests), and the forms against each other bit for bit
+per pattern (each entry's arithmetic is the same)."""
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.cases import dna_case
+from tests.test_gpu_parity import full, lists_and_lengths, make_gpu
+from tests.test_oracle import random_move
+
+pytestmark = pytest.mark.gpu
+
+
+def sequence(c, K, alpha, groups, monkeypatch, squeeze):
+    if groups:
+        monkeypatch.setenv("B3G_F64_GROUPS", str(groups))
+    else:
+        monkeypatch.delenv("B3G_F64_GROUPS", raising=False)
+    g = make_gpu(c.leaves, c.weights, K, "f64")
+    g.set_reversible(c.rates, c.pi)
+    if K > 1:
+        g.set_gamma(alpha)
+    heights = c.tree.heights.copy()
+    if squeeze:  # zero-length internal branches: identity matrices
+        L = c.leaves.shape[0]
+        for v, kids in enumerate(c.tree.children()[2::3]):
+            top = max(kids)
+            if top >= L and heights[top] >= heights[min(kids)]:
+                heights[L + 2 + 3 * v] = heights[top]
+    tree = O.DatedTree(c.tree.parents, heights)
+    tree.mark_all_edges_updated()
+    rng = np.random.default_rng(11)
+    out = []
+    for step in range(4):
+        g.propose_lengths(*lists_and_lengths(tree), 1.0)
+        lnl = g.log_likelihood()
+        out.append((lnl, g.site_log_likelihoods()))
+        g.accept()
+        tree.accept()
+        if not squeeze:
+            random_move(tree, rng)
+        else:
+            tree.mark_all_edges_updated()
+    g.close()
+    return out
+
+
+@pytest.mark.parametrize("taxa,sites,K,alpha,squeeze", [
+    (2, 1, 1, None, False), (5, 33, 1, None, False), (40, 127, 4, 0.5, False),
+    (61, 400, 2, 0.7, True), (33, 300, 3, 0.3, False), (24, 129, 16, 0.5, False),
+    (150, 500, 1, None, True),
+])
+def test_forms_agree(taxa, sites, K, alpha, squeeze, monkeypatch):
+    c = dna_case(taxa, sites, seed=taxa, model="gtr", root_height=1.5, alpha=alpha,
+                 num_categories=K)
+    ref = sequence(c, K, alpha, 1, monkeypatch, squeeze)
+    for groups in (None, 2, 4, 8, 16):
+        got = sequence(c, K, alpha, groups, monkeypatch, squeeze)
+        for (l0, s0), (l1, s1) in zip(ref, got):
+            assert np.array_equal(s0, s1)
+            assert np.isfinite(l0) and abs(l1 - l0) <= 1e-13 * abs(l0)
+    if not squeeze:
+        want = O.GammaLikelihood(c.leaves, c.weights,
+                                 O.DatedTree(c.tree.parents, c.tree.heights),
+                                 O.gtr(c.rates, c.pi), K, alpha if K > 1 else 1.0).cache
+        assert abs(ref[0][0] - want) <= 1e-10 * abs(want)

@@ -56,8 +56,9 @@ int main() {
         const SoftNum t = split(v[0]); // a tip: one table entry
         const uint64_t z = soft_mul_round(((uint64_t)t.hi << 32) | t.lo,
                                           (int32_t)t.e - kSoftBias, b, eb, ok2);
-        std::printf("%016llx %d %016llx %d\n", (unsigned long long)y, ok,
-                    (unsigned long long)z, ok2);
+        const uint64_t w = soft_scale(v[0], split(v[1]));
+        std::printf("%016llx %d %016llx %d %016llx\n", (unsigned long long)y, ok,
+                    (unsigned long long)z, ok2, (unsigned long long)w);
     }
 }
 """
@@ -98,11 +99,12 @@ def test_products_of_sums(spread):
         out = subprocess.run([exe], input=text, capture_output=True, text=True,
                              check=True).stdout.split("\n")
     for row, line in zip(rows[:-2], out):
-        y, ok, z, ok2 = line.split()
+        y, ok, z, ok2, w = line.split()
         f = [Fraction(v) for v in row]
         b = sum(f[8 + k] * f[12 + k] for k in range(4))
         assert ok == "1" and ok2 == "1"
         assert off(int(y, 16), sum(f[k] * f[4 + k] for k in range(4)) * b) < 1
         assert off(int(z, 16), f[0] * b) < 1
+        assert off(int(w, 16), f[0] * f[1]) < 1
     assert out[len(rows) - 2].split()[1] == "0"
     assert out[len(rows) - 1].split()[1] == "0"
