@@ -60,6 +60,7 @@ struct PtabParams {
 	uint32_t C;
 	void *ptab; // R [n][2][C][S+1][S]
 	SoftTab4 *soft; // [n][2][C] beside the four-state FP64 tables, or null
+	void *soft20;   // [n][2][C] beside the 20-state ones (SoftTab20)
 };
 
 struct PruneParams {
@@ -72,6 +73,11 @@ struct PruneParams {
 			      // null (the caller's own tables: plain walk)
 	uint32_t f64_groups;  // with soft: groups a block of the run form (needs
 			      // runs, C * groups <= 16), 1: the serial form
+	// 20-state FP64 form: its integer tables, and the root's value and
+	// count [C][ldp] (ticket then holds a counter a 64-pattern tile)
+	const void *soft20;
+	double *root_val;
+	int32_t *root_exp;
 	const double *pi;
 	const uint32_t *weights;
 	double *site_lnl;   // [ldp]
@@ -259,11 +265,17 @@ cudaError_t launch_ptab20tc(const PtabParams &p, float *tc_tab, cudaStream_t s);
 // category, 4 / p.groups CTAs per SM) then the root's category mixing and
 // fold.
 cudaError_t launch_prune20tc(const Tc20Params &p, cudaStream_t s);
-// 20-state path (prune20.cuh): transition tables [n][2][C][21][20] computed
-// in FP64, then one thread per (pattern, category) column walks the list;
-// blocks of 32 patterns x C (C <= 8) categories.
+// 20-state path: transition tables [n][2][C][21][20] computed in FP64 (FP64
+// form: and their integer form, soft_tab20_bytes() each).
 cudaError_t launch_ptab20(const PtabParams &p, bool f32, cudaStream_t s);
-cudaError_t launch_prune20(const PruneParams &p, bool f32, cudaStream_t s);
+size_t soft_tab20_bytes();
+// FP32 form on the CUDA cores (prune20.cuh): one thread per (pattern,
+// category) column walks the list; blocks of 32 patterns x C (C <= 8).
+cudaError_t launch_prune20(const PruneParams &p, cudaStream_t s);
+// FP64 form (prune20f64.cuh): a block of `groups` (1..4) x 128 threads per
+// 64-pattern tile and category; needs soft20, runs, root buffers, sums_host
+// (a sum a tile) and zeroed tickets (one a tile).
+cudaError_t launch_prune20_f64(const PruneParams &p, uint32_t groups, cudaStream_t s);
 // Fused short-list evaluation: `ctas` persistent blocks over ldp / 128
 // pattern tiles; needs p.n <= kDirectMax and block sums sized for `ctas`.
 cudaError_t launch_prune4_direct(const DirectParams &p, uint32_t ctas,

@@ -231,6 +231,15 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		dev_alloc(d_model_, sizeof(ModelDev), "model");
 		dev_alloc(d_ptab_, (size_t)I_ * 2 * C_ * (S_ + 1) * S_ * rsz,
 			  "transition tables");
+		if (!f32_ && S_ == 20) {
+			dev_alloc(d_soft20_, (size_t)I_ * 2 * C_ * soft_tab20_bytes(),
+				  "integer transition tables");
+			dev_alloc(d_root_val_, (size_t)C_ * ldp_ * sizeof(double), "root values");
+			dev_alloc(d_root_exp_, (size_t)C_ * ldp_ * sizeof(int32_t), "root exponents");
+			dev_alloc(d_tile_tickets_, ldp_ / 64 * sizeof(unsigned), "tile tickets");
+			check_cuda(cudaMemset(d_tile_tickets_, 0, ldp_ / 64 * sizeof(unsigned)),
+				   "zero tickets");
+		}
 		if (!f32_ && S_ == 4)
 			dev_alloc(d_soft_, (size_t)I_ * 2 * C_ * sizeof(SoftTab4),
 				  "integer transition tables");
@@ -253,7 +262,7 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 			   "pinned lnl");
 		check_cuda(cudaHostGetDevicePointer((void **)&d_lnl_host_, h_lnl_, 0),
 			   "mapped lnl");
-		if (S_ == 4) {
+		if (S_ == 4 || !f32_) {
 			check_cuda(cudaHostAlloc((void **)&h_bsums_,
 						 block_sums_cap_ * sizeof(double),
 						 cudaHostAllocMapped),
@@ -340,6 +349,10 @@ void Calculator::release()
 	cudaFree(d_ptab_);
 	cudaFree(d_soft_);
 	d_soft_ = nullptr;
+	cudaFree(d_soft20_);
+	d_soft20_ = nullptr;
+	cudaFree(d_tile_tickets_);
+	d_tile_tickets_ = nullptr;
 	cudaFree(own_d_stage_ ? own_d_stage_ : d_stage_);
 	cudaFreeHost(own_h_stage_ ? own_h_stage_ : h_stage_);
 	own_d_stage_ = nullptr;
@@ -565,6 +578,22 @@ uint32_t Calculator::pick_f64_groups(uint32_t n) const
 	return n_runs_ <= 2048 ? G : 1u;
 }
 
+// Groups a block of the 20-state FP64 walk: doubled while a group's share of
+// a run stays at two thirds of an entry and at most four groups share an SM
+// (us per whole tree with 1 / 2 / 4 groups: 61 taxa x 2,003 patterns x 4
+// categories 378 / 301 / 276, one category 359 / 285 / 261; 64 x 2,500 x 4,
+// 160 blocks: 512 / 489 / 515; 128 x 4,989 x 4, 312 blocks: the same).
+uint32_t Calculator::pick_p20_groups(uint32_t n) const
+{
+	if (f64_groups_)
+		return std::min(f64_groups_, 4u);
+	const uint32_t blocks = ldp_ / 64u * C_;
+	uint32_t G = 1;
+	while (G < 4 && 4 * G * n_runs_ <= 3 * n && 2 * G * blocks <= 4 * num_sms_)
+		G *= 2;
+	return G;
+}
+
 void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 			bool want_cat)
 {
@@ -740,8 +769,7 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 			  bool want_cat, TimingSlot &slot)
 {
-	poll_result_ = false; // result read back by a copy after the kernels
-	++in_flight_;
+	poll_result_ = false; // FP32: result read back by a copy after the kernels
 	PtabParams pt{};
 	pt.lengths = matrices_mode
 			     ? nullptr
@@ -806,6 +834,7 @@ void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 		tp.tips_smem = used + (size_t)L_ * 128u <= budget ? 1u : 0u;
 		tp.log_inv_c = std::log(1.0 / static_cast<double>(C_));
 		check_cuda(launch_prune20tc(tp, stream_), "tensor-core pruning kernel");
+		++in_flight_;
 		record(slot.k1);
 		slot.pending = timing_;
 		ring_next_ += timing_ ? 1 : 0;
@@ -821,6 +850,7 @@ void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 		cat_valid_ = want_cat;
 		return;
 	}
+	pt.soft20 = d_soft20_;
 	check_cuda(launch_ptab20(pt, f32_, stream_), "transition kernel");
 	last_launches_ = 2;
 	record(slot.kmid);
@@ -845,13 +875,27 @@ void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 	pp.scale_threshold = std::exp(-static_cast<double>(scale_ln_));
 	pp.scale_mult = std::exp(static_cast<double>(scale_ln_));
 	pp.log_inv_c = std::log(1.0 / static_cast<double>(C_));
-	check_cuda(launch_prune20(pp, f32_, stream_), "pruning kernel");
+	if (f32_) {
+		check_cuda(launch_prune20(pp, stream_), "pruning kernel");
+	} else {
+		pp.soft20 = d_soft20_;
+		pp.root_val = d_root_val_;
+		pp.root_exp = d_root_exp_;
+		pp.ticket = d_tile_tickets_;
+		pp.runs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
+		pp.n_runs = n_runs_;
+		pp.sums_host = d_bsums_;
+		arm_host_fold(ldp_ / 64u);
+		check_cuda(launch_prune20_f64(pp, pick_p20_groups(n), stream_), "pruning kernel");
+	}
+	++in_flight_;
 	record(slot.k1);
 	slot.pending = timing_;
 	ring_next_ += timing_ ? 1 : 0;
-	check_cuda(cudaMemcpyAsync(h_lnl_, d_lnl_, sizeof(double),
-				   cudaMemcpyDeviceToHost, stream_),
-		   "read lnl");
+	if (f32_)
+		check_cuda(cudaMemcpyAsync(h_lnl_, d_lnl_, sizeof(double),
+					   cudaMemcpyDeviceToHost, stream_),
+			   "read lnl");
 	have_result_ = true;
 	outstanding_ = true;
 	stream_dirty_ = true;

@@ -210,6 +210,9 @@ class Calculator {
 	void *d_ptab_ = nullptr;
 	uint32_t f64_groups_ = 0; // 0: chosen per list
 	uint32_t pick_f64_groups(uint32_t n) const;
+	uint32_t pick_p20_groups(uint32_t n) const;
+	void *d_soft20_ = nullptr;           // 20-state FP64 form: d_ptab_ as integers
+	unsigned *d_tile_tickets_ = nullptr; // [ldp / 64], zero between launches
 	SoftTab4 *d_soft_ = nullptr; // four-state FP64 form: d_ptab_ as integers
 	unsigned char *d_stage_ = nullptr;
 

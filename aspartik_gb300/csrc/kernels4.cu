@@ -423,6 +423,42 @@ __device__ __forceinline__ void neumaier_merge(double &sum, double &comp,
 		comp += comp2;
 }
 
+// log_sum_exp (likelihood/mod.rs:141-151) + ln(1/C) (gamma.rs:155-165) of
+// the FP64 forms' categories: value(k) the root's pi . x, count(k) its
+// e^scale_ln steps (an unsigned 32-bit product with scale_ln, as in the
+// reference).  The values are scaled to the smallest count of those above
+// zero and added, then one logarithm; classes by bit pattern, as the
+// largest-term form treats them: no category above zero -> -inf, else a
+// negative, NaN or infinite one -> NaN.
+template <typename Value, typename Count>
+__device__ __forceinline__ double mix_categories_f64(uint32_t C, Value value, Count count,
+						     uint32_t scale_ln, double log_inv_c)
+{
+	constexpr long long kInf = 0x7FF0000000000000ll;
+	uint32_t least = 0xFFFFFFFFu;
+	bool any = false, bad = false;
+	for (uint32_t k = 0; k < C; k++) {
+		const long long u = __double_as_longlong(value(k));
+		if (u > 0 && u <= kInf) {
+			any = true;
+			least = min(least, (uint32_t)count(k) * scale_ln);
+		}
+		bad = bad || u >= kInf || (u < 0 && (u << 1) != 0);
+	}
+	double acc = value(0);
+	if (C > 1) {
+		acc = 0.0;
+		for (uint32_t k = 0; k < C; k++) {
+			double v = value(k);
+			const uint32_t steps = (uint32_t)count(k) * scale_ln;
+			if (steps > least) // zero or scaled further
+				v *= exp((double)least - (double)steps);
+			acc += v;
+		}
+	}
+	return !any ? -INFINITY : bad ? NAN : log(acc) - (double)least + log_inv_c;
+}
+
 // Root of the schedule: category mixing, pattern weights, block sum and the
 // fold of all block sums by the last block to finish (or by the host).  One
 // `lead` thread per (pattern, category) column reports its root dot product
@@ -487,39 +523,10 @@ __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem
 				       prm.log_inv_c;
 			}
 		} else {
-			// log_sum_exp (likelihood/mod.rs:141-151) + ln(1/C)
-			// (gamma.rs:155-165), scaled to the smallest count (as
-			// unsigned products with scale_ln) of the categories above
-			// zero; classes by bit pattern, as the largest-term form
-			// treats them: no category above zero -> -inf, else a
-			// negative, NaN or infinite one -> NaN
-			constexpr long long kInf = 0x7FF0000000000000ll;
-			uint32_t least = 0xFFFFFFFFu;
-			bool any = false, bad = false;
-			for (uint32_t k = 0; k < C; k++) {
-				const long long u = __double_as_longlong(s_val[k * tp + tid]);
-				if (u > 0 && u <= kInf) {
-					any = true;
-					least = min(least, (uint32_t)s_exp[k * tp + tid] *
-								   prm.scale_ln);
-				}
-				bad = bad || u >= kInf || (u < 0 && (u << 1) != 0);
-			}
-			double acc = s_val[tid];
-			if (C > 1) {
-				acc = 0.0;
-				for (uint32_t k = 0; k < C; k++) {
-					double v = s_val[k * tp + tid];
-					const uint32_t steps =
-						(uint32_t)s_exp[k * tp + tid] * prm.scale_ln;
-					if (steps > least) // zero or scaled further
-						v *= exp((double)least - (double)steps);
-					acc += v;
-				}
-			}
-			site = !any ? -INFINITY
-			       : bad ? NAN
-				     : log(acc) - (double)least + prm.log_inv_c;
+			site = mix_categories_f64(
+				C, [&](uint32_t k) { return s_val[k * tp + tid]; },
+				[&](uint32_t k) { return s_exp[k * tp + tid]; },
+				prm.scale_ln, prm.log_inv_c);
 		}
 		prm.site_lnl[p0 + tid] = site;
 		const uint32_t w = prm.weights[p0 + tid];
@@ -753,6 +760,7 @@ __global__ void __launch_bounds__(512) prune4_plain_kernel(PruneParams prm)
 
 // ---------------------------------------------------------------------------
 #include "prune20.cuh"
+#include "prune20f64.cuh"
 #include "prune20tc.cuh"
 
 } // namespace
@@ -961,25 +969,36 @@ cudaError_t launch_ptab20(const PtabParams &p, bool f32, cudaStream_t s)
 	return cudaGetLastError();
 }
 
-template <typename R, bool kPow2>
-static cudaError_t launch_prune20_t(const PruneParams &p, cudaStream_t s)
+size_t soft_tab20_bytes() { return sizeof(SoftTab20); }
+
+cudaError_t launch_prune20_f64(const PruneParams &p, uint32_t groups, cudaStream_t s)
 {
+	if (p.C == 0 || p.C > 8 || p.ldp % kP20Tile || groups < 1 || groups > 4 || !p.soft20 ||
+	    !p.runs || !p.sums_host)
+		return cudaErrorInvalidValue;
+	const size_t smem =
+		groups * sizeof(P20Group) +
+		(p.n_runs <= kP20RunsSmem ? ((size_t)p.n_runs + 1) * sizeof(uint32_t) : 0);
+	const cudaError_t e = cudaFuncSetAttribute(
+		prune20_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	if (e != cudaSuccess)
+		return e;
+	prune20_f64_kernel<<<dim3(p.ldp / kP20Tile, p.C), 128 * groups, smem, s>>>(p);
+	return cudaGetLastError();
+}
+
+cudaError_t launch_prune20(const PruneParams &p, cudaStream_t s)
+{
+	if (p.C == 0 || p.C > 8 || p.ldp % 32u)
+		return cudaErrorInvalidValue;
 	const dim3 block(32, p.C), grid(p.ldp / 32);
 	const size_t smem = sizeof(double) * (2 * (size_t)block.x * block.y + 32);
 	const bool narrow = (uint64_t)p.num_leaves * 2 * p.C * p.ldp < (1ull << 31);
 	if (narrow)
-		prune20_kernel<R, kPow2, uint32_t><<<grid, block, smem, s>>>(p);
+		prune20_kernel<uint32_t><<<grid, block, smem, s>>>(p);
 	else
-		prune20_kernel<R, kPow2, size_t><<<grid, block, smem, s>>>(p);
+		prune20_kernel<size_t><<<grid, block, smem, s>>>(p);
 	return cudaGetLastError();
-}
-
-cudaError_t launch_prune20(const PruneParams &p, bool f32, cudaStream_t s)
-{
-	if (p.C == 0 || p.C > 8 || p.ldp % 32u)
-		return cudaErrorInvalidValue;
-	return f32 ? launch_prune20_t<float, true>(p, s)
-		   : launch_prune20_t<double, false>(p, s);
 }
 
 cudaError_t launch_ptab20tc(const PtabParams &p, float *tc_tab, cudaStream_t s)

@@ -1,6 +1,7 @@
-// prune20.cuh -- 20-state (protein) pruning on the CUDA cores, both forms.
-// Included by kernels4.cu inside its anonymous namespace (uses finish_root,
-// the Neumaier helpers and the launch plumbing there).
+// prune20.cuh -- 20-state (protein) pruning: the transition tables of both
+// forms and the FP32 form's walk on the CUDA cores.  Included by kernels4.cu
+// inside its anonymous namespace (uses finish_root and the launch plumbing
+// there).
 //
 // The arithmetic generalises the reference's CPU pruner (crates/b3/src/
 // calculator/cpu4.rs:170-433) from 4 to S = 20 states: a tip child
@@ -11,48 +12,95 @@
 // 21st row of ones, so both child kinds read whole 20-element rows.
 //
 // Layouts (S = 20, R = float or double):
-//   partials  R  [2I][C][ldp][20]  80 B (FP32) per (slot, category, pattern)
+//   partials  R  [2I][C][ldp][20]  80 B (FP32), 160 B (FP64)
 //   scales    i32 [2I][C][ldp]
 //   ptab      R  [n][2][C][21][20]
 
 constexpr int kS20 = 20;
+constexpr uint32_t kP20Rows = kS20 + 1;
+// Integer form of an FP64 table (prune20f64.cuh): row k (state or unknown) of
+// the transposed table, states 5 w .. 5 w + 4 together:
+// [w] {e0|e1<<16, e2|e3<<16, e4, plain, hi[5], lo[5], -, -}
+struct __align__(16) SoftTab20 {
+	uint32_t rec[kP20Rows][4][16];
+};
 
-// One block per table (entry, side, category), one thread per element
-// P[i][j], computed in FP64 (the same for both forms: the FP32 form only
-// stores it in single precision) and written transposed.
+// Entry P[i][k] = v of the integer form (its `plain` word is the caller's).
+__device__ __forceinline__ void soft20_store(SoftTab20 *dst, uint32_t k, uint32_t i, double v)
+{
+	const uint32_t dh = (uint32_t)__double2hiint(v), dl = (uint32_t)__double2loint(v);
+	const uint32_t w = i / 5, q = i - 5 * w;
+	uint32_t *r = dst->rec[k][w];
+	reinterpret_cast<uint16_t *>(r)[q] = (uint16_t)(dh >> 20);
+	r[4 + q] = (((dh & 0xFFFFFu) | 0x100000u) << 7) | (dl >> 25);
+	r[9 + q] = dl << 7;
+}
+
+
+// Element (i, j) = (t / 20, t % 20) of the P(t) of table `id` = (entry * 2 +
+// side) * C + category, by thread t < 400 of a block of at least 400 (every
+// thread calls: the block synchronises).  V diag(e) is formed once per table
+// in shared memory, so an element costs 20 FP64 multiply-adds instead of 20
+// products more (the FP64 pipe, 64 cycles an instruction and scheduler
+// partition, bounds this kernel).
+struct Ptab20Smem {
+	double e[kS20];
+	double Ve[kS20 * kS20];
+};
+__device__ __forceinline__ double ptab20_element(const PtabParams &prm, uint32_t id, uint32_t t,
+						 Ptab20Smem &sm)
+{
+	constexpr uint32_t S = kS20;
+	const uint32_t c = id % prm.C, es = id / prm.C;
+	const ModelDev *m = prm.model;
+	const uint32_t i = t / S, j = t - i * S;
+	if (prm.matrices)
+		return t < S * S ? prm.matrices[(size_t)id * S * S + t] : 0.0;
+	const double d = prm.lengths[es] * (prm.clock_rate * m->cat_rates[c]);
+	if (m->shortcuts && d > 20.0) // transition_freqs (substitution.rs:245-252)
+		return t < S * S ? m->pi[j] : 0.0;
+	if (m->shortcuts && d < 1e-10) // transition_q (substitution.rs:258-268)
+		return t >= S * S ? 0.0 : i == j ? 1.0 : m->Q[i * S + j] * d;
+	if (t < S)
+		sm.e[t] = exp(m->lambda[t] * d);
+	__syncthreads();
+	if (t < S * S)
+		sm.Ve[t] = m->V[t] * sm.e[j];
+	__syncthreads();
+	if (t >= S * S)
+		return 0.0;
+	double s = 0.0;
+#pragma unroll
+	for (uint32_t k = 0; k < S; k++)
+		s = fma(sm.Ve[i * S + k], m->Vinv[k * S + j], s);
+	return s;
+}
+
+// One block per table, one thread per element, computed in FP64 (the same
+// for both forms: the FP32 form only stores it in single precision) and
+// written transposed with a 21st row of ones; the FP64 form's integer table
+// beside it.
 template <typename R>
 __global__ void __launch_bounds__(kS20 *kS20) ptab20_kernel(PtabParams prm)
 {
-	constexpr int S = kS20;
-	const uint32_t id = blockIdx.x; // (entry * 2 + side) * C + category
-	const uint32_t c = id % prm.C, es = id / prm.C;
-	const ModelDev *m = prm.model;
-	const uint32_t t = threadIdx.x, i = t / S, j = t - i * S;
-	__shared__ double e[S];
-	double d = 0.0;
-	if (!prm.matrices)
-		d = prm.lengths[es] * (prm.clock_rate * m->cat_rates[c]);
-	if (t < S)
-		e[t] = exp(m->lambda[t] * d);
-	__syncthreads();
-	double P;
-	if (prm.matrices) {
-		P = prm.matrices[(size_t)id * S * S + t];
-	} else if (m->shortcuts && d > 20.0) {
-		P = m->pi[j]; // transition_freqs (substitution.rs:245-252)
-	} else if (m->shortcuts && d < 1e-10) {
-		// transition_q (substitution.rs:258-268): I + Q d, unit diagonal
-		P = i == j ? 1.0 : m->Q[i * S + j] * d;
-	} else {
-		double s = 0.0;
-		for (int k = 0; k < S; k++)
-			s = fma(m->V[i * S + k] * e[k], m->Vinv[k * S + j], s);
-		P = s;
-	}
+	constexpr uint32_t S = kS20;
+	__shared__ Ptab20Smem sm;
+	const uint32_t id = blockIdx.x, t = threadIdx.x, i = t / S, j = t - i * S;
+	const double P = ptab20_element(prm, id, t, sm);
 	R *out = (R *)prm.ptab + (size_t)id * (S + 1) * S;
 	out[j * S + i] = (R)P;
 	if (t < S)
 		out[S * S + t] = (R)1.0;
+	if constexpr (sizeof(R) == 8) {
+		SoftTab20 *st = (SoftTab20 *)prm.soft20 + id;
+		soft20_store(st, j, i, P);
+		if (t < S)
+			soft20_store(st, S, t, 1.0);
+		const int plain = __syncthreads_or(
+			!soft_normal((uint32_t)__double2hiint(P)));
+		if (t == 0)
+			st->rec[0][0][3] = plain ? 1u : 0u;
+	}
 }
 
 // 20 consecutive elements (16-byte aligned) into registers.  kRO: data
@@ -71,18 +119,6 @@ __device__ __forceinline__ void load20(const float *src, float v[20])
 		v[4 * q + 3] = a.w;
 	}
 }
-template <bool kRO>
-__device__ __forceinline__ void load20(const double *src,
-				       double v[20])
-{
-	const double2 *s2 = reinterpret_cast<const double2 *>(src);
-#pragma unroll
-	for (int q = 0; q < 10; q++) {
-		const double2 a = kRO ? __ldg(s2 + q) : s2[q];
-		v[2 * q] = a.x;
-		v[2 * q + 1] = a.y;
-	}
-}
 __device__ __forceinline__ void store20(float *dst, const float v[20])
 {
 	float4 *d4 = reinterpret_cast<float4 *>(dst);
@@ -90,36 +126,26 @@ __device__ __forceinline__ void store20(float *dst, const float v[20])
 	for (int q = 0; q < 5; q++)
 		d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
-__device__ __forceinline__ void store20(double *dst, const double v[20])
-{
-	double2 *d2 = reinterpret_cast<double2 *>(dst);
-#pragma unroll
-	for (int q = 0; q < 10; q++)
-		d2[q] = make_double2(v[2 * q], v[2 * q + 1]);
-}
-
 // One child: tip row lookup or table-times-partial (k-outer, so every
 // table row is one contiguous read shared by the warp's columns).
-template <typename R, typename Idx>
+template <typename Idx>
 __device__ __forceinline__ void child20(const PruneParams &prm, uint32_t id,
-					const R *__restrict__ tab, Idx stride,
-					Idx col, uint32_t p, R out[20],
-					int32_t &sc, bool &tip)
+					const float *__restrict__ tab, Idx stride,
+					Idx col, uint32_t p, float out[20],
+					int32_t &sc)
 {
 	constexpr int S = kS20;
 	if (id & kTipBit) {
 		const uint8_t code = prm.tips[(size_t)(id & ~kTipBit) * prm.ldp + p];
 		load20<true>(tab + (size_t)code * S, out);
 		sc = 0;
-		tip = true;
 		return;
 	}
-	tip = false;
 	const Idx ix = (Idx)id * stride + col;
-	R x[S];
-	load20<false>((const R *)prm.partials + (size_t)ix * S, x);
+	float x[S];
+	load20<false>((const float *)prm.partials + (size_t)ix * S, x);
 	sc = prm.scales[ix];
-	R row[S];
+	float row[S];
 	load20<true>(tab, row);
 #pragma unroll
 	for (int i = 0; i < S; i++)
@@ -162,27 +188,10 @@ __device__ __forceinline__ int32_t rescale_pow2_20(float y[20])
 	return e + shift;
 }
 
-// FP64 form (cpu4.rs:403-433 with S entries): multiply by e^scale_ln when
-// every entry is below e^-scale_ln.
-__device__ __forceinline__ int32_t rescale_threshold_20(double y[20], double thr,
-							double mult)
-{
-	bool all = true;
-#pragma unroll
-	for (int i = 0; i < 20; i++)
-		all = all && y[i] < thr;
-	if (!all)
-		return 0;
-#pragma unroll
-	for (int i = 0; i < 20; i++)
-		y[i] *= mult;
-	return 1;
-}
-
 // One thread per (pattern, category) column walks the whole children-first
 // list.  Block (32, C): 32 patterns of every category, so the root's
 // category mixing stays in the block (finish_root).
-template <typename R, bool kPow2, typename Idx>
+template <typename Idx>
 __global__ void __launch_bounds__(256) prune20_kernel(PruneParams prm)
 {
 	constexpr int S = kS20;
@@ -192,39 +201,32 @@ __global__ void __launch_bounds__(256) prune20_kernel(PruneParams prm)
 	const Idx stride = (Idx)prm.C * prm.ldp;
 	const Idx col = (Idx)c * prm.ldp + p;
 	const size_t tab_stride = (size_t)(S + 1) * S;
-	R y[S];
+	float y[S];
 #pragma unroll
 	for (int i = 0; i < S; i++)
-		y[i] = (R)0;
+		y[i] = 0.0f;
 	int32_t cnt = 0;
 	for (uint32_t e = 0; e < prm.n; ++e) {
 		const NodeOp op = prm.ops[e];
-		const R *tl = (const R *)prm.ptab + ((size_t)(2 * e) * prm.C + c) * tab_stride;
-		const R *tr = tl + (size_t)prm.C * tab_stride;
-		R a[S], b[S];
+		const float *tl = (const float *)prm.ptab + ((size_t)(2 * e) * prm.C + c) * tab_stride;
+		const float *tr = tl + (size_t)prm.C * tab_stride;
+		float a[S], b[S];
 		int32_t sa, sb;
-		bool ta, tb;
-		child20<R, Idx>(prm, op.left, tl, stride, col, p, a, sa, ta);
-		child20<R, Idx>(prm, op.right, tr, stride, col, p, b, sb, tb);
+		child20<Idx>(prm, op.left, tl, stride, col, p, a, sa);
+		child20<Idx>(prm, op.right, tr, stride, col, p, b, sb);
 #pragma unroll
 		for (int i = 0; i < S; i++)
 			y[i] = a[i] * b[i];
-		int32_t own;
-		if constexpr (kPow2)
-			own = rescale_pow2_20(y);
-		else // tip-tip nodes are never rescaled (cpu4.rs:288-318)
-			own = (ta && tb) ? 0
-					 : rescale_threshold_20(y, prm.scale_threshold,
-								prm.scale_mult);
+		const int32_t own = rescale_pow2_20(y);
 		cnt = sa + sb + own;
 		const Idx ox = (Idx)op.out * stride + col;
-		store20((R *)prm.partials + (size_t)ox * S, y);
+		store20((float *)prm.partials + (size_t)ox * S, y);
 		prm.scales[ox] = cnt;
 	}
 	double root_dot = 0.0;
 #pragma unroll
 	for (int i = 0; i < S; i++)
 		root_dot = fma(prm.pi[i], (double)y[i], root_dot);
-	finish_root<kPow2>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, true, root_dot,
+	finish_root<true>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, true, root_dot,
 			   cnt);
 }

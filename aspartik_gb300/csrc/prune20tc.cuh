@@ -76,33 +76,13 @@ __global__ void __launch_bounds__(768) ptab20tc_kernel(PtabParams prm, float *tc
 {
 	constexpr int S = kS20;
 	const uint32_t id = blockIdx.x;
-	const uint32_t c = id % prm.C, es = id / prm.C;
-	const ModelDev *m = prm.model;
 	const uint32_t t = threadIdx.x;
-	__shared__ double e[S];
+	__shared__ Ptab20Smem sm;
 	__shared__ double Ps[S * S];
-	double d = 0.0;
-	if (!prm.matrices)
-		d = prm.lengths[es] * (prm.clock_rate * m->cat_rates[c]);
-	if (t < S)
-		e[t] = exp(m->lambda[t] * d);
-	__syncthreads();
+	const double P = ptab20_element(prm, id, t, sm);
 	float *tip = (float *)prm.ptab + (size_t)id * (S + 1) * S;
 	if (t < S * S) {
 		const uint32_t i = t / S, j = t - i * S;
-		double P;
-		if (prm.matrices) {
-			P = prm.matrices[(size_t)id * S * S + t];
-		} else if (m->shortcuts && d > 20.0) {
-			P = m->pi[j];
-		} else if (m->shortcuts && d < 1e-10) {
-			P = i == j ? 1.0 : m->Q[i * S + j] * d;
-		} else {
-			double s = 0.0;
-			for (int k = 0; k < S; k++)
-				s = fma(m->V[i * S + k] * e[k], m->Vinv[k * S + j], s);
-			P = s;
-		}
 		Ps[t] = P;
 		tip[j * S + i] = (float)P;
 	} else if (t < S * S + S) {

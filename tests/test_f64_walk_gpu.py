@@ -69,3 +69,39 @@ def test_forms_agree(taxa, sites, K, alpha, squeeze, monkeypatch):
                                  O.DatedTree(c.tree.parents, c.tree.heights),
                                  O.gtr(c.rates, c.pi), K, alpha if K > 1 else 1.0).cache
         assert abs(ref[0][0] - want) <= 1e-10 * abs(want)
+
+
+@pytest.mark.parametrize("taxa,sites,K", [(2, 1, 1), (7, 65, 4), (40, 200, 8), (90, 130, 2)])
+def test_protein_groups_agree(taxa, sites, K, monkeypatch):
+    """20 states, FP64: 1, 2 and 4 groups a block give the same bits per
+    pattern, and the generic oracle's likelihood to 1e-10."""
+    from oracle import generic as G
+    from tests.cases import protein_case
+    from aspartik_gb300.calculator import Calculator
+
+    c = protein_case(taxa, sites, seed=taxa, num_categories=K, gaps=0.05)
+    tree = O.DatedTree(c.tree.parents, c.tree.heights)
+    tree.mark_all_edges_updated()
+    lists = lists_and_lengths(tree)
+    got = []
+    for groups in ("", "1", "2", "4"):
+        if groups:
+            monkeypatch.setenv("B3G_F64_GROUPS", groups)
+        else:
+            monkeypatch.delenv("B3G_F64_GROUPS", raising=False)
+        g = Calculator.GB300(0, "f64").make20(c.leaves, c.leaves.shape[1], num_categories=K)
+        g.set_weights(c.weights)
+        g.set_reversible(c.rates, c.pi)
+        if K > 1:
+            g.set_gamma(1.0)
+        for _ in range(2):
+            g.propose_lengths(*lists, 1.0)
+            got.append((g.log_likelihood(), g.site_log_likelihoods()))
+            g.accept()
+        g.close()
+    want = G.log_likelihood(c.leaves, c.weights, c.tree.parents, c.tree.heights,
+                            O.reversible(c.rates, c.pi),
+                            O.gamma_categories(1.0, K) if K > 1 else np.ones(1))
+    for lnl, sites_ in got:
+        assert np.array_equal(sites_, got[0][1])
+        assert abs(lnl - want) <= 1e-10 * abs(want)
