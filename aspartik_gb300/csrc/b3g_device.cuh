@@ -4,6 +4,8 @@
 // Device store of one calculator (one chain), all resident in HBM:
 //   tips      u8  [L][ldp]                   state 0..S-1, S = unknown
 //   partials  R   [2I][C][ldp][S]            slot = (v - L) * 2 + selector
+//                                            (20 states, FP32: [10][128][2]
+//                                            in each 128-pattern tile)
 //   scales    i32 [2I][C][ldp]               cumulative rescale count of the
 //                                            subtree below the slot's node
 //   ptab      R   [n][2][C][S+1][S]          per-step transposed transition
@@ -24,6 +26,11 @@ constexpr uint32_t kTipBit = 0x80000000u;
 constexpr int kMaxStates = 20;
 constexpr int kMaxCategories = 16;
 constexpr uint32_t kPatternAlign = 128;
+
+// Marks of an entry of a depth-first 20-state FP32 list (NodeOp::pad): the
+// right child is multiplied first; the second child is the previous entry's
+// output.
+constexpr uint32_t kS20Swap = 1u, kS20Prev = 2u;
 
 // Shared-memory slot code meaning "global memory only" (run walk).
 constexpr uint32_t kNoSlot = 0xFFu;
@@ -71,8 +78,11 @@ struct PruneParams {
 	const void *ptab;
 	const SoftTab4 *soft; // four-state FP64 form: the tables as integers, or
 			      // null (the caller's own tables: plain walk)
-	uint32_t f64_groups;  // with soft: groups a block of the run form (needs
-			      // runs, C * groups <= 16), 1: the serial form
+	// depth-first order (four-state FP64 and 20-state FP32 walks): with
+	// `groups` > 1 the list has `phases`; in phase ph group g of a block
+	// walks entries [segs[ph groups + g], segs[ph groups + g + 1])
+	const uint32_t *segs;
+	uint32_t groups, phases;
 	// 20-state FP64 form: its integer tables, and the root's value and
 	// count [C][ldp] (ticket then holds a counter a 64-pattern tile)
 	const void *soft20;
@@ -269,9 +279,13 @@ cudaError_t launch_prune20tc(const Tc20Params &p, cudaStream_t s);
 // form: and their integer form, soft_tab20_bytes() each).
 cudaError_t launch_ptab20(const PtabParams &p, bool f32, cudaStream_t s);
 size_t soft_tab20_bytes();
-// FP32 form on the CUDA cores (prune20.cuh): one thread per (pattern,
-// category) column walks the list; blocks of 32 patterns x C (C <= 8).
+// FP32 form with register MMAs (prune20.cuh): a block of p.groups (1..4)
+// warps per 32-pattern tile and category; needs root buffers, sums_host (a
+// sum a tile), zeroed tickets (one a tile), marked entries and, with several
+// groups, segs.
 cudaError_t launch_prune20(const PruneParams &p, cudaStream_t s);
+// Blocks of `groups` warps of that walk that one SM holds.
+uint32_t prune20_blocks_per_sm(uint32_t groups);
 // FP64 form (prune20f64.cuh): a block of `groups` (1..4) x 128 threads per
 // 64-pattern tile and category; needs soft20, runs, root buffers, sums_host
 // (a sum a tile) and zeroed tickets (one a tile).

@@ -124,10 +124,6 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	use_runs_ = f32_ && S_ == 4 && runs_tile_ * C_ <= 512;
 	// fused single-launch evaluation of short lists (B3G_DIRECT=0 turns
 	// it off, e.g. to time the two-kernel path)
-	// 20-state FP32 lists on the tensor cores (B3G_TC20=0: CUDA-core walk)
-	use_tc20_ = f32_ && S_ == 20;
-	if (const char *env = std::getenv("B3G_TC20"))
-		use_tc20_ = use_tc20_ && std::atoi(env) != 0;
 	// groups of 128 threads per tensor-core CTA (B3G_TC20_GROUPS = 1 or 2;
 	// default: chosen per launch from the grid size)
 	if (const char *env = std::getenv("B3G_TC20_CLUSTER")) {
@@ -144,12 +140,22 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 			tc20_groups_fixed_ = true;
 		}
 	}
+	// 20-state FP32 lists on the tensor cores: B3G_TC20=1, or a launch shape
+	// of that engine fixed by one of the two switches above
+	use_tc20_ = f32_ && S_ == 20 && (tc20_cluster_fixed_ || tc20_groups_fixed_);
+	if (const char *env = std::getenv("B3G_TC20"))
+		use_tc20_ = f32_ && S_ == 20 && std::atoi(env) != 0;
 	// groups of the FP64 run form (B3G_F64_GROUPS: 1, 2, 4, 8 or 16 where
 	// they fit a block; default: chosen per list)
 	if (const char *env = std::getenv("B3G_F64_GROUPS")) {
 		const int gr = std::atoi(env);
 		if (gr == 1 || gr == 2 || gr == 4 || gr == 8 || gr == 16)
 			f64_groups_ = static_cast<uint32_t>(gr);
+	}
+	if (const char *env = std::getenv("B3G_S20_GROUPS")) {
+		const int gr = std::atoi(env);
+		if (gr >= 1 && gr <= 4)
+			s20_groups_ = static_cast<uint32_t>(gr);
 	}
 	use_direct_ = f32_ && S_ == 4 && (C_ == 1 || C_ == 2 || C_ == 4);
 	if (const char *env = std::getenv("B3G_DIRECT"))
@@ -160,6 +166,10 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	pos_.assign(2 * L_ - 1, 0);
 	run_of_.assign(I_, 0);
 	smem_of_.assign(2ull * I_, static_cast<uint8_t>(kNoSlot));
+	slot_pos_.assign(2ull * I_, kNone);
+	if (f32_ && S_ == 20)
+		for (uint32_t w = 1; w <= 4; ++w)
+			s20_per_sm_[w] = prune20_blocks_per_sm(w);
 	// shared-memory slots of the run walk (B3G_RUNS_SLOTS=0: children of
 	// listed entries read back from global memory, to time the difference)
 	if (const char *env = std::getenv("B3G_RUNS_SLOTS"))
@@ -216,11 +226,9 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		dev_alloc(d_block_sums_, nblocks * sizeof(double), "block sums");
 		dev_alloc(d_ticket_, sizeof(unsigned), "ticket");
 		dev_alloc(d_lnl_, sizeof(double), "lnl");
-		if (use_tc20_) {
+		if (f32_ && S_ == 20) {
 			dev_alloc(d_tc_tab_, (size_t)I_ * 2 * C_ * 2 * 768 * sizeof(float),
 				  "tensor-core tables");
-			dev_alloc(d_root_val_, (size_t)C_ * ldp_ * sizeof(double), "root values");
-			dev_alloc(d_root_exp_, (size_t)C_ * ldp_ * sizeof(int32_t), "root exponents");
 			dev_alloc(d_status_, sizeof(unsigned), "status");
 			check_cuda(cudaMemset(d_status_, 0, sizeof(unsigned)), "zero status");
 			check_cuda(cudaHostAlloc((void **)&h_status_, sizeof(unsigned),
@@ -228,18 +236,19 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 				   "pinned status");
 			*h_status_ = 0;
 		}
+		if (S_ == 20) {
+			dev_alloc(d_root_val_, (size_t)C_ * ldp_ * sizeof(double), "root values");
+			dev_alloc(d_root_exp_, (size_t)C_ * ldp_ * sizeof(int32_t), "root exponents");
+			dev_alloc(d_tile_tickets_, ldp_ / 32 * sizeof(unsigned), "tile tickets");
+			check_cuda(cudaMemset(d_tile_tickets_, 0, ldp_ / 32 * sizeof(unsigned)),
+				   "zero tickets");
+		}
 		dev_alloc(d_model_, sizeof(ModelDev), "model");
 		dev_alloc(d_ptab_, (size_t)I_ * 2 * C_ * (S_ + 1) * S_ * rsz,
 			  "transition tables");
-		if (!f32_ && S_ == 20) {
+		if (!f32_ && S_ == 20)
 			dev_alloc(d_soft20_, (size_t)I_ * 2 * C_ * soft_tab20_bytes(),
 				  "integer transition tables");
-			dev_alloc(d_root_val_, (size_t)C_ * ldp_ * sizeof(double), "root values");
-			dev_alloc(d_root_exp_, (size_t)C_ * ldp_ * sizeof(int32_t), "root exponents");
-			dev_alloc(d_tile_tickets_, ldp_ / 64 * sizeof(unsigned), "tile tickets");
-			check_cuda(cudaMemset(d_tile_tickets_, 0, ldp_ / 64 * sizeof(unsigned)),
-				   "zero tickets");
-		}
 		if (!f32_ && S_ == 4)
 			dev_alloc(d_soft_, (size_t)I_ * 2 * C_ * sizeof(SoftTab4),
 				  "integer transition tables");
@@ -262,14 +271,11 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 			   "pinned lnl");
 		check_cuda(cudaHostGetDevicePointer((void **)&d_lnl_host_, h_lnl_, 0),
 			   "mapped lnl");
-		if (S_ == 4 || !f32_) {
-			check_cuda(cudaHostAlloc((void **)&h_bsums_,
-						 block_sums_cap_ * sizeof(double),
-						 cudaHostAllocMapped),
-				   "pinned block sums");
-			check_cuda(cudaHostGetDevicePointer((void **)&d_bsums_, h_bsums_, 0),
-				   "mapped block sums");
-		}
+		check_cuda(cudaHostAlloc((void **)&h_bsums_, block_sums_cap_ * sizeof(double),
+					 cudaHostAllocMapped),
+			   "pinned block sums");
+		check_cuda(cudaHostGetDevicePointer((void **)&d_bsums_, h_bsums_, 0),
+			   "mapped block sums");
 
 		// DNA: single bases -> 0..3, everything else -> unknown (4)
 		// (cpu4.rs:117-124).  Protein: states 0..19 as given, anything
@@ -506,6 +512,9 @@ void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
 	runs[n_runs_] = n;
 	if (n_runs_)
 		max_run_ = std::max(max_run_, n - runs[n_runs_ - 1]);
+	depth_first_ = S_ == 4 ? !f32_ : f32_ && !use_tc20_;
+	if (depth_first_)
+		order_depth_first(n);
 }
 
 // Shared-memory slots for the run walk's outputs (at most `capacity`),
@@ -560,22 +569,221 @@ uint32_t Calculator::assign_slots(uint32_t n, uint32_t capacity)
 	return used;
 }
 
-// Groups a block of the FP64 walk's run form, 1 for the serial form.
-uint32_t Calculator::pick_f64_groups(uint32_t n) const
+// Groups a block of the depth-first walks (each walks subtrees of its own
+// before one of them walks the entries above).
+uint32_t Calculator::pick_groups(uint32_t n) const
 {
+	if (S_ == 20) {
+		if (s20_groups_)
+			return s20_groups_;
+		// the most warps with which every block still runs at once: us
+		// per whole tree with 1 / 2 / 3 / 4, 128 taxa x 4,989 patterns x 4
+		// categories (624 blocks): 198 / 165 / 181 / 169; 61 x 2,003 x 4:
+		// 89 / 73 / 70 / 67
+		const uint32_t blocks = ldp_ / 32u * C_;
+		uint32_t G = 1;
+		for (uint32_t w = 2; w <= 4; ++w)
+			if (4 * w <= n && s20_per_sm_[w] * num_sms_ >= blocks)
+				G = w;
+		return G;
+	}
 	if (f64_groups_)
-		return C_ * f64_groups_ <= 16 && n_runs_ <= 2048 ? f64_groups_ : 1u;
-	// doubled while a group's share of a run stays at two thirds of an
-	// entry or more, and every block still runs at once (16 warps an SM at
-	// this kernel's registers): us per whole tree with 1 / 2 / 4 / 8 / 16
-	// groups, 37 taxa x 1,147 patterns: 49 / 41 / 34 / 32 / 32; 64 x 7,855,
-	// one category: 71 / 57 / 47 / 45 / 62, four: 88 / 78 / 94; 128 x 17,764,
-	// one category: 137 / 102 / 81 / 92 / 120.  A path's runs have one entry.
+		return C_ * f64_groups_ <= 16 ? f64_groups_ : 1u;
+	// doubled while every block still runs at once (16 warps an SM at this
+	// kernel's registers): us per whole tree with 1 / 2 / 4 / 8 groups, 37
+	// taxa x 1,147 patterns: 51 / 41 / 35 / 36; 64 x 7,855, one category: 70 /
+	// 54 / 48 / 50, four: 84 / 75 / 92; 128 x 17,764, one category: 130 / 99 /
+	// 80 / 93
 	const uint32_t warps = ldp_ / 32u * C_;
 	uint32_t G = 1;
-	while (2 * G * C_ <= 16 && 4 * G * n_runs_ <= 3 * n && 2 * G * warps <= 16 * num_sms_)
+	while (2 * G * C_ <= 16 && 8 * G <= n && 2 * G * warps <= 16 * num_sms_)
 		G *= 2;
-	return n_runs_ <= 2048 ? G : 1u;
+	return G;
+}
+
+// The phases of G groups (order_, segs_); false where they would not
+// shorten the longest group's work by a fifth.
+template <typename Emit>
+bool Calculator::split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit)
+{
+	// split the costliest subtree until the pieces balance; what is split
+	// belongs to the entries above
+	std::vector<uint32_t> &piece = pieces_, &above = above_;
+	piece.assign(1, n - 1);
+	above.clear();
+	while (!piece.empty() && piece.size() < 4 * G) {
+		size_t top = 0;
+		for (size_t k = 1; k < piece.size(); ++k)
+			if (cost_[piece[k]] > cost_[piece[top]])
+				top = k;
+		const uint32_t v = piece[top];
+		if (v != n - 1 && cost_[v] * 2 * G <= cost_[n - 1])
+			break;
+		above.push_back(v);
+		piece[top] = piece.back();
+		piece.pop_back();
+		for (int j = 0; j < 2; ++j)
+			if (kid_[2 * v + j] != kNone)
+				piece.push_back(kid_[2 * v + j]);
+	}
+	std::sort(piece.begin(), piece.end(), [&](uint32_t a, uint32_t b) {
+		return cost_[a] != cost_[b] ? cost_[a] > cost_[b] : a < b;
+	});
+	std::sort(above.begin(), above.end()); // children first
+	// a piece goes to the least loaded group
+	uint32_t load[16] = {}, owner[80];
+	for (size_t k = 0; k < piece.size(); ++k) {
+		owner[k] = (uint32_t)(std::min_element(load, load + G) - load);
+		load[owner[k]] += cost_[piece[k]];
+	}
+	segs_.clear();
+	for (uint32_t w = 0; w < G; ++w) {
+		segs_.push_back(at);
+		for (size_t k = 0; k < piece.size(); ++k)
+			if (owner[k] == w)
+				emit(piece[k]);
+	}
+	uint32_t longest = *std::max_element(load, load + G);
+	// the entries above: runs of independent entries, each dealt out in
+	// contiguous shares
+	uint32_t phases = 1;
+	for (size_t i = 0; i < above.size();) {
+		size_t j = i;
+		for (; j < above.size(); ++j) {
+			bool free = true;
+			for (size_t k = i; k < j; ++k)
+				free = free && kid_[2 * above[j]] != above[k] &&
+				       kid_[2 * above[j] + 1] != above[k];
+			if (!free)
+				break;
+		}
+		const uint32_t len = (uint32_t)(j - i);
+		for (uint32_t w = 0; w < G; ++w) {
+			segs_.push_back(at + (len * w + G - 1) / G);
+		}
+		for (size_t k = i; k < j; ++k)
+			order_[at++] = above[k];
+		longest += (len + G - 1) / G * 6 + 4; // entries, and the barrier
+		++phases;
+		i = j;
+	}
+	segs_.push_back(at);
+	if (longest * 5 > cost_[n - 1] * 4 || segs_.size() > (size_t)I_ + 1) {
+		segs_.assign({0u, n});
+		return false;
+	}
+	order_groups_ = G;
+	order_phases_ = phases;
+	return true;
+}
+
+// Reorders the staged list depth first, heavier subtree first, so that a
+// child is mostly the previous entry's output, and for several groups splits
+// it into phases (segs_): disjoint subtrees, a balanced share a group, then
+// the entries above them, run by run.  Every entry's arithmetic is the same
+// in any children-first order.  order_[k] = list position of staged entry k.
+// A list that is not one tree under its last entry keeps its order.
+void Calculator::order_depth_first(uint32_t n)
+{
+	NodeOp *ops = reinterpret_cast<NodeOp *>(h_stage_);
+	list_ops_.assign(ops, ops + n);
+	order_.resize(n);
+	kid_.assign(2 * (size_t)n, kNone);
+	parent_.assign(n, kNone);
+	cost_.resize(n);
+	chain_.resize(n);
+	uint32_t linked = 0;
+	bool tree = true;
+	for (uint32_t i = 0; i < n; ++i)
+		slot_pos_[list_ops_[i].out] = i;
+	for (uint32_t i = 0; i < n; ++i) {
+		const uint32_t ids[2] = {list_ops_[i].left, list_ops_[i].right};
+		uint32_t cost = 2; // an entry, and more for each internal child
+		uint32_t below = 0;
+		for (int j = 0; j < 2; ++j) {
+			if (ids[j] & kTipBit)
+				continue;
+			cost += 3;
+			const uint32_t k = slot_pos_[ids[j]];
+			if (k == kNone)
+				continue;
+			tree = tree && parent_[k] == kNone;
+			parent_[k] = i;
+			kid_[2 * i + j] = k;
+			cost += cost_[k];
+			below = std::max(below, chain_[k]);
+			++linked;
+		}
+		chain_[i] = below + 2 + 3 * !(ids[0] & kTipBit) + 3 * !(ids[1] & kTipBit);
+		cost_[i] = cost;
+	}
+	for (uint32_t i = 0; i < n; ++i)
+		slot_pos_[list_ops_[i].out] = kNone;
+	order_groups_ = 1;
+	order_phases_ = 1;
+	segs_.assign({0u, n});
+	uint32_t at = 0;
+	// post-order of the subtree of r, heavier children first
+	auto emit = [&](uint32_t r) {
+		walk_stack_.assign(1, r);
+		const uint32_t begin = at;
+		while (!walk_stack_.empty()) {
+			const uint32_t v = walk_stack_.back();
+			walk_stack_.pop_back();
+			order_[at++] = v; // reversed below: parent, light, heavy
+			uint32_t a = kid_[2 * v], b = kid_[2 * v + 1];
+			if (a != kNone && b != kNone && cost_[a] < cost_[b])
+				std::swap(a, b);
+			if (a != kNone)
+				walk_stack_.push_back(a);
+			if (b != kNone)
+				walk_stack_.push_back(b);
+		}
+		std::reverse(order_.begin() + begin, order_.begin() + at);
+	};
+	if (!tree || linked + 1 != n) {
+		for (uint32_t i = 0; i < n; ++i)
+			order_[i] = i;
+	} else {
+		// at most twice the list's work over its longest chain
+		uint32_t G = pick_groups(n);
+		while (G > 1 && G * chain_[n - 1] > 2 * cost_[n - 1])
+			G = S_ == 20 ? G - 1 : G / 2;
+		if (G == 1 || !split_phases(n, G, at, emit)) {
+			at = 0;
+			emit(n - 1);
+		}
+	}
+	size_t seg = 0; // segs_[seg]: where the current walk began
+	for (uint32_t k = 0; k < n; ++k) {
+		NodeOp op = list_ops_[order_[k]];
+		bool first = false; // of its walk
+		for (; seg < segs_.size() && segs_[seg] <= k; ++seg)
+			first = first || segs_[seg] == k;
+		const uint32_t prev = first ? kNone : ops[k - 1].out;
+		const bool lp = op.left == prev, rp = op.right == prev;
+		const bool lt = (op.left & kTipBit) != 0, rt = (op.right & kTipBit) != 0;
+		// first the child that is not the previous output; of the others a
+		// partial before a tip
+		op.pad = lp ? kS20Swap | kS20Prev : rp ? kS20Prev : lt && !rt ? kS20Swap : 0u;
+		ops[k] = op;
+	}
+	if (order_groups_ > 1)
+		std::memcpy(h_stage_ + off_runs_, segs_.data(), segs_.size() * sizeof(uint32_t));
+}
+
+// The list's edge lengths (two values an entry) or matrices into the staging
+// block, in the staged order.
+void Calculator::stage_inputs(const double *src, uint32_t n, size_t per_entry)
+{
+	double *dst = reinterpret_cast<double *>(h_stage_ + off_in_);
+	if (!depth_first_) {
+		std::memcpy(dst, src, n * per_entry * sizeof(double));
+		return;
+	}
+	for (uint32_t k = 0; k < n; ++k)
+		std::memcpy(dst + k * per_entry, src + order_[k] * per_entry,
+			    per_entry * sizeof(double));
 }
 
 // Groups a block of the 20-state FP64 walk: doubled while a group's share of
@@ -743,11 +951,11 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 	} else {
 		poll_result_ = false;
 		if (pp.soft) { // the blocks' sums go to mapped host memory here too
-			pp.f64_groups = pick_f64_groups(n);
-			pp.runs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
-			pp.n_runs = n_runs_;
+			pp.groups = order_groups_;
+			pp.phases = order_phases_;
+			pp.segs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
 			pp.sums_host = d_bsums_;
-			arm_host_fold(ldp_ / (pp.f64_groups > 1 ? 32u : tile_));
+			arm_host_fold(ldp_ / (pp.groups > 1 ? 32u : tile_));
 		}
 		check_cuda(launch_prune4(pp, f32_, tile_, stream_), "pruning kernel");
 	}
@@ -875,16 +1083,20 @@ void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 	pp.scale_threshold = std::exp(-static_cast<double>(scale_ln_));
 	pp.scale_mult = std::exp(static_cast<double>(scale_ln_));
 	pp.log_inv_c = std::log(1.0 / static_cast<double>(C_));
+	pp.root_val = d_root_val_;
+	pp.root_exp = d_root_exp_;
+	pp.ticket = d_tile_tickets_;
+	pp.runs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
+	pp.n_runs = n_runs_;
+	pp.sums_host = d_bsums_;
 	if (f32_) {
+		pp.groups = order_groups_;
+		pp.phases = order_phases_;
+		pp.segs = pp.runs;
+		arm_host_fold(ldp_ / 32u);
 		check_cuda(launch_prune20(pp, stream_), "pruning kernel");
 	} else {
 		pp.soft20 = d_soft20_;
-		pp.root_val = d_root_val_;
-		pp.root_exp = d_root_exp_;
-		pp.ticket = d_tile_tickets_;
-		pp.runs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
-		pp.n_runs = n_runs_;
-		pp.sums_host = d_bsums_;
 		arm_host_fold(ldp_ / 64u);
 		check_cuda(launch_prune20_f64(pp, pick_p20_groups(n), stream_), "pruning kernel");
 	}
@@ -892,10 +1104,6 @@ void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 	record(slot.k1);
 	slot.pending = timing_;
 	ring_next_ += timing_ ? 1 : 0;
-	if (f32_)
-		check_cuda(cudaMemcpyAsync(h_lnl_, d_lnl_, sizeof(double),
-					   cudaMemcpyDeviceToHost, stream_),
-			   "read lnl");
 	have_result_ = true;
 	outstanding_ = true;
 	stream_dirty_ = true;
@@ -1010,7 +1218,7 @@ void Calculator::propose_matrices(const uint32_t *internals,
 	wait_stage();
 	stage_ops(internals, children, n);
 	std::memcpy(h_stage_ + off_pi_, freqs, S_ * sizeof(double));
-	std::memcpy(h_stage_ + off_in_, matrices, count * sizeof(double));
+	stage_inputs(matrices, n, 2ull * C_ * S_ * S_);
 	launch(n, true, 1.0, true);
 }
 
@@ -1035,7 +1243,7 @@ void Calculator::propose_lengths(const uint32_t *internals,
 		check_cuda(cudaEventSynchronize(batch_done_), "batch stage reuse");
 	stage_ops(internals, children, n);
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
-	std::memcpy(h_stage_ + off_in_, lengths, (size_t)n * 2 * sizeof(double));
+	stage_inputs(lengths, n, 2);
 	staged_ = false;
 	launch(n, false, clock_rate, false);
 }

@@ -161,6 +161,18 @@ class Calculator {
 	size_t off_slots_ = 0;
 	uint32_t assign_slots(uint32_t n, uint32_t capacity);
 	uint32_t stamp_epoch_ = 0;
+	// depth-first order of the staged list (four-state FP64, 20-state FP32)
+	static constexpr uint32_t kNone = 0xFFFFFFFFu;
+	bool depth_first_ = false;
+	uint32_t order_groups_ = 1, order_phases_ = 1;
+	std::vector<uint32_t> order_, segs_, kid_, parent_, cost_, chain_, walk_stack_, pieces_,
+		above_;
+	std::vector<uint32_t> slot_pos_; // by partial slot; kNone outside the call
+	std::vector<NodeOp> list_ops_;
+	void order_depth_first(uint32_t n);
+	template <typename Emit>
+	bool split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit);
+	void stage_inputs(const double *src, uint32_t n, size_t per_entry);
 	uint32_t tip_children_ = 0;      // tip children in the staged list
 	bool model_set_ = false;
 	bool have_result_ = false;
@@ -209,10 +221,12 @@ class Calculator {
 	ModelDev *d_model_ = nullptr;
 	void *d_ptab_ = nullptr;
 	uint32_t f64_groups_ = 0; // 0: chosen per list
-	uint32_t pick_f64_groups(uint32_t n) const;
+	uint32_t pick_groups(uint32_t n) const;
 	uint32_t pick_p20_groups(uint32_t n) const;
+	uint32_t s20_groups_ = 0; // 20-state FP32 walk; 0: chosen per list
+	uint32_t s20_per_sm_[5] = {}; // blocks an SM holds, by warps a block
 	void *d_soft20_ = nullptr;           // 20-state FP64 form: d_ptab_ as integers
-	unsigned *d_tile_tickets_ = nullptr; // [ldp / 64], zero between launches
+	unsigned *d_tile_tickets_ = nullptr; // [ldp / 32], zero between launches
 	SoftTab4 *d_soft_ = nullptr; // four-state FP64 form: d_ptab_ as integers
 	unsigned char *d_stage_ = nullptr;
 

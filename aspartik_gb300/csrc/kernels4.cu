@@ -459,6 +459,24 @@ __device__ __forceinline__ double mix_categories_f64(uint32_t C, Value value, Co
 	return !any ? -INFINITY : bad ? NAN : log(acc) - (double)least + log_inv_c;
 }
 
+// The same for values with power-of-two exponents: sum_c s_c 2^E_c =
+// 2^Emax sum_c s_c 2^(E_c - Emax).
+template <typename Value, typename Count>
+__device__ __forceinline__ double mix_categories_pow2(uint32_t C, Value value, Count count,
+						      double log_inv_c)
+{
+	int32_t emax = INT32_MIN;
+	for (uint32_t k = 0; k < C; k++)
+		if (value(k) > 0.0)
+			emax = max(emax, (int32_t)count(k));
+	if (emax == INT32_MIN)
+		return -INFINITY;
+	double acc = 0.0;
+	for (uint32_t k = 0; k < C; k++)
+		acc += scalbn(value(k), (int32_t)count(k) - emax);
+	return log(acc) + (double)emax * 0.69314718055994530942 + log_inv_c;
+}
+
 // Root of the schedule: category mixing, pattern weights, block sum and the
 // fold of all block sums by the last block to finish (or by the host).  One
 // `lead` thread per (pattern, category) column reports its root dot product
@@ -506,22 +524,10 @@ __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem
 	if (tid < tp) {
 		double site;
 		if constexpr (kPow2) {
-			// sum_c s_c 2^E_c = 2^Emax sum_c s_c 2^(E_c - Emax)
-			int32_t emax = INT32_MIN;
-			for (uint32_t k = 0; k < C; k++)
-				if (s_val[k * tp + tid] > 0.0)
-					emax = max(emax, s_exp[k * tp + tid]);
-			if (emax == INT32_MIN) {
-				site = -INFINITY;
-			} else {
-				double acc = 0.0;
-				for (uint32_t k = 0; k < C; k++)
-					acc += scalbn(s_val[k * tp + tid],
-						      s_exp[k * tp + tid] - emax);
-				site = log(acc) +
-				       (double)emax * 0.69314718055994530942 +
-				       prm.log_inv_c;
-			}
+			site = mix_categories_pow2(
+				C, [&](uint32_t k) { return s_val[k * tp + tid]; },
+				[&](uint32_t k) { return s_exp[k * tp + tid]; },
+				prm.log_inv_c);
 		} else {
 			site = mix_categories_f64(
 				C, [&](uint32_t k) { return s_val[k * tp + tid]; },
@@ -811,20 +817,20 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 	const size_t smem = sizeof(double) * (2 * (size_t)p.C * tile + 32);
 	if (p.soft) {
 		const bool narrow = narrow_index((uint64_t)p.num_leaves * 2, p.C, p.ldp);
-		const uint32_t warps = p.f64_groups > 1 ? p.C * p.f64_groups : p.C * tile / 32u;
+		const uint32_t tp = p.groups > 1 ? 32u : tile;
+		const uint32_t warps = p.C * tp / 32u * p.groups;
+		if (warps > 16 || (p.groups > 1 && !p.segs))
+			return cudaErrorInvalidValue;
 		const size_t bytes = sizeof(double) * (64 * (size_t)warps + 32) +
-				     (size_t)warps * kF64Ring * sizeof(F64Entry);
-		if (p.f64_groups > 1) {
-			if (warps > 16 || !p.runs || p.n_runs > 2048)
-				return cudaErrorInvalidValue;
-			auto kern = narrow ? prune4_f64_runs_kernel<uint32_t>
-					   : prune4_f64_runs_kernel<size_t>;
-			kern<<<p.ldp / 32u, dim3(32, p.C, p.f64_groups),
-			       bytes + (p.n_runs + 1) * sizeof(uint32_t), s>>>(p);
-			return cudaGetLastError();
-		}
-		auto kern = narrow ? prune4_f64_kernel<uint32_t> : prune4_f64_kernel<size_t>;
-		kern<<<grid, block, bytes, s>>>(p);
+				     (size_t)warps * kF64Ring * sizeof(F64Entry) +
+				     (p.groups > 1 ? ((size_t)p.phases * p.groups + 1) * 4 : 0);
+		if (bytes > 48 * 1024)
+			return cudaErrorInvalidValue;
+		auto kern = p.groups > 1 ? (narrow ? prune4_f64_kernel<uint32_t, true>
+						   : prune4_f64_kernel<size_t, true>)
+					 : (narrow ? prune4_f64_kernel<uint32_t, false>
+						   : prune4_f64_kernel<size_t, false>);
+		kern<<<p.ldp / tp, dim3(tp, p.C, p.groups), bytes, s>>>(p);
 		return cudaGetLastError();
 	}
 	prune4_plain_kernel<<<grid, block, smem, s>>>(p);
@@ -987,17 +993,30 @@ cudaError_t launch_prune20_f64(const PruneParams &p, uint32_t groups, cudaStream
 	return cudaGetLastError();
 }
 
+uint32_t prune20_blocks_per_sm(uint32_t groups)
+{
+	int n = 0;
+	const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+		&n, prune20_kernel<uint32_t, true>, (int)(32 * groups),
+		groups * kS20Ring * sizeof(S20Entry));
+	return e == cudaSuccess && n > 0 ? (uint32_t)n : 1u;
+}
+
 cudaError_t launch_prune20(const PruneParams &p, cudaStream_t s)
 {
-	if (p.C == 0 || p.C > 8 || p.ldp % 32u)
+	if (p.C == 0 || p.C > 8 || p.ldp % 128u || p.groups < 1 || p.groups > 4 ||
+	    !p.sums_host || (p.groups > 1 && !p.segs))
 		return cudaErrorInvalidValue;
-	const dim3 block(32, p.C), grid(p.ldp / 32);
-	const size_t smem = sizeof(double) * (2 * (size_t)block.x * block.y + 32);
+	const size_t smem = (size_t)p.groups * kS20Ring * sizeof(S20Entry) +
+			    (p.groups > 1 ? ((size_t)p.phases * p.groups + 1) * 4 : 0);
+	if (smem > 48 * 1024)
+		return cudaErrorInvalidValue;
 	const bool narrow = (uint64_t)p.num_leaves * 2 * p.C * p.ldp < (1ull << 31);
-	if (narrow)
-		prune20_kernel<uint32_t><<<grid, block, smem, s>>>(p);
-	else
-		prune20_kernel<size_t><<<grid, block, smem, s>>>(p);
+	auto kern = p.groups > 1 ? (narrow ? prune20_kernel<uint32_t, true>
+					   : prune20_kernel<size_t, true>)
+				 : (narrow ? prune20_kernel<uint32_t, false>
+					   : prune20_kernel<size_t, false>);
+	kern<<<dim3(p.ldp / 32u, p.C), 32 * p.groups, smem, s>>>(p);
 	return cudaGetLastError();
 }
 

@@ -33,7 +33,6 @@
 // and writes the tile's weighted sum to mapped host memory.
 
 constexpr uint32_t kP20Tile = 64;
-constexpr uint32_t kP20RunsSmem = 2048;
 constexpr uint32_t kTab20Chunks = sizeof(SoftTab20) / 16; // 336
 constexpr uint32_t kXStride = kP20Tile + 1;
 // significands of a child: 2^62 <= X < 2^63; of a table entry 2^59 <= M <

@@ -60,6 +60,35 @@ __host__ __device__ __forceinline__ uint32_t tc_off_a(uint32_t row, uint32_t k)
 	return (row >> 3) * (kTcSboA / 4) + (k >> 2) * 32u + (row & 7u) * 4u + (k & 3u);
 }
 
+// FP32 form: exact power-of-two normalisation of the largest entry into
+// [1, 2); returns the exponent (see rescale_pow2).
+__device__ __forceinline__ int32_t rescale_pow2_20(float y[20])
+{
+	float m = y[0];
+#pragma unroll
+	for (int i = 1; i < 20; i++)
+		m = fmaxf(m, y[i]);
+	if (!(m > 0.0f))
+		return 0; // all zero: the pattern is impossible
+	int32_t shift = 0;
+	uint32_t ex = (__float_as_uint(m) >> 23) & 0xffu;
+	if (ex == 0u) { // subnormal maximum: lift by 2^64 first (exact)
+		const float lift = 18446744073709551616.0f;
+#pragma unroll
+		for (int i = 0; i < 20; i++)
+			y[i] *= lift;
+		shift = -64;
+		m *= lift;
+		ex = (__float_as_uint(m) >> 23) & 0xffu;
+	}
+	const int32_t e = (int32_t)ex - 127;
+	const float f = __uint_as_float((uint32_t)(127 - e) << 23); // 2^-e
+#pragma unroll
+	for (int i = 0; i < 20; i++)
+		y[i] *= f;
+	return e + shift;
+}
+
 // Named barrier of one 128-thread group: id 1 for group 0, 2 for group 1
 // (0 is __syncthreads).  Immediate ids keep the CTA's barrier count at 3.
 __device__ __forceinline__ void group_sync(uint32_t g)
@@ -236,8 +265,6 @@ __global__ void __launch_bounds__(128 * kG, 4 / kG) prune20tc_kernel(Tc20Params 
 		return r == 0 ? 1u : min(r, prm.n - e0);
 	};
 
-	// output rows pass through the left A-hi block (raw [128][20] layout)
-	float *stage = sA;
 	uint32_t lphase = 0, mphase = 0;
 	bool failed = false, pending = false;
 	uint32_t e0 = 0, r = run_len(0);
@@ -261,34 +288,42 @@ __global__ void __launch_bounds__(128 * kG, 4 / kG) prune20tc_kernel(Tc20Params 
 			lphase ^= 1u;
 			pending = false;
 			// this thread's rows: a tip side's final value from its table,
-			// an internal side's partial row from the copied block
+			// an internal side's partial row (state pairs, 128 patterns)
+			// from the copied block
 			float v[2][S];
 			int32_t sc[2];
 #pragma unroll
 			for (uint32_t j = 0; j < 2; j++) {
-				const float *row;
 				if (ids[j] & kTipBit) {
 					const uint32_t leaf = ids[j] & ~kTipBit;
 					const uint32_t code =
 						prm.tips_smem ? sTips[leaf * kTcRows + t]
 							      : sSide[1536 + 128 * j + t];
-					row = sB + j * 2 * kTcB + min(code, (uint32_t)S) * S;
+					const float4 *r4 = reinterpret_cast<const float4 *>(
+						sB + j * 2 * kTcB + min(code, (uint32_t)S) * S);
 					sc[j] = 0;
+#pragma unroll
+					for (int q = 0; q < 5; q++) {
+						const float4 a = r4[q];
+						v[j][4 * q] = a.x;
+						v[j][4 * q + 1] = a.y;
+						v[j][4 * q + 2] = a.z;
+						v[j][4 * q + 3] = a.w;
+					}
 				} else {
-					row = sA + (2 * j + 1) * kTcA + t * S;
+					const float2 *blk = reinterpret_cast<const float2 *>(
+								    sA + (2 * j + 1) * kTcA) +
+							    t;
+#pragma unroll
+					for (int k = 0; k < S / 2; k++) {
+						const float2 a = blk[k * kTcRows];
+						v[j][2 * k] = a.x;
+						v[j][2 * k + 1] = a.y;
+					}
 					sc[j] = reinterpret_cast<const int32_t *>(sSide + 512 + 512 * j)[t];
 				}
-				const float4 *r4 = reinterpret_cast<const float4 *>(row);
-#pragma unroll
-				for (int q = 0; q < 5; q++) {
-					const float4 a = r4[q];
-					v[j][4 * q] = a.x;
-					v[j][4 * q + 1] = a.y;
-					v[j][4 * q + 2] = a.z;
-					v[j][4 * q + 3] = a.w;
-				}
 			}
-			// every copied row read, the previous entry's output stored
+			// every copied row read
 			group_sync(g);
 			const bool next = e + G < e0 + r;
 			if (!any) {
@@ -378,19 +413,13 @@ __global__ void __launch_bounds__(128 * kG, 4 / kG) prune20tc_kernel(Tc20Params 
 				prm.root_val[(size_t)c * prm.ldp + p] = dot;
 				prm.root_exp[(size_t)c * prm.ldp + p] = cnt;
 			}
-			// the output rows through shared memory, then 16-byte stores
-			// of consecutive addresses by consecutive threads
-			float4 *srow = reinterpret_cast<float4 *>(stage + t * S);
+			float2 *dst = reinterpret_cast<float2 *>(
+					      prm.partials +
+					      (size_t)((Idx)op.out * stride + col0) * S) +
+				      t;
 #pragma unroll
-			for (int q = 0; q < 5; q++)
-				srow[q] = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
-			group_sync(g);
-			const float4 *s4 = reinterpret_cast<const float4 *>(stage);
-			float4 *d4 = reinterpret_cast<float4 *>(
-				prm.partials + (size_t)((Idx)op.out * stride + col0) * S);
-#pragma unroll
-			for (uint32_t q = 0; q < 5; q++)
-				d4[t + 128 * q] = s4[t + 128 * q];
+			for (int k = 0; k < S / 2; k++)
+				dst[k * kTcRows] = make_float2(y[2 * k], y[2 * k + 1]);
 		}
 		// the run's outputs are visible to every group of the cluster,
 		// and to the bulk copies of the next run, before those read them
@@ -453,20 +482,9 @@ __global__ void __launch_bounds__(128) finish20_kernel(Tc20Params prm)
 	__shared__ unsigned s_last;
 	const uint32_t t = threadIdx.x, p = blockIdx.x * 128 + t;
 	const uint32_t C = prm.C, ldp = prm.ldp;
-	int32_t emax = INT32_MIN;
-	for (uint32_t k = 0; k < C; k++)
-		if (prm.root_val[(size_t)k * ldp + p] > 0.0)
-			emax = max(emax, prm.root_exp[(size_t)k * ldp + p]);
-	double site;
-	if (emax == INT32_MIN) {
-		site = -INFINITY;
-	} else {
-		double acc = 0.0;
-		for (uint32_t k = 0; k < C; k++)
-			acc += scalbn(prm.root_val[(size_t)k * ldp + p],
-				      prm.root_exp[(size_t)k * ldp + p] - emax);
-		site = log(acc) + (double)emax * 0.69314718055994530942 + prm.log_inv_c;
-	}
+	const double site = mix_categories_pow2(
+		C, [&](uint32_t k) { return prm.root_val[(size_t)k * ldp + p]; },
+		[&](uint32_t k) { return prm.root_exp[(size_t)k * ldp + p]; }, prm.log_inv_c);
 	prm.site_lnl[p] = site;
 	if (prm.cat_lnl)
 		for (uint32_t k = 0; k < C; k++)

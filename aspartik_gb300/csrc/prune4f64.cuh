@@ -2,9 +2,10 @@
 // integer pipes (soft64.cuh).  Included by kernels4.cu inside its anonymous
 // namespace (uses v4_apply, v4_mul, rescale_threshold, finish_root).
 //
-// One thread owns one (pattern, category) column and walks the whole
-// children-first list, as the plain walk does; a warp's columns share one
-// category, so its transition tables are the same for every lane.
+// One thread owns one (pattern, category) column and walks the list depth
+// first; a warp's columns share one category, so its transition tables are
+// the same for every lane.  Where the columns leave the schedulers short of
+// warps, several groups of a block walk disjoint subtrees first.
 //   - Tables: each warp keeps a ring of kF64Ring entries (schedule word and
 //     the two soft tables of its category, 432 bytes) in shared memory,
 //     filled by one 16-byte cp.async a lane and entry, so no table load
@@ -253,140 +254,101 @@ __device__ __forceinline__ double f64_root_dot(const PruneParams &prm, const dou
 	return prm.pi[0] * y.x + prm.pi[1] * y.y + prm.pi[2] * y.z + prm.pi[3] * y.w;
 }
 
-// Serial form: a thread walks its column's whole list.
-template <typename Idx>
+// A block of (tp patterns, C categories, G groups).  Several groups share the
+// list in phases (prm.segs, the host's depth-first order): in phase ph group
+// g walks entries [segs[ph G + g], segs[ph G + g + 1]) of its columns, whole
+// subtrees first, then the entries above them run by run; a barrier ends a
+// phase.  Group 0 walks the last entry, the root.
+template <typename Idx, bool kGroups>
 __global__ void __launch_bounds__(512) prune4_f64_kernel(PruneParams prm)
 {
 	const uint32_t tp = blockDim.x, c = threadIdx.y, C = prm.C;
+	const uint32_t g = kGroups ? threadIdx.z : 0u, G = kGroups ? blockDim.z : 1u;
 	const uint32_t p = blockIdx.x * tp + threadIdx.x;
 	const Idx stride = (Idx)C * prm.ldp, col = (Idx)c * prm.ldp + p;
 	extern __shared__ __align__(16) double smem[];
-	const uint32_t tid = threadIdx.y * tp + threadIdx.x, lane = tid & 31u;
-	F64Entry *ring = reinterpret_cast<F64Entry *>(smem + 2 * tp * C + 32) +
-			 (tid >> 5) * kF64Ring;
-#pragma unroll
-	for (uint32_t e = 0; e < kF64Ring; ++e)
-		f64_fill(prm, ring + e, e, c, lane);
-	cp_async_wait<kF64Ring - 2>(); // entries 0 and 1 have landed
-	__syncwarp();
-	const NodeOp none{kTipBit, kTipBit, kTipBit, 0};
-	NodeOp op = ring[0].op, nop = prm.n > 1 ? ring[1].op : none;
-	F64Child l, r;
-	f64_load<Idx>(prm, op.left, kTipBit, p, stride, col, l);
-	f64_load<Idx>(prm, op.right, kTipBit, p, stride, col, r);
-	const SoftNum mult = soft_split((uint32_t)__double2hiint(prm.scale_mult),
-					(uint32_t)__double2loint(prm.scale_mult));
-	double4_32a y = v4_make<double4_32a, double>(0, 0, 0, 0);
-	int32_t cnt = 0;
-	for (uint32_t i = 0; i < prm.n; ++i) {
-		F64Child nl, nr;
-		if (i + 1 < prm.n) {
-			f64_load<Idx>(prm, nop.left, op.out, p, stride, col, nl);
-			f64_load<Idx>(prm, nop.right, op.out, p, stride, col, nr);
-		}
-		cp_async_wait<kF64Ring - 3>(); // entry i + 2 has landed
-		__syncwarp();
-		const NodeOp nnop = i + 2 < prm.n ? ring[(i + 2) & (kF64Ring - 1)].op : none;
-		const int32_t own = f64_entry(prm, ring[i & (kF64Ring - 1)], op, i, p, c, l, r,
-					      mult, y);
-		cnt = l.s + r.s + own;
-		const Idx ox = (Idx)op.out * stride + col;
-		((double4_32a *)prm.partials)[ox] = y;
-		prm.scales[ox] = cnt;
-		__syncwarp(); // every lane has read the slot that is filled next
-		f64_fill(prm, ring + (i & (kF64Ring - 1)), i + kF64Ring, c, lane);
-		l = nl;
-		r = nr;
-		if (nop.left == op.out) {
-			l.x = y;
-			l.s = cnt;
-		}
-		if (nop.right == op.out) {
-			r.x = y;
-			r.s = cnt;
-		}
-		op = nop;
-		nop = nnop;
+	const uint32_t tid = (g * C + c) * tp + threadIdx.x, lane = tid & 31u;
+	F64Entry *rings = reinterpret_cast<F64Entry *>(smem + 2 * tp * C * G + 32);
+	F64Entry *ring = rings + (tid >> 5) * kF64Ring;
+	uint32_t *s_segs = reinterpret_cast<uint32_t *>(rings + tp / 32u * C * G * kF64Ring);
+	if constexpr (kGroups) {
+		for (uint32_t k = tid; k <= prm.phases * G; k += tp * C * G)
+			s_segs[k] = prm.segs[k];
+		__syncthreads();
 	}
-	finish_root<false>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, true,
-			   f64_root_dot(prm, y), cnt);
-}
-
-// Run form, for problems whose columns leave the schedulers short of warps:
-// a block of (32 patterns, C categories, G groups) walks the list run by run
-// (prm.runs: entries of a run are mutually independent), group g taking
-// entries g, g + G, ... of each run; a barrier ends a run.  A child may be
-// another group's output, so all of them come from memory.
-template <typename Idx>
-__global__ void __launch_bounds__(512) prune4_f64_runs_kernel(PruneParams prm)
-{
-	const uint32_t tp = 32, c = threadIdx.y, C = prm.C;
-	const uint32_t g = threadIdx.z, G = blockDim.z;
-	const uint32_t p = blockIdx.x * tp + threadIdx.x;
-	const Idx stride = (Idx)C * prm.ldp, col = (Idx)c * prm.ldp + p;
-	extern __shared__ __align__(16) double smem[];
-	const uint32_t lane = threadIdx.x, warp = threadIdx.z * C + threadIdx.y;
-	const uint32_t warps = C * G;
-	F64Entry *ring = reinterpret_cast<F64Entry *>(smem + 64 * warps + 32) + warp * kF64Ring;
-	uint32_t *s_runs = reinterpret_cast<uint32_t *>(
-		reinterpret_cast<F64Entry *>(smem + 64 * warps + 32) + warps * kF64Ring);
-	for (uint32_t k = warp * 32u + lane; k <= prm.n_runs; k += warps * 32u)
-		s_runs[k] = prm.runs[k];
-	__syncthreads();
-	// the next entry of this group to copy: entry fe of run fr
-	uint32_t fr = 0, fe = s_runs[0] + g;
-	auto settle = [&] {
-		while (fr < prm.n_runs && fe >= s_runs[fr + 1]) {
-			++fr;
-			fe = s_runs[fr] + g;
+	// this group's next entry to copy: fe of phase fp, until fend
+	uint32_t fp = 0, fe = kGroups ? s_segs[g] : 0, fend = kGroups ? s_segs[g + 1] : prm.n;
+	uint32_t slot = 0;
+	auto fill = [&] {
+		while (kGroups && fe >= fend && fp + 1 < prm.phases) {
+			++fp;
+			fe = s_segs[fp * G + g];
+			fend = s_segs[fp * G + g + 1];
 		}
-	};
-	auto fill = [&](uint32_t slot) {
-		settle();
-		f64_fill(prm, ring + (slot & (kF64Ring - 1)), fr < prm.n_runs ? fe : prm.n, c,
-			 lane);
-		fe += G;
+		f64_fill(prm, ring + slot, fe < fend ? fe : prm.n, c, lane);
+		++fe;
+		slot = (slot + 1) & (kF64Ring - 1);
 	};
 #pragma unroll
 	for (uint32_t e = 0; e < kF64Ring; ++e)
-		fill(e);
+		fill();
+	const NodeOp none{kTipBit, kTipBit, kTipBit, 0};
 	const SoftNum mult = soft_split((uint32_t)__double2hiint(prm.scale_mult),
 					(uint32_t)__double2loint(prm.scale_mult));
 	double4_32a y = v4_make<double4_32a, double>(0, 0, 0, 0);
 	int32_t cnt = 0;
-	uint32_t j = 0; // entries this group has walked
-	for (uint32_t run = 0; run < prm.n_runs; ++run) {
-		const uint32_t lo = s_runs[run], hi = s_runs[run + 1];
+	uint32_t cur = 0; // ring slot of the current entry
+	auto walk = [&](uint32_t lo, uint32_t hi) {
+		if (lo >= hi)
+			return;
+		cp_async_wait<kF64Ring - 2>(); // the first two entries have landed
+		__syncwarp();
+		NodeOp op = ring[cur].op;
+		NodeOp nop = lo + 1 < hi ? ring[(cur + 1) & (kF64Ring - 1)].op : none;
 		F64Child l, r;
-		for (uint32_t i = lo + g; i < hi; i += G, ++j) {
-			// this group's entries j and j + 1 have landed
-			cp_async_wait<kF64Ring - 2>();
-			__syncwarp();
-			const F64Entry &en = ring[j & (kF64Ring - 1)];
-			const NodeOp op = en.op;
-			if (i == lo + g) {
-				f64_load<Idx>(prm, op.left, kTipBit, p, stride, col, l);
-				f64_load<Idx>(prm, op.right, kTipBit, p, stride, col, r);
-			}
+		f64_load<Idx>(prm, op.left, kTipBit, p, stride, col, l);
+		f64_load<Idx>(prm, op.right, kTipBit, p, stride, col, r);
+		for (uint32_t i = lo; i < hi; ++i) {
 			F64Child nl, nr;
-			if (i + G < hi) {
-				const NodeOp &nop = ring[(j + 1) & (kF64Ring - 1)].op;
-				f64_load<Idx>(prm, nop.left, kTipBit, p, stride, col, nl);
-				f64_load<Idx>(prm, nop.right, kTipBit, p, stride, col, nr);
+			if (i + 1 < hi) {
+				f64_load<Idx>(prm, nop.left, op.out, p, stride, col, nl);
+				f64_load<Idx>(prm, nop.right, op.out, p, stride, col, nr);
 			}
-			const int32_t own = f64_entry(prm, en, op, i, p, c, l, r, mult, y);
+			cp_async_wait<kF64Ring - 3>(); // entry i + 2 has landed
+			__syncwarp();
+			const NodeOp nnop =
+				i + 2 < hi ? ring[(cur + 2) & (kF64Ring - 1)].op : none;
+			const int32_t own =
+				f64_entry(prm, ring[cur], op, i, p, c, l, r, mult, y);
 			cnt = l.s + r.s + own;
 			const Idx ox = (Idx)op.out * stride + col;
 			((double4_32a *)prm.partials)[ox] = y;
 			prm.scales[ox] = cnt;
 			__syncwarp(); // every lane has read the slot that is filled next
-			fill(j);
+			fill();
+			cur = (cur + 1) & (kF64Ring - 1);
 			l = nl;
 			r = nr;
+			if (nop.left == op.out) {
+				l.x = y;
+				l.s = cnt;
+			}
+			if (nop.right == op.out) {
+				r.x = y;
+				r.s = cnt;
+			}
+			op = nop;
+			nop = nnop;
 		}
-		__syncthreads(); // the run's outputs are visible to every group
+	};
+	if constexpr (kGroups) {
+		for (uint32_t ph = 0; ph < prm.phases; ++ph) {
+			walk(s_segs[ph * G + g], s_segs[ph * G + g + 1]);
+			__syncthreads(); // the phase's outputs are visible to every group
+		}
+	} else {
+		walk(0, prm.n);
 	}
-	// the last entry (the root) is alone in its run: group 0 walked it
 	finish_root<false>(prm, smem, tp, threadIdx.x, blockIdx.x * tp, c, g == 0,
 			   f64_root_dot(prm, y), cnt);
 }

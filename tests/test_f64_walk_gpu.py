@@ -105,3 +105,49 @@ def test_protein_groups_agree(taxa, sites, K, monkeypatch):
     for lnl, sites_ in got:
         assert np.array_equal(sites_, got[0][1])
         assert abs(lnl - want) <= 1e-10 * abs(want)
+
+
+@pytest.mark.parametrize("taxa,sites,K", [(2, 1, 1), (7, 65, 4), (48, 200, 8), (200, 40, 2)])
+def test_protein_fp32_groups_agree(taxa, sites, K, monkeypatch):
+    """20 states, FP32 register-MMA walk: one to four warps a block (disjoint
+    subtrees, then the entries above them) give the same bits per pattern over
+    whole trees, a dirty path and a list that repeats, and the generic
+    oracle's likelihood to the FP32 bar (1e-6)."""
+    from oracle import generic as G
+    from tests.cases import protein_case
+    from aspartik_gb300.calculator import Calculator
+
+    c = protein_case(taxa, sites, seed=taxa, num_categories=K, gaps=0.05)
+    got = []
+    for groups in ("", "1", "2", "3", "4"):
+        if groups:
+            monkeypatch.setenv("B3G_S20_GROUPS", groups)
+        else:
+            monkeypatch.delenv("B3G_S20_GROUPS", raising=False)
+        tree = O.DatedTree(c.tree.parents, c.tree.heights)
+        g = Calculator.GB300(0, "f32").make20(c.leaves, c.leaves.shape[1], num_categories=K)
+        g.set_weights(c.weights)
+        g.set_reversible(c.rates, c.pi)
+        if K > 1:
+            g.set_gamma(1.0)
+        rng = np.random.default_rng(3)
+        tree.mark_all_edges_updated()
+        mine = []
+        for _ in range(3):
+            lists = lists_and_lengths(tree)
+            for _ in range(2):
+                g.propose_lengths(*lists, 1.0)
+                mine.append((g.log_likelihood(), g.site_log_likelihoods()))
+            g.accept()
+            tree.accept()
+            random_move(tree, rng)
+        g.close()
+        got.append(mine)
+    want = G.log_likelihood(c.leaves, c.weights, c.tree.parents, c.tree.heights,
+                            O.reversible(c.rates, c.pi),
+                            O.gamma_categories(1.0, K) if K > 1 else np.ones(1))
+    assert abs(got[0][0][0] - want) <= 1e-6 * abs(want)
+    for mine in got[1:]:
+        for (l0, s0), (l1, s1) in zip(got[0], mine):
+            assert np.array_equal(s0, s1)
+            assert l0 == l1
