@@ -5,8 +5,9 @@
 // b_l [out].  Hidden layers use GELU in its tanh form (Hendrycks and
 // Gimpel, "Gaussian Error Linear Units", 2016):
 //     gelu(x) = x/2 (1 + tanh(u)),  u = sqrt(2/pi) (x + 0.044715 x^3).
-// Products go through one shared-memory tiled FP32 GEMM kernel with
-// optional transposes; Adam (Kingma and Ba, 2015) updates the parameters.
+// A training step is seven launches: three hidden layers forward, the pair
+// objective with the output layer's backward pass, and three hidden layers
+// backward; Adam (Kingma and Ba, 2015) updates the parameters.
 #include <cooperative_groups.h>
 
 #include "calculator.hpp"
@@ -41,104 +42,404 @@ __device__ __forceinline__ float gelu_grad(float x)
 	       0.5f * x * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * x * x);
 }
 
-// C[M][N] = sum_k A'(m, k) B'(k, n) (+ bias[n]); A'(m, k) = TA ? A[k][m] :
-// A[m][k] with row stride lda, B'(k, n) = TB ? B[n][k] : B[k][n] with row
-// stride ldb.  With `act` the GELU of C goes to Cact and C itself to C.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) gemm_kernel(const float *__restrict__ A,
-						    const float *__restrict__ B,
-						    const float *__restrict__ bias,
-						    float *__restrict__ C,
-						    float *__restrict__ Cact,
-						    uint32_t M, uint32_t N, uint32_t K,
-						    uint32_t lda, uint32_t ldb)
+// ---------------------------------------------------------------------------
+// FP32 matrix products of the training step.
+//
+// A block of 128 threads computes a 32 x 64 tile of C[m][n] = sum_k A'(m, k)
+// B'(k, n), a thread 4 x 4 of it, k in order; operand tiles of 32 k pass
+// through two shared-memory buffers filled by cp.async while the other is
+// used.  A'(m, k) = TA ? A[k][m] : A[m][k] with row stride lda, B'(k, n) = TB ?
+// B[n][k] : B[k][n] with row stride ldb.  The tile is this small because the
+// step is: 1,024 rows x 256 units are 128 tiles for 152 SMs (16 x 16 tiles
+// with one product a thread and shared-memory word pair took 17 to 36 us a
+// product; these take 5 to 8).
+constexpr uint32_t kTm = 32, kTn = 64, kTk = 32;
+// a weight gradient's rows are split over up to kSplits blocks a tile, at
+// least kSplitRows each, whose partial tiles the last one adds in a fixed order
+constexpr uint32_t kSplits = 16, kSplitRows = 128;
+
+struct MlpSmem {
+	// [m][k] or [k][m], rows padded to 36 / 68 floats (16-byte aligned)
+	float a[2][kTk * (kTm + 4)];
+	float b[2][kTn * (kTk + 4)];
+};
+
+__device__ __forceinline__ void mlp_cp16(float *dst, const float *src, bool live)
 {
-	constexpr int T = 16;
-	__shared__ float sa[T][T + 1];
-	__shared__ float sb[T][T + 1];
-	const uint32_t tx = threadIdx.x, ty = threadIdx.y;
-	const uint32_t m = blockIdx.y * T + ty;
-	const uint32_t n = blockIdx.x * T + tx;
-	float acc = 0.0f;
-	for (uint32_t k0 = 0; k0 < K; k0 += T) {
-		// A' tile rows m, columns k0 + tx
-		{
-			const uint32_t mm = blockIdx.y * T + ty, kk = k0 + tx;
-			float v = 0.0f;
-			if (mm < M && kk < K)
-				v = TA ? A[(size_t)kk * lda + mm] : A[(size_t)mm * lda + kk];
-			sa[ty][tx] = v;
-		}
-		// B' tile rows k0 + ty, columns n
-		{
-			const uint32_t kk = k0 + ty, nn = blockIdx.x * T + tx;
-			float v = 0.0f;
-			if (kk < K && nn < N)
-				v = TB ? B[(size_t)nn * ldb + kk] : B[(size_t)kk * ldb + nn];
-			sb[ty][tx] = v;
-		}
-		__syncthreads();
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+			     (uint32_t)__cvta_generic_to_shared(dst)),
+		     "l"(src), "r"(live ? 16 : 0)
+		     : "memory");
+}
+__device__ __forceinline__ void mlp_cp4(float *dst, const float *src, bool live)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+			     (uint32_t)__cvta_generic_to_shared(dst)),
+		     "l"(src), "r"(live ? 4 : 0)
+		     : "memory");
+}
+
+// rows x cols of a row-major matrix from (r0, c0), elements outside [0, R) x
+// [0, C) as zero, into dst with row stride `pitch`.  vec: ld, c0, C and the
+// base are multiples of four floats.
+template <uint32_t rows, uint32_t cols>
+__device__ __forceinline__ void mlp_tile(float *dst, uint32_t pitch, const float *src,
+					 uint32_t r0, uint32_t c0, uint32_t R, uint32_t C,
+					 uint32_t ld, bool vec)
+{
+	if (vec) {
 #pragma unroll
-		for (int k = 0; k < T; ++k)
-			acc = fmaf(sa[ty][k], sb[k][tx], acc);
+		for (uint32_t i = 0; i < rows * cols / 4 / 128; ++i) {
+			const uint32_t at = threadIdx.x + 128 * i;
+			const uint32_t r = at / (cols / 4), c = 4 * (at % (cols / 4));
+			const bool live = r0 + r < R && c0 + c < C;
+			mlp_cp16(dst + r * pitch + c,
+				 live ? src + (size_t)(r0 + r) * ld + c0 + c : src, live);
+		}
+	} else {
+#pragma unroll 4
+		for (uint32_t i = 0; i < rows * cols / 128; ++i) {
+			const uint32_t at = threadIdx.x + 128 * i;
+			const uint32_t r = at / cols, c = at % cols;
+			const bool live = r0 + r < R && c0 + c < C;
+			mlp_cp4(dst + r * pitch + c,
+				live ? src + (size_t)(r0 + r) * ld + c0 + c : src, live);
+		}
+	}
+}
+
+__device__ __forceinline__ bool mlp_vec(const float *p, uint32_t ld)
+{
+	return (ld & 3u) == 0 && ((uintptr_t)p & 15u) == 0;
+}
+
+// The tile's products over k in [k0, k1).  Thread (ty, tx): rows 4 ty + i,
+// columns TB ? tx + 16 j : 4 tx + j.  col_sum (TA): threads 0..31 also add
+// A'(m0 + thread, k) over k.
+template <bool TA, bool TB>
+__device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const float *B,
+					    uint32_t m0, uint32_t n0, uint32_t M, uint32_t N,
+					    uint32_t k0, uint32_t k1, uint32_t lda, uint32_t ldb,
+					    float acc[4][4], float *col_sum = nullptr)
+{
+	constexpr uint32_t pa = TA ? kTm + 4 : kTk + 4, pb = TB ? kTk + 4 : kTn + 4;
+	const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
+	// a row of the operand in memory must be whole vectors up to its end
+	const bool va = mlp_vec(A, lda) && ((TA ? M : k1) & 3u) == 0;
+	const bool vb = mlp_vec(B, ldb) && ((TB ? k1 : N) & 3u) == 0;
+	auto fetch = [&](uint32_t k, uint32_t buf) {
+		if (k < k1) {
+			if (TA)
+				mlp_tile<kTk, kTm>(sm.a[buf], pa, A, k, m0, k1, M, lda, va);
+			else
+				mlp_tile<kTm, kTk>(sm.a[buf], pa, A, m0, k, M, k1, lda, va);
+			if (TB)
+				mlp_tile<kTn, kTk>(sm.b[buf], pb, B, n0, k, N, k1, ldb, vb);
+			else
+				mlp_tile<kTk, kTn>(sm.b[buf], pb, B, k, n0, k1, N, ldb, vb);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+#pragma unroll
+	for (int i = 0; i < 4; ++i)
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+			acc[i][j] = 0.0f;
+	float cs = 0.0f;
+	fetch(k0, 0);
+	uint32_t buf = 0;
+	for (uint32_t k = k0; k < k1; k += kTk, buf ^= 1u) {
+		fetch(k + kTk, buf ^ 1u);
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
 		__syncthreads();
+		const float *sa = sm.a[buf], *sb = sm.b[buf];
+#pragma unroll
+		for (uint32_t kk = 0; kk < kTk; kk += 4) {
+			float a[4][4], b[4][4]; // [k][i], [k][j]
+#pragma unroll
+			for (int i = 0; i < 4; ++i) {
+				if (TA) {
+					const float4 v = *reinterpret_cast<const float4 *>(
+						sa + (kk + i) * pa + 4 * ty);
+					a[i][0] = v.x, a[i][1] = v.y, a[i][2] = v.z, a[i][3] = v.w;
+				} else {
+					const float4 v = *reinterpret_cast<const float4 *>(
+						sa + (4 * ty + i) * pa + kk);
+					a[0][i] = v.x, a[1][i] = v.y, a[2][i] = v.z, a[3][i] = v.w;
+				}
+				if (TB) {
+					const float4 v = *reinterpret_cast<const float4 *>(
+						sb + (tx + 16 * i) * pb + kk);
+					b[0][i] = v.x, b[1][i] = v.y, b[2][i] = v.z, b[3][i] = v.w;
+				} else {
+					const float4 v = *reinterpret_cast<const float4 *>(
+						sb + (kk + i) * pb + 4 * tx);
+					b[i][0] = v.x, b[i][1] = v.y, b[i][2] = v.z, b[i][3] = v.w;
+				}
+			}
+#pragma unroll
+			for (int q = 0; q < 4; ++q)
+#pragma unroll
+				for (int i = 0; i < 4; ++i)
+#pragma unroll
+					for (int j = 0; j < 4; ++j)
+						acc[i][j] = fmaf(a[q][i], b[q][j], acc[i][j]);
+		}
+		if (TA && col_sum && threadIdx.x < kTm)
+			for (uint32_t kk = 0; kk < kTk; ++kk)
+				cs += sa[kk * pa + threadIdx.x];
+		__syncthreads(); // the buffer is free for the next fetch
 	}
-	if (m < M && n < N) {
-		if (bias)
-			acc += bias[n];
-		C[(size_t)m * N + n] = acc;
-		if (Cact)
-			Cact[(size_t)m * N + n] = gelu(acc);
+	if (TA && col_sum)
+		*col_sum = cs;
+}
+
+// Hidden layer: z = x W^T + b and a = gelu(z).  Grid (N / 64, M / 32).
+__global__ void __launch_bounds__(128) mlp_forward_kernel(const float *__restrict__ x,
+							   const float *__restrict__ W,
+							   const float *__restrict__ bias,
+							   float *__restrict__ z,
+							   float *__restrict__ a, uint32_t M,
+							   uint32_t N, uint32_t K)
+{
+	__shared__ __align__(16) MlpSmem sm;
+	const uint32_t m0 = blockIdx.y * kTm, n0 = blockIdx.x * kTn;
+	const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
+	float acc[4][4];
+	mlp_product<false, true>(sm, x, W, m0, n0, M, N, 0, K, K, K, acc);
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const uint32_t n = n0 + tx + 16 * j;
+		if (n >= N)
+			continue;
+		const float bn = bias[n];
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			const uint32_t m = m0 + 4 * ty + i;
+			if (m >= M)
+				continue;
+			const float v = acc[i][j] + bn;
+			z[(size_t)m * N + n] = v;
+			a[(size_t)m * N + n] = gelu(v);
+		}
 	}
 }
 
-// dZ = dA * gelu'(Z), element by element; dZ may be dA (in place), so
-// neither is restrict-qualified
-__global__ void gelu_backward_kernel(const float *dA, const float *__restrict__ Z,
-				     float *dZ, uint32_t count)
+// Sum over lanes of a warp, the same in every lane, in a fixed order.
+__device__ __forceinline__ float warp_sum(float v)
 {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < count)
-		dZ[i] = dA[i] * gelu_grad(Z[i]);
+	for (int off = 16; off > 0; off >>= 1)
+		v += __shfl_xor_sync(0xffffffffu, v, off);
+	return v;
 }
 
-// db[o] = sum_n dZ[n][o], summed in row order
-__global__ void column_sum_kernel(const float *__restrict__ dZ,
-				  float *__restrict__ db, uint32_t rows,
-				  uint32_t cols)
+// y[m] = a[m] . w + b, a warp a row (forward pass only).
+__global__ void __launch_bounds__(256) mlp_out_kernel(const float *__restrict__ a,
+						       const float *__restrict__ w,
+						       float *__restrict__ y, uint32_t rows,
+						       uint32_t H)
 {
-	const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-	if (o >= cols)
+	const uint32_t lane = threadIdx.x & 31u, m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	if (m >= rows)
 		return;
-	float s = 0.0f;
-	for (uint32_t n = 0; n < rows; ++n)
-		s += dZ[(size_t)n * cols + o];
-	db[o] = s;
+	float v = 0.0f;
+	for (uint32_t k = lane; k < H; k += 32)
+		v = fmaf(a[(size_t)m * H + k], w[k], v);
+	v = warp_sum(v);
+	if (lane == 0)
+		y[m] = v + w[H];
 }
 
-// pair objective: rows 0..n-1 hold f(x_new), rows n..2n-1 f(x_old)
-__global__ void pair_loss_kernel(const float *__restrict__ y,
-				 const float *__restrict__ delta,
-				 float *__restrict__ dy, float *__restrict__ loss,
-				 uint32_t n)
+// The pair objective and the last layer's backward pass.  Row i of n holds
+// x_new's third layer, row n + i x_old's; a warp a pair: r = y_new - y_old -
+// delta, the loss's share r^2, dL/dy = +-2 r / n, and dZ of the third layer
+// = dL/dy w gelu'(z).  The block's share of the output weights' gradient
+// (sum of dL/dy a, and of dL/dy) goes to part[block][H + 1].  The last block
+// to finish adds the loss shares in block order.
+constexpr uint32_t kHeadPairs = 8;
+__global__ void __launch_bounds__(32 * kHeadPairs) mlp_head_kernel(
+	const float *__restrict__ a, const float *__restrict__ z, const float *__restrict__ w,
+	const float *__restrict__ delta, float *__restrict__ dz, float *__restrict__ part,
+	float *__restrict__ losses, float *__restrict__ loss, unsigned *ticket, uint32_t n,
+	uint32_t H)
 {
-	__shared__ float s[256];
-	float acc = 0.0f;
-	for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-		const float r = y[i] - y[n + i] - delta[i];
-		dy[i] = 2.0f * r / n;
-		dy[n + i] = -2.0f * r / n;
-		acc += r * r;
+	extern __shared__ float sh[]; // [kHeadPairs][H + 2]
+	__shared__ unsigned s_last;
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t i = blockIdx.x * kHeadPairs + warp;
+	const uint32_t pitch = H + 2;
+	float *mine = sh + warp * pitch;
+	float r = 0.0f, dy = 0.0f;
+	if (i < n) {
+		const float *an = a + (size_t)i * H, *ao = a + (size_t)(n + i) * H;
+		float yn = 0.0f, yo = 0.0f;
+		for (uint32_t k = lane; k < H; k += 32) {
+			yn = fmaf(an[k], w[k], yn);
+			yo = fmaf(ao[k], w[k], yo);
+		}
+		// the output bias cancels in the difference
+		r = warp_sum(yn) - warp_sum(yo) - delta[i];
+		dy = 2.0f * r / n;
+		for (uint32_t k = lane; k < H; k += 32) {
+			const size_t in = (size_t)i * H + k, io = (size_t)(n + i) * H + k;
+			dz[in] = dy * w[k] * gelu_grad(z[in]);
+			dz[io] = -dy * w[k] * gelu_grad(z[io]);
+			mine[k] = dy * an[k] - dy * ao[k];
+		}
+	} else {
+		for (uint32_t k = lane; k < H; k += 32)
+			mine[k] = 0.0f;
 	}
-	s[threadIdx.x] = acc;
+	if (lane == 0) {
+		mine[H] = dy - dy; // the bias gradient: +dy and -dy
+		mine[H + 1] = r * r;
+	}
 	__syncthreads();
-	for (uint32_t st = blockDim.x / 2; st > 0; st >>= 1) {
-		if (threadIdx.x < st)
-			s[threadIdx.x] += s[threadIdx.x + st];
-		__syncthreads();
+	for (uint32_t k = threadIdx.x; k <= H; k += blockDim.x) {
+		float v = 0.0f;
+		for (uint32_t q = 0; q < kHeadPairs; ++q)
+			v += sh[q * pitch + k];
+		part[(size_t)blockIdx.x * (H + 1) + k] = v;
 	}
-	if (threadIdx.x == 0)
-		*loss = s[0] / n;
+	if (threadIdx.x == 0) {
+		float v = 0.0f;
+		for (uint32_t q = 0; q < kHeadPairs; ++q)
+			v += sh[q * pitch + H + 1];
+		losses[blockIdx.x] = v;
+		__threadfence();
+		s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+	}
+	__syncthreads();
+	if (!s_last || warp != 0)
+		return;
+	__threadfence();
+	float v = 0.0f;
+	for (uint32_t k = lane; k < gridDim.x; k += 32)
+		v += __ldcg(losses + k);
+	v = warp_sum(v);
+	if (lane == 0) {
+		*loss = v / n;
+		*ticket = 0u;
+	}
+}
+
+// One hidden layer's backward pass.  Blocks [0, dw_blocks): the weight
+// gradient dW[o][i] = sum_rows dZ[row][o] a[row][i] and the bias gradient,
+// tiles x splits of split_rows rows; with several splits the partial tiles go
+// to `part` and a tile's last block adds them in split order.  Then
+// da_blocks: dZ of the layer below, (dZ W) gelu'(z_below).  Then, where
+// head_part is given, the output layer's gradient from the head kernel's
+// block shares.
+struct MlpBackward {
+	const float *dz, *a, *W, *z_below;
+	float *dW, *db, *dz_below;
+	float *part;       // [tiles][splits][kTm * kTn + kTm]
+	unsigned *tickets; // [tiles], zero between launches
+	const float *head_part;
+	float *head_grad;
+	uint32_t rows, O, I, splits, split_rows, dw_blocks, da_blocks, head_blocks;
+};
+__global__ void __launch_bounds__(128) mlp_backward_kernel(MlpBackward p)
+{
+	__shared__ __align__(16) MlpSmem sm;
+	__shared__ unsigned s_last;
+	const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
+	float acc[4][4];
+	if (blockIdx.x >= p.dw_blocks + p.da_blocks) {
+		// output layer: one column a thread
+		const uint32_t k = (blockIdx.x - p.dw_blocks - p.da_blocks) * 128 + threadIdx.x;
+		if (k > p.O)
+			return;
+		float v = 0.0f;
+#pragma unroll 8
+		for (uint32_t b = 0; b < p.head_blocks; ++b)
+			v += p.head_part[(size_t)b * (p.O + 1) + k];
+		p.head_grad[k] = v;
+		return;
+	}
+	if (blockIdx.x >= p.dw_blocks) {
+		const uint32_t t = blockIdx.x - p.dw_blocks, nt = (p.I + kTn - 1) / kTn;
+		const uint32_t m0 = t / nt * kTm, n0 = t % nt * kTn;
+		mlp_product<false, false>(sm, p.dz, p.W, m0, n0, p.rows, p.I, 0, p.O, p.O, p.I,
+					  acc);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			const uint32_t m = m0 + 4 * ty + i;
+			if (m >= p.rows)
+				continue;
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				const uint32_t n = n0 + 4 * tx + j;
+				if (n < p.I) {
+					const size_t at = (size_t)m * p.I + n;
+					p.dz_below[at] = acc[i][j] * gelu_grad(p.z_below[at]);
+				}
+			}
+		}
+		return;
+	}
+	const uint32_t tile = blockIdx.x / p.splits, split = blockIdx.x - tile * p.splits;
+	const uint32_t nt = (p.I + kTn - 1) / kTn;
+	const uint32_t m0 = tile / nt * kTm, n0 = tile % nt * kTn;
+	const uint32_t k0 = split * p.split_rows, k1 = min(p.rows, k0 + p.split_rows);
+	const bool bias = n0 == 0;
+	float cs = 0.0f;
+	mlp_product<true, false>(sm, p.dz, p.a, m0, n0, p.O, p.I, k0, k1, p.O, p.I, acc,
+				 bias ? &cs : nullptr);
+	if (p.splits > 1) {
+		float *part = p.part + (size_t)tile * p.splits * (kTm * kTn + kTm);
+		float4 *mine = reinterpret_cast<float4 *>(part + split * (kTm * kTn + kTm));
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			mine[(4 * ty + i) * (kTn / 4) + tx] =
+				make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+		if (threadIdx.x < kTm)
+			reinterpret_cast<float *>(mine)[kTm * kTn + threadIdx.x] = cs;
+		__threadfence();
+		__syncthreads();
+		if (threadIdx.x == 0)
+			s_last = atomicAdd(p.tickets + tile, 1u) == p.splits - 1u;
+		__syncthreads();
+		if (!s_last)
+			return;
+		__threadfence();
+		if (threadIdx.x == 0)
+			p.tickets[tile] = 0u;
+		cs = 0.0f;
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+#pragma unroll
+			for (int j = 0; j < 4; ++j)
+				acc[i][j] = 0.0f;
+		for (uint32_t q = 0; q < p.splits; ++q) {
+			const float *from = part + (size_t)q * (kTm * kTn + kTm);
+#pragma unroll
+			for (int i = 0; i < 4; ++i) {
+				const float4 v = __ldcg(reinterpret_cast<const float4 *>(from) +
+							(4 * ty + i) * (kTn / 4) + tx);
+				acc[i][0] += v.x;
+				acc[i][1] += v.y;
+				acc[i][2] += v.z;
+				acc[i][3] += v.w;
+			}
+			if (threadIdx.x < kTm)
+				cs += __ldcg(from + kTm * kTn + threadIdx.x);
+		}
+	}
+#pragma unroll
+	for (int i = 0; i < 4; ++i) {
+		const uint32_t m = m0 + 4 * ty + i;
+		if (m >= p.O)
+			continue;
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const uint32_t n = n0 + 4 * tx + j;
+			if (n < p.I)
+				p.dW[(size_t)m * p.I + n] = acc[i][j];
+		}
+	}
+	if (bias && threadIdx.x < kTm && m0 + threadIdx.x < p.O)
+		p.db[m0 + threadIdx.x] = cs;
 }
 
 __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g,
@@ -298,11 +599,6 @@ __global__ void __cluster_dims__(kDeltaCluster, 1, 1) __launch_bounds__(256)
 	}
 }
 
-dim3 gemm_grid(uint32_t M, uint32_t N)
-{
-	return dim3((N + 15) / 16, (M + 15) / 16);
-}
-
 } // namespace
 
 Mlp::Mlp(uint32_t in_dim, uint32_t hidden, uint64_t seed, int device)
@@ -362,15 +658,7 @@ Mlp::~Mlp()
 	cudaFree(d_grad_);
 	cudaFree(d_m_);
 	cudaFree(d_v_);
-	cudaFree(d_x_);
-	for (uint32_t l = 0; l < kLayers; ++l) {
-		cudaFree(d_z_[l]);
-		cudaFree(d_a_[l]);
-		cudaFree(d_da_[l]);
-	}
-	cudaFree(d_dy_);
-	cudaFree(d_delta_);
-	cudaFree(d_loss_);
+	free_batch();
 	cudaFreeHost(h_pair_);
 	for (InferCtx &c : extra_) {
 		cudaStreamSynchronize(c.stream);
@@ -381,69 +669,122 @@ Mlp::~Mlp()
 		cudaStreamDestroy(stream_);
 }
 
+void Mlp::free_batch()
+{
+	cudaFree(d_x_);
+	for (uint32_t l = 0; l + 1 < kLayers; ++l) {
+		cudaFree(d_z_[l]);
+		cudaFree(d_a_[l]);
+		cudaFree(d_dz_[l]);
+		d_z_[l] = d_a_[l] = d_dz_[l] = nullptr;
+	}
+	cudaFree(d_y_);
+	cudaFree(d_delta_);
+	cudaFree(d_loss_);
+	cudaFree(d_head_);
+	cudaFree(d_part_);
+	cudaFree(d_tickets_);
+	d_x_ = d_y_ = d_delta_ = d_loss_ = d_head_ = d_part_ = nullptr;
+	d_tickets_ = nullptr;
+	cap_ = 0;
+}
+
+namespace {
+uint32_t dw_tiles(uint32_t O, uint32_t I)
+{
+	return ((O + kTm - 1) / kTm) * ((I + kTn - 1) / kTn);
+}
+uint32_t dw_split_rows(uint32_t rows)
+{
+	const uint32_t share = (rows + kSplits - 1) / kSplits;
+	return std::max(kSplitRows, (share + kTk - 1) / kTk * kTk);
+}
+uint32_t head_blocks(uint32_t rows) // rows: two a pair
+{
+	return (rows / 2 + kHeadPairs - 1) / kHeadPairs;
+}
+} // namespace
+
 void Mlp::ensure_batch(uint32_t rows)
 {
 	if (rows <= cap_)
 		return;
-	cudaFree(d_x_);
-	for (uint32_t l = 0; l < kLayers; ++l) {
-		cudaFree(d_z_[l]);
-		cudaFree(d_a_[l]);
-		cudaFree(d_da_[l]);
-	}
-	cudaFree(d_dy_);
-	cudaFree(d_delta_);
-	cudaFree(d_loss_);
-	cap_ = rows;
+	check_cuda(cudaStreamSynchronize(stream_), "sync");
+	free_batch();
 	check_cuda(cudaMalloc(&d_x_, sizeof(float) * rows * in_), "inputs");
-	for (uint32_t l = 0; l < kLayers; ++l) {
+	for (uint32_t l = 0; l + 1 < kLayers; ++l) {
 		const size_t sz = sizeof(float) * rows * dims_[l + 1];
 		check_cuda(cudaMalloc(&d_z_[l], sz), "z");
 		check_cuda(cudaMalloc(&d_a_[l], sz), "a");
-		check_cuda(cudaMalloc(&d_da_[l], sz), "da");
+		check_cuda(cudaMalloc(&d_dz_[l], sz), "dz");
 	}
-	d_y_ = d_z_[kLayers - 1];
-	check_cuda(cudaMalloc(&d_dy_, sizeof(float) * rows), "dy");
+	check_cuda(cudaMalloc(&d_y_, sizeof(float) * rows), "y");
 	check_cuda(cudaMalloc(&d_delta_, sizeof(float) * rows), "delta");
 	check_cuda(cudaMalloc(&d_loss_, sizeof(float)), "loss");
+	// the head kernel's block shares, then its block losses
+	check_cuda(cudaMalloc(&d_head_, sizeof(float) * (head_blocks(rows) + 1) * (hidden_ + 2)),
+		   "output gradient shares");
+	check_cuda(cudaMalloc(&d_part_, sizeof(float) * dw_tiles(hidden_, hidden_) * kSplits *
+						(kTm * kTn + kTm)),
+		   "gradient shares");
+	const size_t tickets = sizeof(unsigned) * (dw_tiles(hidden_, hidden_) + 1);
+	check_cuda(cudaMalloc(&d_tickets_, tickets), "tickets");
+	check_cuda(cudaMemsetAsync(d_tickets_, 0, tickets, stream_), "zero tickets");
+	cap_ = rows;
 }
 
+// d_x_ rows through the hidden layers (z and a of each).
 void Mlp::forward_device(uint32_t rows)
 {
 	const float *in = d_x_;
-	for (uint32_t l = 0; l < kLayers; ++l) {
+	for (uint32_t l = 0; l + 1 < kLayers; ++l) {
 		const uint32_t I = dims_[l], O = dims_[l + 1];
-		const bool act = l + 1 < kLayers;
-		gemm_kernel<false, true><<<gemm_grid(rows, O), dim3(16, 16), 0, stream_>>>(
-			in, d_params_ + w_off_[l], d_params_ + b_off_[l], d_z_[l],
-			act ? d_a_[l] : nullptr, rows, O, I, I, I);
-		in = act ? d_a_[l] : d_z_[l];
+		mlp_forward_kernel<<<dim3((O + kTn - 1) / kTn, (rows + kTm - 1) / kTm), 128, 0,
+				     stream_>>>(in, d_params_ + w_off_[l], d_params_ + b_off_[l],
+						d_z_[l], d_a_[l], rows, O, I);
+		in = d_a_[l];
 	}
 	check_cuda(cudaGetLastError(), "surrogate forward");
 }
 
-void Mlp::backward_device(uint32_t rows)
+// Pair objective of `n` pairs (2 n rows in d_a_, d_delta_) and its gradient:
+// d_loss_, d_grad_.
+void Mlp::backward_device(uint32_t n)
 {
-	// d_dy_ holds dL/dy for every row
-	const float *dz = d_dy_;
-	for (int l = kLayers - 1; l >= 0; --l) {
-		const uint32_t I = dims_[l], O = dims_[l + 1];
-		const float *a_prev = l == 0 ? d_x_ : d_a_[l - 1];
-		// dW = dZ^T a_prev, db = column sums of dZ
-		gemm_kernel<true, false><<<gemm_grid(O, I), dim3(16, 16), 0, stream_>>>(
-			dz, a_prev, nullptr, d_grad_ + w_off_[l], nullptr, O, I, rows, O, I);
-		column_sum_kernel<<<(O + 127) / 128, 128, 0, stream_>>>(
-			dz, d_grad_ + b_off_[l], rows, O);
-		if (l == 0)
-			break;
-		// dA_prev = dZ W, then through GELU into dZ_prev
-		float *da_prev = d_da_[l - 1];
-		gemm_kernel<false, false><<<gemm_grid(rows, I), dim3(16, 16), 0, stream_>>>(
-			dz, d_params_ + w_off_[l], nullptr, da_prev, nullptr, rows, I, O, O, I);
-		const uint32_t count = rows * I;
-		gelu_backward_kernel<<<(count + 255) / 256, 256, 0, stream_>>>(
-			da_prev, d_z_[l - 1], da_prev, count);
-		dz = da_prev;
+	const uint32_t rows = 2 * n, H = hidden_, top = kLayers - 2;
+	const uint32_t hb = head_blocks(rows);
+	float *losses = d_head_ + (size_t)hb * (H + 1);
+	mlp_head_kernel<<<hb, 32 * kHeadPairs, sizeof(float) * kHeadPairs * (H + 2), stream_>>>(
+		d_a_[top], d_z_[top], d_params_ + w_off_[kLayers - 1], d_delta_, d_dz_[top], d_head_,
+		losses, d_loss_, d_tickets_ + dw_tiles(H, H), n, H);
+	for (int l = (int)top; l >= 0; --l) {
+		MlpBackward p{};
+		p.rows = rows;
+		p.O = dims_[l + 1];
+		p.I = dims_[l];
+		p.dz = d_dz_[l];
+		p.a = l == 0 ? d_x_ : d_a_[l - 1];
+		p.W = d_params_ + w_off_[l];
+		p.dW = d_grad_ + w_off_[l];
+		p.db = d_grad_ + b_off_[l];
+		p.part = d_part_;
+		p.tickets = d_tickets_;
+		p.split_rows = dw_split_rows(rows);
+		p.splits = (rows + p.split_rows - 1) / p.split_rows;
+		p.dw_blocks = dw_tiles(p.O, p.I) * p.splits;
+		if (l > 0) {
+			p.z_below = d_z_[l - 1];
+			p.dz_below = d_dz_[l - 1];
+			p.da_blocks = ((rows + kTm - 1) / kTm) * ((p.I + kTn - 1) / kTn);
+		}
+		uint32_t blocks = p.dw_blocks + p.da_blocks;
+		if (l == (int)top) {
+			p.head_part = d_head_;
+			p.head_grad = d_grad_ + w_off_[kLayers - 1]; // weights, then the bias
+			p.head_blocks = hb;
+			blocks += (H + 1 + 127) / 128;
+		}
+		mlp_backward_kernel<<<blocks, 128, 0, stream_>>>(p);
 	}
 	check_cuda(cudaGetLastError(), "surrogate backward");
 }
@@ -475,6 +816,9 @@ void Mlp::forward(const float *x, uint32_t n, float *out)
 				   cudaMemcpyHostToDevice, stream_),
 		   "inputs");
 	forward_device(n);
+	mlp_out_kernel<<<(n + 7) / 8, 256, 0, stream_>>>(
+		d_a_[kLayers - 2], d_params_ + w_off_[kLayers - 1], d_y_, n, hidden_);
+	check_cuda(cudaGetLastError(), "surrogate output");
 	check_cuda(cudaMemcpyAsync(out, d_y_, sizeof(float) * n,
 				   cudaMemcpyDeviceToHost, stream_),
 		   "outputs");
@@ -497,8 +841,7 @@ float Mlp::loss_grad(const float *x_new, const float *x_old,
 				   cudaMemcpyHostToDevice, stream_),
 		   "deltas");
 	forward_device(2 * n);
-	pair_loss_kernel<<<1, 256, 0, stream_>>>(d_y_, d_delta_, d_dy_, d_loss_, n);
-	backward_device(2 * n);
+	backward_device(n);
 	float loss = 0.0f;
 	check_cuda(cudaMemcpyAsync(&loss, d_loss_, sizeof(float),
 				   cudaMemcpyDeviceToHost, stream_),
@@ -556,9 +899,7 @@ float Mlp::train(const float *x_new, const float *x_old, const float *delta,
 			gather_rows_kernel<<<(batch + 255) / 256, 256, 0, stream_>>>(
 				d_dl, d_idx, d_delta_, batch, 1);
 			forward_device(2 * batch);
-			pair_loss_kernel<<<1, 256, 0, stream_>>>(d_y_, d_delta_, d_dy_,
-								 d_loss_, batch);
-			backward_device(2 * batch);
+			backward_device(batch);
 			++adam_t_;
 			const float c1 = 1.0f - std::pow(b1, (float)adam_t_);
 			const float c2 = 1.0f - std::pow(b2, (float)adam_t_);

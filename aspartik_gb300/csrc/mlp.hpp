@@ -57,8 +57,9 @@ class Mlp {
 
       private:
 	void ensure_batch(uint32_t rows);
-	void forward_device(uint32_t rows);   // d_x_ rows -> d_y_
-	void backward_device(uint32_t rows);  // d_dy_ -> d_grad_
+	void free_batch();
+	void forward_device(uint32_t rows); // d_x_ rows -> d_z_, d_a_
+	void backward_device(uint32_t n);   // n pairs -> d_loss_, d_grad_
 	uint32_t in_, hidden_;
 	uint32_t dims_[kLayers + 1];
 	uint32_t w_off_[kLayers], b_off_[kLayers];
@@ -71,11 +72,14 @@ class Mlp {
 	// activations for up to cap_ rows: z (pre) and a (post) per layer
 	uint32_t cap_ = 0;
 	float *d_x_ = nullptr;
-	float *d_z_[kLayers] = {};
-	float *d_a_[kLayers] = {};
-	float *d_da_[kLayers] = {};
-	float *d_y_ = nullptr, *d_dy_ = nullptr, *d_delta_ = nullptr,
-	      *d_loss_ = nullptr;
+	float *d_z_[kLayers - 1] = {};
+	float *d_a_[kLayers - 1] = {};
+	float *d_dz_[kLayers - 1] = {};
+	float *d_y_ = nullptr, *d_delta_ = nullptr, *d_loss_ = nullptr;
+	// workspaces of the backward pass: block shares of the output layer's
+	// gradient and of split weight gradients, and their counters
+	float *d_head_ = nullptr, *d_part_ = nullptr;
+	unsigned *d_tickets_ = nullptr;
 	float *d_pair_ = nullptr, *h_pair_ = nullptr; // inference staging
 	struct InferCtx {
 		cudaStream_t stream;
