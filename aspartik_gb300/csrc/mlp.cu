@@ -45,23 +45,26 @@ __device__ __forceinline__ float gelu_grad(float x)
 // ---------------------------------------------------------------------------
 // FP32 matrix products of the training step.
 //
-// A block of 128 threads computes a 32 x 64 tile of C[m][n] = sum_k A'(m, k)
-// B'(k, n), a thread 4 x 4 of it, k in order; operand tiles of 32 k pass
-// through two shared-memory buffers filled by cp.async while the other is
-// used.  A'(m, k) = TA ? A[k][m] : A[m][k] with row stride lda, B'(k, n) = TB ?
+// A block of 256 threads computes a 32 x 64 tile of C[m][n] = sum_k A'(m, k)
+// B'(k, n): two halves of 128 threads, a thread 4 x 4 products over its
+// half's 16 of every 32 k, the halves added at the end (each keeps two of
+// the four rows); operand tiles of 32 k pass through three shared-memory buffers
+// filled by cp.async two ahead of their use.  A'(m, k) = TA ? A[k][m] : A[m][k] with row stride lda, B'(k, n) = TB ?
 // B[n][k] : B[k][n] with row stride ldb.  The tile is this small because the
-// step is: 1,024 rows x 256 units are 128 tiles for 152 SMs (16 x 16 tiles
-// with one product a thread and shared-memory word pair took 17 to 36 us a
-// product; these take 5 to 8).
-constexpr uint32_t kTm = 32, kTn = 64, kTk = 32;
+// step is: 1,024 rows x 256 units are 128 tiles for 152 SMs, and two halves
+// because one warp a scheduler waits on its own loads (16 x 16 tiles with one
+// product a thread and shared-memory word pair took 17 to 36 us a product,
+// one half 9.7, two 6).
+constexpr uint32_t kTm = 32, kTn = 64, kTk = 32, kTt = 256; // kTt: threads
+constexpr uint32_t kTs = 3; // buffers
 // a weight gradient's rows are split over up to kSplits blocks a tile, at
 // least kSplitRows each, whose partial tiles the last one adds in a fixed order
 constexpr uint32_t kSplits = 16, kSplitRows = 128;
 
 struct MlpSmem {
 	// [m][k] or [k][m], rows padded to 36 / 68 floats (16-byte aligned)
-	float a[2][kTk * (kTm + 4)];
-	float b[2][kTn * (kTk + 4)];
+	float a[kTs][kTk * (kTm + 4)];
+	float b[kTs][kTn * (kTk + 4)];
 };
 
 __device__ __forceinline__ void mlp_cp16(float *dst, const float *src, bool live)
@@ -89,8 +92,8 @@ __device__ __forceinline__ void mlp_tile(float *dst, uint32_t pitch, const float
 {
 	if (vec) {
 #pragma unroll
-		for (uint32_t i = 0; i < rows * cols / 4 / 128; ++i) {
-			const uint32_t at = threadIdx.x + 128 * i;
+		for (uint32_t i = 0; i < rows * cols / 4 / kTt; ++i) {
+			const uint32_t at = threadIdx.x + kTt * i;
 			const uint32_t r = at / (cols / 4), c = 4 * (at % (cols / 4));
 			const bool live = r0 + r < R && c0 + c < C;
 			mlp_cp16(dst + r * pitch + c,
@@ -98,8 +101,8 @@ __device__ __forceinline__ void mlp_tile(float *dst, uint32_t pitch, const float
 		}
 	} else {
 #pragma unroll 4
-		for (uint32_t i = 0; i < rows * cols / 128; ++i) {
-			const uint32_t at = threadIdx.x + 128 * i;
+		for (uint32_t i = 0; i < rows * cols / kTt; ++i) {
+			const uint32_t at = threadIdx.x + kTt * i;
 			const uint32_t r = at / cols, c = at % cols;
 			const bool live = r0 + r < R && c0 + c < C;
 			mlp_cp4(dst + r * pitch + c,
@@ -113,17 +116,18 @@ __device__ __forceinline__ bool mlp_vec(const float *p, uint32_t ld)
 	return (ld & 3u) == 0 && ((uintptr_t)p & 15u) == 0;
 }
 
-// The tile's products over k in [k0, k1).  Thread (ty, tx): rows 4 ty + i,
-// columns TB ? tx + 16 j : 4 tx + j.  col_sum (TA): threads 0..31 also add
+// The tile's products over k in [k0, k1).  Thread (h, ty, tx) leaves with rows
+// 4 ty + 2 h + i, columns TB ? tx + 16 j : 4 tx + j in acc[i][j].  col_sum (TA): threads 0..31 also add
 // A'(m0 + thread, k) over k.
 template <bool TA, bool TB>
 __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const float *B,
 					    uint32_t m0, uint32_t n0, uint32_t M, uint32_t N,
 					    uint32_t k0, uint32_t k1, uint32_t lda, uint32_t ldb,
-					    float acc[4][4], float *col_sum = nullptr)
+					    float acc[2][4], float *col_sum = nullptr)
 {
 	constexpr uint32_t pa = TA ? kTm + 4 : kTk + 4, pb = TB ? kTk + 4 : kTn + 4;
-	const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
+	const uint32_t tx = threadIdx.x & 15u, ty = (threadIdx.x >> 4) & 7u, h = threadIdx.x >> 7;
+	float c[4][4];
 	// a row of the operand in memory must be whole vectors up to its end
 	const bool va = mlp_vec(A, lda) && ((TA ? M : k1) & 3u) == 0;
 	const bool vb = mlp_vec(B, ldb) && ((TB ? k1 : N) & 3u) == 0;
@@ -144,17 +148,19 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 	for (int i = 0; i < 4; ++i)
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
-			acc[i][j] = 0.0f;
+			c[i][j] = 0.0f;
 	float cs = 0.0f;
-	fetch(k0, 0);
-	uint32_t buf = 0;
-	for (uint32_t k = k0; k < k1; k += kTk, buf ^= 1u) {
-		fetch(k + kTk, buf ^ 1u);
-		asm volatile("cp.async.wait_group 1;" ::: "memory");
-		__syncthreads();
+	for (uint32_t q = 0; q + 1 < kTs; ++q)
+		fetch(k0 + q * kTk, q);
+	uint32_t buf = 0, next = kTs - 1;
+	for (uint32_t k = k0; k < k1; k += kTk) {
+		asm volatile("cp.async.wait_group %0;" ::"n"(kTs - 2) : "memory");
+		__syncthreads(); // this tile is there, the one before it used up
+		fetch(k + (kTs - 1) * kTk, next);
 		const float *sa = sm.a[buf], *sb = sm.b[buf];
 #pragma unroll
-		for (uint32_t kk = 0; kk < kTk; kk += 4) {
+		for (uint32_t k4 = 0; k4 < kTk / 2; k4 += 4) {
+			const uint32_t kk = h * (kTk / 2) + k4;
 			float a[4][4], b[4][4]; // [k][i], [k][j]
 #pragma unroll
 			for (int i = 0; i < 4; ++i) {
@@ -183,19 +189,39 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 				for (int i = 0; i < 4; ++i)
 #pragma unroll
 					for (int j = 0; j < 4; ++j)
-						acc[i][j] = fmaf(a[q][i], b[q][j], acc[i][j]);
+						c[i][j] = fmaf(a[q][i], b[q][j], c[i][j]);
 		}
 		if (TA && col_sum && threadIdx.x < kTm)
 			for (uint32_t kk = 0; kk < kTk; ++kk)
 				cs += sa[kk * pa + threadIdx.x];
-		__syncthreads(); // the buffer is free for the next fetch
+		buf = buf + 1 == kTs ? 0 : buf + 1;
+		next = next + 1 == kTs ? 0 : next + 1;
 	}
+	__syncthreads(); // the buffers are free
 	if (TA && col_sum)
 		*col_sum = cs;
+	// the other half's sums of this thread's rows, through shared memory
+	float4 *ex = reinterpret_cast<float4 *>(&sm);
+#pragma unroll
+	for (int i = 0; i < 2; ++i) {
+		const int o = 2 * (1 - (int)h) + i; // what the other half keeps
+		const float *v = o == 0 ? c[0] : o == 1 ? c[1] : o == 2 ? c[2] : c[3];
+		ex[(threadIdx.x ^ 128u) + kTt * i] = make_float4(v[0], v[1], v[2], v[3]);
+	}
+	__syncthreads();
+#pragma unroll
+	for (int i = 0; i < 2; ++i) {
+		const float4 v = ex[threadIdx.x + kTt * i];
+		const float *w = h ? c[2 + i] : c[i];
+		acc[i][0] = w[0] + v.x;
+		acc[i][1] = w[1] + v.y;
+		acc[i][2] = w[2] + v.z;
+		acc[i][3] = w[3] + v.w;
+	}
 }
 
 // Hidden layer: z = x W^T + b and a = gelu(z).  Grid (N / 64, M / 32).
-__global__ void __launch_bounds__(128) mlp_forward_kernel(const float *__restrict__ x,
+__global__ void __launch_bounds__(kTt) mlp_forward_kernel(const float *__restrict__ x,
 							   const float *__restrict__ W,
 							   const float *__restrict__ bias,
 							   float *__restrict__ z,
@@ -204,8 +230,9 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(const float *__restric
 {
 	__shared__ __align__(16) MlpSmem sm;
 	const uint32_t m0 = blockIdx.y * kTm, n0 = blockIdx.x * kTn;
-	const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
-	float acc[4][4];
+	const uint32_t tx = threadIdx.x & 15u;
+	const uint32_t row = 4 * ((threadIdx.x >> 4) & 7u) + 2 * (threadIdx.x >> 7);
+	float acc[2][4];
 	mlp_product<false, true>(sm, x, W, m0, n0, M, N, 0, K, K, K, acc);
 #pragma unroll
 	for (int j = 0; j < 4; ++j) {
@@ -214,8 +241,8 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(const float *__restric
 			continue;
 		const float bn = bias[n];
 #pragma unroll
-		for (int i = 0; i < 4; ++i) {
-			const uint32_t m = m0 + 4 * ty + i;
+		for (int i = 0; i < 2; ++i) {
+			const uint32_t m = m0 + row + i;
 			if (m >= M)
 				continue;
 			const float v = acc[i][j] + bn;
@@ -256,7 +283,7 @@ __global__ void __launch_bounds__(256) mlp_out_kernel(const float *__restrict__ 
 // = dL/dy w gelu'(z).  The block's share of the output weights' gradient
 // (sum of dL/dy a, and of dL/dy) goes to part[block][H + 1].  The last block
 // to finish adds the loss shares in block order.
-constexpr uint32_t kHeadPairs = 8;
+constexpr uint32_t kHeadPairs = 4;
 __global__ void __launch_bounds__(32 * kHeadPairs) mlp_head_kernel(
 	const float *__restrict__ a, const float *__restrict__ z, const float *__restrict__ w,
 	const float *__restrict__ delta, float *__restrict__ dz, float *__restrict__ part,
@@ -272,19 +299,53 @@ __global__ void __launch_bounds__(32 * kHeadPairs) mlp_head_kernel(
 	float r = 0.0f, dy = 0.0f;
 	if (i < n) {
 		const float *an = a + (size_t)i * H, *ao = a + (size_t)(n + i) * H;
+		const float *zn = z + (size_t)i * H, *zo = z + (size_t)(n + i) * H;
 		float yn = 0.0f, yo = 0.0f;
-		for (uint32_t k = lane; k < H; k += 32) {
-			yn = fmaf(an[k], w[k], yn);
-			yo = fmaf(ao[k], w[k], yo);
-		}
-		// the output bias cancels in the difference
-		r = warp_sum(yn) - warp_sum(yo) - delta[i];
-		dy = 2.0f * r / n;
-		for (uint32_t k = lane; k < H; k += 32) {
-			const size_t in = (size_t)i * H + k, io = (size_t)(n + i) * H + k;
-			dz[in] = dy * w[k] * gelu_grad(z[in]);
-			dz[io] = -dy * w[k] * gelu_grad(z[io]);
-			mine[k] = dy * an[k] - dy * ao[k];
+		if (H <= 256) {
+			// everything that does not need dy first, in registers
+			float va[8], vo[8], gn[8], go[8];
+#pragma unroll
+			for (int q = 0; q < 8; ++q) {
+				const uint32_t k = lane + 32 * q;
+				const bool live = k < H;
+				va[q] = live ? an[k] : 0.0f;
+				vo[q] = live ? ao[k] : 0.0f;
+				gn[q] = live ? zn[k] : 0.0f;
+				go[q] = live ? zo[k] : 0.0f;
+			}
+#pragma unroll
+			for (int q = 0; q < 8; ++q) {
+				const uint32_t k = lane + 32 * q;
+				const float wk = k < H ? w[k] : 0.0f;
+				yn = fmaf(va[q], wk, yn);
+				yo = fmaf(vo[q], wk, yo);
+				gn[q] = wk * gelu_grad(gn[q]);
+				go[q] = wk * gelu_grad(go[q]);
+			}
+			// the output bias cancels in the difference
+			r = warp_sum(yn) - warp_sum(yo) - delta[i];
+			dy = 2.0f * r / n;
+#pragma unroll
+			for (int q = 0; q < 8; ++q) {
+				const uint32_t k = lane + 32 * q;
+				if (k < H) {
+					dz[(size_t)i * H + k] = dy * gn[q];
+					dz[(size_t)(n + i) * H + k] = -dy * go[q];
+					mine[k] = dy * va[q] - dy * vo[q];
+				}
+			}
+		} else {
+			for (uint32_t k = lane; k < H; k += 32) {
+				yn = fmaf(an[k], w[k], yn);
+				yo = fmaf(ao[k], w[k], yo);
+			}
+			r = warp_sum(yn) - warp_sum(yo) - delta[i];
+			dy = 2.0f * r / n;
+			for (uint32_t k = lane; k < H; k += 32) {
+				dz[(size_t)i * H + k] = dy * (w[k] * gelu_grad(zn[k]));
+				dz[(size_t)(n + i) * H + k] = -dy * (w[k] * gelu_grad(zo[k]));
+				mine[k] = dy * an[k] - dy * ao[k];
+			}
 		}
 	} else {
 		for (uint32_t k = lane; k < H; k += 32)
@@ -339,15 +400,16 @@ struct MlpBackward {
 	float *head_grad;
 	uint32_t rows, O, I, splits, split_rows, dw_blocks, da_blocks, head_blocks;
 };
-__global__ void __launch_bounds__(128) mlp_backward_kernel(MlpBackward p)
+__global__ void __launch_bounds__(kTt) mlp_backward_kernel(MlpBackward p)
 {
 	__shared__ __align__(16) MlpSmem sm;
 	__shared__ unsigned s_last;
-	const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
-	float acc[4][4];
+	const uint32_t tx = threadIdx.x & 15u;
+	const uint32_t row = 4 * ((threadIdx.x >> 4) & 7u) + 2 * (threadIdx.x >> 7);
+	float acc[2][4];
 	if (blockIdx.x >= p.dw_blocks + p.da_blocks) {
 		// output layer: one column a thread
-		const uint32_t k = (blockIdx.x - p.dw_blocks - p.da_blocks) * 128 + threadIdx.x;
+		const uint32_t k = (blockIdx.x - p.dw_blocks - p.da_blocks) * kTt + threadIdx.x;
 		if (k > p.O)
 			return;
 		float v = 0.0f;
@@ -363,8 +425,8 @@ __global__ void __launch_bounds__(128) mlp_backward_kernel(MlpBackward p)
 		mlp_product<false, false>(sm, p.dz, p.W, m0, n0, p.rows, p.I, 0, p.O, p.O, p.I,
 					  acc);
 #pragma unroll
-		for (int i = 0; i < 4; ++i) {
-			const uint32_t m = m0 + 4 * ty + i;
+		for (int i = 0; i < 2; ++i) {
+			const uint32_t m = m0 + row + i;
 			if (m >= p.rows)
 				continue;
 #pragma unroll
@@ -390,8 +452,8 @@ __global__ void __launch_bounds__(128) mlp_backward_kernel(MlpBackward p)
 		float *part = p.part + (size_t)tile * p.splits * (kTm * kTn + kTm);
 		float4 *mine = reinterpret_cast<float4 *>(part + split * (kTm * kTn + kTm));
 #pragma unroll
-		for (int i = 0; i < 4; ++i)
-			mine[(4 * ty + i) * (kTn / 4) + tx] =
+		for (int i = 0; i < 2; ++i)
+			mine[(row + i) * (kTn / 4) + tx] =
 				make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
 		if (threadIdx.x < kTm)
 			reinterpret_cast<float *>(mine)[kTm * kTn + threadIdx.x] = cs;
@@ -407,16 +469,17 @@ __global__ void __launch_bounds__(128) mlp_backward_kernel(MlpBackward p)
 			p.tickets[tile] = 0u;
 		cs = 0.0f;
 #pragma unroll
-		for (int i = 0; i < 4; ++i)
+		for (int i = 0; i < 2; ++i)
 #pragma unroll
 			for (int j = 0; j < 4; ++j)
 				acc[i][j] = 0.0f;
+#pragma unroll 4
 		for (uint32_t q = 0; q < p.splits; ++q) {
 			const float *from = part + (size_t)q * (kTm * kTn + kTm);
 #pragma unroll
-			for (int i = 0; i < 4; ++i) {
+			for (int i = 0; i < 2; ++i) {
 				const float4 v = __ldcg(reinterpret_cast<const float4 *>(from) +
-							(4 * ty + i) * (kTn / 4) + tx);
+							(row + i) * (kTn / 4) + tx);
 				acc[i][0] += v.x;
 				acc[i][1] += v.y;
 				acc[i][2] += v.z;
@@ -427,8 +490,8 @@ __global__ void __launch_bounds__(128) mlp_backward_kernel(MlpBackward p)
 		}
 	}
 #pragma unroll
-	for (int i = 0; i < 4; ++i) {
-		const uint32_t m = m0 + 4 * ty + i;
+	for (int i = 0; i < 2; ++i) {
+		const uint32_t m = m0 + row + i;
 		if (m >= p.O)
 			continue;
 #pragma unroll
@@ -739,7 +802,7 @@ void Mlp::forward_device(uint32_t rows)
 	const float *in = d_x_;
 	for (uint32_t l = 0; l + 1 < kLayers; ++l) {
 		const uint32_t I = dims_[l], O = dims_[l + 1];
-		mlp_forward_kernel<<<dim3((O + kTn - 1) / kTn, (rows + kTm - 1) / kTm), 128, 0,
+		mlp_forward_kernel<<<dim3((O + kTn - 1) / kTn, (rows + kTm - 1) / kTm), kTt, 0,
 				     stream_>>>(in, d_params_ + w_off_[l], d_params_ + b_off_[l],
 						d_z_[l], d_a_[l], rows, O, I);
 		in = d_a_[l];
@@ -782,9 +845,9 @@ void Mlp::backward_device(uint32_t n)
 			p.head_part = d_head_;
 			p.head_grad = d_grad_ + w_off_[kLayers - 1]; // weights, then the bias
 			p.head_blocks = hb;
-			blocks += (H + 1 + 127) / 128;
+			blocks += (H + kTt) / kTt; // H + 1 columns
 		}
-		mlp_backward_kernel<<<blocks, 128, 0, stream_>>>(p);
+		mlp_backward_kernel<<<blocks, kTt, 0, stream_>>>(p);
 	}
 	check_cuda(cudaGetLastError(), "surrogate backward");
 }
