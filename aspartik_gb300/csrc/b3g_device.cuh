@@ -217,10 +217,9 @@ struct DirectParams {
 	// memory is read only on the shortcut paths)
 	float eig[40];
 	double rate[4];
+	// pad: where the left (bits 0-7) and right (8-15) child comes from (kSrc*)
 	NodeOp ops[kDirectMax];
 	double lengths[2 * kDirectMax]; // [n][2] time lengths
-	// where entry i's left (0) and right (1) child comes from (kSrc*)
-	uint8_t src[kDirectMax][2];
 };
 
 // Sources of a child in the fused short-list walk, set by the host: a tip

@@ -1150,9 +1150,10 @@ void Calculator::launch_direct(uint32_t n, double clock_rate)
 	// where each child comes from in the walk
 	for (uint32_t i = 0; i < n; ++i) {
 		const uint32_t ids[2] = {dp.ops[i].left, dp.ops[i].right};
+		uint32_t marks = 0;
 		for (int j = 0; j < 2; ++j) {
 			const uint32_t id = ids[j];
-			uint8_t src = kSrcClean;
+			uint32_t src = kSrcClean;
 			if (id & kTipBit) {
 				src = kSrcTip;
 			} else if (i >= 1 && id == dp.ops[i - 1].out) {
@@ -1166,8 +1167,9 @@ void Calculator::launch_direct(uint32_t n, double clock_rate)
 						break;
 					}
 			}
-			dp.src[i][j] = src;
+			marks |= src << (8 * j);
 		}
+		dp.ops[i].pad = marks;
 	}
 	// bytes that reach the device with the launch
 	last_upload_bytes_ = (uint64_t)n * (sizeof(NodeOp) + 2 * sizeof(double)) +

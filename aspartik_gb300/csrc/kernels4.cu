@@ -837,6 +837,35 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 	return cudaGetLastError();
 }
 
+// Allows a kernel the device's whole opt-in shared memory, once per kernel
+// and device (a permission, not a reservation: no call lowers another's
+// limit and later launches pay nothing).
+struct SmemOptIn {
+	std::atomic<bool> done[64] = {};
+};
+template <typename Kernel> static cudaError_t opt_in_smem(Kernel kern, SmemOptIn &state)
+{
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess)
+		return e;
+	if (dev >= 0 && dev < 64 && state.done[dev].load(std::memory_order_acquire))
+		return cudaSuccess;
+	int most = 0;
+	e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+	if (e != cudaSuccess)
+		return e;
+	cudaFuncAttributes fa{};
+	e = cudaFuncGetAttributes(&fa, kern);
+	if (e != cudaSuccess)
+		return e;
+	e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				 most - (int)fa.sharedSizeBytes);
+	if (e == cudaSuccess && dev >= 0 && dev < 64)
+		state.done[dev].store(true, std::memory_order_release);
+	return e;
+}
+
 size_t prune4_runs_smem(const PruneParams &p)
 {
 	const uint32_t cols = p.tile * p.C;
@@ -880,35 +909,11 @@ cudaError_t launch_prune4_runs(const PruneParams &p, uint32_t ctas,
 			    : (narrow ? prune4_runs_kernel<uint32_t, 512>
 				      : prune4_runs_kernel<size_t, 512>);
 	if (smem > 48 * 1024) {
-		// once per (kernel variant, device): allow the device's whole
-		// opt-in shared memory (a permission, not a reservation), so no
-		// call lowers another's limit and later launches pay nothing
-		static std::atomic<bool> opted[4][64];
-		int dev = 0;
-		cudaError_t e = cudaGetDevice(&dev);
+		static SmemOptIn opted[4];
+		const cudaError_t e =
+			opt_in_smem(kern, opted[(block == 1024 ? 2 : 0) + (narrow ? 0 : 1)]);
 		if (e != cudaSuccess)
 			return e;
-		const int v = (block == 1024 ? 2 : 0) + (narrow ? 0 : 1);
-		if (dev < 0 || dev >= 64 || !opted[v][dev].load(std::memory_order_acquire)) {
-			int most = 0;
-			e = cudaDeviceGetAttribute(
-				&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-			if (e != cudaSuccess)
-				return e;
-			cudaFuncAttributes fa{};
-			e = cudaFuncGetAttributes(&fa, kern);
-			if (e != cudaSuccess)
-				return e;
-			most -= (int)fa.sharedSizeBytes; // static + dynamic <= opt-in
-			if ((int)smem > most)
-				return cudaErrorInvalidValue;
-			e = cudaFuncSetAttribute(
-				kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-			if (e != cudaSuccess)
-				return e;
-			if (dev >= 0 && dev < 64)
-				opted[v][dev].store(true, std::memory_order_release);
-		}
 	}
 	kern<<<ctas, threads, smem, s>>>(p);
 	return cudaGetLastError();
@@ -940,29 +945,33 @@ cudaError_t launch_prune4_batch(const BatchParams &p, uint32_t ctas,
 	return cudaGetLastError();
 }
 
+template <typename Idx, uint32_t kC>
+static cudaError_t launch_direct_batch_t(const BatchParams &p, uint32_t ctas, cudaStream_t s)
+{
+	static SmemOptIn opted;
+	auto kern = prune4_direct_batch_kernel<Idx, kC>;
+	const cudaError_t e = opt_in_smem(kern, opted);
+	if (e != cudaSuccess)
+		return e;
+	kern<<<ctas, 128 * kC, DirectSmem<kC, kBatchAhead>::bytes(kDirectMax), s>>>(p);
+	return cudaGetLastError();
+}
+
 cudaError_t launch_prune4_direct_batch(const BatchParams &p, uint32_t C,
 				       uint32_t ctas, cudaStream_t s)
 {
-	const uint32_t threads = 128 * C;
-	if (C == 4) {
-		if (p.narrow)
-			prune4_direct_batch_kernel<uint32_t, 4><<<ctas, threads, 0, s>>>(p);
-		else
-			prune4_direct_batch_kernel<size_t, 4><<<ctas, threads, 0, s>>>(p);
-	} else if (C == 2) {
-		if (p.narrow)
-			prune4_direct_batch_kernel<uint32_t, 2><<<ctas, threads, 0, s>>>(p);
-		else
-			prune4_direct_batch_kernel<size_t, 2><<<ctas, threads, 0, s>>>(p);
-	} else if (C == 1) {
-		if (p.narrow)
-			prune4_direct_batch_kernel<uint32_t, 1><<<ctas, threads, 0, s>>>(p);
-		else
-			prune4_direct_batch_kernel<size_t, 1><<<ctas, threads, 0, s>>>(p);
-	} else {
-		return cudaErrorInvalidValue;
+	switch (C) {
+	case 4:
+		return p.narrow ? launch_direct_batch_t<uint32_t, 4>(p, ctas, s)
+				: launch_direct_batch_t<size_t, 4>(p, ctas, s);
+	case 2:
+		return p.narrow ? launch_direct_batch_t<uint32_t, 2>(p, ctas, s)
+				: launch_direct_batch_t<size_t, 2>(p, ctas, s);
+	case 1:
+		return p.narrow ? launch_direct_batch_t<uint32_t, 1>(p, ctas, s)
+				: launch_direct_batch_t<size_t, 1>(p, ctas, s);
 	}
-	return cudaGetLastError();
+	return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_ptab20(const PtabParams &p, bool f32, cudaStream_t s)
@@ -1078,31 +1087,36 @@ cudaError_t launch_prune20tc(const Tc20Params &p, cudaStream_t s)
 	return cudaGetLastError();
 }
 
+template <typename Idx, uint32_t kC>
+static cudaError_t launch_direct_t(const DirectParams &p, uint32_t ctas, cudaStream_t s)
+{
+	static SmemOptIn opted;
+	auto kern = prune4_direct_kernel<Idx, kC>;
+	const cudaError_t e = opt_in_smem(kern, opted);
+	if (e != cudaSuccess)
+		return e;
+	kern<<<ctas, 128 * kC, DirectSmem<kC, kDirectAhead>::bytes(p.n), s>>>(p);
+	return cudaGetLastError();
+}
+
 cudaError_t launch_prune4_direct(const DirectParams &p, uint32_t ctas,
 				 cudaStream_t s)
 {
-	if (p.n == 0 || p.n > kDirectMax || p.ldp % 128u ||
-	    (p.C != 1 && p.C != 2 && p.C != 4))
+	if (p.n == 0 || p.n > kDirectMax || p.ldp % 128u)
 		return cudaErrorInvalidValue;
 	const bool narrow = (uint64_t)p.L * 2 * p.C * p.ldp < (1ull << 31);
-	const uint32_t threads = 128 * p.C;
-	if (p.C == 4) {
-		if (narrow)
-			prune4_direct_kernel<uint32_t, 4><<<ctas, threads, 0, s>>>(p);
-		else
-			prune4_direct_kernel<size_t, 4><<<ctas, threads, 0, s>>>(p);
-	} else if (p.C == 2) {
-		if (narrow)
-			prune4_direct_kernel<uint32_t, 2><<<ctas, threads, 0, s>>>(p);
-		else
-			prune4_direct_kernel<size_t, 2><<<ctas, threads, 0, s>>>(p);
-	} else {
-		if (narrow)
-			prune4_direct_kernel<uint32_t, 1><<<ctas, threads, 0, s>>>(p);
-		else
-			prune4_direct_kernel<size_t, 1><<<ctas, threads, 0, s>>>(p);
+	switch (p.C) {
+	case 4:
+		return narrow ? launch_direct_t<uint32_t, 4>(p, ctas, s)
+			      : launch_direct_t<size_t, 4>(p, ctas, s);
+	case 2:
+		return narrow ? launch_direct_t<uint32_t, 2>(p, ctas, s)
+			      : launch_direct_t<size_t, 2>(p, ctas, s);
+	case 1:
+		return narrow ? launch_direct_t<uint32_t, 1>(p, ctas, s)
+			      : launch_direct_t<size_t, 1>(p, ctas, s);
 	}
-	return cudaGetLastError();
+	return cudaErrorInvalidValue;
 }
 
 

@@ -371,6 +371,16 @@ __device__ double tile_walk(const TileArgs &a, uint32_t t, float *s_dot,
 	return tile_root(a, t, s_dot, s_cnt, s_red);
 }
 
+// x 2^e for e <= 0 (zero below 2^-252, which no sum with a term of at least
+// 2^-126 beside it notices): two exact powers of two instead of ldexpf's
+// cases.
+__device__ __forceinline__ float scale_down(float x, int32_t e)
+{
+	const int32_t lo = max(e, -126), hi = max(e - lo, -126);
+	x *= __uint_as_float((uint32_t)(127 + lo) << 23);
+	return x * __uint_as_float((uint32_t)(127 + hi) << 23);
+}
+
 // Root of tile t after its walk left pi . x and the exponent of every
 // column in s_dot / s_cnt: category mixing per pattern (threads 0 ..
 // tile-1), site values, and the tile's weighted sum in a fixed order,
@@ -395,8 +405,8 @@ __device__ double tile_root(const TileArgs &a, uint32_t t, const float *s_dot,
 			// the exact exponent term and the constant join in FP64
 			float acc = 0.f;
 			for (uint32_t k = 0; k < C; k++)
-				acc += ldexpf(s_dot[k * tile + tid],
-					      s_cnt[k * tile + tid] - emax);
+				acc += scale_down(s_dot[k * tile + tid],
+						  s_cnt[k * tile + tid] - emax);
 			site = (double)logf(acc) +
 			       fma((double)emax, 0.69314718055994530942,
 				   a.log_inv_c);
@@ -594,138 +604,183 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 // The walk is a chain: each entry needs the previous one's output, and its
 // other child is a clean partial written long ago (mostly in DRAM) or a tip
 // code.  Every clean input and tip code is known before the walk starts
-// (the host marks each child's source in DirectParams::src), so they are
-// loaded kDirectAhead entries ahead of their use, the first ones before the
-// tables are built.  The two previous outputs stay in registers; an older
-// output is read back when needed (written by the same thread earlier).
-// Two entries ahead fit 64 registers, so two blocks share an SM and
-// several chains' launches can overlap on the same SMs.  (One, two and four
-// entries ahead measured within 2 % of each other on one chain and on
-// eight: the walk is not bound by these loads.)
-constexpr uint32_t kDirectAhead = 2;
+// (the host marks each child's source in NodeOp::pad), so they are copied to
+// shared memory kDirectAhead entries ahead of their use by cp.async, each
+// thread for its own column (no barrier), the first ones before the tables
+// are built.  The two previous outputs stay in registers; an older output is
+// read back when needed (written by the same thread earlier).
+//
+// Every word the walk reads is staged in shared memory first: a kernel
+// parameter read through the constant bank costs a cache miss of about 30 ns
+// for each 64-byte line, one after another along the chain (reading the
+// parameters through their generic address costs one load latency in all).
+// (Four entries ahead cover a DRAM round trip at the walk's 500 cycles an
+// entry; the batched kernel, whose blocks hold the largest list's tables,
+// takes two so that two blocks share an SM.)
+constexpr uint32_t kDirectAhead = 4, kBatchAhead = 2;
 
-template <typename Idx>
-__device__ __forceinline__ void direct_fetch(const NodeOp *ops, const uint8_t (*src)[2],
-					     uint32_t i, uint32_t ldp,
-					     const float4 *part, const int32_t *scales,
-					     const uint8_t *tips_p, Idx stride, Idx col_off,
-					     float4 (&v)[2], int32_t (&s)[2])
+// Rounds up to whole 16-byte words.
+__host__ __device__ constexpr uint32_t direct_align(uint32_t bytes)
 {
-	const NodeOp &op = ops[i];
+	return (bytes + 15u) & ~15u;
+}
+
+// Dynamic shared memory of the short-list kernels: tables of n entries, the
+// list, the columns' root values and counts, and the input ring.
+template <uint32_t kC, uint32_t kA> struct DirectSmem {
+	static constexpr uint32_t kCols = 128 * kC;
+	float4 *tab;
+	NodeOp *ops;
+	float4 *ring_x; // [kA][2][kCols]
+	int32_t *ring_s;
+	float *dot;
+	int32_t *cnt;
+	__device__ DirectSmem(unsigned char *base, uint32_t n)
+	{
+		tab = reinterpret_cast<float4 *>(base);
+		ring_x = tab + n * 2 * kC * 5;
+		ops = reinterpret_cast<NodeOp *>(ring_x + kA * 2 * kCols);
+		ring_s = reinterpret_cast<int32_t *>(ops + n);
+		dot = reinterpret_cast<float *>(ring_s + kA * 2 * kCols);
+		cnt = reinterpret_cast<int32_t *>(dot + kCols);
+	}
+	static constexpr size_t bytes(uint32_t n)
+	{
+		return (size_t)n * (2 * kC * 5 * sizeof(float4) + sizeof(NodeOp)) +
+		       kA * 2 * kCols * (sizeof(float4) + 4) + 8 * kCols;
+	}
+};
+
+__device__ __forceinline__ void cp_async4(void *dst, const void *src)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+			     (uint32_t)__cvta_generic_to_shared(dst)),
+		     "l"(src)
+		     : "memory");
+}
+
+// Per-thread constants of one tile's walk.
+template <typename Idx, uint32_t kC> struct DirectCtx {
+	const uint8_t *tips;  // tips + first pattern of this thread's 4-byte word
+	const float4 *part;
+	const int32_t *scales;
+	uint32_t ldp, tip_shift; // bit position of this pattern's code in a word
+	Idx stride, col_off;
+	__device__ DirectCtx(const uint8_t *all_tips, const float4 *p, const int32_t *s,
+			     uint32_t ldp_, uint32_t t)
+	    : part(p), scales(s), ldp(ldp_)
+	{
+		const uint32_t c = threadIdx.x >> 7, pl = threadIdx.x & 127u;
+		const uint32_t pat = t * 128u + pl;
+		tips = all_tips + (pat & ~3u);
+		tip_shift = 8u * (pat & 3u);
+		stride = (Idx)kC * ldp_;
+		col_off = (Idx)c * ldp_ + pat;
+	}
+};
+
+// Copies entry i's clean inputs (and tip words) of this thread's column into
+// the ring; one cp.async group in any case.
+template <typename Idx, uint32_t kC, uint32_t kA>
+__device__ __forceinline__ void direct_issue(const DirectCtx<Idx, kC> &w, const NodeOp &op,
+					     uint32_t i, const DirectSmem<kC, kA> &sm)
+{
 	const uint32_t ids[2] = {op.left, op.right};
 #pragma unroll
-	for (int j = 0; j < 2; ++j) {
-		const uint32_t sr = src[i][j];
+	for (uint32_t j = 0; j < 2; ++j) {
+		const uint32_t sr = (op.pad >> (8 * j)) & 0xFFu;
+		const uint32_t at =
+			((i & (kA - 1)) * 2 + j) * (128 * kC) + threadIdx.x;
 		if (sr == kSrcTip) {
-			s[j] = tips_p[(size_t)(ids[j] & ~kTipBit) * ldp];
+			cp_async4(sm.ring_s + at,
+				  w.tips + (size_t)(ids[j] & ~kTipBit) * w.ldp);
 		} else if (sr == kSrcClean) {
-			const Idx ix = (Idx)ids[j] * stride + col_off;
-			v[j] = part[ix];
-			s[j] = scales[ix];
+			const Idx ix = (Idx)ids[j] * w.stride + w.col_off;
+			cp_async16(sm.ring_x + at, w.part + ix);
+			cp_async4(sm.ring_s + at, w.scales + ix);
 		}
 	}
 }
 
-// The first kDirectAhead entries' clean inputs of tile t for this thread's
-// column (c, pl).
-template <typename Idx, uint32_t kC>
-__device__ __forceinline__ void direct_prefetch(const NodeOp *ops, const uint8_t (*src)[2],
-						uint32_t n, uint32_t ldp, const uint8_t *tips,
-						const float4 *part, const int32_t *scales,
-						uint32_t t, float4 (&pv)[kDirectAhead][2],
-						int32_t (&ps)[kDirectAhead][2])
+// The first kA entries' inputs of a tile.
+template <typename Idx, uint32_t kC, uint32_t kA>
+__device__ __forceinline__ void direct_prefetch(const DirectCtx<Idx, kC> &w, const NodeOp *ops,
+						uint32_t n, const DirectSmem<kC, kA> &sm)
 {
-	constexpr uint32_t kTile = 128;
-	const uint32_t c = threadIdx.x / kTile, pl = threadIdx.x - c * kTile;
-	const Idx stride = (Idx)kC * ldp;
-	const Idx col_off = (Idx)c * ldp + t * kTile + pl;
-	const uint8_t *tips_p = tips + t * kTile + pl;
 #pragma unroll
-	for (uint32_t u = 0; u < kDirectAhead; ++u)
-		if (u < n)
-			direct_fetch<Idx>(ops, src, u, ldp, part, scales, tips_p, stride,
-					  col_off, pv[u], ps[u]);
+	for (uint32_t i = 0; i < kA; ++i) {
+		if (i < n)
+			direct_issue<Idx, kC, kA>(w, ops[i], i, sm);
+		cp_async_commit();
+	}
 }
 
-// The serial walk of tile t (one thread per column) after direct_prefetch:
-// leaves pi . x and the exponent of the root in s_dot / s_cnt (not
+// The serial walk of a tile (one thread per column) after direct_prefetch:
+// leaves pi . x and the exponent of the root in sm.dot / sm.cnt (not
 // synchronised).
-template <typename Idx, uint32_t kC>
-__device__ __forceinline__ void direct_walk(const NodeOp *ops, const uint8_t (*src)[2],
-					    uint32_t n, uint32_t ldp, const uint8_t *tips,
-					    float4 *part, int32_t *scales, const float4 *s_tab,
-					    const float *s_pi, uint32_t t, float *s_dot,
-					    int32_t *s_cnt, float4 (&pv)[kDirectAhead][2],
-					    int32_t (&ps)[kDirectAhead][2])
+template <typename Idx, uint32_t kC, uint32_t kA>
+__device__ __forceinline__ void direct_walk(const DirectCtx<Idx, kC> &w, uint32_t n,
+					    float4 *part, int32_t *scales,
+					    const DirectSmem<kC, kA> &sm, const float *s_pi)
 {
-	constexpr uint32_t kTile = 128;
-	const uint32_t tid = threadIdx.x;
-	const uint32_t c = tid / kTile, pl = tid - c * kTile;
-	const Idx stride = (Idx)kC * ldp;
-	const Idx col_off = (Idx)c * ldp + t * kTile + pl;
-	const uint8_t *tips_p = tips + t * kTile + pl;
+	const uint32_t tid = threadIdx.x, c = tid >> 7;
 	float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
 	int32_t c0 = 0, c1 = 0;
-	for (uint32_t i0 = 0; i0 < n; i0 += kDirectAhead) {
+	for (uint32_t i = 0; i < n; ++i) {
+		const NodeOp op = sm.ops[i];
+		const float4 *tl = sm.tab + ((size_t)(2 * i) * kC + c) * 5;
+		float4 in[2];
+		int32_t sc[2];
+		const uint32_t ids[2] = {op.left, op.right};
+		cp_async_wait<kA - 1>(); // this entry's inputs
 #pragma unroll
-		for (uint32_t u = 0; u < kDirectAhead; ++u) {
-			const uint32_t i = i0 + u;
-			if (i < n) {
-				const NodeOp op = ops[i];
-				const float4 *tl = s_tab + ((size_t)(2 * i) * kC + c) * 5;
-				const float4 *tr = tl + 5 * kC;
-				float4 in[2];
-				int32_t sc[2];
-				const uint32_t ids[2] = {op.left, op.right};
-#pragma unroll
-				for (int j = 0; j < 2; ++j) {
-					const float4 *tb = j ? tr : tl;
-					const uint32_t sr = src[i][j];
-					if (sr == kSrcTip) {
-						in[j] = tb[ps[u][j]];
-						sc[j] = 0;
-					} else {
-						// the internal child's vector, then one product
-						// (one copy of the code for every source)
-						float4 x;
-						int32_t s;
-						if (sr == kSrcClean) {
-							x = pv[u][j];
-							s = ps[u][j];
-						} else if (sr == kSrcPrev) {
-							x = y0;
-							s = c0;
-						} else if (sr == kSrcPrev2) {
-							x = y1;
-							s = c1;
-						} else {
-							const Idx ix = (Idx)ids[j] * stride + col_off;
-							x = part[ix];
-							s = scales[ix];
-						}
-						in[j] = v4_apply(tb, x);
-						sc[j] = s;
-					}
+		for (uint32_t j = 0; j < 2; ++j) {
+			const float4 *tb = tl + 5 * kC * j;
+			const uint32_t sr = (op.pad >> (8 * j)) & 0xFFu;
+			const uint32_t at =
+				((i & (kA - 1)) * 2 + j) * (128 * kC) + tid;
+			if (sr == kSrcTip) {
+				in[j] = tb[((uint32_t)sm.ring_s[at] >> w.tip_shift) & 0xFFu];
+				sc[j] = 0;
+			} else {
+				// the internal child's vector, then one product (one
+				// copy of the code for every source)
+				float4 x;
+				int32_t s;
+				if (sr == kSrcClean) {
+					x = sm.ring_x[at];
+					s = sm.ring_s[at];
+				} else if (sr == kSrcPrev) {
+					x = y0;
+					s = c0;
+				} else if (sr == kSrcPrev2) {
+					x = y1;
+					s = c1;
+				} else {
+					const Idx ix = (Idx)ids[j] * w.stride + w.col_off;
+					x = part[ix];
+					s = scales[ix];
 				}
-				// the slot just consumed takes entry i + ahead
-				if (i + kDirectAhead < n)
-					direct_fetch<Idx>(ops, src, i + kDirectAhead, ldp, part,
-							  scales, tips_p, stride, col_off, pv[u],
-							  ps[u]);
-				float4 y = v4_mul(in[0], in[1]);
-				const int32_t cnt = sc[0] + sc[1] + rescale_pow2(y);
-				const Idx ox = (Idx)op.out * stride + col_off;
-				part[ox] = y;
-				scales[ox] = cnt;
-				y1 = y0;
-				c1 = c0;
-				y0 = y;
-				c0 = cnt;
+				in[j] = v4_apply(tb, x);
+				sc[j] = s;
 			}
 		}
+		// the ring slot just consumed takes entry i + kA
+		if (i + kA < n)
+			direct_issue<Idx, kC, kA>(w, sm.ops[i + kA], i, sm);
+		cp_async_commit();
+		float4 y = v4_mul(in[0], in[1]);
+		const int32_t cnt = sc[0] + sc[1] + rescale_pow2(y);
+		const Idx ox = (Idx)op.out * w.stride + w.col_off;
+		part[ox] = y;
+		scales[ox] = cnt;
+		y1 = y0;
+		c1 = c0;
+		y0 = y;
+		c0 = cnt;
 	}
-	s_dot[tid] = root_dot4(s_pi, y0);
-	s_cnt[tid] = c0;
+	sm.dot[tid] = root_dot4(s_pi, y0);
+	sm.cnt[tid] = c0;
 }
 
 // The list's transition tables (entry, side, category) in shared memory,
@@ -734,20 +789,19 @@ __device__ __forceinline__ void direct_walk(const NodeOp *ops, const uint8_t (*s
 // kernels).
 template <uint32_t kC>
 __device__ __forceinline__ void direct_tables(const ModelDev *m, const float *s_eig,
-					      const double *s_rate, const double *lengths,
-					      uint32_t n, float4 *s_tab)
+					      const double *s_rate, double length, uint32_t n,
+					      float4 *s_tab)
 {
+	// one table a thread; `length`: of entry and side tid / kC
 	const uint32_t tid = threadIdx.x;
 	if (tid < n * 2 * kC) {
-		const uint32_t cc = tid % kC, es = tid / kC;
 		float P[16];
-		transition4f_eig(m, s_eig, lengths[es] * s_rate[cc], P);
-		float *out = reinterpret_cast<float *>(s_tab + tid * 5);
+		transition4f_eig(m, s_eig, length * s_rate[tid % kC], P);
+		float4 *out = s_tab + tid * 5;
+#pragma unroll
 		for (int k = 0; k < 4; k++)
-			for (int j = 0; j < 4; j++)
-				out[k * 4 + j] = P[j * 4 + k];
-		for (int j = 0; j < 4; j++)
-			out[16 + j] = 1.0f;
+			out[k] = make_float4(P[k], P[4 + k], P[8 + k], P[12 + k]);
+		out[4] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
 	}
 }
 
@@ -755,36 +809,41 @@ template <typename Idx, uint32_t kC>
 __global__ void __launch_bounds__(128 * kC, 8 / kC)
 prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 {
-	constexpr uint32_t kTile = 128, kCols = kTile * kC;
-	__shared__ float4 s_tab[kDirectMax * 2 * kC * 5];
+	constexpr uint32_t kTile = 128;
+	extern __shared__ __align__(16) unsigned char direct_smem[];
 	__shared__ float s_eig[37];
 	__shared__ double s_rate[kC];
 	__shared__ float s_pi[4];
-	__shared__ float s_dot[kCols];
-	__shared__ int32_t s_cnt[kCols];
 	__shared__ double s_red[32];
 	__shared__ unsigned s_last;
 	const uint32_t tid = threadIdx.x;
 	const uint32_t n = prm.n;
 	const uint32_t ntiles = prm.ldp / kTile;
+	const DirectSmem<kC, kDirectAhead> sm(direct_smem, n);
 	float4 *part = (float4 *)prm.partials;
-
+	// the parameters through their generic address (the constant bank would
+	// serve a warp's different words one after another)
+	const DirectParams *gp = &prm;
+	asm volatile("" : "+l"(gp));
+	double length = 0.0;
+	if (tid < n * 2 * kC)
+		length = gp->lengths[tid / kC];
+	if (tid < n)
+		sm.ops[tid] = gp->ops[tid];
+	else if (tid >= 64 && tid < 64 + 37)
+		s_eig[tid - 64] = gp->eig[tid - 64];
+	else if (tid >= 104 && tid < 104 + kC)
+		s_rate[tid - 104] = gp->rate[tid - 104];
+	else if (tid >= 112 && tid < 116)
+		s_pi[tid - 112] = (float)gp->pi[tid - 112];
+	__syncthreads();
 	// clean inputs of the first entries of the first tile, in flight while
 	// the tables are built
-	float4 pv[kDirectAhead][2];
-	int32_t ps[kDirectAhead][2];
 	if (blockIdx.x < ntiles)
-		direct_prefetch<Idx, kC>(prm.ops, prm.src, n, prm.ldp, prm.tips, part,
-					 prm.scales, blockIdx.x, pv, ps);
-	// from the parameters: no global-memory round trip before the tables
-	if (tid < 37)
-		s_eig[tid] = prm.eig[tid];
-	else if (tid < 37 + kC)
-		s_rate[tid - 37] = prm.rate[tid - 37];
-	else if (tid >= 64 && tid < 68)
-		s_pi[tid - 64] = (float)prm.pi[tid - 64];
-	__syncthreads();
-	direct_tables<kC>(prm.model, s_eig, s_rate, prm.lengths, n, s_tab);
+		direct_prefetch<Idx, kC, kDirectAhead>(DirectCtx<Idx, kC>(prm.tips, part, prm.scales, prm.ldp,
+							    blockIdx.x),
+					 sm.ops, n, sm);
+	direct_tables<kC>(prm.model, s_eig, s_rate, length, n, sm.tab);
 	__syncthreads();
 
 	TileArgs a{};
@@ -797,13 +856,16 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 	a.log_inv_c = prm.log_inv_c;
 	double cta_sum = 0.0, cta_comp = 0.0; // thread 0: this block's tiles
 	for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+		const DirectCtx<Idx, kC> w(prm.tips, part, prm.scales, prm.ldp, t);
 		if (t != blockIdx.x)
-			direct_prefetch<Idx, kC>(prm.ops, prm.src, n, prm.ldp, prm.tips,
-						 part, prm.scales, t, pv, ps);
-		direct_walk<Idx, kC>(prm.ops, prm.src, n, prm.ldp, prm.tips, part,
-				     prm.scales, s_tab, s_pi, t, s_dot, s_cnt, pv, ps);
+			direct_prefetch<Idx, kC, kDirectAhead>(w, sm.ops, n, sm);
+		direct_walk<Idx, kC, kDirectAhead>(w, n, part, prm.scales, sm, s_pi);
 		__syncthreads();
-		const double tsum = tile_root(a, t, s_dot, s_cnt, s_red);
+		const double tsum = tile_root(a, t, sm.dot, sm.cnt, s_red);
+		if (gridDim.x >= ntiles) { // this block's only tile
+			cta_sum = tsum;
+			break;
+		}
 		if (tid == 0)
 			neumaier_add(cta_sum, cta_comp, tsum);
 	}
@@ -836,7 +898,7 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 // items of the members whose step is direct and has kC categories from
 // their own counter (work_next[1], [2], [3] for 4, 2, 1 categories;
 // costliest member first); a block that moves to another
-// member copies its list, classifies every child's source, converts the
+// member copies its list, marks every child's source, converts the
 // member's eigensystem to FP32 and builds the list's tables (as the
 // single-calculator kernel does, so values match it), then walks the tile
 // serially with clean inputs loaded four entries ahead.  Each tile's
@@ -846,16 +908,14 @@ template <typename Idx, uint32_t kC>
 __global__ void __launch_bounds__(128 * kC, 8 / kC)
 prune4_direct_batch_kernel(BatchParams bp)
 {
-	constexpr uint32_t kTile = 128, kCols = kTile * kC;
+	constexpr uint32_t kTile = 128;
 	constexpr uint32_t kMaxMembers = 256;
-	__shared__ float4 s_tab[kDirectMax * 2 * kC * 5];
-	__shared__ NodeOp s_ops[kDirectMax];
-	__shared__ uint8_t s_src[kDirectMax][2];
+	extern __shared__ __align__(16) unsigned char direct_smem[];
+	const DirectSmem<kC, kBatchAhead> sm(direct_smem, kDirectMax);
+	NodeOp *const s_ops = sm.ops;
 	__shared__ float s_eig[37];
 	__shared__ double s_rate[kC];
 	__shared__ float s_pi[4];
-	__shared__ float s_dot[kCols];
-	__shared__ int32_t s_cnt[kCols];
 	__shared__ double s_red[32];
 	__shared__ uint32_t s_prefix[kMaxMembers + 1];
 	__shared__ uint32_t s_work;
@@ -880,8 +940,6 @@ prune4_direct_batch_kernel(BatchParams bp)
 	a.C = kC;
 	a.tile = kTile;
 	a.cat_lnl = nullptr;
-	float4 pv[kDirectAhead][2];
-	int32_t ps[kDirectAhead][2];
 	// items come in chunks of consecutive tiles (mostly of one member), so
 	// that a block rebuilds a member's tables less often
 	constexpr uint32_t kChunk = 4;
@@ -929,12 +987,13 @@ prune4_direct_batch_kernel(BatchParams bp)
 			__syncthreads();
 			// where each child comes from (as the host classifies it for
 			// the single-calculator kernel)
+			uint32_t marks = 0;
 			if (tid < n) {
 				const NodeOp op = s_ops[tid];
 				const uint32_t ids[2] = {op.left, op.right};
 				for (int j = 0; j < 2; ++j) {
 					const uint32_t id = ids[j];
-					uint8_t sr = kSrcClean;
+					uint32_t sr = kSrcClean;
 					if (id & kTipBit) {
 						sr = kSrcTip;
 					} else if (tid >= 1 && id == s_ops[tid - 1].out) {
@@ -948,32 +1007,40 @@ prune4_direct_batch_kernel(BatchParams bp)
 								break;
 							}
 					}
-					s_src[tid][j] = sr;
+					marks |= sr << (8 * j);
 				}
 			}
+			__syncthreads();
+			if (tid < n)
+				s_ops[tid].pad = marks;
 			__syncthreads();
 			a.pi = (const double *)(md->stage + md->off_pi);
 			a.weights = md->weights;
 			a.site_lnl = md->site_lnl;
 			a.ldp = md->ldp;
 			a.log_inv_c = md->log_inv_c;
-			direct_prefetch<Idx, kC>(s_ops, s_src, n, md->ldp, md->tips,
-						 (const float4 *)md->partials, md->scales, t, pv,
-						 ps);
+			direct_prefetch<Idx, kC, kBatchAhead>(
+				DirectCtx<Idx, kC>(md->tips, (const float4 *)md->partials,
+						   md->scales, md->ldp, t),
+				s_ops, n, sm);
 			direct_tables<kC>(mod, s_eig, s_rate,
-					  (const double *)(md->stage + md->off_in), n, s_tab);
+					  tid < n * 2 * kC
+						  ? ((const double *)(md->stage + md->off_in))[tid / kC]
+						  : 0.0,
+					  n, sm.tab);
 			cur = m;
 			__syncthreads();
 		} else {
-			direct_prefetch<Idx, kC>(s_ops, s_src, n, md->ldp, md->tips,
-						 (const float4 *)md->partials, md->scales, t, pv,
-						 ps);
+			direct_prefetch<Idx, kC, kBatchAhead>(
+				DirectCtx<Idx, kC>(md->tips, (const float4 *)md->partials,
+						   md->scales, md->ldp, t),
+				s_ops, n, sm);
 		}
-		direct_walk<Idx, kC>(s_ops, s_src, n, md->ldp, md->tips,
-				     (float4 *)md->partials, md->scales, s_tab, s_pi, t,
-				     s_dot, s_cnt, pv, ps);
+		direct_walk<Idx, kC, kBatchAhead>(DirectCtx<Idx, kC>(md->tips, (const float4 *)md->partials,
+							md->scales, md->ldp, t),
+				     n, (float4 *)md->partials, md->scales, sm, s_pi);
 		__syncthreads();
-		const double tsum = tile_root(a, t, s_dot, s_cnt, s_red);
+		const double tsum = tile_root(a, t, sm.dot, sm.cnt, s_red);
 		const uint32_t tiles = md->ldp / kTile;
 		if (tid == 0) {
 			md->tile_sums[t] = tsum;
