@@ -953,7 +953,7 @@ static cudaError_t launch_direct_batch_t(const BatchParams &p, uint32_t ctas, cu
 	const cudaError_t e = opt_in_smem(kern, opted);
 	if (e != cudaSuccess)
 		return e;
-	kern<<<ctas, 128 * kC, DirectSmem<kC, kBatchAhead>::bytes(kDirectMax), s>>>(p);
+	kern<<<ctas, kDirectThreads<kC>, DirectSmem<kC, kBatchAhead>::bytes(kDirectMax), s>>>(p);
 	return cudaGetLastError();
 }
 
@@ -1095,7 +1095,7 @@ static cudaError_t launch_direct_t(const DirectParams &p, uint32_t ctas, cudaStr
 	const cudaError_t e = opt_in_smem(kern, opted);
 	if (e != cudaSuccess)
 		return e;
-	kern<<<ctas, 128 * kC, DirectSmem<kC, kDirectAhead>::bytes(p.n), s>>>(p);
+	kern<<<ctas, kDirectThreads<kC>, DirectSmem<kC, kDirectAhead>::bytes(p.n), s>>>(p);
 	return cudaGetLastError();
 }
 

@@ -619,12 +619,6 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 // takes two so that two blocks share an SM.)
 constexpr uint32_t kDirectAhead = 4, kBatchAhead = 2;
 
-// Rounds up to whole 16-byte words.
-__host__ __device__ constexpr uint32_t direct_align(uint32_t bytes)
-{
-	return (bytes + 15u) & ~15u;
-}
-
 // Dynamic shared memory of the short-list kernels: tables of n entries, the
 // list, the columns' root values and counts, and the input ring.
 template <uint32_t kC, uint32_t kA> struct DirectSmem {
@@ -659,45 +653,63 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src)
 		     : "memory");
 }
 
+// Columns a thread walks: two (patterns pl and pl + 64 of one category) where
+// a tile has 512.  The walk's shared-memory reads are then shared (eight
+// 16-byte table rows an entry and thread took 830 cycles of an SM's load path
+// for 512 threads); with fewer columns the chain's latency, not the load
+// path, sets the time.
+template <uint32_t kC> constexpr uint32_t kDirectCols = kC == 4 ? 2 : 1;
+template <uint32_t kC> constexpr uint32_t kDirectThreads = 128 * kC / kDirectCols<kC>;
+
 // Per-thread constants of one tile's walk.
 template <typename Idx, uint32_t kC> struct DirectCtx {
-	const uint8_t *tips;  // tips + first pattern of this thread's 4-byte word
-	const float4 *part;
-	const int32_t *scales;
-	uint32_t ldp, tip_shift; // bit position of this pattern's code in a word
-	Idx stride, col_off;
-	__device__ DirectCtx(const uint8_t *all_tips, const float4 *p, const int32_t *s,
-			     uint32_t ldp_, uint32_t t)
-	    : part(p), scales(s), ldp(ldp_)
+	static constexpr uint32_t kR = kDirectCols<kC>, kHalf = 128 / kR;
+	const uint8_t *tips; // tips + the first pattern of this thread's 4-byte word
+	float4 *part;        // the first column's element of slot 0
+	int32_t *scales;
+	uint32_t ldp, tip_shift; // bit position of the pattern's code in its word
+	uint32_t col;            // first column inside the tile
+	__device__ DirectCtx(const uint8_t *all_tips, float4 *p, int32_t *s, uint32_t ldp_,
+			     uint32_t t)
+	    : ldp(ldp_)
 	{
-		const uint32_t c = threadIdx.x >> 7, pl = threadIdx.x & 127u;
+		const uint32_t c = threadIdx.x / kHalf, pl = threadIdx.x % kHalf;
 		const uint32_t pat = t * 128u + pl;
 		tips = all_tips + (pat & ~3u);
-		tip_shift = 8u * (pat & 3u);
-		stride = (Idx)kC * ldp_;
-		col_off = (Idx)c * ldp_ + pat;
+		tip_shift = 8u * (pat & 3u); // the same 64 patterns further
+		part = p + ((Idx)c * ldp_ + pat);
+		scales = s + ((Idx)c * ldp_ + pat);
+		col = c * 128u + pl;
 	}
+	__device__ Idx slot(uint32_t id) const { return (Idx)id * ((Idx)kC * ldp); }
 };
 
-// Copies entry i's clean inputs (and tip words) of this thread's column into
+// Copies entry i's clean inputs (and tip words) of this thread's columns into
 // the ring; one cp.async group in any case.
 template <typename Idx, uint32_t kC, uint32_t kA>
 __device__ __forceinline__ void direct_issue(const DirectCtx<Idx, kC> &w, const NodeOp &op,
 					     uint32_t i, const DirectSmem<kC, kA> &sm)
 {
+	typedef DirectCtx<Idx, kC> W;
 	const uint32_t ids[2] = {op.left, op.right};
 #pragma unroll
 	for (uint32_t j = 0; j < 2; ++j) {
 		const uint32_t sr = (op.pad >> (8 * j)) & 0xFFu;
-		const uint32_t at =
-			((i & (kA - 1)) * 2 + j) * (128 * kC) + threadIdx.x;
+		const uint32_t at = ((i & (kA - 1)) * 2 + j) * (128 * kC) + w.col;
 		if (sr == kSrcTip) {
-			cp_async4(sm.ring_s + at,
-				  w.tips + (size_t)(ids[j] & ~kTipBit) * w.ldp);
+			const uint8_t *tips = w.tips + (size_t)(ids[j] & ~kTipBit) * w.ldp;
+#pragma unroll
+			for (uint32_t r = 0; r < W::kR; ++r)
+				cp_async4(sm.ring_s + at + W::kHalf * r, tips + W::kHalf * r);
 		} else if (sr == kSrcClean) {
-			const Idx ix = (Idx)ids[j] * w.stride + w.col_off;
-			cp_async16(sm.ring_x + at, w.part + ix);
-			cp_async4(sm.ring_s + at, w.scales + ix);
+			const Idx ix = w.slot(ids[j]);
+#pragma unroll
+			for (uint32_t r = 0; r < W::kR; ++r) {
+				cp_async16(sm.ring_x + at + W::kHalf * r,
+					   w.part + ix + W::kHalf * r);
+				cp_async4(sm.ring_s + at + W::kHalf * r,
+					  w.scales + ix + W::kHalf * r);
+			}
 		}
 	}
 }
@@ -715,72 +727,148 @@ __device__ __forceinline__ void direct_prefetch(const DirectCtx<Idx, kC> &w, con
 	}
 }
 
-// The serial walk of a tile (one thread per column) after direct_prefetch:
-// leaves pi . x and the exponent of the root in sm.dot / sm.cnt (not
-// synchronised).
+// The serial walk of a tile after direct_prefetch: leaves pi . x and the
+// exponent of the root in sm.dot / sm.cnt (not synchronised).
 template <typename Idx, uint32_t kC, uint32_t kA>
 __device__ __forceinline__ void direct_walk(const DirectCtx<Idx, kC> &w, uint32_t n,
-					    float4 *part, int32_t *scales,
 					    const DirectSmem<kC, kA> &sm, const float *s_pi)
 {
-	const uint32_t tid = threadIdx.x, c = tid >> 7;
-	float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
-	int32_t c0 = 0, c1 = 0;
+	typedef DirectCtx<Idx, kC> W;
+	constexpr uint32_t kR = W::kR, kHalf = W::kHalf;
+	const uint32_t c = w.col >> 7;
+	float4 y0[kR], y1[kR];
+	int32_t c0[kR], c1[kR];
+#pragma unroll
+	for (uint32_t r = 0; r < kR; ++r) {
+		y0[r] = y1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+		c0[r] = c1[r] = 0;
+	}
 	for (uint32_t i = 0; i < n; ++i) {
 		const NodeOp op = sm.ops[i];
 		const float4 *tl = sm.tab + ((size_t)(2 * i) * kC + c) * 5;
-		float4 in[2];
-		int32_t sc[2];
+		float4 in[2][kR];
+		int32_t cnt[kR];
+#pragma unroll
+		for (uint32_t r = 0; r < kR; ++r)
+			cnt[r] = 0;
 		const uint32_t ids[2] = {op.left, op.right};
 		cp_async_wait<kA - 1>(); // this entry's inputs
 #pragma unroll
 		for (uint32_t j = 0; j < 2; ++j) {
 			const float4 *tb = tl + 5 * kC * j;
 			const uint32_t sr = (op.pad >> (8 * j)) & 0xFFu;
-			const uint32_t at =
-				((i & (kA - 1)) * 2 + j) * (128 * kC) + tid;
+			const uint32_t at = ((i & (kA - 1)) * 2 + j) * (128 * kC) + w.col;
 			if (sr == kSrcTip) {
-				in[j] = tb[((uint32_t)sm.ring_s[at] >> w.tip_shift) & 0xFFu];
-				sc[j] = 0;
+#pragma unroll
+				for (uint32_t r = 0; r < kR; ++r)
+					in[j][r] = tb[((uint32_t)sm.ring_s[at + kHalf * r] >>
+						       w.tip_shift) &
+						      0xFFu];
 			} else {
-				// the internal child's vector, then one product (one
+				// the internal child's vectors, then one product (one
 				// copy of the code for every source)
-				float4 x;
-				int32_t s;
+				float4 x[kR];
+				int32_t sc[kR];
 				if (sr == kSrcClean) {
-					x = sm.ring_x[at];
-					s = sm.ring_s[at];
+#pragma unroll
+					for (uint32_t r = 0; r < kR; ++r) {
+						x[r] = sm.ring_x[at + kHalf * r];
+						sc[r] = sm.ring_s[at + kHalf * r];
+					}
 				} else if (sr == kSrcPrev) {
-					x = y0;
-					s = c0;
+#pragma unroll
+					for (uint32_t r = 0; r < kR; ++r) {
+						x[r] = y0[r];
+						sc[r] = c0[r];
+					}
 				} else if (sr == kSrcPrev2) {
-					x = y1;
-					s = c1;
+#pragma unroll
+					for (uint32_t r = 0; r < kR; ++r) {
+						x[r] = y1[r];
+						sc[r] = c1[r];
+					}
 				} else {
-					const Idx ix = (Idx)ids[j] * w.stride + w.col_off;
-					x = part[ix];
-					s = scales[ix];
+					const Idx ix = w.slot(ids[j]);
+#pragma unroll
+					for (uint32_t r = 0; r < kR; ++r) {
+						x[r] = w.part[ix + kHalf * r];
+						sc[r] = w.scales[ix + kHalf * r];
+					}
 				}
-				in[j] = v4_apply(tb, x);
-				sc[j] = s;
+				const float4 rows[4] = {tb[0], tb[1], tb[2], tb[3]};
+#pragma unroll
+				for (uint32_t r = 0; r < kR; ++r) {
+					in[j][r] = v4_apply(rows, x[r]);
+					cnt[r] += sc[r];
+				}
 			}
 		}
 		// the ring slot just consumed takes entry i + kA
 		if (i + kA < n)
 			direct_issue<Idx, kC, kA>(w, sm.ops[i + kA], i, sm);
 		cp_async_commit();
-		float4 y = v4_mul(in[0], in[1]);
-		const int32_t cnt = sc[0] + sc[1] + rescale_pow2(y);
-		const Idx ox = (Idx)op.out * w.stride + w.col_off;
-		part[ox] = y;
-		scales[ox] = cnt;
-		y1 = y0;
-		c1 = c0;
-		y0 = y;
-		c0 = cnt;
+		const Idx ox = w.slot(op.out);
+#pragma unroll
+		for (uint32_t r = 0; r < kR; ++r) {
+			float4 y = v4_mul(in[0][r], in[1][r]);
+			cnt[r] += rescale_pow2(y);
+			w.part[ox + kHalf * r] = y;
+			w.scales[ox + kHalf * r] = cnt[r];
+			y1[r] = y0[r];
+			c1[r] = c0[r];
+			y0[r] = y;
+			c0[r] = cnt[r];
+		}
 	}
-	sm.dot[tid] = root_dot4(s_pi, y0);
-	sm.cnt[tid] = c0;
+#pragma unroll
+	for (uint32_t r = 0; r < kR; ++r) {
+		sm.dot[w.col + kHalf * r] = root_dot4(s_pi, y0[r]);
+		sm.cnt[w.col + kHalf * r] = c0[r];
+	}
+}
+
+// Root of a tile, thread = pattern (tid < 128) with its weight: tile_root's
+// arithmetic with everything it needs at hand.  Returns the tile's sum in
+// thread 0; ends with the block synchronised.
+template <uint32_t kC>
+__device__ __forceinline__ double direct_root(const float *s_dot, const int32_t *s_cnt,
+					      double *site_lnl, uint32_t p, uint32_t weight,
+					      double log_inv_c, double *s_red)
+{
+	const uint32_t tid = threadIdx.x;
+	if (tid < 128) {
+		float dot[kC];
+		int32_t cnt[kC], emax = INT32_MIN;
+#pragma unroll
+		for (uint32_t k = 0; k < kC; k++) {
+			dot[k] = s_dot[k * 128 + tid];
+			cnt[k] = s_cnt[k * 128 + tid];
+			if (dot[k] > 0.f)
+				emax = max(emax, cnt[k]);
+		}
+		double site = -INFINITY;
+		if (emax != INT32_MIN) {
+			float acc = 0.f;
+#pragma unroll
+			for (uint32_t k = 0; k < kC; k++)
+				acc += scale_down(dot[k], cnt[k] - emax);
+			site = (double)logf(acc) +
+			       fma((double)emax, 0.69314718055994530942, log_inv_c);
+		}
+		site_lnl[p] = site;
+		double contrib = weight ? site * (double)weight : 0.0;
+		for (int off = 16; off > 0; off >>= 1)
+			contrib += __shfl_down_sync(0xffffffffu, contrib, off);
+		if ((tid & 31u) == 0)
+			s_red[tid >> 5] = contrib;
+	}
+	__syncthreads();
+	double tsum = 0.0;
+	if (tid == 0)
+		for (uint32_t q = 0; q < 4; q++)
+			tsum += s_red[q];
+	__syncthreads();
+	return tsum;
 }
 
 // The list's transition tables (entry, side, category) in shared memory,
@@ -789,24 +877,38 @@ __device__ __forceinline__ void direct_walk(const DirectCtx<Idx, kC> &w, uint32_
 // kernels).
 template <uint32_t kC>
 __device__ __forceinline__ void direct_tables(const ModelDev *m, const float *s_eig,
-					      const double *s_rate, double length, uint32_t n,
+					      const double *s_rate,
+					      const double (&length)[kDirectCols<kC>], uint32_t n,
 					      float4 *s_tab)
 {
-	// one table a thread; `length`: of entry and side tid / kC
-	const uint32_t tid = threadIdx.x;
-	if (tid < n * 2 * kC) {
+	// a table a thread and round; `length`: of the table's entry and side
+#pragma unroll
+	for (uint32_t r = 0; r < kDirectCols<kC>; ++r) {
+		const uint32_t at = threadIdx.x + r * kDirectThreads<kC>;
+		if (at >= n * 2 * kC)
+			break;
 		float P[16];
-		transition4f_eig(m, s_eig, length * s_rate[tid % kC], P);
-		float4 *out = s_tab + tid * 5;
+		transition4f_eig(m, s_eig, length[r] * s_rate[at % kC], P);
+		float4 *out = s_tab + at * 5;
 #pragma unroll
 		for (int k = 0; k < 4; k++)
 			out[k] = make_float4(P[k], P[4 + k], P[8 + k], P[12 + k]);
 		out[4] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
 	}
 }
+template <uint32_t kC>
+__device__ __forceinline__ void direct_lengths(const double *lengths, uint32_t n,
+					       double (&length)[kDirectCols<kC>])
+{
+#pragma unroll
+	for (uint32_t r = 0; r < kDirectCols<kC>; ++r) {
+		const uint32_t at = threadIdx.x + r * kDirectThreads<kC>;
+		length[r] = at < n * 2 * kC ? lengths[at / kC] : 0.0;
+	}
+}
 
 template <typename Idx, uint32_t kC>
-__global__ void __launch_bounds__(128 * kC, 8 / kC)
+__global__ void __launch_bounds__(kDirectThreads<kC>, 8 / kC)
 prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 {
 	constexpr uint32_t kTile = 128;
@@ -825,9 +927,8 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 	// serve a warp's different words one after another)
 	const DirectParams *gp = &prm;
 	asm volatile("" : "+l"(gp));
-	double length = 0.0;
-	if (tid < n * 2 * kC)
-		length = gp->lengths[tid / kC];
+	double length[kDirectCols<kC>];
+	direct_lengths<kC>(gp->lengths, n, length);
 	if (tid < n)
 		sm.ops[tid] = gp->ops[tid];
 	else if (tid >= 64 && tid < 64 + 37)
@@ -836,32 +937,36 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 		s_rate[tid - 104] = gp->rate[tid - 104];
 	else if (tid >= 112 && tid < 116)
 		s_pi[tid - 112] = (float)gp->pi[tid - 112];
+	// the first pattern tile's addresses and weights, and the constants the
+	// root needs, under the same wait
+	DirectCtx<Idx, kC> w(prm.tips, part, prm.scales, prm.ldp, blockIdx.x);
+	uint32_t weight = 0;
+	if (tid < kTile && blockIdx.x < ntiles)
+		weight = prm.weights[blockIdx.x * kTile + tid];
+	const double log_inv_c = prm.log_inv_c;
+	double *site_lnl = prm.site_lnl, *sums_host = prm.sums_host;
+	asm volatile("" ::"l"(w.tips), "l"(w.part), "l"(w.scales), "r"(w.ldp), "d"(log_inv_c),
+		     "l"(site_lnl), "l"(sums_host));
 	__syncthreads();
 	// clean inputs of the first entries of the first tile, in flight while
 	// the tables are built
 	if (blockIdx.x < ntiles)
-		direct_prefetch<Idx, kC, kDirectAhead>(DirectCtx<Idx, kC>(prm.tips, part, prm.scales, prm.ldp,
-							    blockIdx.x),
-					 sm.ops, n, sm);
+		direct_prefetch<Idx, kC, kDirectAhead>(w, sm.ops, n, sm);
 	direct_tables<kC>(prm.model, s_eig, s_rate, length, n, sm.tab);
 	__syncthreads();
 
-	TileArgs a{};
-	a.pi = prm.pi;
-	a.weights = prm.weights;
-	a.site_lnl = prm.site_lnl;
-	a.cat_lnl = nullptr;
-	a.C = kC;
-	a.tile = kTile;
-	a.log_inv_c = prm.log_inv_c;
 	double cta_sum = 0.0, cta_comp = 0.0; // thread 0: this block's tiles
 	for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-		const DirectCtx<Idx, kC> w(prm.tips, part, prm.scales, prm.ldp, t);
-		if (t != blockIdx.x)
+		if (t != blockIdx.x) {
+			w = DirectCtx<Idx, kC>(prm.tips, part, prm.scales, prm.ldp, t);
+			if (tid < kTile)
+				weight = prm.weights[t * kTile + tid];
 			direct_prefetch<Idx, kC, kDirectAhead>(w, sm.ops, n, sm);
-		direct_walk<Idx, kC, kDirectAhead>(w, n, part, prm.scales, sm, s_pi);
+		}
+		direct_walk<Idx, kC, kDirectAhead>(w, n, sm, s_pi);
 		__syncthreads();
-		const double tsum = tile_root(a, t, sm.dot, sm.cnt, s_red);
+		const double tsum = direct_root<kC>(sm.dot, sm.cnt, site_lnl, t * kTile + tid,
+						    weight, log_inv_c, s_red);
 		if (gridDim.x >= ntiles) { // this block's only tile
 			cta_sum = tsum;
 			break;
@@ -869,9 +974,9 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 		if (tid == 0)
 			neumaier_add(cta_sum, cta_comp, tsum);
 	}
-	if (prm.sums_host) { // the host folds the blocks' sums
+	if (sums_host) { // the host folds the blocks' sums
 		if (tid == 0)
-			prm.sums_host[blockIdx.x] =
+			sums_host[blockIdx.x] =
 				isfinite(cta_sum) ? cta_sum + cta_comp : cta_sum;
 		return;
 	}
@@ -905,7 +1010,7 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 // weighted sum goes to the member's tile slot; the block finishing a
 // member's last tile folds its sums (fixed order).
 template <typename Idx, uint32_t kC>
-__global__ void __launch_bounds__(128 * kC, 8 / kC)
+__global__ void __launch_bounds__(kDirectThreads<kC>, 8 / kC)
 prune4_direct_batch_kernel(BatchParams bp)
 {
 	constexpr uint32_t kTile = 128;
@@ -936,10 +1041,7 @@ prune4_direct_batch_kernel(BatchParams bp)
 	const uint32_t total = s_prefix[M];
 	uint32_t cur = 0xFFFFFFFFu, n = 0;
 	const MemberDesc *md = nullptr;
-	TileArgs a{};
-	a.C = kC;
-	a.tile = kTile;
-	a.cat_lnl = nullptr;
+	double log_inv_c = 0.0;
 	// items come in chunks of consecutive tiles (mostly of one member), so
 	// that a block rebuilds a member's tables less often
 	constexpr uint32_t kChunk = 4;
@@ -1014,33 +1116,29 @@ prune4_direct_batch_kernel(BatchParams bp)
 			if (tid < n)
 				s_ops[tid].pad = marks;
 			__syncthreads();
-			a.pi = (const double *)(md->stage + md->off_pi);
-			a.weights = md->weights;
-			a.site_lnl = md->site_lnl;
-			a.ldp = md->ldp;
-			a.log_inv_c = md->log_inv_c;
+			log_inv_c = md->log_inv_c;
+			double length[kDirectCols<kC>];
+			direct_lengths<kC>((const double *)(md->stage + md->off_in), n, length);
 			direct_prefetch<Idx, kC, kBatchAhead>(
-				DirectCtx<Idx, kC>(md->tips, (const float4 *)md->partials,
-						   md->scales, md->ldp, t),
+				DirectCtx<Idx, kC>(md->tips, (float4 *)md->partials, md->scales,
+						   md->ldp, t),
 				s_ops, n, sm);
-			direct_tables<kC>(mod, s_eig, s_rate,
-					  tid < n * 2 * kC
-						  ? ((const double *)(md->stage + md->off_in))[tid / kC]
-						  : 0.0,
-					  n, sm.tab);
+			direct_tables<kC>(mod, s_eig, s_rate, length, n, sm.tab);
 			cur = m;
 			__syncthreads();
 		} else {
 			direct_prefetch<Idx, kC, kBatchAhead>(
-				DirectCtx<Idx, kC>(md->tips, (const float4 *)md->partials,
-						   md->scales, md->ldp, t),
+				DirectCtx<Idx, kC>(md->tips, (float4 *)md->partials, md->scales,
+						   md->ldp, t),
 				s_ops, n, sm);
 		}
-		direct_walk<Idx, kC, kBatchAhead>(DirectCtx<Idx, kC>(md->tips, (const float4 *)md->partials,
-							md->scales, md->ldp, t),
-				     n, (float4 *)md->partials, md->scales, sm, s_pi);
+		const uint32_t weight = tid < kTile ? md->weights[t * kTile + tid] : 0u;
+		direct_walk<Idx, kC, kBatchAhead>(
+			DirectCtx<Idx, kC>(md->tips, (float4 *)md->partials, md->scales, md->ldp, t),
+			n, sm, s_pi);
 		__syncthreads();
-		const double tsum = tile_root(a, t, sm.dot, sm.cnt, s_red);
+		const double tsum = direct_root<kC>(sm.dot, sm.cnt, md->site_lnl, t * kTile + tid,
+						    weight, log_inv_c, s_red);
 		const uint32_t tiles = md->ldp / kTile;
 		if (tid == 0) {
 			md->tile_sums[t] = tsum;
