@@ -279,13 +279,27 @@ void Batch::release()
 	stream_ = nullptr;
 }
 
+// A list that the short-list kernels take.
+bool Batch::short_list(const Calculator &c)
+{
+	return c.staged_n_ <= kDirectMax && (c.C_ == 1 || c.C_ == 2 || c.C_ == 4);
+}
+
 void Batch::run()
 {
 	check_cuda(cudaSetDevice(device_), "cudaSetDevice");
 	// the previous replay reads h_steps_: it must be done
-	if (ran_)
-		check_cuda(cudaEventSynchronize(ev1_), "previous batch");
+	wait();
 	const uint32_t M = (uint32_t)members_.size();
+	// long lists' tiles: the members' own size, halved while every tile still
+	// gets a block at once (a tile's serial chain of runs shortens with it:
+	// its entries are spread over more thread groups)
+	uint32_t tiles = 0, shrink = 0;
+	for (Calculator *c : members_)
+		if (c->staged_ && !short_list(*c))
+			tiles += c->ldp_ / c->staged_tile_;
+	while (tiles && (tiles << (shrink + 1)) <= ctas_)
+		++shrink;
 	for (uint32_t k = 0; k < M; ++k) {
 		Calculator *c = members_[order_[k]];
 		MemberStep &s = h_steps_[k];
@@ -295,13 +309,10 @@ void Batch::run()
 			c->wait_stage();
 			s.n = c->staged_n_;
 			s.n_runs = c->n_runs_;
-			s.tile = c->staged_tile_;
+			s.tile = std::max(16u, c->staged_tile_ >> shrink);
 			s.tips_smem = c->staged_tips_smem_;
 			s.clock_rate = c->staged_clock_;
-			s.direct = (c->staged_n_ <= kDirectMax &&
-				    (c->C_ == 1 || c->C_ == 2 || c->C_ == 4))
-					   ? 1u
-					   : 0u;
+			s.direct = short_list(*c) ? 1u : 0u;
 			c->staged_ = false;
 		} else {
 			s.n = 0;
@@ -319,10 +330,13 @@ void Batch::run()
 			c->stream_dirty_ = false;
 		}
 	check_cuda(cudaGraphLaunch(exec_, stream_), "graph launch");
-	if (!ran_) // from now on members wait for the replay before restaging
-		for (Calculator *c : members_)
-			c->batch_done_ = ev1_;
+	// members wait for the replay before restaging
+	for (Calculator *c : members_) {
+		c->batch_done_ = ev1_;
+		c->batch_running_ = true;
+	}
 	ran_ = true;
+	running_ = true;
 }
 
 void Batch::log_likelihoods(double *out)
@@ -332,7 +346,7 @@ void Batch::log_likelihoods(double *out)
 	if (!ran_)
 		throw Error(B3G_ERR_STATE, "the batch has not run");
 	check_cuda(cudaSetDevice(device_), "cudaSetDevice");
-	check_cuda(cudaEventSynchronize(ev1_), "batch");
+	wait();
 	const uint32_t M = (uint32_t)members_.size();
 	for (uint32_t k = 0; k < M; ++k) {
 		const uint32_t m = order_[k];
@@ -340,11 +354,22 @@ void Batch::log_likelihoods(double *out)
 	}
 }
 
+// Waits for the last replay's end, once.
+void Batch::wait()
+{
+	if (!running_)
+		return;
+	check_cuda(cudaEventSynchronize(ev1_), "batch");
+	running_ = false;
+	for (Calculator *c : members_)
+		c->batch_running_ = false;
+}
+
 float Batch::last_ms()
 {
 	if (!ran_)
 		throw Error(B3G_ERR_STATE, "the batch has not run");
-	check_cuda(cudaEventSynchronize(ev1_), "batch");
+	wait();
 	float ms = 0.0f;
 	check_cuda(cudaEventElapsedTime(&ms, ev0_, ev1_), "elapsed");
 	return ms;

@@ -45,7 +45,9 @@ class Batch {
 	unsigned char *h_block_ = nullptr, *d_block_ = nullptr;
 	size_t block_bytes_ = 0;
 	bool direct_c_[5] = {}; // members with 1, 2 or 4 categories present
-	bool ran_ = false;
+	bool ran_ = false, running_ = false; // running_: the last replay was not waited for
+	void wait();
+	static bool short_list(const Calculator &c);
 	std::vector<uint8_t> evaluated_;
 };
 

@@ -1241,8 +1241,7 @@ void Calculator::propose_lengths(const uint32_t *internals,
 	if (!std::isfinite(clock_rate))
 		throw Error(B3G_ERR_NUMERIC, "non-finite clock rate");
 	wait_stage();
-	if (batch_done_)
-		check_cuda(cudaEventSynchronize(batch_done_), "batch stage reuse");
+	wait_batch();
 	stage_ops(internals, children, n);
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
 	stage_inputs(lengths, n, 2);
@@ -1275,8 +1274,7 @@ void Calculator::stage_lengths(const uint32_t *internals,
 	// the batch's previous copy of this staging buffer must be done, and
 	// so must this calculator's own last launch
 	wait_stage();
-	if (batch_done_)
-		check_cuda(cudaEventSynchronize(batch_done_), "batch stage reuse");
+	wait_batch();
 	stage_ops(internals, children, n);
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
 	std::memcpy(h_stage_ + off_in_, lengths, (size_t)n * 2 * sizeof(double));
@@ -1460,6 +1458,16 @@ void Calculator::wait_stage()
 	if (upload_pending_) {
 		check_cuda(cudaEventSynchronize(ev_stage_free_), "stage reuse");
 		upload_pending_ = false;
+	}
+}
+
+// A replay of the batch may still read this calculator's slice of the
+// staging block, until its results have been read (Batch::log_likelihoods).
+void Calculator::wait_batch()
+{
+	if (batch_done_ && batch_running_) {
+		check_cuda(cudaEventSynchronize(batch_done_), "batch stage reuse");
+		batch_running_ = false;
 	}
 }
 

@@ -262,6 +262,8 @@ class Calculator {
 	}
 	double staged_clock_ = 1.0;
 	cudaEvent_t batch_done_ = nullptr;
+	bool batch_running_ = false; // replayed, its end not waited for yet
+	void wait_batch();
 	// work was queued on this calculator's own stream since a batch last
 	// synchronised with it (model uploads, eigen kernel, own proposals)
 	bool stream_dirty_ = false;
