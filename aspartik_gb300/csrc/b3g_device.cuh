@@ -35,6 +35,39 @@ constexpr uint32_t kS20Swap = 1u, kS20Prev = 2u;
 // Shared-memory slot code meaning "global memory only" (run walk).
 constexpr uint32_t kNoSlot = 0xFFu;
 
+// Schedule of the four-state FP32 depth-first walk (tree4.cuh).
+constexpr uint32_t kTreeInA = 1u, kTreeInB = 2u; // the child is no tip
+constexpr uint32_t kTreePrev = 4u;   // the first child is the previous output
+constexpr uint32_t kTreeMemA = 8u, kTreeMemB = 16u; // read from global memory
+constexpr uint32_t kTreeKeep = 32u;    // the output goes to its slot
+constexpr uint32_t kTreeBarrier = 64u; // a phase ends behind the entry
+constexpr uint32_t kTreeCleanA = 1u, kTreeCleanB = 2u; // (more) copied to its slot
+// the kinds with code of their own
+constexpr uint32_t kTreeKind = kTreeInA | kTreeInB | kTreePrev | kTreeMemA | kTreeMemB;
+constexpr uint32_t kTreeTipTip = 0u, kTreePrevTip = kTreeInA | kTreePrev;
+constexpr uint32_t kTreePrevSlot = kTreeInA | kTreePrev | kTreeInB;
+// Leaves are given as tile times their number where the tip codes are in
+// shared memory, a slot or memory child as the row behind them (else kTreeNoTip).
+constexpr uint32_t kTreeNoTip = 0xFFFFFFFFu;
+struct __align__(16) TreeOp {
+	uint32_t out;
+	uint32_t code;     // flags above, the output's slot (bits 8-15), and the base
+			   // of the next entry's second child (16-31): 16-byte units
+			   // in its category's part of shared memory
+	uint32_t next_a;   // the next entry's first child's leaf
+	uint32_t after_b;  // the second child's leaf of the entry after that
+	uint32_t id[2];    // the children's partials slots
+	uint32_t more;     // clean children, the children's slots (8-15, 16-23)
+	uint32_t barriers; // phases that end behind the entry
+};
+// What entry 0 finds in the words before it in the others' case.
+struct TreeHead {
+	uint32_t tip[3];   // first child's leaf, second's, entry 1's second's
+	uint32_t base;
+	uint32_t barriers; // phases without an entry before it
+};
+constexpr uint32_t kTreeChunk = 4;   // entries copied together
+
 // One entry of the children-first schedule: output slot and the two
 // children, each either a partial slot or (kTipBit | leaf id).
 struct NodeOp {
@@ -234,6 +267,18 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 			  cudaStream_t s);
 // Run-synchronous FP32 walk: `ctas` persistent blocks over ldp / p.tile
 // pattern tiles.  Needs p.runs; block sums sized for `ctas`.
+// The depth-first FP32 walk (tree4.cuh): `tile` patterns (64 or 128) a block,
+// `groups` x C warps (at most 16); needs ptab, sums_host, and the schedule for n_slots
+// shared-memory slots, group after group.  segs: the groups' first entries, n,
+// then their heads.
+size_t prune4_tree_smem(const PruneParams &p);
+// bases (16-byte units in a category's part of shared memory) of the second
+// child's rows of a group's entry k, and of a slot's vectors
+uint32_t prune4_tree_entry(uint32_t group, uint32_t k);
+uint32_t prune4_tree_slot(uint32_t groups, uint32_t tile, uint32_t slot);
+cudaError_t launch_prune4_tree(const PruneParams &p, bool clean, cudaStream_t s);
+cudaError_t launch_ptab4_rows(const PtabParams &p, cudaStream_t s);
+
 // dynamic shared memory of prune4_runs_kernel for these parameters
 size_t prune4_runs_smem(const PruneParams &p);
 // block: 512 (two blocks per SM) or 1024 threads (one per SM)

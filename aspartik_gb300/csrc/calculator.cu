@@ -161,6 +161,32 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	if (const char *env = std::getenv("B3G_DIRECT"))
 		use_direct_ = use_direct_ && std::atoi(env) != 0;
 
+	use_tree_ = f32_ && S_ == 4 && C_ <= 16 && (uint64_t)C_ * ldp_ < (1ull << 28);
+	// the switches of the run walk's form select the run walk
+	for (const char *name : {"B3G_RUNS_TILE", "B3G_RUNS_BLOCK", "B3G_RUNS_SLOTS",
+				 "B3G_RUNS_INLINE"})
+		use_tree_ = use_tree_ && !std::getenv(name);
+	if (const char *env = std::getenv("B3G_TREE"))
+		use_tree_ = use_tree_ && std::atoi(env) != 0, tree_always_ = std::atoi(env) == 2;
+	if (const char *env = std::getenv("B3G_TREE_GROUPS")) {
+		const int gr = std::atoi(env);
+		if (gr >= 1 && gr <= 16)
+			tree_groups_ = static_cast<uint32_t>(gr);
+	}
+	if (use_tree_) { // the first list finds its workspaces
+		tree_swap_.assign(I_, 0);
+		list_ops_.resize(I_);
+		for (auto *v : {&order_, &parent_, &cost_, &chain_, &tree_order_, &tree_ends_,
+				&walk_stack_, &segs_})
+			v->assign(I_, 0);
+		kid_.assign(2ull * I_, 0);
+		tree_pools_.resize(16);
+		for (auto &pool : tree_pools_)
+			pool.reserve(256);
+	}
+	if (const char *env = std::getenv("B3G_TREE_TILE"))
+		tree_tile_fixed_ = std::atoi(env) == 128 ? 128u : 64u;
+
 	selectors_.assign(I_, 0);
 	stamp_.assign(2 * L_ - 1, 0);
 	pos_.assign(2 * L_ - 1, 0);
@@ -256,7 +282,10 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		off_pi_ = align_up((size_t)I_ * sizeof(NodeOp), 256);
 		off_runs_ = align_up(off_pi_ + S_ * sizeof(double), 256);
 		off_slots_ = align_up(off_runs_ + (size_t)(I_ + 1) * sizeof(uint32_t), 256);
-		off_in_ = align_up(off_slots_ + (size_t)I_ * sizeof(uint32_t), 256);
+		off_tree_ = align_up(off_slots_ + (size_t)I_ * sizeof(uint32_t), 256);
+		off_in_ = off_tree_;
+		if (use_tree_)
+			off_in_ = align_up(off_tree_ + (size_t)I_ * sizeof(TreeOp), 256);
 		stage_bytes_ = off_in_ + (size_t)I_ * 2 * C_ * S_ * S_ * sizeof(double);
 		dev_alloc(d_stage_, stage_bytes_, "stage");
 		check_cuda(cudaHostAlloc((void **)&h_stage_, stage_bytes_,
@@ -460,7 +489,7 @@ void Calculator::validate_lists(const uint32_t *internals,
 // set_selectors, cpu4.rs:93-98) and writes the schedule: output slot of each
 // listed node and the slot or leaf of each child.
 void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
-			   uint32_t n)
+			   uint32_t n, bool tree)
 {
 	for (uint32_t i = 0; i < n; ++i)
 		set_edited(selectors_[internals[i] - L_]);
@@ -469,6 +498,23 @@ void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
 		const uint32_t k = v - L_;
 		return k * 2 + (selectors_[k] & 1u);
 	};
+	if (tree) {
+		list_ops_.resize(n);
+		tip_children_ = 0;
+		for (uint32_t i = 0; i < n; ++i) {
+			const uint32_t l = children[2 * i], r = children[2 * i + 1];
+			NodeOp &op = list_ops_[i];
+			op.out = slot_of(internals[i]);
+			op.left = l < L_ ? (kTipBit | l) : slot_of(l);
+			op.right = r < L_ ? (kTipBit | r) : slot_of(r);
+			tip_children_ += (l < L_) + (r < L_);
+		}
+		depth_first_ = order_depth_first(n);
+		if (depth_first_) {
+			stage_tree(n);
+			return;
+		}
+	}
 	// Runs of mutually independent entries: entry i opens a new run when
 	// one of its children is listed inside the current run.  validate_lists
 	// left stamp_[v] == stamp_epoch_ on every listed internal.
@@ -513,8 +559,198 @@ void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
 	if (n_runs_)
 		max_run_ = std::max(max_run_, n - runs[n_runs_ - 1]);
 	depth_first_ = S_ == 4 ? !f32_ : f32_ && !use_tc20_;
-	if (depth_first_)
-		order_depth_first(n);
+	if (!depth_first_)
+		return;
+	list_ops_.assign(ops, ops + n);
+	order_depth_first(n);
+	stage_order(n);
+}
+
+// Schedule of the depth-first FP32 walk (tree4.cuh) for the ordered list:
+// group after group, child sources, and shared-memory slots for the outputs
+// that the group's next entry does not take from registers and for the clean
+// children.  Follows the kernel's order of events: before the first entry of
+// chunk q the clean children of chunk q + 2 are copied; an entry's slots are
+// read before its output is stored.  A slot returns to the group that read it
+// (a slot that another group filled was read behind a barrier), so no other
+// group can still be reading it when it is written again.  What finds no slot
+// is read from global memory.
+void Calculator::stage_tree(uint32_t n)
+{
+	const uint32_t G = order_groups_, phases = order_phases_;
+	PruneParams pp{};
+	pp.C = C_;
+	pp.groups = G;
+	pp.num_leaves = L_;
+	const uint32_t tile = tree_tile_, budget = tree_budget(G);
+	pp.tile = tile;
+	pp.n_slots = 1;
+	pp.tips_smem = 4ull * tip_children_ >= L_ &&
+		       prune4_tree_smem(pp) + (size_t)tile * (L_ + 1) <= budget;
+	TreeOp *ops = reinterpret_cast<TreeOp *>(h_stage_ + off_tree_);
+	uint32_t *segs = reinterpret_cast<uint32_t *>(h_stage_ + off_runs_);
+	TreeHead *heads = reinterpret_cast<TreeHead *>(segs + G + 1);
+	// phase-major (order_, segs_) to group-major
+	tree_order_.resize(n);
+	tree_ends_.resize((size_t)G * phases);
+	uint32_t at = 0;
+	for (uint32_t g = 0; g < G; ++g) {
+		segs[g] = at;
+		for (uint32_t ph = 0; ph < phases; ++ph) {
+			for (uint32_t k = segs_[ph * G + g]; k < segs_[ph * G + g + 1]; ++k)
+				tree_order_[at++] = order_[k];
+			tree_ends_[ph * G + g] = at;
+		}
+	}
+	segs[G] = n;
+	order_.swap(tree_order_);
+	// children's kinds: the group's previous output first, a tip last
+	for (uint32_t g = 0; g < G; ++g)
+		for (uint32_t e = segs[g]; e < segs[g + 1]; ++e) {
+			const NodeOp &in = list_ops_[order_[e]];
+			const uint32_t prev = e > segs[g] ? ops[e - 1].out : kNone;
+			const bool lt = (in.left & kTipBit) != 0, rt = (in.right & kTipBit) != 0;
+			const bool swap = in.right == prev || (in.left != prev && lt && !rt);
+			TreeOp op{};
+			op.out = in.out;
+			op.id[0] = swap ? in.right : in.left;
+			op.id[1] = swap ? in.left : in.right;
+			op.code = (op.id[0] & kTipBit ? 0u : kTreeInA) |
+				  (op.id[1] & kTipBit ? 0u : kTreeInB) |
+				  (op.id[0] == prev ? kTreePrev : 0u);
+			tree_swap_[e] = swap;
+			ops[e] = op;
+		}
+	tree_pools_.resize(std::max<size_t>(tree_pools_.size(), G));
+	uint32_t used = 0, capacity = 0, missing = 0;
+	auto take = [&](uint32_t g) -> uint32_t {
+		auto &pool = tree_pools_[g];
+		if (!pool.empty()) {
+			const uint32_t s = pool.back();
+			pool.pop_back();
+			return s;
+		}
+		if (used < capacity)
+			return used++;
+		++missing;
+		return kNoSlot;
+	};
+	auto fetch = [&](uint32_t g, uint32_t chunk) { // its clean children
+		const uint32_t lo = segs[g] + chunk * kTreeChunk;
+		for (uint32_t e = lo; e < std::min(lo + kTreeChunk, segs[g + 1]); ++e) {
+			const uint32_t *kid = &kid_[2 * (size_t)order_[e]];
+			for (uint32_t j = 0; j < 2; ++j) {
+				if (!(ops[e].code & (j ? kTreeInB : kTreeInA)) ||
+				    kid[j ^ tree_swap_[e]] != kNone)
+					continue;
+				const uint32_t s = take(g);
+				if (s == kNoSlot) {
+					ops[e].code |= j ? kTreeMemB : kTreeMemA;
+					continue;
+				}
+				ops[e].more |= (j ? kTreeCleanB : kTreeCleanA) |
+					       s << (j ? 16 : 8);
+				tree_clean_ = true;
+			}
+		}
+	};
+	auto assign = [&] {
+		const size_t rest = prune4_tree_smem(pp);
+		capacity = 1 + static_cast<uint32_t>(std::min<size_t>(
+				       254, rest < budget ? (budget - rest) / (tile * 20 * C_) : 0));
+		for (auto &pool : tree_pools_)
+			pool.clear();
+		used = missing = 0;
+		tree_clean_ = false;
+		for (uint32_t g = 0; g < G; ++g) {
+			fetch(g, 0);
+			fetch(g, 1);
+		}
+		for (uint32_t ph = 0; ph < phases; ++ph)
+			for (uint32_t g = 0; g < G; ++g)
+				for (uint32_t e = ph ? tree_ends_[(ph - 1) * G + g] : segs[g];
+				     e < tree_ends_[ph * G + g]; ++e) {
+					if ((e - segs[g]) % kTreeChunk == 0)
+						fetch(g, (e - segs[g]) / kTreeChunk + 2);
+					TreeOp &op = ops[e];
+					for (uint32_t j = 0; j < 2; ++j) {
+						if (!(op.code & (j ? kTreeInB : kTreeInA)) ||
+						    (j == 0 && (op.code & kTreePrev)) ||
+						    (op.code & (j ? kTreeMemB : kTreeMemA)))
+							continue;
+						if (!(op.more & (j ? kTreeCleanB : kTreeCleanA))) {
+							const uint32_t s = smem_of_[op.id[j]];
+							if (s == kNoSlot) {
+								op.code |= j ? kTreeMemB : kTreeMemA;
+								continue;
+							}
+							op.more |= s << (j ? 16 : 8);
+						}
+						tree_pools_[g].push_back(static_cast<uint8_t>(
+							op.more >> (j ? 16 : 8)));
+					}
+					// the root, and what the next entry takes from registers,
+					// need no slot
+					if (order_[e] == n - 1 ||
+					    (e + 1 < segs[g + 1] && (ops[e + 1].code & kTreePrev)))
+						continue;
+					const uint32_t s = take(g);
+					smem_of_[op.out] = static_cast<uint8_t>(s);
+					if (s != kNoSlot)
+						op.code |= kTreeKeep | s << 8;
+				}
+	};
+	assign();
+	if (missing && pp.tips_smem) { // the tips' room for slots
+		pp.tips_smem = 0;
+		for (uint32_t e = 0; e < n; ++e) {
+			ops[e].code &= kTreeInA | kTreeInB | kTreePrev;
+			ops[e].more = 0;
+			smem_of_[ops[e].out] = static_cast<uint8_t>(kNoSlot);
+		}
+		assign();
+	}
+	for (uint32_t i = 0; i < n; ++i)
+		smem_of_[ops[i].out] = static_cast<uint8_t>(kNoSlot);
+	tree_slots_ = std::max(1u, used);
+	tree_tips_ = pp.tips_smem;
+	// what the words and heads read ahead, and the ends of the phases
+	const uint32_t other = pp.tips_smem ? L_ * tile : kTreeNoTip;
+	auto tip = [&](uint32_t e, uint32_t j) {
+		const uint32_t id = ops[e].id[j];
+		return !(id & kTipBit) ? other : (id & ~kTipBit) * (pp.tips_smem ? tile : 1u);
+	};
+	auto base = [&](uint32_t g, uint32_t e) {
+		if (!(ops[e].code & kTreeInB))
+			return prune4_tree_entry(g, e - segs[g]);
+		return prune4_tree_slot(G, tile, ops[e].more >> 16 & 0xFFu);
+	};
+	for (uint32_t g = 0; g < G; ++g) {
+		const uint32_t lo = segs[g], hi = segs[g + 1];
+		TreeHead &h = heads[g];
+		h = TreeHead{};
+		if (hi > lo) {
+			h.tip[0] = tip(lo, 0);
+			h.tip[1] = tip(lo, 1);
+			h.base = base(g, lo);
+		}
+		h.tip[2] = hi > lo + 1 ? tip(lo + 1, 1) : 0;
+		for (uint32_t e = lo; e < hi; ++e) {
+			ops[e].next_a = e + 1 < hi ? tip(e + 1, 0) : 0;
+			ops[e].code |= (e + 1 < hi ? base(g, e + 1) : 0) << 16;
+			ops[e].after_b = e + 2 < hi ? tip(e + 2, 1) : 0;
+		}
+		// (the last phase needs no barrier)
+		for (uint32_t ph = 0; ph + 1 < phases; ++ph) {
+			const uint32_t end = tree_ends_[ph * G + g];
+			if (end == lo) {
+				++h.barriers;
+			} else {
+				ops[end - 1].code |= kTreeBarrier;
+				++ops[end - 1].barriers;
+			}
+		}
+	}
 }
 
 // Shared-memory slots for the run walk's outputs (at most `capacity`),
@@ -569,10 +805,59 @@ uint32_t Calculator::assign_slots(uint32_t n, uint32_t capacity)
 	return used;
 }
 
+// Tile and groups of the depth-first FP32 walk.  128 patterns a block where
+// there are more 64-pattern tiles than SMs (the table rows are read once for
+// four columns instead of two), and groups until an SM has its warps (12, or
+// 16 of the smaller tile) or the list's tips and slots fit the block's share
+// of shared memory.  Us per whole tree at 64 / 128 patterns (4 categories):
+// 256 taxa x 17,764 patterns 98 / 88, 128 x 30,000 94 / 84, 256 x 12,000 91 /
+// 84; 256 x 8,000, 125 small tiles, 61 / 83, 64 x 7,855 34 / 37.  With 1 / 2 /
+// 4 groups of the smaller tile: 256 x 8,000 94 / 72 / 62; of the larger: 256 x
+// 17,764 118 / 88 / 91.
+uint32_t Calculator::pick_tree(uint32_t n)
+{
+	PruneParams pp{};
+	pp.C = C_;
+	pp.num_leaves = L_;
+	pp.tips_smem = 4ull * tip_children_ >= L_;
+	uint32_t G = 1;
+	for (uint32_t tile = ldp_ / 64u > num_sms_ ? 128u : 64u;; tile = 64u) {
+		if (tree_tile_fixed_)
+			tile = tree_tile_fixed_;
+		tree_tile_ = pp.tile = tile;
+		const uint32_t blocks = ldp_ / tile, warps = tile == 128 ? 12 : 16;
+		for (G = 1;; G *= 2) {
+			if (tree_groups_)
+				return tree_groups_ = std::min(tree_groups_, 16u / C_);
+			const bool more = 2 * G * C_ <= 16 && 8 * G <= n;
+			if (more && 2 * G * C_ * blocks <= warps * num_sms_)
+				continue;
+			pp.groups = G;
+			pp.n_slots = 5 + 3 * G;
+			if (prune4_tree_smem(pp) <= tree_budget(G))
+				return G;
+			if (!more)
+				break;
+		}
+		if (tile == 64 || tree_tile_fixed_)
+			return G;
+	}
+}
+
+// Shared memory of a block of that walk.
+uint32_t Calculator::tree_budget(uint32_t G) const
+{
+	const uint32_t warps = tree_tile_ == 128 ? 12 : 16;
+	const uint32_t rounds = (ldp_ / tree_tile_ + num_sms_ - 1) / num_sms_;
+	return smem_budget(1024u / std::max(1u, std::min(warps / (G * C_), rounds)));
+}
+
 // Groups a block of the depth-first walks (each walks subtrees of its own
 // before one of them walks the entries above).
-uint32_t Calculator::pick_groups(uint32_t n) const
+uint32_t Calculator::pick_groups(uint32_t n)
 {
+	if (S_ == 4 && f32_)
+		return pick_tree(n);
 	if (S_ == 20) {
 		if (s20_groups_)
 			return s20_groups_;
@@ -677,16 +962,14 @@ bool Calculator::split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit)
 	return true;
 }
 
-// Reorders the staged list depth first, heavier subtree first, so that a
+// Orders the list (list_ops_) depth first, heavier subtree first, so that a
 // child is mostly the previous entry's output, and for several groups splits
 // it into phases (segs_): disjoint subtrees, a balanced share a group, then
 // the entries above them, run by run.  Every entry's arithmetic is the same
 // in any children-first order.  order_[k] = list position of staged entry k.
-// A list that is not one tree under its last entry keeps its order.
-void Calculator::order_depth_first(uint32_t n)
+// A list that is not one tree under its last entry keeps its order (false).
+bool Calculator::order_depth_first(uint32_t n)
 {
-	NodeOp *ops = reinterpret_cast<NodeOp *>(h_stage_);
-	list_ops_.assign(ops, ops + n);
 	order_.resize(n);
 	kid_.assign(2 * (size_t)n, kNone);
 	parent_.assign(n, kNone);
@@ -754,6 +1037,13 @@ void Calculator::order_depth_first(uint32_t n)
 			emit(n - 1);
 		}
 	}
+	return tree && linked + 1 == n;
+}
+
+// The ordered list's schedule words (the walks but the FP32 four-state one).
+void Calculator::stage_order(uint32_t n)
+{
+	NodeOp *ops = reinterpret_cast<NodeOp *>(h_stage_);
 	size_t seg = 0; // segs_[seg]: where the current walk began
 	for (uint32_t k = 0; k < n; ++k) {
 		NodeOp op = list_ops_[order_[k]];
@@ -779,6 +1069,15 @@ void Calculator::stage_inputs(const double *src, uint32_t n, size_t per_entry)
 	double *dst = reinterpret_cast<double *>(h_stage_ + off_in_);
 	if (!depth_first_) {
 		std::memcpy(dst, src, n * per_entry * sizeof(double));
+		return;
+	}
+	if (S_ == 4 && f32_) { // children in the schedule's order
+		const size_t half = per_entry / 2;
+		for (uint32_t k = 0; k < n; ++k)
+			for (uint32_t j = 0; j < 2; ++j)
+				std::memcpy(dst + k * per_entry + j * half,
+					    src + order_[k] * per_entry + (j ^ tree_swap_[k]) * half,
+					    half * sizeof(double));
 		return;
 	}
 	for (uint32_t k = 0; k < n; ++k)
@@ -813,7 +1112,8 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 	}
 	// run walk configuration, decided before the upload because the slot
 	// codes travel with the schedule
-	const bool runs = S_ == 4 && use_runs_ && n <= 4096;
+	const bool tree = S_ == 4 && f32_ && depth_first_;
+	const bool runs = S_ == 4 && use_runs_ && n <= 4096 && !tree;
 	PruneParams pp{};
 	uint32_t block = 512;
 	if (runs) {
@@ -860,8 +1160,10 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 	const size_t in_bytes =
 		matrices_mode ? (size_t)n * 2 * C_ * S_ * S_ * sizeof(double)
 			      : (size_t)n * 2 * sizeof(double);
-	last_upload_bytes_ = off_in_ + in_bytes;
-	check_cuda(cudaMemcpyAsync(d_stage_, h_stage_, last_upload_bytes_,
+	// (the depth-first FP32 walk's schedule lies behind the list's)
+	const size_t from = tree ? off_pi_ : 0;
+	last_upload_bytes_ = off_in_ + in_bytes - from;
+	check_cuda(cudaMemcpyAsync(d_stage_ + from, h_stage_ + from, last_upload_bytes_,
 				   cudaMemcpyHostToDevice, stream_),
 		   "upload step");
 	check_cuda(cudaEventRecord(ev_stage_free_, stream_), "event");
@@ -896,7 +1198,8 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 		pp.clock_rate = clock_rate;
 		last_launches_ = 1;
 	} else {
-		check_cuda(launch_ptab4(pt, f32_, stream_), "transition kernel");
+		check_cuda(tree ? launch_ptab4_rows(pt, stream_) : launch_ptab4(pt, f32_, stream_),
+			   "transition kernel");
 		last_launches_ = 2;
 	}
 	record(slot.kmid);
@@ -932,7 +1235,18 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 	pp.log_inv_c = std::log(1.0 / static_cast<double>(C_));
 	// the run-synchronous walk stages the schedule in shared memory: keep
 	// it for lists up to 4,096 entries
-	if (runs) {
+	if (tree) {
+		pp.ops = reinterpret_cast<const NodeOp *>(d_stage_ + off_tree_);
+		pp.n_slots = tree_slots_;
+		pp.tips_smem = tree_tips_;
+		pp.groups = order_groups_;
+		pp.phases = order_phases_;
+		pp.segs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
+		pp.sums_host = d_bsums_;
+		arm_host_fold(ldp_ / tree_tile_);
+		pp.tile = tree_tile_;
+		check_cuda(launch_prune4_tree(pp, tree_clean_, stream_), "pruning kernel");
+	} else if (runs) {
 		pp.runs = reinterpret_cast<const uint32_t *>(d_stage_ + off_runs_);
 		pp.slots = reinterpret_cast<const uint32_t *>(d_stage_ + off_slots_);
 		const uint32_t tiles = ldp_ / pp.tile;
@@ -1218,7 +1532,7 @@ void Calculator::propose_matrices(const uint32_t *internals,
 		if (!std::isfinite(freqs[s]))
 			throw Error(B3G_ERR_NUMERIC, "non-finite frequency");
 	wait_stage();
-	stage_ops(internals, children, n);
+	stage_ops(internals, children, n, tree_list(n));
 	std::memcpy(h_stage_ + off_pi_, freqs, S_ * sizeof(double));
 	stage_inputs(matrices, n, 2ull * C_ * S_ * S_);
 	launch(n, true, 1.0, true);
@@ -1242,7 +1556,8 @@ void Calculator::propose_lengths(const uint32_t *internals,
 		throw Error(B3G_ERR_NUMERIC, "non-finite clock rate");
 	wait_stage();
 	wait_batch();
-	stage_ops(internals, children, n);
+	stage_ops(internals, children, n,
+		  tree_list(n) && !(use_direct_ && n <= kDirectMax));
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
 	stage_inputs(lengths, n, 2);
 	staged_ = false;
@@ -1275,7 +1590,7 @@ void Calculator::stage_lengths(const uint32_t *internals,
 	// so must this calculator's own last launch
 	wait_stage();
 	wait_batch();
-	stage_ops(internals, children, n);
+	stage_ops(internals, children, n, false);
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
 	std::memcpy(h_stage_ + off_in_, lengths, (size_t)n * 2 * sizeof(double));
 	staged_ = true;
@@ -1608,6 +1923,10 @@ uint32_t Calculator::autotune(const uint32_t *internals,
 	// category per thread: a warp spans 32 / (tile / 2) categories, so
 	// tiles of 16 and 32 patterns put four and two categories in a warp
 	// (and give small alignments more blocks), 64 and 128 one.
+	// (The run walk's shape, for batches and lists of several trees; the
+	// depth-first walk has none.)
+	const Restore walk{use_tree_, use_tree_};
+	use_tree_ = false;
 	uint32_t best_tile = runs_tile_, best_block = runs_block_;
 	float best_ms = INFINITY;
 	const uint32_t cand[][2] = {{16, 512},  {32, 512},  {64, 512},

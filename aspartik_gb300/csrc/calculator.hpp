@@ -98,7 +98,21 @@ class Calculator {
 	void validate_lists(const uint32_t *internals,
 			    const uint32_t *children, uint32_t n);
 	void stage_ops(const uint32_t *internals, const uint32_t *children,
-		       uint32_t n);
+		       uint32_t n, bool tree);
+	void stage_tree(uint32_t n);
+	void stage_order(uint32_t n);
+	// Whether a single-tree list takes the depth-first FP32 walk: where its
+	// 64-pattern tiles reach half of the SMs, or the list is small.  Us per
+	// whole tree, run walk / depth first: 256 taxa x 8,000 patterns x 4
+	// categories 75 / 61, 100 x 5,000 x 8 61 / 50, 500 x 5,000 x 1 57 / 56;
+	// with fewer tiles an SM has all of a tile's entries and the run walk's
+	// smaller tiles win, 256 x 3,000 x 4 55 / 58, 256 x 300 x 4 45 / 57, 100 x
+	// 1,500 x 4 32 / 36; small lists 64 x 1,000 x 4 32 / 31, 60 x 500 x 3 29 /
+	// 28.
+	bool tree_list(uint32_t n) const
+	{
+		return use_tree_ && (tree_always_ || 128 * num_sms_ <= 4 * ldp_ || n * C_ <= 256);
+	}
 	void launch(uint32_t n, bool matrices_mode, double clock_rate,
 		    bool want_cat);
 	void launch_direct(uint32_t n, double clock_rate);
@@ -158,18 +172,27 @@ class Calculator {
 	uint32_t runs_block_ = 512;
 	bool use_slots_ = true;
 	bool use_inline_ = true;
-	size_t off_slots_ = 0;
+	size_t off_slots_ = 0, off_tree_ = 0;
 	uint32_t assign_slots(uint32_t n, uint32_t capacity);
 	uint32_t stamp_epoch_ = 0;
 	// depth-first order of the staged list (four-state FP64, 20-state FP32)
 	static constexpr uint32_t kNone = 0xFFFFFFFFu;
 	bool depth_first_ = false;
+	// the four-state FP32 form's depth-first walk of single-tree lists
+	// (B3G_TREE=0: the run walk), and the staged list's shared-memory slots
+	bool use_tree_ = false, tree_always_ = false;
+	uint32_t tree_slots_ = 0, tree_tips_ = 0, tree_groups_ = 0, tree_tile_ = 64;
+	uint32_t tree_tile_fixed_ = 0;
+	bool tree_clean_ = false;
+	std::vector<uint32_t> tree_order_, tree_ends_;
+	std::vector<uint8_t> tree_swap_; // staged entry: first child is the right one
+	std::vector<std::vector<uint8_t>> tree_pools_;
 	uint32_t order_groups_ = 1, order_phases_ = 1;
 	std::vector<uint32_t> order_, segs_, kid_, parent_, cost_, chain_, walk_stack_, pieces_,
 		above_;
 	std::vector<uint32_t> slot_pos_; // by partial slot; kNone outside the call
 	std::vector<NodeOp> list_ops_;
-	void order_depth_first(uint32_t n);
+	bool order_depth_first(uint32_t n);
 	template <typename Emit>
 	bool split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit);
 	void stage_inputs(const double *src, uint32_t n, size_t per_entry);
@@ -221,7 +244,9 @@ class Calculator {
 	ModelDev *d_model_ = nullptr;
 	void *d_ptab_ = nullptr;
 	uint32_t f64_groups_ = 0; // 0: chosen per list
-	uint32_t pick_groups(uint32_t n) const;
+	uint32_t pick_groups(uint32_t n);
+	uint32_t pick_tree(uint32_t n);
+	uint32_t tree_budget(uint32_t groups) const;
 	uint32_t pick_p20_groups(uint32_t n) const;
 	uint32_t s20_groups_ = 0; // 20-state FP32 walk; 0: chosen per list
 	uint32_t s20_per_sm_[5] = {}; // blocks an SM holds, by warps a block

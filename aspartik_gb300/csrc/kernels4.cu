@@ -307,6 +307,67 @@ __global__ void __launch_bounds__(32) ptab4_kernel(PtabParams prm)
 		out[16 + j] = 1.0f;
 }
 
+// FP32 tables of the depth-first walk (tree4.cuh), four lanes a table: lane i
+// takes exp(lambda_i d) and row i of P, with transition4f_eig's arithmetic.
+// The eigensystem is converted once a block.  The walk may be launched beside
+// this kernel (it waits for the tables itself).
+__global__ void __launch_bounds__(128) ptab4_rows_kernel(PtabParams prm)
+{
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	const uint32_t t = blockIdx.x * 128u + threadIdx.x;
+	const uint32_t id = t >> 2, i = t & 3u;
+	const bool live = id < prm.n * 2u * prm.C;
+	const uint32_t c = id % prm.C, es = id / prm.C;
+	const ModelDev *m = prm.model;
+	float P[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+	if (prm.matrices) {
+		if (live)
+			for (int j = 0; j < 4; j++)
+				P[j] = (float)prm.matrices[(size_t)id * 16 + i * 4 + j];
+	} else {
+		__shared__ float eig[40];
+		if (threadIdx.x < 37) {
+			const uint32_t k = threadIdx.x;
+			eig[k] = k < 16   ? (float)m->V[k]
+				 : k < 32 ? (float)m->Vinv[k - 16]
+				 : k < 36 ? (float)m->lambda[k - 32]
+					  : (m->shortcuts ? 1.0f : 0.0f);
+		}
+		const double d = live ? prm.lengths[es] * (prm.clock_rate * m->cat_rates[c])
+				      : 0.0;
+		__syncthreads();
+		const float mine = expf(eig[32 + i] * (float)d);
+		float e[4];
+#pragma unroll
+		for (int k = 0; k < 4; k++)
+			e[k] = __shfl_sync(0xffffffffu, mine, k, 4);
+		const bool shortcuts = eig[36] != 0.0f;
+		if (shortcuts && d > 20.0) {
+			for (int j = 0; j < 4; j++)
+				P[j] = (float)m->pi[j];
+		} else if (shortcuts && d < 1e-10) {
+			for (int j = 0; j < 4; j++)
+				P[j] = (int)i == j ? 1.0f : (float)(m->Q[i * 4 + j] * d);
+		} else {
+			const float t0 = eig[i * 4 + 0] * e[0], t1 = eig[i * 4 + 1] * e[1];
+			const float t2 = eig[i * 4 + 2] * e[2], t3 = eig[i * 4 + 3] * e[3];
+			for (int j = 0; j < 4; j++) {
+				float s = t0 * eig[16 + 0 * 4 + j];
+				s = fmaf(t1, eig[16 + 1 * 4 + j], s);
+				s = fmaf(t2, eig[16 + 2 * 4 + j], s);
+				s = fmaf(t3, eig[16 + 3 * 4 + j], s);
+				P[j] = s;
+			}
+		}
+	}
+	if (!live)
+		return;
+	float *out = (float *)prm.ptab + (size_t)id * 20;
+	for (int j = 0; j < 4; j++)
+		out[j * 4 + i] = P[j];
+	out[16 + i] = 1.0f;
+}
+
 // ---------------------------------------------------------------------------
 // pruning
 
@@ -763,6 +824,7 @@ __global__ void __launch_bounds__(512) prune4_plain_kernel(PruneParams prm)
 // ---------------------------------------------------------------------------
 #include "prune4f64.cuh"
 #include "runs4.cuh"
+#include "tree4.cuh"
 
 // ---------------------------------------------------------------------------
 #include "prune20.cuh"
@@ -916,6 +978,68 @@ cudaError_t launch_prune4_runs(const PruneParams &p, uint32_t ctas,
 			return e;
 	}
 	kern<<<ctas, threads, smem, s>>>(p);
+	return cudaGetLastError();
+}
+
+size_t prune4_tree_smem(const PruneParams &p)
+{
+	return p.C * (p.tile * (sizeof(float) + sizeof(int32_t)) + p.groups * kTreeRingBytes +
+		      (size_t)p.n_slots * p.tile * kTreeColBytes) +
+	       (p.tips_smem ? (size_t)(p.num_leaves + 1) * p.tile : 0);
+}
+
+uint32_t prune4_tree_entry(uint32_t group, uint32_t k)
+{
+	return (uint32_t)(group * kTreeRingBytes + (k & (kTreeRing - 1)) * sizeof(TreeEntry) +
+			  5 * sizeof(float4)) /
+	       16u;
+}
+
+uint32_t prune4_tree_slot(uint32_t groups, uint32_t tile, uint32_t slot)
+{
+	return (groups * kTreeRingBytes) / 16u + slot * tile;
+}
+
+cudaError_t launch_prune4_tree(const PruneParams &p, bool clean, cudaStream_t s)
+{
+	if (p.n == 0 || p.C == 0 || p.groups == 0 || p.groups * p.C > 16 ||
+	    (p.tile != 64 && p.tile != 128) || p.ldp % p.tile ||
+	    !p.sums_host || !p.segs || p.n_slots > 255 || (uint64_t)p.C * p.ldp >= (1ull << 28))
+		return cudaErrorInvalidValue;
+	const size_t smem = prune4_tree_smem(p);
+	const int v = (p.tile == 128 ? 4 : 0) + (p.tips_smem ? 2 : 0) + (clean ? 1 : 0);
+	void (*const kerns[8])(PruneParams) = {
+		prune4_tree_kernel<1, false, false>, prune4_tree_kernel<1, false, true>,
+		prune4_tree_kernel<1, true, false>,  prune4_tree_kernel<1, true, true>,
+		prune4_tree_kernel<2, false, false>, prune4_tree_kernel<2, false, true>,
+		prune4_tree_kernel<2, true, false>,  prune4_tree_kernel<2, true, true>};
+	void (*const kern)(PruneParams) = kerns[v];
+	if (smem > 48 * 1024) {
+		static SmemOptIn opted[8];
+		const cudaError_t e = opt_in_smem(kern, opted[v]);
+		if (e != cudaSuccess)
+			return e;
+	}
+	// may start while the transition kernel runs
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3(p.ldp / p.tile);
+	cfg.blockDim = dim3(32 * p.C * p.groups);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = s;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+cudaError_t launch_ptab4_rows(const PtabParams &p, cudaStream_t s)
+{
+	const uint32_t total = p.n * 2u * p.C;
+	if (total == 0)
+		return cudaSuccess;
+	ptab4_rows_kernel<<<(4u * total + 127u) / 128u, 128, 0, s>>>(p);
 	return cudaGetLastError();
 }
 

@@ -381,46 +381,52 @@ __device__ __forceinline__ float scale_down(float x, int32_t e)
 	return x * __uint_as_float((uint32_t)(127 + hi) << 23);
 }
 
-// Root of tile t after its walk left pi . x and the exponent of every
-// column in s_dot / s_cnt: category mixing per pattern (threads 0 ..
-// tile-1), site values, and the tile's weighted sum in a fixed order,
-// returned in thread 0.  Ends with the block synchronised.
+// Root of the pattern at column k of a tile (p of the whole) after the walk
+// left pi . x and the exponent of every column in s_dot / s_cnt: category
+// mixing and site values.  Returns the weighted site value.
+__device__ __forceinline__ double
+pattern_root(const float *s_dot, const int32_t *s_cnt, uint32_t tile, uint32_t C, uint32_t k,
+	     uint32_t ldp, uint32_t p, double log_inv_c, double *site_lnl, double *cat_lnl,
+	     const uint32_t *weights)
+{
+	const uint32_t wgt = weights[p];
+	int32_t emax = INT32_MIN;
+	for (uint32_t c = 0; c < C; c++)
+		if (s_dot[c * tile + k] > 0.f)
+			emax = max(emax, s_cnt[c * tile + k]);
+	double site;
+	if (emax == INT32_MIN) {
+		site = -INFINITY;
+	} else {
+		// categories mixed in FP32 at the largest exponent; only the
+		// exact exponent term and the constant join in FP64
+		float acc = 0.f;
+		for (uint32_t c = 0; c < C; c++)
+			acc += scale_down(s_dot[c * tile + k], s_cnt[c * tile + k] - emax);
+		site = (double)logf(acc) +
+		       fma((double)emax, 0.69314718055994530942, log_inv_c);
+	}
+	site_lnl[p] = site;
+	if (cat_lnl)
+		for (uint32_t c = 0; c < C; c++)
+			cat_lnl[(size_t)c * ldp + p] =
+				log((double)s_dot[c * tile + k]) +
+				(double)s_cnt[c * tile + k] * 0.69314718055994530942;
+	return wgt ? site * (double)wgt : 0.0;
+}
+
+// Root of tile t: threads 0 .. tile-1 a pattern each, and the tile's weighted
+// sum in a fixed order, returned in thread 0.  Ends with the block
+// synchronised.
 __device__ double tile_root(const TileArgs &a, uint32_t t, const float *s_dot,
 			    const int32_t *s_cnt, double *s_red)
 {
-	const uint32_t tile = a.tile, C = a.C;
+	const uint32_t tile = a.tile;
 	const uint32_t tid = threadIdx.x;
 	double contrib = 0.0;
-	if (tid < tile) {
-		const uint32_t pp = t * tile + tid;
-		int32_t emax = INT32_MIN;
-		for (uint32_t k = 0; k < C; k++)
-			if (s_dot[k * tile + tid] > 0.f)
-				emax = max(emax, s_cnt[k * tile + tid]);
-		double site;
-		if (emax == INT32_MIN) {
-			site = -INFINITY;
-		} else {
-			// categories mixed in FP32 at the largest exponent; only
-			// the exact exponent term and the constant join in FP64
-			float acc = 0.f;
-			for (uint32_t k = 0; k < C; k++)
-				acc += scale_down(s_dot[k * tile + tid],
-						  s_cnt[k * tile + tid] - emax);
-			site = (double)logf(acc) +
-			       fma((double)emax, 0.69314718055994530942,
-				   a.log_inv_c);
-		}
-		a.site_lnl[pp] = site;
-		if (a.cat_lnl)
-			for (uint32_t k = 0; k < C; k++)
-				a.cat_lnl[(size_t)k * a.ldp + pp] =
-					log((double)s_dot[k * tile + tid]) +
-					(double)s_cnt[k * tile + tid] *
-						0.69314718055994530942;
-		const uint32_t wgt = a.weights[pp];
-		contrib = wgt ? site * (double)wgt : 0.0;
-	}
+	if (tid < tile)
+		contrib = pattern_root(s_dot, s_cnt, tile, a.C, tid, a.ldp, t * tile + tid,
+				       a.log_inv_c, a.site_lnl, a.cat_lnl, a.weights);
 	// tile sum in a fixed order (warp shuffles, then warps in order)
 	for (int off = 16; off > 0; off >>= 1)
 		contrib += __shfl_down_sync(0xffffffffu, contrib, off);
