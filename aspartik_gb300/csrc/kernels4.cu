@@ -37,6 +37,38 @@ namespace {
 
 namespace cg = cooperative_groups;
 
+// A walk may be launched beside the kernel that writes its transition tables
+// (launch_beside): the table kernel lets it start at once, the walk waits
+// before it reads a table.  Its launch and prologue are then off the chain of
+// a short evaluation (FP64, 64 taxa x 7,855 patterns x 4 categories, paths of
+// 8 entries: 34.7 -> 32.6 us each; 37 x 1,147, whole tree: 57 -> 55 us).  The
+// 20-state FP32 walk, whose early blocks take the table kernel's place on the
+// SMs, gained nothing (350 / 351, a whole tree 168 / 165 us) and waits.
+__device__ __forceinline__ void tables_started()
+{
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_tables()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename P>
+cudaError_t launch_beside(void (*kern)(P), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+			  const P &p)
+{
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = s;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
 // ---------------------------------------------------------------------------
 // 4-vectors: double4_32a (one 256-bit access) and float4 (one 128-bit access)
 
@@ -209,6 +241,7 @@ __device__ void transition4f(const ModelDev *__restrict__ m, double d,
 // as the matrix form V diag(e) V^-1 row by row.  With `soft` the integer form of the table is written too.
 __global__ void __launch_bounds__(32) ptab4_f64_kernel(PtabParams prm)
 {
+	tables_started();
 	const uint32_t t = blockIdx.x * 32u + threadIdx.x;
 	const uint32_t id = t >> 2, i = t & 3u;
 	const bool live = id < prm.n * 2u * prm.C;
@@ -313,7 +346,7 @@ __global__ void __launch_bounds__(32) ptab4_kernel(PtabParams prm)
 // this kernel (it waits for the tables itself).
 __global__ void __launch_bounds__(128) ptab4_rows_kernel(PtabParams prm)
 {
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	tables_started();
 	const uint32_t t = blockIdx.x * 128u + threadIdx.x;
 	const uint32_t id = t >> 2, i = t & 3u;
 	const bool live = id < prm.n * 2u * prm.C;
@@ -892,8 +925,7 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 						   : prune4_f64_kernel<size_t, true>)
 					 : (narrow ? prune4_f64_kernel<uint32_t, false>
 						   : prune4_f64_kernel<size_t, false>);
-		kern<<<p.ldp / tp, dim3(tp, p.C, p.groups), bytes, s>>>(p);
-		return cudaGetLastError();
+		return launch_beside(kern, dim3(p.ldp / tp), dim3(tp, p.C, p.groups), bytes, s, p);
 	}
 	prune4_plain_kernel<<<grid, block, smem, s>>>(p);
 	return cudaGetLastError();
@@ -1020,18 +1052,7 @@ cudaError_t launch_prune4_tree(const PruneParams &p, bool clean, cudaStream_t s)
 		if (e != cudaSuccess)
 			return e;
 	}
-	// may start while the transition kernel runs
-	cudaLaunchAttribute attr{};
-	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr.val.programmaticStreamSerializationAllowed = 1;
-	cudaLaunchConfig_t cfg{};
-	cfg.gridDim = dim3(p.ldp / p.tile);
-	cfg.blockDim = dim3(32 * p.C * p.groups);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = s;
-	cfg.attrs = &attr;
-	cfg.numAttrs = 1;
-	return cudaLaunchKernelEx(&cfg, kern, p);
+	return launch_beside(kern, dim3(p.ldp / p.tile), dim3(32 * p.C * p.groups), smem, s, p);
 }
 
 cudaError_t launch_ptab4_rows(const PtabParams &p, cudaStream_t s)
@@ -1122,8 +1143,8 @@ cudaError_t launch_prune20_f64(const PruneParams &p, uint32_t groups, cudaStream
 		prune20_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess)
 		return e;
-	prune20_f64_kernel<<<dim3(p.ldp / kP20Tile, p.C), 128 * groups, smem, s>>>(p);
-	return cudaGetLastError();
+	return launch_beside(prune20_f64_kernel, dim3(p.ldp / kP20Tile, p.C), dim3(128 * groups),
+			     smem, s, p);
 }
 
 uint32_t prune20_blocks_per_sm(uint32_t groups)

@@ -86,6 +86,8 @@ template <typename R>
 __global__ void __launch_bounds__(kS20 *kS20) ptab20_kernel(PtabParams prm)
 {
 	constexpr uint32_t S = kS20;
+	if constexpr (sizeof(R) == 8)
+		tables_started();
 	__shared__ Ptab20Smem sm;
 	const uint32_t id = blockIdx.x, t = threadIdx.x, i = t / S, j = t - i * S;
 	const double P = ptab20_element(prm, id, t, sm);

@@ -289,6 +289,7 @@ __global__ void __launch_bounds__(512) prune4_f64_kernel(PruneParams prm)
 		++fe;
 		slot = (slot + 1) & (kF64Ring - 1);
 	};
+	wait_for_tables();
 #pragma unroll
 	for (uint32_t e = 0; e < kF64Ring; ++e)
 		fill();

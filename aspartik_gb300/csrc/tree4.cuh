@@ -206,8 +206,7 @@ __global__ void __launch_bounds__(512) prune4_tree_kernel(PruneParams prm)
 			((uint16_t *)(s_tips + prm.num_leaves * kTreeTile))[h * 32 + lane] =
 				(uint16_t)((h * 64 + lane) | (h * 64 + lane + 32u) << 8);
 	}
-	// the transition kernel's tables (this kernel may start beside it)
-	asm volatile("griddepcontrol.wait;" ::: "memory");
+	wait_for_tables();
 	fill(0);
 	if (kClean) { // chunk 0's words
 		cp_async_wait<0>();
