@@ -181,10 +181,17 @@ struct MemberDesc {
 	double *site_lnl;
 	double *tile_sums;   // one per tile, owned by the batch
 	unsigned *ticket;    // tiles finished, owned by the batch
-	uint32_t off_pi, off_runs, off_in;
+	uint32_t off_pi, off_runs, off_in, off_tree;
 	uint32_t ldp, C, L, tile;
 	double log_inv_c;
 };
+
+// The run walk; the short-list kernel (n <= kDirectMax, C of 1, 2 or 4); the
+// depth-first walk (other single-tree lists).
+constexpr uint32_t kListRuns = 0, kListShort = 1, kListTree = 2;
+// Shared memory of a block of the batched depth-first walk: beside it fits one
+// block of the short-list kernel.
+constexpr uint32_t kBatchTreeSmem = 144u * 1024u;
 
 // Per step and member, written by the host before every batched launch.
 struct MemberStep {
@@ -192,9 +199,9 @@ struct MemberStep {
 	uint32_t n_runs;
 	uint32_t tips_smem;
 	uint32_t tile; // patterns per tile for this step (divides ldp)
-	// a short list (n <= kDirectMax, C of 1, 2 or 4): walked by the
-	// batched short-list kernel instead of the run walk
-	uint32_t direct;
+	uint32_t kind; // the kernel that walks the list
+	// a depth-first list's schedule (kListTree)
+	uint32_t groups, phases, n_slots, clean;
 	double clock_rate;
 };
 
@@ -343,6 +350,7 @@ cudaError_t launch_prune4_direct(const DirectParams &p, uint32_t ctas,
 // max_entries = largest member n * 2 * C.
 cudaError_t launch_ptab4_batch(const BatchParams &p, uint32_t max_entries,
 			       cudaStream_t s);
+cudaError_t launch_prune4_tree_batch(const BatchParams &p, uint32_t ctas, cudaStream_t s);
 cudaError_t launch_prune4_batch(const BatchParams &p, uint32_t ctas,
 				cudaStream_t s);
 // Batched short lists: every member whose step is direct and has C

@@ -57,24 +57,23 @@ Batch::Batch(Calculator *const *members, uint32_t count)
 		return (uint64_t)x->I_ * x->ldp_ * x->C_ > (uint64_t)y->I_ * y->ldp_ * y->C_;
 	});
 	try {
-		check_cuda(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking),
+		int low = 0, high = 0;
+		check_cuda(cudaDeviceGetStreamPriorityRange(&low, &high), "priorities");
+		check_cuda(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, high),
 			   "stream");
-		check_cuda(cudaStreamCreateWithFlags(&stream2_, cudaStreamNonBlocking),
+		check_cuda(cudaStreamCreateWithPriority(&stream2_, cudaStreamNonBlocking, low),
 			   "stream");
 		check_cuda(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming), "event");
 		check_cuda(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming), "event");
 		check_cuda(cudaEventCreate(&ev0_), "event");
 		check_cuda(cudaEventCreate(&ev1_), "event");
 		check_cuda(cudaMalloc(&d_desc_, sizeof(MemberDesc) * M), "descriptors");
-		check_cuda(cudaMalloc(&d_steps_, sizeof(MemberStep) * M), "steps");
-		check_cuda(cudaHostAlloc((void **)&h_steps_, sizeof(MemberStep) * M,
-					 cudaHostAllocDefault),
-			   "pinned steps");
-		check_cuda(cudaMalloc(&d_lnl_, sizeof(double) * M), "lnl");
+		// the members' last blocks write here (mapped; read after the
+		// step's end event)
 		check_cuda(cudaHostAlloc((void **)&h_lnl_, sizeof(double) * M,
-					 cudaHostAllocDefault),
+					 cudaHostAllocMapped),
 			   "pinned lnl");
-		check_cuda(cudaMalloc(&d_work_, 4 * sizeof(unsigned)), "work counters");
+		check_cuda(cudaHostGetDevicePointer((void **)&d_lnl_, h_lnl_, 0), "mapped lnl");
 		// one sum per tile of a member, for tiles as small as 16 patterns
 		// (whatever tile the member's autotuner picks later)
 		size_t total_tiles = 0;
@@ -105,6 +104,7 @@ Batch::Batch(Calculator *const *members, uint32_t count)
 			d.off_pi = (uint32_t)c->off_pi_;
 			d.off_runs = (uint32_t)c->off_runs_;
 			d.off_in = (uint32_t)c->off_in_;
+			d.off_tree = (uint32_t)c->off_tree_;
 			d.ldp = c->ldp_;
 			d.C = c->C_;
 			d.L = c->L_;
@@ -126,7 +126,10 @@ Batch::Batch(Calculator *const *members, uint32_t count)
 		}
 		// the members' staging slices: each member's layout up to the end
 		// of its edge lengths (lengths-mode proposals only while batched)
+		// in front of them the zeroed work counters and the steps, so that
+		// one copy brings all of a step's inputs
 		std::vector<size_t> slice(M);
+		block_bytes_ = (256 + sizeof(MemberStep) * M + 255) & ~(size_t)255;
 		for (uint32_t k = 0; k < M; ++k) {
 			const Calculator *c = members_[order_[k]];
 			slice[k] = block_bytes_;
@@ -136,6 +139,10 @@ Batch::Batch(Calculator *const *members, uint32_t count)
 		check_cuda(cudaHostAlloc((void **)&h_block_, block_bytes_, cudaHostAllocDefault),
 			   "pinned staging block");
 		check_cuda(cudaMalloc(&d_block_, block_bytes_), "staging block");
+		std::memset(h_block_, 0, 256);
+		d_work_ = reinterpret_cast<unsigned *>(d_block_);
+		h_steps_ = reinterpret_cast<MemberStep *>(h_block_ + 256);
+		d_steps_ = reinterpret_cast<MemberStep *>(d_block_ + 256);
 		for (uint32_t k = 0; k < M; ++k) {
 			Calculator *c = members_[order_[k]];
 			// the member's own last launch must be done with its buffer
@@ -164,49 +171,50 @@ Batch::Batch(Calculator *const *members, uint32_t count)
 		ctas_ = 2 * members_[0]->num_sms_;
 		evaluated_.assign(M, 0);
 
-		// capture one step as a graph
-		check_cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal),
-			   "begin capture");
-		// external event-record nodes: the events are recorded each time
-		// the graph runs and can be waited on outside it
-		check_cuda(cudaEventRecordWithFlags(ev0_, stream_,
-						    cudaEventRecordExternal),
-			   "event");
-		check_cuda(cudaMemcpyAsync(d_steps_, h_steps_, sizeof(MemberStep) * M,
-					   cudaMemcpyHostToDevice, stream_),
-			   "steps copy");
-		check_cuda(cudaMemcpyAsync(d_block_, h_block_, block_bytes_,
-					   cudaMemcpyHostToDevice, stream_),
-			   "staging block copy");
-		check_cuda(cudaMemsetAsync(d_work_, 0, 4 * sizeof(unsigned), stream_),
-			   "work counters");
-		// two branches: the run walk of long lists on this stream, the
-		// short-list kernels on the second, joined before the read-back
-		check_cuda(cudaEventRecord(ev_fork_, stream_), "fork");
-		check_cuda(cudaStreamWaitEvent(stream2_, ev_fork_, 0), "fork");
-		check_cuda(launch_ptab4_batch(bp_, max_entries_, stream_),
-			   "batched transition kernel");
-		check_cuda(launch_prune4_batch(bp_, ctas_, stream_),
-			   "batched pruning kernel");
-		for (uint32_t C : {4u, 2u, 1u})
-			if (direct_c_[C])
-				check_cuda(launch_prune4_direct_batch(
-						   bp_, C, (8u / C) * members_[0]->num_sms_, stream2_),
-					   "batched short-list kernel");
-		check_cuda(cudaEventRecord(ev_join_, stream2_), "join");
-		check_cuda(cudaStreamWaitEvent(stream_, ev_join_, 0), "join");
-		check_cuda(cudaMemcpyAsync(h_lnl_, d_lnl_, sizeof(double) * M,
-					   cudaMemcpyDeviceToHost, stream_),
-			   "lnl copy");
-		check_cuda(cudaEventRecordWithFlags(ev1_, stream_,
-						    cudaEventRecordExternal),
-			   "event");
-		check_cuda(cudaStreamEndCapture(stream_, &graph_), "end capture");
-		check_cuda(cudaGraphInstantiate(&exec_, graph_, 0), "instantiate");
+		for (uint32_t form = 0; form < 4; ++form)
+			capture(form);
 	} catch (...) {
 		release();
 		throw;
 	}
+}
+
+// One step as a graph, for steps with (1) and without lists for the run walk,
+// with (2) and without lists for the depth-first walk.
+void Batch::capture(uint32_t form)
+{
+	check_cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal),
+		   "begin capture");
+	// external event-record nodes: the events are recorded each time
+	// the graph runs and can be waited on outside it
+	check_cuda(cudaEventRecordWithFlags(ev0_, stream_, cudaEventRecordExternal), "event");
+	check_cuda(cudaMemcpyAsync(d_block_, h_block_, block_bytes_, cudaMemcpyHostToDevice,
+				   stream_),
+		   "staging block copy");
+	// two branches: the long lists on this stream, the short-list kernels on
+	// the second (of lower priority), joined at the end.  The second starts
+	// beside the long lists' tables: behind them, a step of two whole trees and
+	// 30 short lists took 75.6 us instead of 68.6.
+	check_cuda(cudaEventRecord(ev_fork_, stream_), "fork");
+	check_cuda(cudaStreamWaitEvent(stream2_, ev_fork_, 0), "fork");
+	if (form)
+		check_cuda(launch_ptab4_batch(bp_, max_entries_, stream_),
+			   "batched transition kernel");
+	if (form & 2u)
+		check_cuda(launch_prune4_tree_batch(bp_, members_[0]->num_sms_, stream_),
+			   "batched depth-first kernel");
+	if (form & 1u)
+		check_cuda(launch_prune4_batch(bp_, ctas_, stream_), "batched pruning kernel");
+	for (uint32_t C : {4u, 2u, 1u})
+		if (direct_c_[C])
+			check_cuda(launch_prune4_direct_batch(
+					   bp_, C, (8u / C) * members_[0]->num_sms_, stream2_),
+				   "batched short-list kernel");
+	check_cuda(cudaEventRecord(ev_join_, stream2_), "join");
+	check_cuda(cudaStreamWaitEvent(stream_, ev_join_, 0), "join");
+	check_cuda(cudaEventRecordWithFlags(ev1_, stream_, cudaEventRecordExternal), "event");
+	check_cuda(cudaStreamEndCapture(stream_, &graph_[form]), "end capture");
+	check_cuda(cudaGraphInstantiate(&exec_[form], graph_[form], 0), "instantiate");
 }
 
 Batch::~Batch() { release(); }
@@ -241,16 +249,16 @@ void Batch::release()
 	cudaFree(d_block_);
 	h_block_ = nullptr;
 	d_block_ = nullptr;
-	if (exec_)
-		cudaGraphExecDestroy(exec_);
-	if (graph_)
-		cudaGraphDestroy(graph_);
+	for (uint32_t form = 0; form < 4; ++form) {
+		if (exec_[form])
+			cudaGraphExecDestroy(exec_[form]);
+		if (graph_[form])
+			cudaGraphDestroy(graph_[form]);
+		exec_[form] = nullptr;
+		graph_[form] = nullptr;
+	}
 	cudaFree(d_desc_);
-	cudaFree(d_steps_);
-	cudaFreeHost(h_steps_);
-	cudaFree(d_lnl_);
 	cudaFreeHost(h_lnl_);
-	cudaFree(d_work_);
 	cudaFree(d_tile_sums_);
 	cudaFree(d_tickets_);
 	if (ev0_)
@@ -267,8 +275,6 @@ void Batch::release()
 		cudaStreamDestroy(stream2_);
 	ev_fork_ = ev_join_ = nullptr;
 	stream2_ = nullptr;
-	exec_ = nullptr;
-	graph_ = nullptr;
 	d_desc_ = nullptr;
 	d_steps_ = h_steps_ = nullptr;
 	d_lnl_ = h_lnl_ = nullptr;
@@ -279,10 +285,12 @@ void Batch::release()
 	stream_ = nullptr;
 }
 
-// A list that the short-list kernels take.
-bool Batch::short_list(const Calculator &c)
+// The kernel that takes a member's staged list.
+uint32_t Batch::kind_of(const Calculator &c)
 {
-	return c.staged_n_ <= kDirectMax && (c.C_ == 1 || c.C_ == 2 || c.C_ == 4);
+	if (c.staged_n_ <= kDirectMax && (c.C_ == 1 || c.C_ == 2 || c.C_ == 4))
+		return kListShort;
+	return c.staged_tree_ ? kListTree : kListRuns;
 }
 
 void Batch::run()
@@ -294,9 +302,9 @@ void Batch::run()
 	// long lists' tiles: the members' own size, halved while every tile still
 	// gets a block at once (a tile's serial chain of runs shortens with it:
 	// its entries are spread over more thread groups)
-	uint32_t tiles = 0, shrink = 0;
+	uint32_t tiles = 0, shrink = 0, form = 0;
 	for (Calculator *c : members_)
-		if (c->staged_ && !short_list(*c))
+		if (c->staged_ && kind_of(*c) == kListRuns)
 			tiles += c->ldp_ / c->staged_tile_;
 	while (tiles && (tiles << (shrink + 1)) <= ctas_)
 		++shrink;
@@ -312,14 +320,22 @@ void Batch::run()
 			s.tile = std::max(16u, c->staged_tile_ >> shrink);
 			s.tips_smem = c->staged_tips_smem_;
 			s.clock_rate = c->staged_clock_;
-			s.direct = short_list(*c) ? 1u : 0u;
+			s.kind = kind_of(*c);
+			if (s.kind == kListTree) {
+				s.tips_smem = c->tree_tips_;
+				s.groups = c->order_groups_;
+				s.phases = c->order_phases_;
+				s.n_slots = c->tree_slots_;
+				s.clean = c->tree_clean_ ? 1u : 0u;
+			}
+			form |= s.kind == kListRuns ? 1u : s.kind == kListTree ? 2u : 0u;
 			c->staged_ = false;
 		} else {
 			s.n = 0;
 			s.n_runs = 0;
 			s.tile = c->runs_tile_;
 			s.tips_smem = 0;
-			s.direct = 0;
+			s.kind = kListRuns;
 			s.clock_rate = 1.0;
 		}
 	}
@@ -329,7 +345,7 @@ void Batch::run()
 			check_cuda(cudaStreamSynchronize(c->stream_), "member stream");
 			c->stream_dirty_ = false;
 		}
-	check_cuda(cudaGraphLaunch(exec_, stream_), "graph launch");
+	check_cuda(cudaGraphLaunch(exec_[form], stream_), "graph launch");
 	// members wait for the replay before restaging
 	for (Calculator *c : members_) {
 		c->batch_done_ = ev1_;

@@ -35,8 +35,8 @@ class Batch {
 	unsigned *d_work_ = nullptr;
 	double *d_tile_sums_ = nullptr;
 	unsigned *d_tickets_ = nullptr;
-	cudaGraph_t graph_ = nullptr;
-	cudaGraphExec_t exec_ = nullptr;
+	cudaGraph_t graph_[4] = {};     // by the kernels a step needs (capture)
+	cudaGraphExec_t exec_[4] = {};
 	BatchParams bp_{};
 	uint32_t max_entries_ = 0, ctas_ = 0;
 	// one contiguous staging block for every member (copied by one graph
@@ -47,7 +47,8 @@ class Batch {
 	bool direct_c_[5] = {}; // members with 1, 2 or 4 categories present
 	bool ran_ = false, running_ = false; // running_: the last replay was not waited for
 	void wait();
-	static bool short_list(const Calculator &c);
+	static uint32_t kind_of(const Calculator &c);
+	void capture(uint32_t form);
 	std::vector<uint8_t> evaluated_;
 };
 

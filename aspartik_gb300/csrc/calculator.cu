@@ -821,6 +821,11 @@ uint32_t Calculator::pick_tree(uint32_t n)
 	pp.num_leaves = L_;
 	pp.tips_smem = 4ull * tip_children_ >= L_;
 	uint32_t G = 1;
+	if (tree_batch_) {
+		tree_tile_ = 64;
+		G = tree_groups_ ? tree_groups_ : std::max(1u, n / 8);
+		return std::min(G, 16u / C_);
+	}
 	for (uint32_t tile = ldp_ / 64u > num_sms_ ? 128u : 64u;; tile = 64u) {
 		if (tree_tile_fixed_)
 			tile = tree_tile_fixed_;
@@ -844,9 +849,28 @@ uint32_t Calculator::pick_tree(uint32_t n)
 	}
 }
 
+// Whether a batched list takes that walk: where its tips and slots fit a
+// block.  Us a step, run walk / depth first, every member a whole tree of 4
+// categories: 32 of 184 taxa x 1,172 patterns 276 / 183, 4 of 256 x 1,418 90 /
+// 72, 8 of 64 x 857 46 / 39, 2 of 256 x 285 61 / 58; 2 of 700 x 300, too large,
+// 114 / 132.
+bool Calculator::batch_tree(uint32_t n) const
+{
+	PruneParams pp{};
+	pp.C = C_;
+	pp.num_leaves = L_;
+	pp.tile = 64;
+	pp.tips_smem = 1;
+	pp.groups = std::min(std::max(1u, n / 8), 16u / C_);
+	pp.n_slots = 3 + 5 * pp.groups / 2;
+	return prune4_tree_smem(pp) <= kBatchTreeSmem;
+}
+
 // Shared memory of a block of that walk.
 uint32_t Calculator::tree_budget(uint32_t G) const
 {
+	if (tree_batch_)
+		return kBatchTreeSmem;
 	const uint32_t warps = tree_tile_ == 128 ? 12 : 16;
 	const uint32_t rounds = (ldp_ / tree_tile_ + num_sms_ - 1) / num_sms_;
 	return smem_budget(1024u / std::max(1u, std::min(warps / (G * C_), rounds)));
@@ -1590,9 +1614,13 @@ void Calculator::stage_lengths(const uint32_t *internals,
 	// so must this calculator's own last launch
 	wait_stage();
 	wait_batch();
-	stage_ops(internals, children, n, false);
+	tree_batch_ = true;
+	stage_ops(internals, children, n,
+		  use_tree_ && !(use_direct_ && n <= kDirectMax) && batch_tree(n));
+	tree_batch_ = false;
+	staged_tree_ = depth_first_;
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
-	std::memcpy(h_stage_ + off_in_, lengths, (size_t)n * 2 * sizeof(double));
+	stage_inputs(lengths, n, 2);
 	staged_ = true;
 	staged_n_ = n;
 	staged_clock_ = clock_rate;

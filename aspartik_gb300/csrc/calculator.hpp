@@ -181,9 +181,10 @@ class Calculator {
 	// the four-state FP32 form's depth-first walk of single-tree lists
 	// (B3G_TREE=0: the run walk), and the staged list's shared-memory slots
 	bool use_tree_ = false, tree_always_ = false;
+	bool staged_tree_ = false; // the batch's staged list takes it
 	uint32_t tree_slots_ = 0, tree_tips_ = 0, tree_groups_ = 0, tree_tile_ = 64;
 	uint32_t tree_tile_fixed_ = 0;
-	bool tree_clean_ = false;
+	bool tree_clean_ = false, tree_batch_ = false; // (staging for a batch)
 	std::vector<uint32_t> tree_order_, tree_ends_;
 	std::vector<uint8_t> tree_swap_; // staged entry: first child is the right one
 	std::vector<std::vector<uint8_t>> tree_pools_;
@@ -247,6 +248,7 @@ class Calculator {
 	uint32_t pick_groups(uint32_t n);
 	uint32_t pick_tree(uint32_t n);
 	uint32_t tree_budget(uint32_t groups) const;
+	bool batch_tree(uint32_t n) const;
 	uint32_t pick_p20_groups(uint32_t n) const;
 	uint32_t s20_groups_ = 0; // 20-state FP32 walk; 0: chosen per list
 	uint32_t s20_per_sm_[5] = {}; // blocks an SM holds, by warps a block

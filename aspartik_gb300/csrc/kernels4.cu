@@ -1072,6 +1072,16 @@ cudaError_t launch_ptab4_batch(const BatchParams &p, uint32_t max_entries,
 	return cudaGetLastError();
 }
 
+cudaError_t launch_prune4_tree_batch(const BatchParams &p, uint32_t ctas, cudaStream_t s)
+{
+	static SmemOptIn opted;
+	const cudaError_t e = opt_in_smem(prune4_tree_batch_kernel, opted);
+	if (e != cudaSuccess)
+		return e;
+	prune4_tree_batch_kernel<<<ctas, 512, kBatchTreeSmem, s>>>(p);
+	return cudaGetLastError();
+}
+
 cudaError_t launch_prune4_batch(const BatchParams &p, uint32_t ctas,
 				cudaStream_t s)
 {

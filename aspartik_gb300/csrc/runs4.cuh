@@ -1005,6 +1005,50 @@ prune4_direct_kernel(const __grid_constant__ DirectParams prm)
 	}
 }
 
+constexpr uint32_t kBatchMembers = 256;
+
+// prefix[m] = items of the members before m, for m up to M, by warp 0; ends
+// with the block synchronised.  (One thread adding them up waited for a load a
+// member: the short-list kernel of 32 members took 45 us, now 33.)
+template <typename F>
+__device__ __forceinline__ void member_prefix(uint32_t M, uint32_t *prefix, F items)
+{
+	if (threadIdx.x < 32) {
+		uint32_t before = 0;
+		for (uint32_t m0 = 0; m0 < M; m0 += 32) {
+			const uint32_t m = m0 + threadIdx.x;
+			const uint32_t mine = m < M ? items(m) : 0u;
+			uint32_t sum = mine;
+			for (uint32_t off = 1; off < 32; off *= 2) {
+				const uint32_t v = __shfl_up_sync(0xffffffffu, sum, off);
+				sum += threadIdx.x >= off ? v : 0u;
+			}
+			if (m < M)
+				prefix[m] = before + sum - mine;
+			before += __shfl_sync(0xffffffffu, sum, 31);
+		}
+		if (threadIdx.x == 0)
+			prefix[M] = before;
+	}
+	__syncthreads();
+}
+
+// The member whose items hold w.
+__device__ __forceinline__ uint32_t member_of(const uint32_t *prefix, uint32_t M, uint32_t w)
+{
+	uint32_t lo = 0, hi = M;
+	while (hi - lo > 1) {
+		const uint32_t mid = (lo + hi) >> 1;
+		if (prefix[mid] <= w)
+			lo = mid;
+		else
+			hi = mid;
+	}
+	while (lo + 1 < M && prefix[lo + 1] <= w)
+		++lo;
+	return lo;
+}
+
 // Batched short lists: persistent blocks take (member, 128-pattern tile)
 // items of the members whose step is direct and has kC categories from
 // their own counter (work_next[1], [2], [3] for 4, 2, 1 categories;
@@ -1020,7 +1064,6 @@ __global__ void __launch_bounds__(kDirectThreads<kC>, 8 / kC)
 prune4_direct_batch_kernel(BatchParams bp)
 {
 	constexpr uint32_t kTile = 128;
-	constexpr uint32_t kMaxMembers = 256;
 	extern __shared__ __align__(16) unsigned char direct_smem[];
 	const DirectSmem<kC, kBatchAhead> sm(direct_smem, kDirectMax);
 	NodeOp *const s_ops = sm.ops;
@@ -1028,49 +1071,36 @@ prune4_direct_batch_kernel(BatchParams bp)
 	__shared__ double s_rate[kC];
 	__shared__ float s_pi[4];
 	__shared__ double s_red[32];
-	__shared__ uint32_t s_prefix[kMaxMembers + 1];
+	__shared__ uint32_t s_prefix[kBatchMembers + 1];
 	__shared__ uint32_t s_work;
 	__shared__ unsigned s_last;
 	const uint32_t tid = threadIdx.x;
 	const uint32_t M = bp.num_members;
-	if (tid == 0) {
-		uint32_t acc = 0;
-		for (uint32_t m = 0; m < M; ++m) {
-			s_prefix[m] = acc;
-			const MemberStep &st = bp.steps[m];
-			if (st.n && st.direct && bp.members[m].C == kC)
-				acc += bp.members[m].ldp / kTile;
-		}
-		s_prefix[M] = acc;
-	}
-	__syncthreads();
+	member_prefix(M, s_prefix, [&](uint32_t m) {
+		const MemberStep &st = bp.steps[m];
+		return st.n && st.kind == kListShort && bp.members[m].C == kC
+			       ? bp.members[m].ldp / kTile
+			       : 0u;
+	});
 	const uint32_t total = s_prefix[M];
 	uint32_t cur = 0xFFFFFFFFu, n = 0;
 	const MemberDesc *md = nullptr;
 	double log_inv_c = 0.0;
 	// items come in chunks of consecutive tiles (mostly of one member), so
-	// that a block rebuilds a member's tables less often
-	constexpr uint32_t kChunk = 4;
+	// that a block rebuilds a member's tables less often: as many as a block
+	// gets, at most four (30 members of 13 tiles on 304 blocks, this kernel
+	// alone: 65 us with always four, 45 with two)
+	const uint32_t chunk = min(4u, max(1u, (total + gridDim.x - 1u) / gridDim.x));
 	for (;;) {
 		if (tid == 0)
-			s_work = atomicAdd(bp.work_next + (kC == 4 ? 1 : kC == 2 ? 2 : 3), kChunk);
+			s_work = atomicAdd(bp.work_next + (kC == 4 ? 1 : kC == 2 ? 2 : 3), chunk);
 		__syncthreads();
 		const uint32_t w0 = s_work;
 		__syncthreads();
 		if (w0 >= total)
 			break;
-	for (uint32_t w = w0; w < min(w0 + kChunk, total); ++w) {
-		uint32_t lo = 0, hi = M;
-		while (hi - lo > 1) {
-			const uint32_t mid = (lo + hi) >> 1;
-			if (s_prefix[mid] <= w)
-				lo = mid;
-			else
-				hi = mid;
-		}
-		while (lo + 1 < M && s_prefix[lo + 1] <= w)
-			++lo;
-		const uint32_t m = lo, t = w - s_prefix[m];
+	for (uint32_t w = w0; w < min(w0 + chunk, total); ++w) {
+		const uint32_t m = member_of(s_prefix, M, w), t = w - s_prefix[m];
 		md = &bp.members[m];
 		if (m != cur) {
 			const MemberStep st = bp.steps[m];
@@ -1173,7 +1203,7 @@ __global__ void __launch_bounds__(32) ptab4_batch_kernel(BatchParams bp)
 {
 	const uint32_t m = blockIdx.y;
 	const MemberStep st = bp.steps[m];
-	if (st.n == 0 || st.direct)
+	if (st.n == 0 || st.kind == kListShort)
 		return;
 	const MemberDesc &md = bp.members[m];
 	const uint32_t C = md.C;
@@ -1201,8 +1231,7 @@ __global__ void __launch_bounds__(32) ptab4_batch_kernel(BatchParams bp)
 template <typename Idx>
 __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 {
-	constexpr uint32_t kMaxMembers = 256;
-	__shared__ uint32_t s_prefix[kMaxMembers + 1];
+	__shared__ uint32_t s_prefix[kBatchMembers + 1];
 	__shared__ uint32_t s_work;
 	__shared__ unsigned s_last;
 	extern __shared__ double smem[];
@@ -1216,16 +1245,10 @@ __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 	float4 *s_ptab = (float4 *)(((uintptr_t)s_tips + bp.smem_tips_bytes + 15) &
 				    ~(uintptr_t)15);
 
-	if (tid == 0) {
-		uint32_t acc = 0;
-		for (uint32_t m = 0; m < M; ++m) {
-			s_prefix[m] = acc;
-			if (bp.steps[m].n && !bp.steps[m].direct)
-				acc += bp.members[m].ldp / bp.steps[m].tile;
-		}
-		s_prefix[M] = acc;
-	}
-	__syncthreads();
+	member_prefix(M, s_prefix, [&](uint32_t m) {
+		const MemberStep &st = bp.steps[m];
+		return st.n && st.kind == kListRuns ? bp.members[m].ldp / st.tile : 0u;
+	});
 	const uint32_t total = s_prefix[M];
 	uint32_t cur = 0xFFFFFFFFu;
 	TileArgs a;
@@ -1238,18 +1261,7 @@ __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 		__syncthreads();
 		if (w >= total)
 			break;
-		// the member whose tile range holds w
-		uint32_t lo = 0, hi = M;
-		while (hi - lo > 1) {
-			const uint32_t mid = (lo + hi) >> 1;
-			if (s_prefix[mid] <= w)
-				lo = mid;
-			else
-				hi = mid;
-		}
-		while (lo + 1 < M && s_prefix[lo + 1] <= w)
-			++lo;
-		const uint32_t m = lo, t = w - s_prefix[m];
+		const uint32_t m = member_of(s_prefix, M, w), t = w - s_prefix[m];
 		const MemberDesc &md = bp.members[m];
 		if (m != cur) {
 			const MemberStep st = bp.steps[m];

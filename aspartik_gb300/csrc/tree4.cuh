@@ -99,7 +99,9 @@ __device__ __forceinline__ void apply_rows(const float4 *tab, float4 (&x)[kV])
 		x[v] = v4_apply(r, x[v]);
 }
 
-// Block = `groups` x C warps, 64 kR patterns (lane l: 2l and 2l + 1 of every
+// One tile of a list: returns its weighted site sum in thread 0, the block
+// synchronised.  Block = `groups` x C warps (further ones only keep the
+// barriers), 64 kR patterns (lane l: 2l and 2l + 1 of every
 // 64).  Dynamic shared memory: [dot: C x tile floats][cnt: C x tile][a part a
 // category: its groups' rings, its slots' vectors (for every 64 columns the
 // even ones, then the odd ones), their counts][tips: num_leaves + 1 rows,
@@ -113,14 +115,13 @@ __device__ __forceinline__ void apply_rows(const float4 *tab, float4 (&x)[kV])
 // each column, the codes of a slot child being the lane's place in it (the
 // row behind the last leaf's).
 template <uint32_t kR, bool kTips, bool kClean>
-__global__ void __launch_bounds__(512) prune4_tree_kernel(PruneParams prm)
+__device__ __forceinline__ double tree_tile(const PruneParams &prm, uint32_t t, double *smem)
 {
-	extern __shared__ __align__(16) double smem[];
 	const uint32_t C = prm.C, G = prm.groups;
 	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
 	const uint32_t g = wid / C, c = wid - g * C;
 	constexpr uint32_t kTreeTile = 64 * kR;
-	const uint32_t p0 = blockIdx.x * kTreeTile;
+	const uint32_t p0 = t * kTreeTile;
 	float *s_dot = (float *)smem;
 	int32_t *s_cnt = (int32_t *)(s_dot + C * kTreeTile);
 	const uint32_t part_bytes = G * kTreeRingBytes + prm.n_slots * (kTreeTile * kTreeColBytes);
@@ -131,8 +132,14 @@ __global__ void __launch_bounds__(512) prune4_tree_kernel(PruneParams prm)
 	int2 *sc = (int2 *)(base + G * kTreeRingBytes + prm.n_slots * (kTreeTile * 16u)) + lane;
 
 	// segs: first entry of every group, n, then the groups' heads
-	const uint32_t first = prm.segs[g], count = prm.segs[g + 1] - first;
-	const TreeHead head = ((const TreeHead *)(prm.segs + G + 1))[g];
+	const bool walks = g < G;
+	const uint32_t first = walks ? prm.segs[g] : 0u;
+	const uint32_t count = walks ? prm.segs[g + 1] - first : 0u;
+	TreeHead head{};
+	if (walks)
+		head = ((const TreeHead *)(prm.segs + G + 1))[g];
+	else
+		head.barriers = prm.phases - 1;
 	const size_t col = (size_t)c * prm.ldp + p0 + 2 * lane;
 	const uint32_t stride = C * prm.ldp;
 	float4 *part = (float4 *)prm.partials + col;
@@ -398,10 +405,77 @@ __global__ void __launch_bounds__(512) prune4_tree_kernel(PruneParams prm)
 			s_red[h] = sum;
 	}
 	__syncthreads();
-	if (threadIdx.x == 0) {
-		double sum = 0.0;
-		for (uint32_t h = 0; h < 2 * kR; ++h)
-			sum += s_red[h];
+	double sum = 0.0;
+	for (uint32_t h = 0; h < 2 * kR; ++h)
+		sum += s_red[h];
+	return sum;
+}
+
+template <uint32_t kR, bool kTips, bool kClean>
+__global__ void __launch_bounds__(512) prune4_tree_kernel(PruneParams prm)
+{
+	extern __shared__ __align__(16) double smem[];
+	const double sum = tree_tile<kR, kTips, kClean>(prm, blockIdx.x, smem);
+	if (threadIdx.x == 0)
 		prm.sums_host[blockIdx.x] = sum;
+}
+
+// The long single-tree lists of a batch, 64 patterns and as many groups as a
+// block of 16 warps has: two lists of 183 entries x 1,664 patterns x 4
+// categories 37 us on 52 SMs, where the run walk's tiles took 62 us on all of
+// them; the short lists' blocks run on the others meanwhile (a step of 32
+// chains, two whole trees and 30 paths, 105 -> 69 us on the device).
+__global__ void __launch_bounds__(512) prune4_tree_batch_kernel(BatchParams bp)
+{
+	extern __shared__ __align__(16) double smem[];
+	__shared__ uint32_t s_prefix[kBatchMembers + 1];
+	__shared__ unsigned s_last;
+	const uint32_t M = bp.num_members;
+	member_prefix(M, s_prefix, [&](uint32_t m) {
+		const MemberStep &st = bp.steps[m];
+		return st.n && st.kind == kListTree ? bp.members[m].ldp / 64u : 0u;
+	});
+	const uint32_t total = s_prefix[M];
+	for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
+		const uint32_t m = member_of(s_prefix, M, w), t = w - s_prefix[m];
+		const MemberDesc &md = bp.members[m];
+		const MemberStep &st = bp.steps[m];
+		PruneParams prm{};
+		prm.tips = md.tips;
+		prm.partials = md.partials;
+		prm.scales = md.scales;
+		prm.ops = (const NodeOp *)(md.stage + md.off_tree);
+		prm.ptab = md.ptab;
+		prm.segs = (const uint32_t *)(md.stage + md.off_runs);
+		prm.groups = st.groups;
+		prm.phases = st.phases;
+		prm.pi = (const double *)(md.stage + md.off_pi);
+		prm.weights = md.weights;
+		prm.site_lnl = md.site_lnl;
+		prm.n = st.n;
+		prm.ldp = md.ldp;
+		prm.C = md.C;
+		prm.num_leaves = md.L;
+		prm.n_slots = st.n_slots;
+		prm.log_inv_c = md.log_inv_c;
+		const double sum = !st.tips_smem ? tree_tile<1, false, true>(prm, t, smem)
+				   : st.clean    ? tree_tile<1, true, true>(prm, t, smem)
+						 : tree_tile<1, true, false>(prm, t, smem);
+		const uint32_t tiles = md.ldp / 64u;
+		if (threadIdx.x == 0) {
+			md.tile_sums[t] = sum;
+			__threadfence();
+			s_last = atomicAdd(md.ticket, 1u) == tiles - 1u;
+		}
+		__syncthreads();
+		if (s_last) {
+			__threadfence();
+			const double lnl = block_fold(md.tile_sums, tiles, nullptr);
+			if (threadIdx.x == 0) {
+				bp.lnl_out[m] = lnl;
+				*md.ticket = 0u;
+			}
+		}
+		__syncthreads();
 	}
 }

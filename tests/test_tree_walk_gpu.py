@@ -71,6 +71,54 @@ def test_forms_agree(taxa, sites, K, alpha, monkeypatch):
             assert np.isfinite(l0) and abs(l1 - l0) <= 1e-13 * abs(l0)
 
 
+def test_batched_lists(monkeypatch):
+    """Whole trees and paths of members of several sizes in one batch, walked
+    depth first there, against calculators of their own on the run walk: sums
+    of the same bits per pattern, to 1e-13."""
+    from aspartik_gb300.calculator import Batch
+    shapes = [(60, 300, 4, 0.5), (53, 129, 1, None), (80, 700, 5, 0.6), (150, 64, 16, 0.5),
+              (260, 500, 3, 0.4), (9, 200, 2, 0.5), (700, 40, 4, 0.7)]
+    cases = [dna_case(t, s, seed=t, model="gtr", root_height=1.5, alpha=a, num_categories=K)
+             for t, s, K, a in shapes]
+
+    def make(batched):
+        monkeypatch.setenv("B3G_TREE", "1" if batched else "0")
+        out = []
+        for c, (_, _, K, a) in zip(cases, shapes):
+            g = make_gpu(c.leaves, c.weights, K, "f32")
+            g.set_reversible(c.rates, c.pi)
+            if K > 1:
+                g.set_gamma(a)
+            out.append(g)
+        return out
+
+    alone, members = make(False), make(True)
+    batch = Batch(members)
+    trees = [O.DatedTree(c.tree.parents, c.tree.heights.copy()) for c in cases]
+    for t in trees:
+        t.mark_all_edges_updated()
+    rng = np.random.default_rng(3)
+    for step in range(4):
+        want = []
+        for g, m, t in zip(alone, members, trees):
+            lists = lists_and_lengths(t)
+            g.propose_lengths(*lists, 1.0)
+            want.append(g.log_likelihood())
+            m.stage_lengths(*lists, 1.0)
+        batch.run()
+        got = batch.log_likelihoods()
+        for lnl, l in zip(want, got):
+            assert abs(l - lnl) <= 1e-13 * abs(lnl)
+        for g, m, t in zip(alone, members, trees):
+            g.accept()
+            m.accept()
+            t.accept()
+            if step == 1:
+                t.mark_all_edges_updated()
+            else:
+                random_move(t, rng)
+
+
 def test_impossible_patterns(monkeypatch):
     """Patterns of likelihood zero (identity matrices under different bases)
     give -inf."""
