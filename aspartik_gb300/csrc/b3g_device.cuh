@@ -103,6 +103,8 @@ struct PtabParams {
 	void *soft20;   // [n][2][C] beside the 20-state ones (SoftTab20)
 };
 
+constexpr uint32_t kScalePow = 8;
+
 struct PruneParams {
 	const uint8_t *tips;
 	void *partials;
@@ -165,6 +167,9 @@ struct PruneParams {
 	uint32_t lengths_smem; // stage the lengths in shared memory
 	double scale_threshold;
 	double scale_mult;
+	// e^(-scale_ln d) for d = 1 ..., or zeros: the FP64 form's root mixes the
+	// categories with them
+	double scale_pow[kScalePow];
 	double log_inv_c;
 };
 

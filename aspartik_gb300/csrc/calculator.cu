@@ -90,6 +90,8 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	C_ = cfg.num_categories;
 	f32_ = cfg.precision == B3G_PRECISION_F32;
 	scale_ln_ = cfg.scale_ln;
+	for (uint32_t d = 0; d < kScalePow; ++d)
+		scale_pow_[d] = std::exp(-static_cast<double>(scale_ln_) * (d + 1));
 	device_ = cfg.device;
 	ldp_ = static_cast<uint32_t>(align_up(P_, kPatternAlign));
 	// patterns per block: 128 threads for up to 4 categories, one warp of
@@ -1256,6 +1258,7 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 				       : 0u;
 	pp.scale_threshold = std::exp(-static_cast<double>(scale_ln_));
 	pp.scale_mult = std::exp(static_cast<double>(scale_ln_));
+	std::copy(scale_pow_, scale_pow_ + kScalePow, pp.scale_pow);
 	pp.log_inv_c = std::log(1.0 / static_cast<double>(C_));
 	// the run-synchronous walk stages the schedule in shared memory: keep
 	// it for lists up to 4,096 entries
@@ -1420,6 +1423,7 @@ void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 	pp.num_leaves = L_;
 	pp.scale_threshold = std::exp(-static_cast<double>(scale_ln_));
 	pp.scale_mult = std::exp(static_cast<double>(scale_ln_));
+	std::copy(scale_pow_, scale_pow_ + kScalePow, pp.scale_pow);
 	pp.log_inv_c = std::log(1.0 / static_cast<double>(C_));
 	pp.root_val = d_root_val_;
 	pp.root_exp = d_root_exp_;

@@ -148,6 +148,7 @@ class Calculator {
 	uint32_t L_ = 0, I_ = 0, P_ = 0, ldp_ = 0, S_ = 0, C_ = 0, tile_ = 0;
 	bool f32_ = false;
 	uint32_t scale_ln_ = 0;
+	double scale_pow_[kScalePow] = {}; // e^(-scale_ln d)
 	int device_ = -1;
 
 	// host state

@@ -526,16 +526,22 @@ __device__ __forceinline__ void neumaier_merge(double &sum, double &comp,
 // negative, NaN or infinite one -> NaN.
 template <typename Value, typename Count>
 __device__ __forceinline__ double mix_categories_f64(uint32_t C, Value value, Count count,
-						     uint32_t scale_ln, double log_inv_c)
+						     uint32_t scale_ln, double log_inv_c,
+						     const double *scale_pow,
+						     const double *known_log = nullptr)
 {
 	constexpr long long kInf = 0x7FF0000000000000ll;
-	uint32_t least = 0xFFFFFFFFu;
+	uint32_t least = 0xFFFFFFFFu, least_count = 0;
 	bool any = false, bad = false;
 	for (uint32_t k = 0; k < C; k++) {
 		const long long u = __double_as_longlong(value(k));
 		if (u > 0 && u <= kInf) {
 			any = true;
-			least = min(least, (uint32_t)count(k) * scale_ln);
+			const uint32_t n = (uint32_t)count(k);
+			if (n * scale_ln <= least) {
+				least = n * scale_ln;
+				least_count = n;
+			}
 		}
 		bad = bad || u >= kInf || (u < 0 && (u << 1) != 0);
 	}
@@ -545,12 +551,21 @@ __device__ __forceinline__ double mix_categories_f64(uint32_t C, Value value, Co
 		for (uint32_t k = 0; k < C; k++) {
 			double v = value(k);
 			const uint32_t steps = (uint32_t)count(k) * scale_ln;
-			if (steps > least) // zero or scaled further
-				v *= exp((double)least - (double)steps);
+			if (steps > least) { // zero or scaled further
+				const uint32_t d = (uint32_t)count(k) - least_count;
+				double f = 0.0;
+				if (d - 1u < kScalePow && d * scale_ln == steps - least)
+					f = scale_pow[d - 1u];
+				if (f == 0.0) // further apart, or no table
+					f = exp((double)least - (double)steps);
+				v *= f;
+			}
 			acc += v;
 		}
 	}
-	return !any ? -INFINITY : bad ? NAN : log(acc) - (double)least + log_inv_c;
+	return !any ? -INFINITY
+	       : bad ? NAN
+		     : (known_log ? *known_log : log(acc)) - (double)least + log_inv_c;
 }
 
 // The same for values with power-of-two exponents: sum_c s_c 2^E_c =
@@ -566,8 +581,13 @@ __device__ __forceinline__ double mix_categories_pow2(uint32_t C, Value value, C
 	if (emax == INT32_MIN)
 		return -INFINITY;
 	double acc = 0.0;
-	for (uint32_t k = 0; k < C; k++)
-		acc += scalbn(value(k), (int32_t)count(k) - emax);
+	for (uint32_t k = 0; k < C; k++) {
+		// by one exact product where the power is a normal number
+		const int32_t e = (int32_t)count(k) - emax;
+		acc += e <= 0 && e > -1000
+			       ? value(k) * __hiloint2double((1023 + e) << 20, 0)
+			       : scalbn(value(k), e);
+	}
 	return log(acc) + (double)emax * 0.69314718055994530942 + log_inv_c;
 }
 
@@ -583,7 +603,12 @@ __device__ __forceinline__ double mix_categories_pow2(uint32_t C, Value value, C
 // logarithm a pattern: an FP64 logarithm or exponential is 30 to 40
 // instructions of 64 cycles each here, and a logarithm a category, an
 // exponential a category and a logarithm on top (the log-sum-exp this
-// equals) took 15,000 to 20,000 cycles of a launch against 4,000.
+// equals) took 15,000 to 20,000 cycles of a launch.  The factors of the sum
+// are powers of e^-scale_ln and come as parameters (as exponentials, one
+// after another for the categories scaled further, they were 5,300 of the
+// root's 10,800 cycles; an FP64 dirty path of 8 entries, 64 taxa x 7,855
+// patterns x 4 categories: 21.2 -> 19.1 us).  With one category the logarithm
+// of its value is the site's too.
 template <bool kPow2>
 __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem,
 					    uint32_t tp, uint32_t pl, uint32_t p0,
@@ -597,6 +622,7 @@ __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem
 	double *s_warp = smem + 2 * nthr;             // [32]
 	__shared__ unsigned s_last;
 
+	double col_log = 0.0;
 	if (lead) {
 		s_val[c * tp + pl] = root_dot;
 		s_exp[c * tp + pl] = cnt;
@@ -606,13 +632,15 @@ __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem
 			const double off =
 				kPow2 ? (double)cnt * 0.69314718055994530942
 				      : -(double)((uint32_t)cnt * prm.scale_ln);
-			prm.cat_lnl[(size_t)c * ldp + p0 + pl] = log(root_dot) + off;
+			col_log = log(root_dot);
+			prm.cat_lnl[(size_t)c * ldp + p0 + pl] = col_log + off;
 		}
 	}
-	__syncthreads();
-
 	const uint32_t tid =
 		(threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+	const uint32_t w = tid < tp ? prm.weights[p0 + tid] : 0u;
+	__syncthreads();
+
 	const uint32_t lane = tid & 31u, warp = tid >> 5;
 	double contrib = 0.0;
 	if (tid < tp) {
@@ -626,10 +654,11 @@ __device__ __forceinline__ void finish_root(const PruneParams &prm, double *smem
 			site = mix_categories_f64(
 				C, [&](uint32_t k) { return s_val[k * tp + tid]; },
 				[&](uint32_t k) { return s_exp[k * tp + tid]; },
-				prm.scale_ln, prm.log_inv_c);
+				prm.scale_ln, prm.log_inv_c, prm.scale_pow,
+				// one category: thread tid was its pattern's lead
+				C == 1 && prm.cat_lnl ? &col_log : nullptr);
 		}
 		prm.site_lnl[p0 + tid] = site;
-		const uint32_t w = prm.weights[p0 + tid];
 		contrib = w ? site * (double)w : 0.0;
 	}
 

@@ -107,6 +107,31 @@ __global__ void __launch_bounds__(kS20 *kS20) ptab20_kernel(PtabParams prm)
 	}
 }
 
+// The C <= 8 categories' root values and counts of pattern p, read together
+// (they are used three times over) into this thread's shared-memory words: at
+// [k * pitch] of `words`, the counts behind 8 * pitch doubles.
+struct RootColumns {
+	double *v;
+	uint32_t pitch;
+	__device__ RootColumns(const PruneParams &prm, uint32_t p, double *words, uint32_t pitch_)
+	    : v(words), pitch(pitch_)
+	{
+#pragma unroll 4
+		for (uint32_t k = 0; k < prm.C; ++k) {
+			const size_t at = (size_t)k * prm.ldp + p;
+			const double x = __ldcg(prm.root_val + at);
+			const int32_t n = __ldcg(prm.root_exp + at);
+			v[k * pitch] = x;
+			((int32_t *)(v + (8 + k) * pitch))[0] = n;
+		}
+	}
+	__device__ double val(uint32_t k) const { return v[k * pitch]; }
+	__device__ int32_t exp(uint32_t k) const
+	{
+		return ((const int32_t *)(v + (8 + k) * pitch))[0];
+	}
+};
+
 // ---------------------------------------------------------------------------
 // FP32 walk with register matrix instructions.
 //
@@ -525,10 +550,10 @@ __global__ void __launch_bounds__(128, 3) prune20_kernel(PruneParams prm)
 	__syncwarp();
 	if (!s_last)
 		return;
+	const RootColumns root(prm, p, (double *)s20_smem + lane, 32);
 	const double site = mix_categories_pow2(
-		C, [&](uint32_t k) { return __ldcg(prm.root_val + (size_t)k * ldp + p); },
-		[&](uint32_t k) { return __ldcg(prm.root_exp + (size_t)k * ldp + p); },
-		prm.log_inv_c);
+		C, [&](uint32_t k) { return root.val(k); },
+		[&](uint32_t k) { return root.exp(k); }, prm.log_inv_c);
 	prm.site_lnl[p] = site;
 	const uint32_t w = prm.weights[p];
 	double contrib = w ? site * (double)w : 0.0;

@@ -379,10 +379,11 @@ __global__ void __launch_bounds__(512) prune20_f64_kernel(PruneParams prm)
 	double contrib = 0.0;
 	if (threadIdx.x < kP20Tile) {
 		const uint32_t p = p0 + threadIdx.x;
+		const RootColumns root(prm, p, (double *)p20_smem + threadIdx.x, kP20Tile);
 		double site = mix_categories_f64(
-			C, [&](uint32_t k) { return __ldcg(prm.root_val + (size_t)k * ldp + p); },
-			[&](uint32_t k) { return __ldcg(prm.root_exp + (size_t)k * ldp + p); },
-			prm.scale_ln, prm.log_inv_c);
+			C, [&](uint32_t k) { return root.val(k); },
+			[&](uint32_t k) { return root.exp(k); }, prm.scale_ln, prm.log_inv_c,
+			prm.scale_pow);
 		prm.site_lnl[p] = site;
 		const uint32_t wgt = prm.weights[p];
 		contrib = wgt ? site * (double)wgt : 0.0;
