@@ -1161,10 +1161,13 @@ cudaError_t launch_prune4_direct_batch(const BatchParams &p, uint32_t C,
 cudaError_t launch_ptab20(const PtabParams &p, bool f32, cudaStream_t s)
 {
 	const uint32_t tables = p.n * 2u * p.C;
-	if (f32)
-		ptab20_kernel<float><<<tables, kS20 * kS20, 0, s>>>(p);
+	if (!f32)
+		ptab20_kernel<double, 1><<<tables, kS20 * kS20, 0, s>>>(p);
+	// (FP32) four blocks a table up to two blocks an SM of a 152-SM part
+	else if (4 * tables <= 304)
+		ptab20_kernel<float, 4><<<4 * tables, kS20 * kS20 / 4, 0, s>>>(p);
 	else
-		ptab20_kernel<double><<<tables, kS20 * kS20, 0, s>>>(p);
+		ptab20_kernel<float, 1><<<tables, kS20 * kS20, 0, s>>>(p);
 	return cudaGetLastError();
 }
 

@@ -39,61 +39,67 @@ __device__ __forceinline__ void soft20_store(SoftTab20 *dst, uint32_t k, uint32_
 }
 
 
-// Element (i, j) = (t / 20, t % 20) of the P(t) of table `id` = (entry * 2 +
-// side) * C + category, by thread t < 400 of a block of at least 400 (every
-// thread calls: the block synchronises).  V diag(e) is formed once per table
-// in shared memory, so an element costs 20 FP64 multiply-adds instead of 20
-// products more (the FP64 pipe, 64 cycles an instruction and scheduler
-// partition, bounds this kernel).
+// Element base + t = (i, j) of the P(t) of table `id` = (entry * 2 + side) * C
+// + category, row by row, by thread t < count (whole rows) of a block of at
+// least 20 threads (every thread calls: the block synchronises).  V diag(e) is
+// formed once per table in shared memory, so an element costs 20 FP64
+// multiply-adds instead of 20 products more (the FP64 pipe, 64 cycles an
+// instruction and scheduler partition, bounds this kernel).
 struct Ptab20Smem {
 	double e[kS20];
 	double Ve[kS20 * kS20];
 };
 __device__ __forceinline__ double ptab20_element(const PtabParams &prm, uint32_t id, uint32_t t,
-						 Ptab20Smem &sm)
+						 Ptab20Smem &sm, uint32_t base = 0,
+						 uint32_t count = kS20 * kS20)
 {
 	constexpr uint32_t S = kS20;
 	const uint32_t c = id % prm.C, es = id / prm.C;
 	const ModelDev *m = prm.model;
-	const uint32_t i = t / S, j = t - i * S;
+	const uint32_t i = (base + t) / S, j = (base + t) - i * S;
 	if (prm.matrices)
-		return t < S * S ? prm.matrices[(size_t)id * S * S + t] : 0.0;
+		return t < count ? prm.matrices[(size_t)id * S * S + base + t] : 0.0;
 	const double d = prm.lengths[es] * (prm.clock_rate * m->cat_rates[c]);
 	if (m->shortcuts && d > 20.0) // transition_freqs (substitution.rs:245-252)
-		return t < S * S ? m->pi[j] : 0.0;
+		return t < count ? m->pi[j] : 0.0;
 	if (m->shortcuts && d < 1e-10) // transition_q (substitution.rs:258-268)
-		return t >= S * S ? 0.0 : i == j ? 1.0 : m->Q[i * S + j] * d;
+		return t >= count ? 0.0 : i == j ? 1.0 : m->Q[i * S + j] * d;
 	if (t < S)
 		sm.e[t] = exp(m->lambda[t] * d);
 	__syncthreads();
-	if (t < S * S)
-		sm.Ve[t] = m->V[t] * sm.e[j];
+	if (t < count)
+		sm.Ve[t] = m->V[base + t] * sm.e[j];
 	__syncthreads();
-	if (t >= S * S)
+	if (t >= count)
 		return 0.0;
+	const double *Ve = sm.Ve + (t - j);
 	double s = 0.0;
 #pragma unroll
 	for (uint32_t k = 0; k < S; k++)
-		s = fma(sm.Ve[i * S + k], m->Vinv[k * S + j], s);
+		s = fma(Ve[k], m->Vinv[k * S + j], s);
 	return s;
 }
 
-// One block per table, one thread per element, computed in FP64 (the same
-// for both forms: the FP32 form only stores it in single precision) and
-// written transposed with a 21st row of ones; the FP64 form's integer table
-// beside it.
-template <typename R>
-__global__ void __launch_bounds__(kS20 *kS20) ptab20_kernel(PtabParams prm)
+// One thread per element, computed in FP64 (the same for both forms: the FP32
+// form only stores it in single precision) and written transposed with a 21st
+// row of ones; the FP64 form's integer table beside it.  A table is one block,
+// or in the FP32 form kParts blocks of 20 / kParts rows each where the list's
+// tables would leave SMs idle (64 tables of a path of 8 entries: 7.5 -> 6.7 us
+// beside 2.2 of an empty event pair; an evaluation 39.2 -> 37.5 us).
+template <typename R, uint32_t kParts>
+__global__ void __launch_bounds__(kS20 *kS20 / kParts) ptab20_kernel(PtabParams prm)
 {
-	constexpr uint32_t S = kS20;
+	constexpr uint32_t S = kS20, kCount = S * S / kParts;
+	static_assert(kParts == 1 || sizeof(R) == 4, "the integer table's flag is one block's");
 	if constexpr (sizeof(R) == 8)
 		tables_started();
 	__shared__ Ptab20Smem sm;
-	const uint32_t id = blockIdx.x, t = threadIdx.x, i = t / S, j = t - i * S;
-	const double P = ptab20_element(prm, id, t, sm);
+	const uint32_t id = blockIdx.x / kParts, base = (blockIdx.x % kParts) * kCount;
+	const uint32_t t = threadIdx.x, i = (base + t) / S, j = (base + t) - i * S;
+	const double P = ptab20_element(prm, id, t, sm, base, kCount);
 	R *out = (R *)prm.ptab + (size_t)id * (S + 1) * S;
 	out[j * S + i] = (R)P;
-	if (t < S)
+	if (t < S && base == 0)
 		out[S * S + t] = (R)1.0;
 	if constexpr (sizeof(R) == 8) {
 		SoftTab20 *st = (SoftTab20 *)prm.soft20 + id;
@@ -514,6 +520,13 @@ __global__ void __launch_bounds__(128, 3) prune20_kernel(PruneParams prm)
 	}
 	double *root_val = prm.root_val + (size_t)c * ldp + p0;
 	int32_t *root_exp = prm.root_exp + (size_t)c * ldp + p0;
+	double pi[3][2]; // read together
+#pragma unroll
+	for (int s = 0; s < 3; s++) {
+		const bool pad = s == 2 && q >= 2;
+		pi[s][0] = pad ? 0.0 : prm.pi[8 * s + 2 * q];
+		pi[s][1] = pad ? 0.0 : prm.pi[8 * s + 2 * q + 1];
+	}
 #pragma unroll
 	for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -522,9 +535,8 @@ __global__ void __launch_bounds__(128, 3) prune20_kernel(PruneParams prm)
 #pragma unroll
 			for (int s = 0; s < 3; s++)
 				if (s < 2 || q < 2) {
-					dot = fma(prm.pi[8 * s + 2 * q], (double)y.v[m][h][s].x, dot);
-					dot = fma(prm.pi[8 * s + 2 * q + 1], (double)y.v[m][h][s].y,
-						  dot);
+					dot = fma(pi[s][0], (double)y.v[m][h][s].x, dot);
+					dot = fma(pi[s][1], (double)y.v[m][h][s].y, dot);
 				}
 			dot += __shfl_xor_sync(0xffffffffu, dot, 1);
 			dot += __shfl_xor_sync(0xffffffffu, dot, 2);
