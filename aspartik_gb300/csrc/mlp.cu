@@ -19,6 +19,7 @@
 #include <cstring>
 #include <numeric>
 #include <random>
+#include <type_traits>
 
 namespace b3g {
 namespace {
@@ -48,13 +49,15 @@ __device__ __forceinline__ float gelu_grad(float x)
 // A block of 256 threads computes a 32 x 64 tile of C[m][n] = sum_k A'(m, k)
 // B'(k, n): two halves of 128 threads, a thread 4 x 4 products over its
 // half's 16 of every 32 k, the halves added at the end (each keeps two of
-// the four rows); operand tiles of 32 k pass through three shared-memory buffers
-// filled by cp.async two ahead of their use.  A'(m, k) = TA ? A[k][m] : A[m][k] with row stride lda, B'(k, n) = TB ?
-// B[n][k] : B[k][n] with row stride ldb.  The tile is this small because the
-// step is: 1,024 rows x 256 units are 128 tiles for 152 SMs, and two halves
-// because one warp a scheduler waits on its own loads (16 x 16 tiles with one
-// product a thread and shared-memory word pair took 17 to 36 us a product,
-// one half 9.7, two 6).
+// the four rows), or (kHalves false) 2 x 4 products over every k in order;
+// operand tiles of 32 k pass through three shared-memory buffers filled by
+// cp.async two ahead of their use.  A'(m, k) = TA ? A[k][m] : A[m][k] with row
+// stride lda, B'(k, n) = TB ? B[n][k] : B[k][n] with row stride ldb.  The tile
+// is this small because the step is: 1,024 rows x 256 units are 128 tiles for
+// 152 SMs, and 256 threads because one warp a scheduler waits on its own
+// loads (16 x 16 tiles with one product a thread and shared-memory word pair
+// took 17 to 36 us a product, 128 threads 9.7, two halves 6, 256 threads over
+// every k 7).
 constexpr uint32_t kTm = 32, kTn = 64, kTk = 32, kTt = 256; // kTt: threads
 constexpr uint32_t kTs = 3; // buffers
 // a weight gradient's rows are split over up to kSplits blocks a tile, at
@@ -119,7 +122,7 @@ __device__ __forceinline__ bool mlp_vec(const float *p, uint32_t ld)
 // The tile's products over k in [k0, k1).  Thread (h, ty, tx) leaves with rows
 // 4 ty + 2 h + i, columns TB ? tx + 16 j : 4 tx + j in acc[i][j].  col_sum (TA): threads 0..31 also add
 // A'(m0 + thread, k) over k.
-template <bool TA, bool TB>
+template <bool TA, bool TB, bool kHalves = true>
 __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const float *B,
 					    uint32_t m0, uint32_t n0, uint32_t M, uint32_t N,
 					    uint32_t k0, uint32_t k1, uint32_t lda, uint32_t ldb,
@@ -127,7 +130,9 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 {
 	constexpr uint32_t pa = TA ? kTm + 4 : kTk + 4, pb = TB ? kTk + 4 : kTn + 4;
 	const uint32_t tx = threadIdx.x & 15u, ty = (threadIdx.x >> 4) & 7u, h = threadIdx.x >> 7;
-	float c[4][4];
+	constexpr int kRows = kHalves ? 4 : 2; // a thread's rows, from row 4 ty (+ 2 h)
+	const uint32_t r0 = 4 * ty + (kHalves ? 0u : 2 * h);
+	float c[kRows][4];
 	// a row of the operand in memory must be whole vectors up to its end
 	const bool va = mlp_vec(A, lda) && ((TA ? M : k1) & 3u) == 0;
 	const bool vb = mlp_vec(B, ldb) && ((TB ? k1 : N) & 3u) == 0;
@@ -145,7 +150,7 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
 #pragma unroll
-	for (int i = 0; i < 4; ++i)
+	for (int i = 0; i < kRows; ++i)
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 			c[i][j] = 0.0f;
@@ -159,8 +164,8 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 		fetch(k + (kTs - 1) * kTk, next);
 		const float *sa = sm.a[buf], *sb = sm.b[buf];
 #pragma unroll
-		for (uint32_t k4 = 0; k4 < kTk / 2; k4 += 4) {
-			const uint32_t kk = h * (kTk / 2) + k4;
+		for (uint32_t k4 = 0; k4 < (kHalves ? kTk / 2 : kTk); k4 += 4) {
+			const uint32_t kk = kHalves ? h * (kTk / 2) + k4 : k4;
 			float a[4][4], b[4][4]; // [k][i], [k][j]
 #pragma unroll
 			for (int i = 0; i < 4; ++i) {
@@ -168,9 +173,9 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 					const float4 v = *reinterpret_cast<const float4 *>(
 						sa + (kk + i) * pa + 4 * ty);
 					a[i][0] = v.x, a[i][1] = v.y, a[i][2] = v.z, a[i][3] = v.w;
-				} else {
+				} else if (i < kRows) {
 					const float4 v = *reinterpret_cast<const float4 *>(
-						sa + (4 * ty + i) * pa + kk);
+						sa + (r0 + i) * pa + kk);
 					a[0][i] = v.x, a[1][i] = v.y, a[2][i] = v.z, a[3][i] = v.w;
 				}
 				if (TB) {
@@ -186,7 +191,7 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 #pragma unroll
 			for (int q = 0; q < 4; ++q)
 #pragma unroll
-				for (int i = 0; i < 4; ++i)
+				for (int i = 0; i < kRows; ++i)
 #pragma unroll
 					for (int j = 0; j < 4; ++j)
 						c[i][j] = fmaf(a[q][i], b[q][j], c[i][j]);
@@ -200,27 +205,39 @@ __device__ __forceinline__ void mlp_product(MlpSmem &sm, const float *A, const f
 	__syncthreads(); // the buffers are free
 	if (TA && col_sum)
 		*col_sum = cs;
-	// the other half's sums of this thread's rows, through shared memory
-	float4 *ex = reinterpret_cast<float4 *>(&sm);
+	if constexpr (!kHalves) {
+		static_assert(!TA || kHalves, "whole k: rows of A' only");
 #pragma unroll
-	for (int i = 0; i < 2; ++i) {
-		const int o = 2 * (1 - (int)h) + i; // what the other half keeps
-		const float *v = o == 0 ? c[0] : o == 1 ? c[1] : o == 2 ? c[2] : c[3];
-		ex[(threadIdx.x ^ 128u) + kTt * i] = make_float4(v[0], v[1], v[2], v[3]);
-	}
-	__syncthreads();
+		for (int i = 0; i < 2; ++i)
 #pragma unroll
-	for (int i = 0; i < 2; ++i) {
-		const float4 v = ex[threadIdx.x + kTt * i];
-		const float *w = h ? c[2 + i] : c[i];
-		acc[i][0] = w[0] + v.x;
-		acc[i][1] = w[1] + v.y;
-		acc[i][2] = w[2] + v.z;
-		acc[i][3] = w[3] + v.w;
+			for (int j = 0; j < 4; ++j)
+				acc[i][j] = c[i][j];
+		return;
+	} else {
+		// the other half's sums of this thread's rows, through shared memory
+		float4 *ex = reinterpret_cast<float4 *>(&sm);
+#pragma unroll
+		for (int i = 0; i < 2; ++i) {
+			const int o = 2 * (1 - (int)h) + i; // what the other half keeps
+			const float *v = o == 0 ? c[0] : o == 1 ? c[1] : o == 2 ? c[2] : c[3];
+			ex[(threadIdx.x ^ 128u) + kTt * i] = make_float4(v[0], v[1], v[2], v[3]);
+		}
+		__syncthreads();
+#pragma unroll
+		for (int i = 0; i < 2; ++i) {
+			const float4 v = ex[threadIdx.x + kTt * i];
+			const float *w = h ? c[2 + i] : c[i];
+			acc[i][0] = w[0] + v.x;
+			acc[i][1] = w[1] + v.y;
+			acc[i][2] = w[2] + v.z;
+			acc[i][3] = w[3] + v.w;
+		}
 	}
 }
 
-// Hidden layer: z = x W^T + b and a = gelu(z).  Grid (N / 64, M / 32).
+// Hidden layer: z = x W^T + b and a = gelu(z), each product one chain over k in
+// order (not halves): the residuals, whose rounding the output bias's gradient
+// consists of (below), do not depend on the tiling.  Grid (N / 64, M / 32).
 __global__ void __launch_bounds__(kTt) mlp_forward_kernel(const float *__restrict__ x,
 							   const float *__restrict__ W,
 							   const float *__restrict__ bias,
@@ -233,7 +250,7 @@ __global__ void __launch_bounds__(kTt) mlp_forward_kernel(const float *__restric
 	const uint32_t tx = threadIdx.x & 15u;
 	const uint32_t row = 4 * ((threadIdx.x >> 4) & 7u) + 2 * (threadIdx.x >> 7);
 	float acc[2][4];
-	mlp_product<false, true>(sm, x, W, m0, n0, M, N, 0, K, K, K, acc);
+	mlp_product<false, true, false>(sm, x, W, m0, n0, M, N, 0, K, K, K, acc);
 #pragma unroll
 	for (int j = 0; j < 4; ++j) {
 		const uint32_t n = n0 + tx + 16 * j;
@@ -279,93 +296,108 @@ __global__ void __launch_bounds__(256) mlp_out_kernel(const float *__restrict__ 
 
 // The pair objective and the last layer's backward pass.  Row i of n holds
 // x_new's third layer, row n + i x_old's; a warp a pair: r = y_new - y_old -
-// delta, the loss's share r^2, dL/dy = +-2 r / n, and dZ of the third layer
-// = dL/dy w gelu'(z).  The block's share of the output weights' gradient
-// (sum of dL/dy a, and of dL/dy) goes to part[block][H + 1].  The last block
-// to finish adds the loss shares in block order.
+// delta, the loss's share r^2, dL/dy = +-2 r / n (dys: the new rows'), and dZ
+// of the third layer = dL/dy w gelu'(z).  The last block to finish adds the
+// loss shares in block order.  y is one chain over the units in order, then
+// the bias, as a forward product forms it: the output layer's gradients are
+// small differences of large sums, and hold each value's rounding.
 constexpr uint32_t kHeadPairs = 4;
+// floats of a staged row (none above 256 units: rows are read in place)
+__host__ __device__ constexpr uint32_t head_row(uint32_t H)
+{
+	return H <= 256 ? (H + 3u) & ~3u : 0u;
+}
 __global__ void __launch_bounds__(32 * kHeadPairs) mlp_head_kernel(
 	const float *__restrict__ a, const float *__restrict__ z, const float *__restrict__ w,
-	const float *__restrict__ delta, float *__restrict__ dz, float *__restrict__ part,
+	const float *__restrict__ delta, float *__restrict__ dz, float *__restrict__ dys,
 	float *__restrict__ losses, float *__restrict__ loss, unsigned *ticket, uint32_t n,
 	uint32_t H)
 {
-	extern __shared__ float sh[]; // [kHeadPairs][H + 2]
+	extern __shared__ __align__(16) float sh[]; // [w: Hs][kHeadPairs][2][Hs], H <= 256
+	__shared__ float s_loss[kHeadPairs];
 	__shared__ unsigned s_last;
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	const uint32_t i = blockIdx.x * kHeadPairs + warp;
-	const uint32_t pitch = H + 2;
-	float *mine = sh + warp * pitch;
-	float r = 0.0f, dy = 0.0f;
+	const uint32_t i = blockIdx.x * kHeadPairs + warp, Hs = head_row(H);
+	float *rows = sh + (2 * warp + 1) * Hs; // this warp's new and old row
+	if (Hs)
+		for (uint32_t k = threadIdx.x; k < H; k += blockDim.x)
+			sh[k] = w[k];
+	__syncthreads();
+	auto value = [&](const float *row, const float *ww) {
+		float acc = 0.0f;
+		uint32_t k = 0;
+		if (Hs)
+#pragma unroll 8
+			for (; k + 4 <= H; k += 4) {
+				const float4 x = *reinterpret_cast<const float4 *>(row + k);
+				const float4 y = *reinterpret_cast<const float4 *>(ww + k);
+				acc = fmaf(x.x, y.x, acc);
+				acc = fmaf(x.y, y.y, acc);
+				acc = fmaf(x.z, y.z, acc);
+				acc = fmaf(x.w, y.w, acc);
+			}
+#pragma unroll 16
+		for (; k < H; ++k)
+			acc = fmaf(row[k], ww[k], acc);
+		return acc + w[H];
+	};
+	float r = 0.0f;
 	if (i < n) {
 		const float *an = a + (size_t)i * H, *ao = a + (size_t)(n + i) * H;
 		const float *zn = z + (size_t)i * H, *zo = z + (size_t)(n + i) * H;
-		float yn = 0.0f, yo = 0.0f;
-		if (H <= 256) {
-			// everything that does not need dy first, in registers
-			float va[8], vo[8], gn[8], go[8];
+		float gn[8], go[8];
+		float f = 0.0f;
+		if (Hs) {
+			// everything that does not need dL/dy first
 #pragma unroll
 			for (int q = 0; q < 8; ++q) {
 				const uint32_t k = lane + 32 * q;
 				const bool live = k < H;
-				va[q] = live ? an[k] : 0.0f;
-				vo[q] = live ? ao[k] : 0.0f;
 				gn[q] = live ? zn[k] : 0.0f;
 				go[q] = live ? zo[k] : 0.0f;
+				if (live) {
+					rows[k] = an[k];
+					rows[Hs + k] = ao[k];
+				}
 			}
+			__syncwarp();
+			if (lane < 2)
+				f = value(rows + lane * Hs, sh);
 #pragma unroll
 			for (int q = 0; q < 8; ++q) {
-				const uint32_t k = lane + 32 * q;
-				const float wk = k < H ? w[k] : 0.0f;
-				yn = fmaf(va[q], wk, yn);
-				yo = fmaf(vo[q], wk, yo);
-				gn[q] = wk * gelu_grad(gn[q]);
-				go[q] = wk * gelu_grad(go[q]);
+				gn[q] = gelu_grad(gn[q]);
+				go[q] = gelu_grad(go[q]);
 			}
-			// the output bias cancels in the difference
-			r = warp_sum(yn) - warp_sum(yo) - delta[i];
-			dy = 2.0f * r / n;
+		} else if (lane < 2) {
+			f = value(lane ? ao : an, w);
+		}
+		r = __shfl_sync(0xffffffffu, f, 0) - __shfl_sync(0xffffffffu, f, 1) - delta[i];
+		const float dy = 2.0f * r / n;
+		if (lane == 0)
+			dys[i] = dy;
+		if (Hs) {
 #pragma unroll
 			for (int q = 0; q < 8; ++q) {
 				const uint32_t k = lane + 32 * q;
 				if (k < H) {
-					dz[(size_t)i * H + k] = dy * gn[q];
-					dz[(size_t)(n + i) * H + k] = -dy * go[q];
-					mine[k] = dy * va[q] - dy * vo[q];
+					dz[(size_t)i * H + k] = dy * sh[k] * gn[q];
+					dz[(size_t)(n + i) * H + k] = -dy * sh[k] * go[q];
 				}
 			}
 		} else {
 			for (uint32_t k = lane; k < H; k += 32) {
-				yn = fmaf(an[k], w[k], yn);
-				yo = fmaf(ao[k], w[k], yo);
-			}
-			r = warp_sum(yn) - warp_sum(yo) - delta[i];
-			dy = 2.0f * r / n;
-			for (uint32_t k = lane; k < H; k += 32) {
-				dz[(size_t)i * H + k] = dy * (w[k] * gelu_grad(zn[k]));
-				dz[(size_t)(n + i) * H + k] = -dy * (w[k] * gelu_grad(zo[k]));
-				mine[k] = dy * an[k] - dy * ao[k];
+				dz[(size_t)i * H + k] = dy * w[k] * gelu_grad(zn[k]);
+				dz[(size_t)(n + i) * H + k] = -dy * w[k] * gelu_grad(zo[k]);
 			}
 		}
-	} else {
-		for (uint32_t k = lane; k < H; k += 32)
-			mine[k] = 0.0f;
 	}
-	if (lane == 0) {
-		mine[H] = dy - dy; // the bias gradient: +dy and -dy
-		mine[H + 1] = r * r;
-	}
+	if (lane == 0)
+		s_loss[warp] = r * r;
 	__syncthreads();
-	for (uint32_t k = threadIdx.x; k <= H; k += blockDim.x) {
-		float v = 0.0f;
-		for (uint32_t q = 0; q < kHeadPairs; ++q)
-			v += sh[q * pitch + k];
-		part[(size_t)blockIdx.x * (H + 1) + k] = v;
-	}
 	if (threadIdx.x == 0) {
 		float v = 0.0f;
 		for (uint32_t q = 0; q < kHeadPairs; ++q)
-			v += sh[q * pitch + H + 1];
+			v += s_loss[q];
 		losses[blockIdx.x] = v;
 		__threadfence();
 		s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
@@ -384,21 +416,79 @@ __global__ void __launch_bounds__(32 * kHeadPairs) mlp_head_kernel(
 	}
 }
 
-// One hidden layer's backward pass.  Blocks [0, dw_blocks): the weight
-// gradient dW[o][i] = sum_rows dZ[row][o] a[row][i] and the bias gradient,
+// Sums over the rows, one chain in row order, of columns c0 .. c0 + 15 of src
+// [R][C]: with dys the rows weighted by +dys[row] (first half) and -dys[row -
+// R / 2], and their own sum in *weights.  128 rows a tile, three tiles ahead
+// (tiles of 64 columns and 32 rows, two ahead, took 35 us for 1,024 rows: a
+// memory latency a tile).
+constexpr uint32_t kChainCols = 16, kChainRows = 128, kChainTiles = 4;
+__device__ __forceinline__ void mlp_column_chain(MlpSmem &sm, const float *src, uint32_t c0,
+						 uint32_t R, uint32_t C, const float *dys,
+						 float *out, float *weights)
+{
+	constexpr uint32_t kTile = kChainRows * kChainCols;
+	static_assert(kChainTiles * (kTile + kChainRows) * sizeof(float) <= sizeof(MlpSmem), "");
+	float *tiles = reinterpret_cast<float *>(&sm), *scales = tiles + kChainTiles * kTile;
+	const uint32_t t = threadIdx.x, n = R / 2;
+	const bool vec = mlp_vec(src, C);
+	auto fetch = [&](uint32_t k, uint32_t buf) {
+		if (k < R) {
+			mlp_tile<kChainRows, kChainCols>(tiles + buf * kTile, kChainCols, src, k, c0,
+							 R, C, C, vec);
+			const uint32_t row = k + t;
+			if (dys && t < kChainRows)
+				mlp_cp4(scales + buf * kChainRows + t,
+					dys + (row < n ? row : row < R ? row - n : 0u), row < R);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	for (uint32_t q = 0; q + 1 < kChainTiles; ++q)
+		fetch(q * kChainRows, q);
+	float acc = 0.0f;
+	uint32_t buf = 0;
+	for (uint32_t k = 0; k < R; k += kChainRows) {
+		asm volatile("cp.async.wait_group %0;" ::"n"(kChainTiles - 2) : "memory");
+		__syncthreads(); // this tile is there, the one before it used up
+		fetch(k + (kChainTiles - 1) * kChainRows, (buf + kChainTiles - 1) % kChainTiles);
+		const float *v = tiles + buf * kTile + t, *w = scales + buf * kChainRows;
+		const uint32_t rows = min(kChainRows, R - k);
+		if (t < kChainCols) {
+			if (!dys) {
+#pragma unroll 16
+				for (uint32_t r = 0; r < rows; ++r)
+					acc += v[r * kChainCols];
+			} else {
+#pragma unroll 16
+				for (uint32_t r = 0; r < rows; ++r)
+					acc = fmaf(k + r < n ? w[r] : -w[r], v[r * kChainCols], acc);
+			}
+		} else if (t == 32 && weights) {
+#pragma unroll 16
+			for (uint32_t r = 0; r < rows; ++r)
+				acc += k + r < n ? w[r] : -w[r];
+		}
+		buf = (buf + 1) % kChainTiles;
+	}
+	if (t < kChainCols && c0 + t < C)
+		out[c0 + t] = acc;
+	else if (t == 32 && weights)
+		*weights = acc;
+}
+
+// One hidden layer's backward pass.  Where dys is given (the last hidden
+// layer), first the output layer's gradients and this layer's bias gradient as
+// chains over the rows.  Then dw_blocks: the weight gradient dW[o][i] = sum_rows dZ[row][o] a[row][i] and the bias gradient,
 // tiles x splits of split_rows rows; with several splits the partial tiles go
 // to `part` and a tile's last block adds them in split order.  Then
-// da_blocks: dZ of the layer below, (dZ W) gelu'(z_below).  Then, where
-// head_part is given, the output layer's gradient from the head kernel's
-// block shares.
+// da_blocks: dZ of the layer below, (dZ W) gelu'(z_below).
 struct MlpBackward {
 	const float *dz, *a, *W, *z_below;
 	float *dW, *db, *dz_below;
 	float *part;       // [tiles][splits][kTm * kTn + kTm]
 	unsigned *tickets; // [tiles], zero between launches
-	const float *head_part;
+	const float *dys, *a_out; // dL/dy, this layer's outputs
 	float *head_grad;
-	uint32_t rows, O, I, splits, split_rows, dw_blocks, da_blocks, head_blocks;
+	uint32_t rows, O, I, splits, split_rows, dw_blocks, da_blocks;
 };
 __global__ void __launch_bounds__(kTt) mlp_backward_kernel(MlpBackward p)
 {
@@ -407,20 +497,20 @@ __global__ void __launch_bounds__(kTt) mlp_backward_kernel(MlpBackward p)
 	const uint32_t tx = threadIdx.x & 15u;
 	const uint32_t row = 4 * ((threadIdx.x >> 4) & 7u) + 2 * (threadIdx.x >> 7);
 	float acc[2][4];
-	if (blockIdx.x >= p.dw_blocks + p.da_blocks) {
-		// output layer: one column a thread
-		const uint32_t k = (blockIdx.x - p.dw_blocks - p.da_blocks) * kTt + threadIdx.x;
-		if (k > p.O)
-			return;
-		float v = 0.0f;
-#pragma unroll 8
-		for (uint32_t b = 0; b < p.head_blocks; ++b)
-			v += p.head_part[(size_t)b * (p.O + 1) + k];
-		p.head_grad[k] = v;
+	// (the chains first: they are the longest blocks)
+	const uint32_t chains = p.dys ? 2 * ((p.O + kChainCols - 1) / kChainCols) : 0u;
+	if (blockIdx.x < chains) {
+		const uint32_t t = blockIdx.x >> 1;
+		if (blockIdx.x & 1u)
+			mlp_column_chain(sm, p.dz, t * kChainCols, p.rows, p.O, nullptr, p.db, nullptr);
+		else
+			mlp_column_chain(sm, p.a_out, t * kChainCols, p.rows, p.O, p.dys, p.head_grad,
+					 t == 0 ? p.head_grad + p.O : nullptr);
 		return;
 	}
-	if (blockIdx.x >= p.dw_blocks) {
-		const uint32_t t = blockIdx.x - p.dw_blocks, nt = (p.I + kTn - 1) / kTn;
+	const uint32_t block = blockIdx.x - chains;
+	if (block >= p.dw_blocks) {
+		const uint32_t t = block - p.dw_blocks, nt = (p.I + kTn - 1) / kTn;
 		const uint32_t m0 = t / nt * kTm, n0 = t % nt * kTn;
 		mlp_product<false, false>(sm, p.dz, p.W, m0, n0, p.rows, p.I, 0, p.O, p.O, p.I,
 					  acc);
@@ -440,11 +530,11 @@ __global__ void __launch_bounds__(kTt) mlp_backward_kernel(MlpBackward p)
 		}
 		return;
 	}
-	const uint32_t tile = blockIdx.x / p.splits, split = blockIdx.x - tile * p.splits;
+	const uint32_t tile = block / p.splits, split = block - tile * p.splits;
 	const uint32_t nt = (p.I + kTn - 1) / kTn;
 	const uint32_t m0 = tile / nt * kTm, n0 = tile % nt * kTn;
 	const uint32_t k0 = split * p.split_rows, k1 = min(p.rows, k0 + p.split_rows);
-	const bool bias = n0 == 0;
+	const bool bias = n0 == 0 && !p.dys;
 	float cs = 0.0f;
 	mlp_product<true, false>(sm, p.dz, p.a, m0, n0, p.O, p.I, k0, k1, p.O, p.I, acc,
 				 bias ? &cs : nullptr);
@@ -734,20 +824,11 @@ Mlp::~Mlp()
 
 void Mlp::free_batch()
 {
-	cudaFree(d_x_);
-	for (uint32_t l = 0; l + 1 < kLayers; ++l) {
-		cudaFree(d_z_[l]);
-		cudaFree(d_a_[l]);
-		cudaFree(d_dz_[l]);
+	cudaFree(d_batch_);
+	d_batch_ = nullptr;
+	for (uint32_t l = 0; l + 1 < kLayers; ++l)
 		d_z_[l] = d_a_[l] = d_dz_[l] = nullptr;
-	}
-	cudaFree(d_y_);
-	cudaFree(d_delta_);
-	cudaFree(d_loss_);
-	cudaFree(d_head_);
-	cudaFree(d_part_);
-	cudaFree(d_tickets_);
-	d_x_ = d_y_ = d_delta_ = d_loss_ = d_head_ = d_part_ = nullptr;
+	d_x_ = d_y_ = d_delta_ = d_dys_ = d_loss_ = d_head_ = d_part_ = nullptr;
 	d_tickets_ = nullptr;
 	cap_ = 0;
 }
@@ -774,25 +855,38 @@ void Mlp::ensure_batch(uint32_t rows)
 		return;
 	check_cuda(cudaStreamSynchronize(stream_), "sync");
 	free_batch();
-	check_cuda(cudaMalloc(&d_x_, sizeof(float) * rows * in_), "inputs");
-	for (uint32_t l = 0; l + 1 < kLayers; ++l) {
-		const size_t sz = sizeof(float) * rows * dims_[l + 1];
-		check_cuda(cudaMalloc(&d_z_[l], sz), "z");
-		check_cuda(cudaMalloc(&d_a_[l], sz), "a");
-		check_cuda(cudaMalloc(&d_dz_[l], sz), "dz");
-	}
-	check_cuda(cudaMalloc(&d_y_, sizeof(float) * rows), "y");
-	check_cuda(cudaMalloc(&d_delta_, sizeof(float) * rows), "delta");
-	check_cuda(cudaMalloc(&d_loss_, sizeof(float)), "loss");
-	// the head kernel's block shares, then its block losses
-	check_cuda(cudaMalloc(&d_head_, sizeof(float) * (head_blocks(rows) + 1) * (hidden_ + 2)),
-		   "output gradient shares");
-	check_cuda(cudaMalloc(&d_part_, sizeof(float) * dw_tiles(hidden_, hidden_) * kSplits *
-						(kTm * kTn + kTm)),
-		   "gradient shares");
-	const size_t tickets = sizeof(unsigned) * (dw_tiles(hidden_, hidden_) + 1);
-	check_cuda(cudaMalloc(&d_tickets_, tickets), "tickets");
-	check_cuda(cudaMemsetAsync(d_tickets_, 0, tickets, stream_), "zero tickets");
+	// one allocation, carved up (sixteen calls were half of the first
+	// evaluation's time at small sizes)
+	const uint32_t tiles = dw_tiles(hidden_, hidden_);
+	size_t bytes = 0;
+	auto carve = [&](auto *&p, size_t count) {
+		const size_t at = bytes;
+		bytes += (count * sizeof(*p) + 255) & ~(size_t)255;
+		if (d_batch_)
+			p = reinterpret_cast<std::decay_t<decltype(p)>>(d_batch_ + at);
+	};
+	auto all = [&] {
+		bytes = 0;
+		carve(d_tickets_, tiles + 1);
+		carve(d_x_, (size_t)rows * in_);
+		for (uint32_t l = 0; l + 1 < kLayers; ++l) {
+			const size_t count = (size_t)rows * dims_[l + 1];
+			carve(d_z_[l], count);
+			carve(d_a_[l], count);
+			carve(d_dz_[l], count);
+		}
+		carve(d_y_, rows);
+		carve(d_delta_, rows);
+		carve(d_dys_, rows);
+		carve(d_loss_, 1);
+		carve(d_head_, head_blocks(rows)); // the head kernel's block losses
+		carve(d_part_, (size_t)tiles * kSplits * (kTm * kTn + kTm));
+	};
+	all();
+	check_cuda(cudaMalloc(&d_batch_, bytes), "batch workspace");
+	all();
+	check_cuda(cudaMemsetAsync(d_tickets_, 0, sizeof(unsigned) * (tiles + 1), stream_),
+		   "zero tickets");
 	cap_ = rows;
 }
 
@@ -816,10 +910,10 @@ void Mlp::backward_device(uint32_t n)
 {
 	const uint32_t rows = 2 * n, H = hidden_, top = kLayers - 2;
 	const uint32_t hb = head_blocks(rows);
-	float *losses = d_head_ + (size_t)hb * (H + 1);
-	mlp_head_kernel<<<hb, 32 * kHeadPairs, sizeof(float) * kHeadPairs * (H + 2), stream_>>>(
-		d_a_[top], d_z_[top], d_params_ + w_off_[kLayers - 1], d_delta_, d_dz_[top], d_head_,
-		losses, d_loss_, d_tickets_ + dw_tiles(H, H), n, H);
+	mlp_head_kernel<<<hb, 32 * kHeadPairs, sizeof(float) * (2 * kHeadPairs + 1) * head_row(H),
+			  stream_>>>(d_a_[top], d_z_[top], d_params_ + w_off_[kLayers - 1], d_delta_,
+				     d_dz_[top], d_dys_, d_head_, d_loss_,
+				     d_tickets_ + dw_tiles(H, H), n, H);
 	for (int l = (int)top; l >= 0; --l) {
 		MlpBackward p{};
 		p.rows = rows;
@@ -842,10 +936,10 @@ void Mlp::backward_device(uint32_t n)
 		}
 		uint32_t blocks = p.dw_blocks + p.da_blocks;
 		if (l == (int)top) {
-			p.head_part = d_head_;
+			p.dys = d_dys_;
+			p.a_out = d_a_[l];
 			p.head_grad = d_grad_ + w_off_[kLayers - 1]; // weights, then the bias
-			p.head_blocks = hb;
-			blocks += (H + kTt) / kTt; // H + 1 columns
+			blocks += 2 * ((H + kChainCols - 1) / kChainCols);
 		}
 		mlp_backward_kernel<<<blocks, kTt, 0, stream_>>>(p);
 	}

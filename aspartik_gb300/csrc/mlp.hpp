@@ -71,6 +71,7 @@ class Mlp {
 	uint32_t adam_t_ = 0;
 	// activations for up to cap_ rows: z (pre) and a (post) per layer
 	uint32_t cap_ = 0;
+	unsigned char *d_batch_ = nullptr; // holds the buffers below up to d_tickets_
 	float *d_x_ = nullptr;
 	float *d_z_[kLayers - 1] = {};
 	float *d_a_[kLayers - 1] = {};
@@ -78,7 +79,7 @@ class Mlp {
 	float *d_y_ = nullptr, *d_delta_ = nullptr, *d_loss_ = nullptr;
 	// workspaces of the backward pass: block shares of the output layer's
 	// gradient and of split weight gradients, and their counters
-	float *d_head_ = nullptr, *d_part_ = nullptr;
+	float *d_head_ = nullptr, *d_part_ = nullptr, *d_dys_ = nullptr;
 	unsigned *d_tickets_ = nullptr;
 	float *d_pair_ = nullptr, *h_pair_ = nullptr; // inference staging
 	struct InferCtx {
