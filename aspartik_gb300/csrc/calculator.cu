@@ -1957,7 +1957,8 @@ uint32_t Calculator::autotune(const uint32_t *internals,
 	// (and give small alignments more blocks), 64 and 128 one.
 	// (The run walk's shape, for batches and lists of several trees; the
 	// depth-first walk has none.)
-	const Restore walk{use_tree_, use_tree_};
+	const bool tree = tree_list(n);
+	Restore walk{use_tree_, use_tree_};
 	use_tree_ = false;
 	uint32_t best_tile = runs_tile_, best_block = runs_block_;
 	float best_ms = INFINITY;
@@ -1978,6 +1979,9 @@ uint32_t Calculator::autotune(const uint32_t *internals,
 	}
 	runs_tile_ = best_tile;
 	runs_block_ = best_block;
+	use_tree_ = walk.value;
+	if (tree) // leave the walk that the list takes in the caches
+		(void)trial();
 	return best_tile;
 }
 
