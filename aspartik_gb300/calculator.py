@@ -173,7 +173,8 @@ class GpuCalculator:
     def autotune(self, internals, children, lengths, clock_rate: float = 1.0) -> int:
         """Time the list with each launch configuration of this form and keep
         the fastest (no counterpart in the reference); returns the patterns
-        per tile (4 states), 1 / 0 for tensor / CUDA cores (20 states), 0 for
+        per tile of the run walk (4 states), 1 / 0 for the tcgen05 / the register
+        walk (20 states), 0 for
         the FP64 form.  Trial proposals are rejected: call between steps."""
         internals = nat.u32(internals)
         children = nat.u32(children).reshape(-1)

@@ -1,10 +1,15 @@
 // kernels4.cu -- sm_103a kernels of the 4-state (DNA) pruning likelihood.
 //
-//   ptab4_kernel   transition-matrix builder: P = V diag(exp(lambda d)) V^-1
+//   ptab4_kernel, ptab4_rows_kernel, ptab4_f64_kernel
+//                  transition-matrix builders: P = V diag(exp(lambda d)) V^-1
 //                  per (dirty node, child side, rate category), written
 //                  transposed with a trailing row of ones so that both the
 //                  internal-child product (sum_k x_k PT[k]) and the tip
 //                  lookup (PT[code]) are one 4-vector access each.
+//   prune4_tree_kernel
+//                  FP32 depth-first walk of whole trees (tree4.cuh).
+//   prune4_f64_kernel
+//                  FP64 walk on the integer pipes (prune4f64.cuh).
 //   prune4_kernel  Felsenstein pruning over the children-first dirty list.
 //                  One thread owns one (pattern, category) column and walks
 //                  the whole list, so no inter-block synchronisation exists;

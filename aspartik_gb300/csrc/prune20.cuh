@@ -150,16 +150,15 @@ struct RootColumns {
 // fragment the next product reads: values never change lanes, and a chain of
 // entries passes through registers.
 //
-// Whole tree, 128 taxa x 4,989 patterns, four categories: 90 us (about 2,100
+// Whole tree, 128 taxa x 4,989 patterns, four categories: 124 us (about 2,100
 // cycles an entry and warp alone, 2,650 with two warps a scheduler), dirty
-// path of ten entries 10 us; 44,000 patterns: 760 us.
+// path of eight entries 10 us of walk; 44,000 patterns: 767 us.
 // Why not the other two engines: scalar FMAs need a broadcast shared-memory
-// word per multiply-add and warp (131 us for a whole tree of 128 taxa x 4,989
-// patterns, the load path 70 % busy), and on the fifth-generation tensor
-// cores (prune20tc.cuh) an entry is a chain of a bulk copy, a split through
-// shared memory, an MMA round trip and a tensor-memory read of about 5,000
-// cycles for at most 0.1 of them of tensor work (137 us; 840 us at 44,000
-// patterns).  Here an internal
+// word per multiply-add and warp (the load path 70 % busy), and on the
+// fifth-generation tensor cores (prune20tc.cuh) an entry is a chain of a bulk
+// copy, a split through shared memory, an MMA round trip and a tensor-memory
+// read of about 5,000 cycles for at most 0.1 of them of tensor work (168 us
+// with its root kernel; 853 us at 44,000 patterns).  Here an internal
 // child of 32 patterns takes 54 instructions of 8 cycles each (measured) of
 // its scheduler's matrix pipe and about as many issue slots beside them.
 //

@@ -1056,7 +1056,7 @@ __device__ __forceinline__ uint32_t member_of(const uint32_t *prefix, uint32_t M
 // member copies its list, marks every child's source, converts the
 // member's eigensystem to FP32 and builds the list's tables (as the
 // single-calculator kernel does, so values match it), then walks the tile
-// serially with clean inputs loaded four entries ahead.  Each tile's
+// serially with clean inputs copied two entries ahead.  Each tile's
 // weighted sum goes to the member's tile slot; the block finishing a
 // member's last tile folds its sums (fixed order).
 template <typename Idx, uint32_t kC>

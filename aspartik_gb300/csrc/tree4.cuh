@@ -29,10 +29,11 @@
 // Kernel time of a whole tree, the run walk -> this: 256 taxa x 17,764 patterns
 // x 4 categories 106 -> 69 us (362 MB stored, 5.2 TB/s; 42 us is what the SMs'
 // store ports need, 50 us DRAM); 64 x 7,855 x 4 30 -> 20 us, of which the
-// tables, the prologue and the root are half.  It is bound by the latency of
-// its shared-memory reads at 12 to 16 warps an SM, with the load path (60 %),
-// the store port (57 %) and the issue slots (46 %) all half busy; more warps
-// at fewer registers spill and were slower (96 -> 113 us).
+// tables, the prologue and the root are half.  No unit is full (of the active
+// cycles at 8 warps an SM: busiest L1 unit 67 %, issue slots 43 %); its warps
+// wait on fixed latencies and shared-memory reads.  16 warps an SM (four
+// groups) were no faster (91 against 88 us a call), more at fewer registers
+// spill and were slower (96 -> 113 us).
 constexpr uint32_t kTreeRing = 4 * kTreeChunk;
 
 struct __align__(16) TreeEntry {

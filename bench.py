@@ -59,12 +59,12 @@ WORKLOADS = {
                            root_height=0.5, pi_conc=10.0),
 }
 DEFAULT_WORKLOAD = "dna256x20000_gtr_g4"
-# DRAM bytes (read + write) of one whole-tree launch of prune4_runs_kernel on
-# the default workload, from an ncu capture (dram__bytes_read.sum 17.47 MB +
-# dram__bytes_write.sum 304.28 MB): children written earlier in the same pass
-# are read from shared-memory slots or from L2, tables are built on chip, so
-# the traffic is mostly the partials' writes, 43 % of the algorithmic bytes.
-TRAFFIC_RUNS_BYTES = 321_756_416
+# DRAM bytes (read + write) of one whole-tree launch of prune4_tree_kernel on
+# the default workload, from an ncu capture (dram__bytes_read.sum 4.85 MB +
+# dram__bytes_write.sum 301.74 MB): children written earlier in the same pass
+# stay in registers and shared-memory slots, so the traffic is the partials'
+# writes, 41 % of the algorithmic bytes.
+TRAFFIC_TREE_BYTES = 306_590_000
 
 
 def make_workload(name: str, seed: int = 4) -> dict:
@@ -390,12 +390,14 @@ def protein20(device: int, steps: int, warmup: int, seed: int = 4, L: int = 128,
         calc.set_weights(weights)
         calc.set_reversible(rates, pi)
         calc.set_gamma(1.0)
-        engine = "CUDA cores" if form == "f32_cuda_cores" else None
+        engine = ("register matrix instructions" if form == "f32_cuda_cores"
+                  else None)
         if form == "f32":
             calc.propose_lengths(*lists, 1.0)
             calc.log_likelihood()
             calc.accept()
-            engine = "tensor cores" if calc.autotune(*lists, 1.0) else "CUDA cores"
+            engine = ("tcgen05" if calc.autotune(*lists, 1.0)
+                      else "register matrix instructions")
         k = steps if precision == "f32" else max(3, min(steps, 20))
         ms, _, prune_ms, _ = device_throughput(calc, lists, k, warmup, 1)
         lnl = calc.log_likelihood()
@@ -908,11 +910,11 @@ def run_ours(args):
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": pk["hbm_gbs"],
                      "unit": "GB/s", "frac": round(achieved / pk["hbm_gbs"], 4),
-                     "traffic": TRAFFIC_RUNS_BYTES if args.workload == DEFAULT_WORKLOAD else None,
+                     "traffic": TRAFFIC_TREE_BYTES if args.workload == DEFAULT_WORKLOAD else None,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, "
                                        "one whole-tree launch of this workload",
                      "peak_source": pk["source"],
-                     "kernel": "prune4_runs_kernel (FP32, run-synchronous)",
+                     "kernel": "prune4_tree_kernel (FP32, depth first)",
                      "tile_patterns": tile,
                      "kernel_ms": round(t_pr, 5), "transition_kernel_ms": round(t_tr, 5)},
         "e2e": {"value": round(e2e, 2), "unit": UNIT,

@@ -197,8 +197,8 @@ B3G_API b3g_status b3g_calculator_last_upload_bytes(b3g_calculator *calc,
 						    uint64_t *bytes);
 /* Kernels the last evaluation launched on the calculator's stream (one
  * fused launch for a short FP32 list or a run walk that builds its own
- * tables; tables + pruning otherwise; three for 20 states on the tensor
- * cores). */
+ * tables; tables + pruning otherwise; three for the 20-state tcgen05
+ * walk). */
 B3G_API b3g_status b3g_calculator_last_launches(b3g_calculator *calc,
 						uint32_t *kernels);
 /* Device time between two markers on the calculator's stream: span_begin
@@ -212,12 +212,13 @@ B3G_API b3g_status b3g_calculator_span_end(b3g_calculator *calc, float *ms);
  * calculator's form and keeps the fastest: patterns per tile of the
  * run-synchronous walk (16, 32, 64 or 128, with 512- or 1,024-thread
  * blocks; a thread owns two pattern columns of one category, so a warp
- * spans four, two, one or one categories; four-state FP32), or tensor
- * cores (one or two thread groups per CTA) against CUDA cores (20-state
- * FP32).
+ * spans four, two, one or one categories; four-state FP32: batches and
+ * lists that do not take the depth-first walk use it), or the tcgen05 walk
+ * (one or two thread groups per CTA) against the walk with register matrix
+ * instructions (20-state FP32).
  * Every trial proposal is rejected, so
  * call it between steps; the accepted state is unchanged.  `choice`
- * receives the tile, or 1 (tensor cores) / 0 (CUDA cores); the FP64 form
+ * receives the tile, or 1 (tcgen05) / 0 (register walk); the FP64 form
  * has nothing to tune and returns 0. */
 B3G_API b3g_status b3g_calculator_autotune(b3g_calculator *calc,
 					   const uint32_t *internals,
