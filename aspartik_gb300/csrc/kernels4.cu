@@ -47,8 +47,10 @@ namespace cg = cooperative_groups;
 // before it reads a table.  Its launch and prologue are then off the chain of
 // a short evaluation (FP64, 64 taxa x 7,855 patterns x 4 categories, paths of
 // 8 entries: 34.7 -> 32.6 us each; 37 x 1,147, whole tree: 57 -> 55 us).  The
-// 20-state FP32 walk, whose early blocks take the table kernel's place on the
-// SMs, gained nothing (350 / 351, a whole tree 168 / 165 us) and waits.
+// 20-state walks do without: the table kernel's blocks fill the SMs, and the
+// walk's then crowd on the few that become free first (FP64, 128 taxa x 4,989
+// patterns x 4 categories: 1,280 us behind the tables, 1,630 beside them; a
+// path of 61 x 2,003 80 / 96).
 __device__ __forceinline__ void tables_started()
 {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1190,8 +1192,8 @@ cudaError_t launch_prune20_f64(const PruneParams &p, uint32_t groups, cudaStream
 		prune20_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess)
 		return e;
-	return launch_beside(prune20_f64_kernel, dim3(p.ldp / kP20Tile, p.C), dim3(128 * groups),
-			     smem, s, p);
+	prune20_f64_kernel<<<dim3(p.ldp / kP20Tile, p.C), 128 * groups, smem, s>>>(p);
+	return cudaGetLastError();
 }
 
 uint32_t prune20_blocks_per_sm(uint32_t groups)

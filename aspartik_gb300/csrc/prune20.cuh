@@ -91,8 +91,6 @@ __global__ void __launch_bounds__(kS20 *kS20 / kParts) ptab20_kernel(PtabParams 
 {
 	constexpr uint32_t S = kS20, kCount = S * S / kParts;
 	static_assert(kParts == 1 || sizeof(R) == 4, "the integer table's flag is one block's");
-	if constexpr (sizeof(R) == 8)
-		tables_started();
 	__shared__ Ptab20Smem sm;
 	const uint32_t id = blockIdx.x / kParts, base = (blockIdx.x % kParts) * kCount;
 	const uint32_t t = threadIdx.x, i = (base + t) / S, j = (base + t) - i * S;

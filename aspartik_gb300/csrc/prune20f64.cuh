@@ -219,7 +219,6 @@ __global__ void __launch_bounds__(512) prune20_f64_kernel(PruneParams prm)
 			}
 			e = runs[r] + g;
 		}
-		wait_for_tables();
 		fill(e, 0);
 	}
 	int32_t cnt[2] = {0, 0};
