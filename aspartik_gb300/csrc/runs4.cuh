@@ -371,11 +371,16 @@ __device__ double tile_walk(const TileArgs &a, uint32_t t, float *s_dot,
 	return tile_root(a, t, s_dot, s_cnt, s_red);
 }
 
-// x 2^e for e <= 0 (zero below 2^-252, which no sum with a term of at least
-// 2^-126 beside it notices): two exact powers of two instead of ldexpf's
-// cases.
-__device__ __forceinline__ float scale_down(float x, int32_t e)
+// x 2^e.  A category's count lies above the largest of the positive ones only
+// where its own value is zero or below: an invariant class keeps the count 0
+// of its all-zero vectors while the others' fall with the tree, and by two
+// factors 2^128 would be an infinity, its product with zero NaN.  For e <= 0
+// (zero below 2^-252, which no sum with a term of at least 2^-126 beside it
+// notices) two exact powers of two instead of ldexpf's cases.
+__device__ __forceinline__ float scale_to(float x, int32_t e)
 {
+	if (e > 0)
+		return ldexpf(x, e);
 	const int32_t lo = max(e, -126), hi = max(e - lo, -126);
 	x *= __uint_as_float((uint32_t)(127 + lo) << 23);
 	return x * __uint_as_float((uint32_t)(127 + hi) << 23);
@@ -402,7 +407,7 @@ pattern_root(const float *s_dot, const int32_t *s_cnt, uint32_t tile, uint32_t C
 		// exact exponent term and the constant join in FP64
 		float acc = 0.f;
 		for (uint32_t c = 0; c < C; c++)
-			acc += scale_down(s_dot[c * tile + k], s_cnt[c * tile + k] - emax);
+			acc += scale_to(s_dot[c * tile + k], s_cnt[c * tile + k] - emax);
 		site = (double)logf(acc) +
 		       fma((double)emax, 0.69314718055994530942, log_inv_c);
 	}
@@ -857,7 +862,7 @@ __device__ __forceinline__ double direct_root(const float *s_dot, const int32_t 
 			float acc = 0.f;
 #pragma unroll
 			for (uint32_t k = 0; k < kC; k++)
-				acc += scale_down(dot[k], cnt[k] - emax);
+				acc += scale_to(dot[k], cnt[k] - emax);
 			site = (double)logf(acc) +
 			       fma((double)emax, 0.69314718055994530942, log_inv_c);
 		}
