@@ -352,8 +352,9 @@ __global__ void __launch_bounds__(512) prune20_f64_kernel(PruneParams prm)
 		}
 		__syncthreads(); // the run's outputs are visible to every group
 	}
-	// the last entry (the root) is alone in its run: group 0 walked it
-	if (g == 0 && t < kP20Tile) {
+	// the group that walked the last entry, the root (group 0 unless the list
+	// is not one tree and unrelated entries share the root's run)
+	if (g == (prm.n - 1 - runs[prm.n_runs - 1]) % G && t < kP20Tile) {
 		// w is 0 or 1 here: patterns t = lane + 32 w
 		const int32_t n = w ? cnt[1] : cnt[0];
 		const double dot = sm.dot[t];
