@@ -285,14 +285,6 @@ void Batch::release()
 	stream_ = nullptr;
 }
 
-// The kernel that takes a member's staged list.
-uint32_t Batch::kind_of(const Calculator &c)
-{
-	if (c.staged_n_ <= kDirectMax && (c.C_ == 1 || c.C_ == 2 || c.C_ == 4))
-		return kListShort;
-	return c.staged_tree_ ? kListTree : kListRuns;
-}
-
 void Batch::run()
 {
 	check_cuda(cudaSetDevice(device_), "cudaSetDevice");
@@ -304,7 +296,7 @@ void Batch::run()
 	// its entries are spread over more thread groups)
 	uint32_t tiles = 0, shrink = 0, form = 0;
 	for (Calculator *c : members_)
-		if (c->staged_ && kind_of(*c) == kListRuns)
+		if (c->staged_ && c->staged_kind_ == kListRuns)
 			tiles += c->ldp_ / c->staged_tile_;
 	while (tiles && (tiles << (shrink + 1)) <= ctas_)
 		++shrink;
@@ -320,7 +312,7 @@ void Batch::run()
 			s.tile = std::max(16u, c->staged_tile_ >> shrink);
 			s.tips_smem = c->staged_tips_smem_;
 			s.clock_rate = c->staged_clock_;
-			s.kind = kind_of(*c);
+			s.kind = c->staged_kind_;
 			if (s.kind == kListTree) {
 				s.tips_smem = c->tree_tips_;
 				s.groups = c->order_groups_;

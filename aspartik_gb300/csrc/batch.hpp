@@ -47,7 +47,6 @@ class Batch {
 	bool direct_c_[5] = {}; // members with 1, 2 or 4 categories present
 	bool ran_ = false, running_ = false; // running_: the last replay was not waited for
 	void wait();
-	static uint32_t kind_of(const Calculator &c);
 	void capture(uint32_t form);
 	std::vector<uint8_t> evaluated_;
 };

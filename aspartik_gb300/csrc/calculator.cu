@@ -1618,11 +1618,12 @@ void Calculator::stage_lengths(const uint32_t *internals,
 	// so must this calculator's own last launch
 	wait_stage();
 	wait_batch();
+	// (a batch takes short lists by one launch whatever B3G_DIRECT says)
+	const bool is_short = n <= kDirectMax && (C_ == 1 || C_ == 2 || C_ == 4);
 	tree_batch_ = true;
-	stage_ops(internals, children, n,
-		  use_tree_ && !(use_direct_ && n <= kDirectMax) && batch_tree(n));
+	stage_ops(internals, children, n, !is_short && use_tree_ && batch_tree(n));
 	tree_batch_ = false;
-	staged_tree_ = depth_first_;
+	staged_kind_ = is_short ? kListShort : depth_first_ ? kListTree : kListRuns;
 	std::memcpy(h_stage_ + off_pi_, model_host_.pi, S_ * sizeof(double));
 	stage_inputs(lengths, n, 2);
 	staged_ = true;

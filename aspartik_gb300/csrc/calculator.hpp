@@ -182,7 +182,7 @@ class Calculator {
 	// the four-state FP32 form's depth-first walk of single-tree lists
 	// (B3G_TREE=0: the run walk), and the staged list's shared-memory slots
 	bool use_tree_ = false, tree_always_ = false;
-	bool staged_tree_ = false; // the batch's staged list takes it
+	uint32_t staged_kind_ = 0; // the kernel that the staged list is laid out for (kList*)
 	uint32_t tree_slots_ = 0, tree_tips_ = 0, tree_groups_ = 0, tree_tile_ = 64;
 	uint32_t tree_tile_fixed_ = 0;
 	bool tree_clean_ = false, tree_batch_ = false; // (staging for a batch)
