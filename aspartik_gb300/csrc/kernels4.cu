@@ -915,6 +915,37 @@ cudaError_t launch_ptab4(const PtabParams &p, bool f32, cudaStream_t s)
 	return cudaGetLastError();
 }
 
+// Allows a kernel the device's whole opt-in shared memory, once per kernel
+// and device (a permission, not a reservation: no call lowers another's
+// limit and later launches pay nothing).  A limit set to each launch's own
+// size would be the process's too: a second thread with a smaller list could
+// lower it between this one's call and its launch.
+struct SmemOptIn {
+	std::atomic<bool> done[64] = {};
+};
+template <typename Kernel> static cudaError_t opt_in_smem(Kernel kern, SmemOptIn &state)
+{
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess)
+		return e;
+	if (dev >= 0 && dev < 64 && state.done[dev].load(std::memory_order_acquire))
+		return cudaSuccess;
+	int most = 0;
+	e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+	if (e != cudaSuccess)
+		return e;
+	cudaFuncAttributes fa{};
+	e = cudaFuncGetAttributes(&fa, kern);
+	if (e != cudaSuccess)
+		return e;
+	e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				 most - (int)fa.sharedSizeBytes);
+	if (e == cudaSuccess && dev >= 0 && dev < 64)
+		state.done[dev].store(true, std::memory_order_release);
+	return e;
+}
+
 template <typename VT, bool kPow2>
 static cudaError_t launch_prune4_t(const PruneParams &p, uint32_t tile,
 				   cudaStream_t s)
@@ -930,8 +961,8 @@ static cudaError_t launch_prune4_t(const PruneParams &p, uint32_t tile,
 	auto kern = narrow ? prune4_kernel<VT, kPow2, uint32_t>
 			   : prune4_kernel<VT, kPow2, size_t>;
 	if (smem > 48 * 1024) {
-		const cudaError_t e = cudaFuncSetAttribute(
-			kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		static SmemOptIn opted[2];
+		const cudaError_t e = opt_in_smem(kern, opted[narrow ? 0 : 1]);
 		if (e != cudaSuccess)
 			return e;
 	}
@@ -965,35 +996,6 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 	}
 	prune4_plain_kernel<<<grid, block, smem, s>>>(p);
 	return cudaGetLastError();
-}
-
-// Allows a kernel the device's whole opt-in shared memory, once per kernel
-// and device (a permission, not a reservation: no call lowers another's
-// limit and later launches pay nothing).
-struct SmemOptIn {
-	std::atomic<bool> done[64] = {};
-};
-template <typename Kernel> static cudaError_t opt_in_smem(Kernel kern, SmemOptIn &state)
-{
-	int dev = 0;
-	cudaError_t e = cudaGetDevice(&dev);
-	if (e != cudaSuccess)
-		return e;
-	if (dev >= 0 && dev < 64 && state.done[dev].load(std::memory_order_acquire))
-		return cudaSuccess;
-	int most = 0;
-	e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-	if (e != cudaSuccess)
-		return e;
-	cudaFuncAttributes fa{};
-	e = cudaFuncGetAttributes(&fa, kern);
-	if (e != cudaSuccess)
-		return e;
-	e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				 most - (int)fa.sharedSizeBytes);
-	if (e == cudaSuccess && dev >= 0 && dev < 64)
-		state.done[dev].store(true, std::memory_order_release);
-	return e;
 }
 
 size_t prune4_runs_smem(const PruneParams &p)
@@ -1127,8 +1129,8 @@ cudaError_t launch_prune4_batch(const BatchParams &p, uint32_t ctas,
 	auto kern = p.narrow ? prune4_batch_kernel<uint32_t>
 			     : prune4_batch_kernel<size_t>;
 	if (smem > 48 * 1024) {
-		const cudaError_t e = cudaFuncSetAttribute(
-			kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		static SmemOptIn opted[2];
+		const cudaError_t e = opt_in_smem(kern, opted[p.narrow ? 0 : 1]);
 		if (e != cudaSuccess)
 			return e;
 	}
@@ -1188,8 +1190,8 @@ cudaError_t launch_prune20_f64(const PruneParams &p, uint32_t groups, cudaStream
 	const size_t smem =
 		groups * sizeof(P20Group) +
 		(p.n_runs <= kP20RunsSmem ? ((size_t)p.n_runs + 1) * sizeof(uint32_t) : 0);
-	const cudaError_t e = cudaFuncSetAttribute(
-		prune20_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	static SmemOptIn opted;
+	const cudaError_t e = opt_in_smem(prune20_f64_kernel, opted);
 	if (e != cudaSuccess)
 		return e;
 	prune20_f64_kernel<<<dim3(p.ldp / kP20Tile, p.C), 128 * groups, smem, s>>>(p);
@@ -1242,8 +1244,8 @@ static cudaError_t launch_prune20tc_g(const Tc20Params &p, bool narrow, int smem
 				      cudaStream_t s)
 {
 	auto kern = narrow ? prune20tc_kernel<uint32_t, kG> : prune20tc_kernel<size_t, kG>;
-	cudaError_t e = cudaFuncSetAttribute(
-		kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	static SmemOptIn opted[2];
+	cudaError_t e = opt_in_smem(kern, opted[narrow ? 0 : 1]);
 	if (e != cudaSuccess)
 		return e;
 	// grid (K, tiles, C), clusters of the K CTAs of one work item
