@@ -912,6 +912,14 @@ uint32_t Calculator::pick_groups(uint32_t n)
 	return G;
 }
 
+// Whether the walk of G groups holds the phases (the 20-state FP32 and the
+// four-state FP64 walk keep them in shared memory).
+bool Calculator::segs_fit(uint32_t G) const
+{
+	return S_ == 20 ? segs_.size() <= prune20_seg_words(G)
+			: f32_ || segs_.size() <= prune4_f64_seg_words(G * C_);
+}
+
 // The phases of G groups (order_, segs_); false where they would not
 // shorten the longest group's work by a fifth.
 template <typename Emit>
@@ -1058,8 +1066,17 @@ bool Calculator::order_depth_first(uint32_t n)
 		uint32_t G = pick_groups(n);
 		while (G > 1 && G * chain_[n - 1] > 2 * cost_[n - 1])
 			G = S_ == 20 ? G - 1 : G / 2;
-		if (G == 1 || !split_phases(n, G, at, emit)) {
+		bool split = G > 1 && split_phases(n, G, at, emit);
+		// a long ladder's phases may be too many: fewer groups hold more
+		while (split && !segs_fit(G)) {
+			G = S_ == 20 ? G - 1 : G / 2;
 			at = 0;
+			split = G > 1 && split_phases(n, G, at, emit);
+		}
+		if (!split) {
+			at = 0;
+			order_groups_ = order_phases_ = 1;
+			segs_.assign({0u, n});
 			emit(n - 1);
 		}
 	}

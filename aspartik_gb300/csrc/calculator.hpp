@@ -197,6 +197,7 @@ class Calculator {
 	bool order_depth_first(uint32_t n);
 	template <typename Emit>
 	bool split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit);
+	bool segs_fit(uint32_t G) const;
 	void stage_inputs(const double *src, uint32_t n, size_t per_entry);
 	uint32_t tip_children_ = 0;      // tip children in the staged list
 	bool model_set_ = false;

@@ -970,6 +970,24 @@ static cudaError_t launch_prune4_t(const PruneParams &p, uint32_t tile,
 	return cudaGetLastError();
 }
 
+// Shared memory of a block of the FP64 walk without its phases.
+static size_t f64_smem(uint32_t warps)
+{
+	return sizeof(double) * (64 * (size_t)warps + 32) +
+	       (size_t)warps * kF64Ring * sizeof(F64Entry);
+}
+
+uint32_t prune4_f64_seg_words(uint32_t warps)
+{
+	const size_t rest = f64_smem(warps);
+	return rest < kSegSmem ? (uint32_t)((kSegSmem - rest) / 4) : 0u;
+}
+
+uint32_t prune20_seg_words(uint32_t groups)
+{
+	return (uint32_t)((kSegSmem - groups * kS20Ring * sizeof(S20Entry)) / 4);
+}
+
 cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 			  cudaStream_t s)
 {
@@ -983,11 +1001,10 @@ cudaError_t launch_prune4(const PruneParams &p, bool f32, uint32_t tile,
 		const uint32_t warps = p.C * tp / 32u * p.groups;
 		if (warps > 16 || (p.groups > 1 && !p.segs))
 			return cudaErrorInvalidValue;
-		const size_t bytes = sizeof(double) * (64 * (size_t)warps + 32) +
-				     (size_t)warps * kF64Ring * sizeof(F64Entry) +
-				     (p.groups > 1 ? ((size_t)p.phases * p.groups + 1) * 4 : 0);
-		if (bytes > 48 * 1024)
+		const size_t words = p.groups > 1 ? (size_t)p.phases * p.groups + 1 : 0;
+		if (words > prune4_f64_seg_words(warps))
 			return cudaErrorInvalidValue;
+		const size_t bytes = f64_smem(warps) + words * 4;
 		auto kern = p.groups > 1 ? (narrow ? prune4_f64_kernel<uint32_t, true>
 						   : prune4_f64_kernel<size_t, true>)
 					 : (narrow ? prune4_f64_kernel<uint32_t, false>
@@ -1212,10 +1229,10 @@ cudaError_t launch_prune20(const PruneParams &p, cudaStream_t s)
 	if (p.C == 0 || p.C > 8 || p.ldp % 128u || p.groups < 1 || p.groups > 4 ||
 	    !p.sums_host || (p.groups > 1 && !p.segs))
 		return cudaErrorInvalidValue;
-	const size_t smem = (size_t)p.groups * kS20Ring * sizeof(S20Entry) +
-			    (p.groups > 1 ? ((size_t)p.phases * p.groups + 1) * 4 : 0);
-	if (smem > 48 * 1024)
+	const size_t words = p.groups > 1 ? (size_t)p.phases * p.groups + 1 : 0;
+	if (words > prune20_seg_words(p.groups))
 		return cudaErrorInvalidValue;
+	const size_t smem = (size_t)p.groups * kS20Ring * sizeof(S20Entry) + words * 4;
 	const bool narrow = (uint64_t)p.num_leaves * 2 * p.C * p.ldp < (1ull << 31);
 	auto kern = p.groups > 1 ? (narrow ? prune20_kernel<uint32_t, true>
 					   : prune20_kernel<size_t, true>)
