@@ -80,6 +80,12 @@ __device__ __forceinline__ double ptab20_element(const PtabParams &prm, uint32_t
 	return s;
 }
 
+// NaN with a payload that split_tf32_int keeps.
+__device__ __forceinline__ float quiet_nan(float x)
+{
+	return x != x ? __uint_as_float(0x7FC00000u) : x;
+}
+
 // One thread per element, computed in FP64 (the same for both forms: the FP32
 // form only stores it in single precision) and written transposed with a 21st
 // row of ones; the FP64 form's integer table beside it.  A table is one block,
@@ -96,7 +102,10 @@ __global__ void __launch_bounds__(kS20 *kS20 / kParts) ptab20_kernel(PtabParams 
 	const uint32_t t = threadIdx.x, i = (base + t) / S, j = (base + t) - i * S;
 	const double P = ptab20_element(prm, id, t, sm, base, kCount);
 	R *out = (R *)prm.ptab + (size_t)id * (S + 1) * S;
-	out[j * S + i] = (R)P;
+	if constexpr (sizeof(R) == 4)
+		out[j * S + i] = quiet_nan((float)P);
+	else
+		out[j * S + i] = P;
 	if (t < S && base == 0)
 		out[S * S + t] = (R)1.0;
 	if constexpr (sizeof(R) == 8) {
@@ -215,7 +224,8 @@ __device__ __forceinline__ void mma_tf32_k8(float c[4], const uint32_t a[4], uin
 
 // TF32 head and tail of x as tc::split_tf32 makes them (round to nearest,
 // halves away from zero), in integer arithmetic: a conversion instruction
-// issues at an eighth of its rate.
+// issues at an eighth of its rate.  A NaN must be quiet_nan's: arithmetic's own
+// (0x7FFFFFFF) would wrap to -0, so the tables and s20_rescale replace it.
 __device__ __forceinline__ void split_tf32_int(float x, uint32_t &hi, uint32_t &lo)
 {
 	hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
@@ -299,52 +309,83 @@ __device__ __forceinline__ void s20_apply(const float *__restrict__ tab, uint32_
 		}
 }
 
+// Largest of three, NaN if one of them is.
+__device__ __forceinline__ float max3_nan(float a, float b, float c)
+{
+	float r;
+	asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+	return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+	float r;
+	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+
 // Exact power-of-two normalisation of each row's largest entry (20 states
 // over four lanes) into [1, 2), adding the exponent to the row's count (see
-// rescale_pow2).  The four rows' exchanges overlap.
+// rescale_pow2).  The four rows' exchanges overlap.  Of a row with an overflow
+// or NaN every entry that is not finite leaves as quiet_nan's NaN (an infinity
+// has no tail to split: what is multiplied with one is NaN).
 __device__ __forceinline__ void s20_rescale(S20Frag &y, int32_t cnt[2][2])
 {
 	float m[4];
 #pragma unroll
 	for (int k = 0; k < 4; k++) {
 		const float2 *v = y.v[k >> 1][k & 1];
-		m[k] = fmaxf(fmaxf(fmaxf(v[0].x, v[0].y), fmaxf(v[1].x, v[1].y)),
-			     fmaxf(v[2].x, v[2].y));
+		m[k] = max3_nan(max3_nan(v[0].x, v[0].y, v[1].x), max_nan(v[1].y, v[2].x), v[2].y);
 	}
 #pragma unroll
 	for (int k = 0; k < 4; k++)
-		m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], 1));
+		m[k] = max_nan(m[k], __shfl_xor_sync(0xffffffffu, m[k], 1));
 #pragma unroll
 	for (int k = 0; k < 4; k++)
-		m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], 2));
-	constexpr float kTiny = 1.17549435e-38f; // smallest normal number
-	if (__any_sync(0xffffffffu, (m[0] < kTiny) | (m[1] < kTiny) | (m[2] < kTiny) |
-					    (m[3] < kTiny))) {
+		m[k] = max_nan(m[k], __shfl_xor_sync(0xffffffffu, m[k], 2));
+	uint32_t rare = 0; // a maximum that is not a positive normal number
 #pragma unroll
-		for (int k = 0; k < 4; k++)
-			if (m[k] < kTiny && m[k] > 0.0f) {
-				// subnormal maximum: lift by 2^64 first (exact)
-				const float lift = 18446744073709551616.0f;
+	for (int k = 0; k < 4; k++)
+		rare = max(rare, __float_as_uint(m[k]) - 0x00800000u);
+	if (!__any_sync(0xffffffffu, rare >= 0x7F000000u)) {
 #pragma unroll
-				for (int s = 0; s < 3; s++) {
-					y.v[k >> 1][k & 1][s].x *= lift;
-					y.v[k >> 1][k & 1][s].y *= lift;
-				}
-				m[k] *= lift;
-				cnt[k >> 1][k & 1] -= 64;
+		for (int k = 0; k < 4; k++) {
+			const uint32_t e = __float_as_uint(m[k]) & 0x7F800000u;
+			const float f = __uint_as_float(0x7F000000u - e); // 2^-exponent
+			cnt[k >> 1][k & 1] += (int32_t)(e >> 23) - 127;
+#pragma unroll
+			for (int s = 0; s < 3; s++) {
+				y.v[k >> 1][k & 1][s].x *= f;
+				y.v[k >> 1][k & 1][s].y *= f;
 			}
+		}
+		return;
 	}
+	constexpr float kTiny = 1.17549435e-38f; // smallest normal number
 #pragma unroll
 	for (int k = 0; k < 4; k++) {
+		if (m[k] < kTiny && m[k] > 0.0f) {
+			// subnormal maximum: lift by 2^64 first (exact)
+			const float lift = 18446744073709551616.0f;
+#pragma unroll
+			for (int s = 0; s < 3; s++) {
+				y.v[k >> 1][k & 1][s].x *= lift;
+				y.v[k >> 1][k & 1][s].y *= lift;
+			}
+			m[k] *= lift;
+			cnt[k >> 1][k & 1] -= 64;
+		}
 		// all zero (the pattern is impossible): no scaling
 		const int32_t e =
 			m[k] > 0.0f ? (int32_t)((__float_as_uint(m[k]) >> 23) & 0xffu) - 127 : 0;
-		const float f = __uint_as_float((uint32_t)(127 - e) << 23); // 2^-e
+		const float f = __uint_as_float((uint32_t)(127 - e) << 23);
 		cnt[k >> 1][k & 1] += e;
 #pragma unroll
 		for (int s = 0; s < 3; s++) {
-			y.v[k >> 1][k & 1][s].x *= f;
-			y.v[k >> 1][k & 1][s].y *= f;
+			float2 &v = y.v[k >> 1][k & 1][s];
+			v.x *= f;
+			v.y *= f;
+			v.x = fabsf(v.x) <= 3.402823466e+38f ? v.x : quiet_nan(NAN);
+			v.y = fabsf(v.y) <= 3.402823466e+38f ? v.y : quiet_nan(NAN);
 		}
 	}
 }

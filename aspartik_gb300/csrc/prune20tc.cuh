@@ -419,7 +419,9 @@ __global__ void __launch_bounds__(128 * kG, 4 / kG) prune20tc_kernel(Tc20Params 
 				      t;
 #pragma unroll
 			for (int k = 0; k < S / 2; k++)
-				dst[k * kTcRows] = make_float2(y[2 * k], y[2 * k + 1]);
+				// (a NaN as the register walk takes it)
+				dst[k * kTcRows] =
+					make_float2(quiet_nan(y[2 * k]), quiet_nan(y[2 * k + 1]));
 		}
 		// the run's outputs are visible to every group of the cluster,
 		// and to the bulk copies of the next run, before those read them
