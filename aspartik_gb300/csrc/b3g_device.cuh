@@ -204,6 +204,7 @@ struct MemberStep {
 	uint32_t n_runs;
 	uint32_t tips_smem;
 	uint32_t tile; // patterns per tile for this step (divides ldp)
+	uint32_t fold; // the member's own tile, a multiple of it: order of the sum
 	uint32_t kind; // the kernel that walks the list
 	// a depth-first list's schedule (kListTree)
 	uint32_t groups, phases, n_slots, clean;

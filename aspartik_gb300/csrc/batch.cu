@@ -309,7 +309,8 @@ void Batch::run()
 			c->wait_stage();
 			s.n = c->staged_n_;
 			s.n_runs = c->n_runs_;
-			s.tile = std::max(16u, c->staged_tile_ >> shrink);
+			s.fold = c->staged_tile_;
+			s.tile = std::max(16u, s.fold >> shrink);
 			s.tips_smem = c->staged_tips_smem_;
 			s.clock_rate = c->staged_clock_;
 			s.kind = c->staged_kind_;
@@ -325,7 +326,7 @@ void Batch::run()
 		} else {
 			s.n = 0;
 			s.n_runs = 0;
-			s.tile = c->runs_tile_;
+			s.tile = s.fold = c->runs_tile_;
 			s.tips_smem = 0;
 			s.kind = kListRuns;
 			s.clock_rate = 1.0;

@@ -452,15 +452,21 @@ __device__ double tile_root(const TileArgs &a, uint32_t t, const float *s_dot,
 // is unused).  Pairwise FP64 over a few hundred block sums loses nothing at
 // the FP32 form's accuracy, and keeps the serial tail of the launch to a
 // few dependent FP64 adds (the pipe runs at 1/64 of the FP32 rate here).
-__device__ double block_fold(const double *sums, uint32_t count, double *s_red)
+// With `parts` > 1 every sum is given as that many parts, added in order first.
+__device__ double block_fold(const double *sums, uint32_t count, double *s_red,
+			     uint32_t parts = 1)
 {
 	(void)s_red;
 	const uint32_t tid = threadIdx.x;
 	if (tid >= 32)
 		return 0.0;
 	double sum = 0.0;
-	for (uint32_t k = tid; k < count; k += 32)
-		sum += __ldcg(sums + k);
+	for (uint32_t k = tid; k < count; k += 32) {
+		double one = 0.0;
+		for (uint32_t u = 0; u < parts; ++u)
+			one += __ldcg(sums + k * parts + u);
+		sum += one;
+	}
 	for (int off = 16; off > 0; off >>= 1)
 		sum += __shfl_down_sync(0xffffffffu, sum, off);
 	return sum;
@@ -1231,8 +1237,9 @@ __global__ void __launch_bounds__(32) ptab4_batch_kernel(BatchParams bp)
 // Persistent blocks take (member, tile) work items from a counter; members
 // are visited in the order of the descriptor array (the host puts the
 // costliest first).  Each tile's weighted sum goes to the member's tile
-// slot; the block that finishes a member's last tile folds that member's
-// sums (fixed order, so the result does not depend on scheduling).
+// slots; the block that finishes a member's last tile folds that member's
+// sums (in the order of its own tiles, MemberStep::fold, so that the result
+// depends neither on scheduling nor on the other members).
 template <typename Idx>
 __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 {
@@ -1257,6 +1264,7 @@ __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 	const uint32_t total = s_prefix[M];
 	uint32_t cur = 0xFFFFFFFFu;
 	TileArgs a;
+	uint32_t fold = 0;
 	uint32_t *s_runs = nullptr;
 	for (;;) {
 		if (tid == 0)
@@ -1282,6 +1290,7 @@ __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 			a.C = md.C;
 			a.L = md.L;
 			a.tile = st.tile;
+			fold = st.fold;
 			a.n = st.n;
 			a.n_runs = st.n_runs;
 			a.tips_smem = st.tips_smem;
@@ -1307,20 +1316,35 @@ __global__ void __launch_bounds__(512, 2) prune4_batch_kernel(BatchParams bp)
 			cur = m;
 			__syncthreads();
 		}
-		const double tsum =
-			tile_walk<Idx>(a, t, (float *)s_dot, s_cnt, s_red, s_ops,
-				       s_runs, s_tips);
-		const uint32_t tiles = md.ldp / a.tile;
-		if (tid == 0) {
-			md.tile_sums[t] = tsum;
+		tile_walk<Idx>(a, t, (float *)s_dot, s_cnt, s_red, s_ops, s_runs, s_tips);
+		// the sums of every 32 patterns, or of a tile of 16
+		const uint32_t tiles = md.ldp / a.tile, units = (a.tile + 31u) / 32u;
+		if (tid < 32) {
+			if (tid < units)
+				md.tile_sums[t * units + tid] = s_red[tid];
 			__threadfence();
-			const unsigned tk = atomicAdd(md.ticket, 1u);
-			s_last = (tk == tiles - 1u);
+			__syncwarp();
+			if (tid == 0)
+				s_last = atomicAdd(md.ticket, 1u) == tiles - 1u;
 		}
 		__syncthreads();
 		if (s_last) {
 			__threadfence();
-			const double lnl = block_fold(md.tile_sums, tiles, s_red);
+			if (a.tile < min(fold, 32u)) {
+				// halves of a warp's patterns: its sum over again, from
+				// the site values, in tile_root's order
+				for (uint32_t p = tid; p < md.ldp; p += blockDim.x) {
+					const uint32_t wgt = md.weights[p];
+					double sum = wgt ? __ldcg(md.site_lnl + p) * (double)wgt : 0.0;
+					for (int off = 16; off > 0; off >>= 1)
+						sum += __shfl_down_sync(0xffffffffu, sum, off);
+					if ((tid & 31u) == 0)
+						md.tile_sums[p / 32u] = sum;
+				}
+				__syncthreads();
+			}
+			const double lnl = block_fold(md.tile_sums, md.ldp / fold, s_red,
+						      (fold + 31u) / 32u);
 			if (tid == 0) {
 				bp.lnl_out[m] = lnl;
 				*md.ticket = 0u;
