@@ -67,6 +67,7 @@ struct TreeHead {
 	uint32_t barriers; // phases without an entry before it
 };
 constexpr uint32_t kTreeChunk = 4;   // entries copied together
+constexpr uint32_t kTreeRing = 4 * kTreeChunk; // entries in a group's ring
 
 // One entry of the children-first schedule: output slot and the two
 // children, each either a partial slot or (kTipBit | leaf id).

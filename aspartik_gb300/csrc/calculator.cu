@@ -178,13 +178,10 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	if (use_tree_) { // the first list finds its workspaces
 		tree_swap_.assign(I_, 0);
 		list_ops_.resize(I_);
-		for (auto *v : {&order_, &parent_, &cost_, &chain_, &tree_order_, &tree_ends_,
-				&walk_stack_, &segs_})
-			v->assign(I_, 0);
+		for (auto *v : {&order_, &pos_of_, &tree_order_, &tree_ends_, &segs_})
+			v->assign(I_ + 1, 0);
+		nodes_.resize(I_ + 1);
 		kid_.assign(2ull * I_, 0);
-		tree_pools_.resize(16);
-		for (auto &pool : tree_pools_)
-			pool.reserve(256);
 	}
 	if (const char *env = std::getenv("B3G_TREE_TILE"))
 		tree_tile_fixed_ = std::atoi(env) == 128 ? 128u : 64u;
@@ -193,8 +190,7 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	stamp_.assign(2 * L_ - 1, 0);
 	pos_.assign(2 * L_ - 1, 0);
 	run_of_.assign(I_, 0);
-	smem_of_.assign(2ull * I_, static_cast<uint8_t>(kNoSlot));
-	slot_pos_.assign(2ull * I_, kNone);
+	smem_of_.assign(2ull * I_ + 1, static_cast<uint8_t>(kNoSlot));
 	if (f32_ && S_ == 20)
 		for (uint32_t w = 1; w <= 4; ++w)
 			s20_per_sm_[w] = prune20_blocks_per_sm(w);
@@ -487,6 +483,22 @@ void Calculator::validate_lists(const uint32_t *internals,
 	}
 }
 
+namespace {
+// c ? a : b without a branch.  Branches on a list's shape are mispredicted
+// unless the same list comes again: with them the schedules of 32 whole trees of
+// 184 taxa took 10.1 us each, more than the batch's depth-first kernel saved, now
+// 5.5 (a step of such lists, 1,172 patterns x 4 categories: 566 us by the run
+// walk, 643, 488); one tree over and over took 4.8 and takes 5.1.
+uint32_t pick(bool c, uint32_t a, uint32_t b) { return b ^ ((a ^ b) & (0u - (uint32_t)c)); }
+
+// At least n elements (growing again and again would clear them every time).
+template <typename T> void fit(std::vector<T> &v, size_t n)
+{
+	if (v.size() < n)
+		v.resize(n);
+}
+} // namespace
+
 // Flips the selectors of the listed internals (Cpu4Calculator::
 // set_selectors, cpu4.rs:93-98) and writes the schedule: output slot of each
 // listed node and the slot or leaf of each child.
@@ -501,17 +513,7 @@ void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
 		return k * 2 + (selectors_[k] & 1u);
 	};
 	if (tree) {
-		list_ops_.resize(n);
-		tip_children_ = 0;
-		for (uint32_t i = 0; i < n; ++i) {
-			const uint32_t l = children[2 * i], r = children[2 * i + 1];
-			NodeOp &op = list_ops_[i];
-			op.out = slot_of(internals[i]);
-			op.left = l < L_ ? (kTipBit | l) : slot_of(l);
-			op.right = r < L_ ? (kTipBit | r) : slot_of(r);
-			tip_children_ += (l < L_) + (r < L_);
-		}
-		depth_first_ = order_depth_first(n);
+		depth_first_ = order_depth_first(internals, children, n);
 		if (depth_first_) {
 			stage_tree(n);
 			return;
@@ -563,8 +565,7 @@ void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
 	depth_first_ = S_ == 4 ? !f32_ : f32_ && !use_tc20_;
 	if (!depth_first_)
 		return;
-	list_ops_.assign(ops, ops + n);
-	order_depth_first(n);
+	order_depth_first(internals, children, n);
 	stage_order(n);
 }
 
@@ -593,8 +594,8 @@ void Calculator::stage_tree(uint32_t n)
 	uint32_t *segs = reinterpret_cast<uint32_t *>(h_stage_ + off_runs_);
 	TreeHead *heads = reinterpret_cast<TreeHead *>(segs + G + 1);
 	// phase-major (order_, segs_) to group-major
-	tree_order_.resize(n);
-	tree_ends_.resize((size_t)G * phases);
+	fit(tree_order_, n);
+	fit(tree_ends_, (size_t)G * phases);
 	uint32_t at = 0;
 	for (uint32_t g = 0; g < G; ++g) {
 		segs[g] = at;
@@ -607,141 +608,162 @@ void Calculator::stage_tree(uint32_t n)
 	segs[G] = n;
 	order_.swap(tree_order_);
 	// children's kinds: the group's previous output first, a tip last
-	for (uint32_t g = 0; g < G; ++g)
+	const NodeOp *const words = list_ops_.data();
+	uint8_t *const swaps = tree_swap_.data();
+	for (uint32_t g = 0; g < G; ++g) {
+		uint32_t prev = kNone;
 		for (uint32_t e = segs[g]; e < segs[g + 1]; ++e) {
-			const NodeOp &in = list_ops_[order_[e]];
-			const uint32_t prev = e > segs[g] ? ops[e - 1].out : kNone;
-			const bool lt = (in.left & kTipBit) != 0, rt = (in.right & kTipBit) != 0;
-			const bool swap = in.right == prev || (in.left != prev && lt && !rt);
-			TreeOp op{};
-			op.out = in.out;
-			op.id[0] = swap ? in.right : in.left;
-			op.id[1] = swap ? in.left : in.right;
-			op.code = (op.id[0] & kTipBit ? 0u : kTreeInA) |
-				  (op.id[1] & kTipBit ? 0u : kTreeInB) |
-				  (op.id[0] == prev ? kTreePrev : 0u);
-			tree_swap_[e] = swap;
-			ops[e] = op;
+			const NodeOp &in = words[order_[e]];
+			const uint32_t l = in.left, r = in.right;
+			const uint32_t swap = (uint32_t)(r == prev) |
+					      ((uint32_t)(l != prev) & ((l & ~r) / kTipBit));
+			const uint32_t flip = (l ^ r) & (0u - swap), a = l ^ flip, b = r ^ flip;
+			const uint32_t code = (~a / kTipBit) * kTreeInA | (~b / kTipBit) * kTreeInB |
+					      (uint32_t)(a == prev) * kTreePrev;
+			swaps[e] = static_cast<uint8_t>(swap);
+			ops[e] = TreeOp{in.out, code, 0, 0, {a, b}, 0, 0};
+			prev = in.out;
 		}
-	tree_pools_.resize(std::max<size_t>(tree_pools_.size(), G));
-	uint32_t used = 0, capacity = 0, missing = 0;
-	auto take = [&](uint32_t g) -> uint32_t {
-		auto &pool = tree_pools_[g];
-		if (!pool.empty()) {
-			const uint32_t s = pool.back();
-			pool.pop_back();
-			return s;
-		}
-		if (used < capacity)
-			return used++;
-		++missing;
-		return kNoSlot;
-	};
-	auto fetch = [&](uint32_t g, uint32_t chunk) { // its clean children
-		const uint32_t lo = segs[g] + chunk * kTreeChunk;
-		for (uint32_t e = lo; e < std::min(lo + kTreeChunk, segs[g + 1]); ++e) {
-			const uint32_t *kid = &kid_[2 * (size_t)order_[e]];
-			for (uint32_t j = 0; j < 2; ++j) {
-				if (!(ops[e].code & (j ? kTreeInB : kTreeInA)) ||
-				    kid[j ^ tree_swap_[e]] != kNone)
-					continue;
-				const uint32_t s = take(g);
-				if (s == kNoSlot) {
-					ops[e].code |= j ? kTreeMemB : kTreeMemA;
-					continue;
-				}
-				ops[e].more |= (j ? kTreeCleanB : kTreeCleanA) |
-					       s << (j ? 16 : 8);
-				tree_clean_ = true;
-			}
-		}
-	};
-	auto assign = [&] {
+	}
+	// (a whole tree's list has no child outside it)
+	const bool any_clean = 2 * n - tip_children_ != n - 1;
+	const uint32_t none = 2 * I_; // smem_of_ holds kNoSlot there
+	uint32_t slots_used = 0;
+	// (byte stores may alias the members)
+	uint8_t *const smem = smem_of_.data();
+	const uint32_t *const order = order_.data();
+	auto assign = [&]() -> uint32_t { // entries and children without a slot
 		const size_t rest = prune4_tree_smem(pp);
-		capacity = 1 + static_cast<uint32_t>(std::min<size_t>(
-				       254, rest < budget ? (budget - rest) / (tile * 20 * C_) : 0));
-		for (auto &pool : tree_pools_)
-			pool.clear();
-		used = missing = 0;
+		const uint32_t capacity =
+			1 + static_cast<uint32_t>(std::min<size_t>(
+				    254, rest < budget ? (budget - rest) / (tile * 20 * C_) : 0));
+		uint32_t used = 0, missing = 0, have[16] = {};
+		uint8_t pool[16][258]; // a group's free slots: [1] .. [have]
 		tree_clean_ = false;
-		for (uint32_t g = 0; g < G; ++g) {
+		auto take = [&](const uint8_t *free, uint32_t &h, bool want) -> uint32_t {
+			const bool old = want & (h != 0), fresh = want & !old & (used < capacity);
+			const uint32_t s = pick(old, free[h], pick(fresh, used, kNoSlot));
+			h -= old;
+			used += fresh;
+			missing += want & !old & !fresh;
+			return s;
+		};
+		auto fetch = [&](uint32_t g, uint32_t chunk) { // its clean children
+			const uint32_t lo = segs[g] + chunk * kTreeChunk;
+			for (uint32_t e = lo; e < std::min(lo + kTreeChunk, segs[g + 1]); ++e) {
+				const uint32_t *kid = &kid_[2 * (size_t)order[e]];
+				for (uint32_t j = 0; j < 2; ++j) {
+					if (!(ops[e].code & (j ? kTreeInB : kTreeInA)) ||
+					    kid[j ^ tree_swap_[e]] != n)
+						continue;
+					const uint32_t s = take(pool[g], have[g], true);
+					if (s == kNoSlot) {
+						ops[e].code |= j ? kTreeMemB : kTreeMemA;
+						continue;
+					}
+					ops[e].more |= (j ? kTreeCleanB : kTreeCleanA) |
+						       s << (j ? 16 : 8);
+					tree_clean_ = true;
+				}
+			}
+		};
+		for (auto &free : pool)
+			free[0] = 0;
+		for (uint32_t g = 0; any_clean && g < G; ++g) {
 			fetch(g, 0);
 			fetch(g, 1);
 		}
+		// a child that waits in a slot: its slot is free behind the entry
+		auto read = [&](const TreeOp &op, uint32_t j, uint32_t &code, uint32_t &more,
+				uint8_t *free, uint32_t &h) {
+			const uint32_t mem = j ? kTreeMemB : kTreeMemA, shift = j ? 16 : 8;
+			const bool need = ((code & (j ? kTreeInB : kTreeInA)) != 0) &
+					  ((code & mem) == 0);
+			const bool clean = more & (j ? kTreeCleanB : kTreeCleanA);
+			const uint32_t kept = smem[pick(need & !clean, op.id[j], none)];
+			const uint32_t s = pick(clean, more >> shift & 0xFFu, kept);
+			if (need & (s == kNoSlot)) {
+				code |= mem;
+				return;
+			}
+			more |= pick(need & !clean, s << shift, 0u);
+			free[h + 1] = static_cast<uint8_t>(s);
+			h += need;
+		};
 		for (uint32_t ph = 0; ph < phases; ++ph)
-			for (uint32_t g = 0; g < G; ++g)
-				for (uint32_t e = ph ? tree_ends_[(ph - 1) * G + g] : segs[g];
-				     e < tree_ends_[ph * G + g]; ++e) {
-					if ((e - segs[g]) % kTreeChunk == 0)
+			for (uint32_t g = 0; g < G; ++g) {
+				uint8_t *const free = pool[g];
+				uint32_t h = have[g];
+				const uint32_t from = ph ? tree_ends_[(ph - 1) * G + g] : segs[g];
+				const uint32_t to = tree_ends_[ph * G + g], end = segs[g + 1];
+				for (uint32_t e = from; e < to; ++e) {
+					if (any_clean && (e - segs[g]) % kTreeChunk == 0) {
+						have[g] = h;
 						fetch(g, (e - segs[g]) / kTreeChunk + 2);
-					TreeOp &op = ops[e];
-					for (uint32_t j = 0; j < 2; ++j) {
-						if (!(op.code & (j ? kTreeInB : kTreeInA)) ||
-						    (j == 0 && (op.code & kTreePrev)) ||
-						    (op.code & (j ? kTreeMemB : kTreeMemA)))
-							continue;
-						if (!(op.more & (j ? kTreeCleanB : kTreeCleanA))) {
-							const uint32_t s = smem_of_[op.id[j]];
-							if (s == kNoSlot) {
-								op.code |= j ? kTreeMemB : kTreeMemA;
-								continue;
-							}
-							op.more |= s << (j ? 16 : 8);
-						}
-						tree_pools_[g].push_back(static_cast<uint8_t>(
-							op.more >> (j ? 16 : 8)));
+						h = have[g];
 					}
+					TreeOp &op = ops[e];
+					uint32_t code = op.code, more = op.more;
+					// (rare but for clean children)
+					if ((code & (kTreeInA | kTreePrev)) == kTreeInA)
+						read(op, 0, code, more, free, h);
+					read(op, 1, code, more, free, h);
 					// the root, and what the next entry takes from registers,
 					// need no slot
-					if (order_[e] == n - 1 ||
-					    (e + 1 < segs[g + 1] && (ops[e + 1].code & kTreePrev)))
-						continue;
-					const uint32_t s = take(g);
-					smem_of_[op.out] = static_cast<uint8_t>(s);
-					if (s != kNoSlot)
-						op.code |= kTreeKeep | s << 8;
+					const bool last = e + 1 == end;
+					const bool keep = (order[e] != n - 1) &
+							  (last | !(ops[e + !last].code & kTreePrev));
+					const uint32_t s = take(free, h, keep);
+					smem[op.out] = static_cast<uint8_t>(s);
+					op.code = code | pick(s != kNoSlot, kTreeKeep | s << 8, 0u);
+					op.more = more;
 				}
+				have[g] = h;
+			}
+		slots_used = used;
+		return missing;
 	};
-	assign();
-	if (missing && pp.tips_smem) { // the tips' room for slots
+	if (assign() && pp.tips_smem) { // the tips' room for slots
 		pp.tips_smem = 0;
 		for (uint32_t e = 0; e < n; ++e) {
 			ops[e].code &= kTreeInA | kTreeInB | kTreePrev;
 			ops[e].more = 0;
 			smem_of_[ops[e].out] = static_cast<uint8_t>(kNoSlot);
 		}
-		assign();
+		(void)assign();
 	}
 	for (uint32_t i = 0; i < n; ++i)
 		smem_of_[ops[i].out] = static_cast<uint8_t>(kNoSlot);
-	tree_slots_ = std::max(1u, used);
+	tree_slots_ = std::max(1u, slots_used);
 	tree_tips_ = pp.tips_smem;
 	// what the words and heads read ahead, and the ends of the phases
 	const uint32_t other = pp.tips_smem ? L_ * tile : kTreeNoTip;
-	auto tip = [&](uint32_t e, uint32_t j) {
-		const uint32_t id = ops[e].id[j];
-		return !(id & kTipBit) ? other : (id & ~kTipBit) * (pp.tips_smem ? tile : 1u);
-	};
-	auto base = [&](uint32_t g, uint32_t e) {
-		if (!(ops[e].code & kTreeInB))
-			return prune4_tree_entry(g, e - segs[g]);
-		return prune4_tree_slot(G, tile, ops[e].more >> 16 & 0xFFu);
-	};
+	const uint32_t row = pp.tips_smem ? tile : 1u;
+	auto tip = [&](uint32_t id) { return pick(id / kTipBit, (id & ~kTipBit) * row, other); };
+	const uint32_t slot0 = prune4_tree_slot(G, tile, 0);
+	const uint32_t pitch = prune4_tree_slot(G, tile, 1) - slot0;
+	const uint32_t step = prune4_tree_entry(0, 1) - prune4_tree_entry(0, 0);
 	for (uint32_t g = 0; g < G; ++g) {
 		const uint32_t lo = segs[g], hi = segs[g + 1];
 		TreeHead &h = heads[g];
 		h = TreeHead{};
-		if (hi > lo) {
-			h.tip[0] = tip(lo, 0);
-			h.tip[1] = tip(lo, 1);
-			h.base = base(g, lo);
-		}
-		h.tip[2] = hi > lo + 1 ? tip(lo + 1, 1) : 0;
+		const uint32_t entry0 = prune4_tree_entry(g, 0);
+		TreeOp first[2] = {}; // stand for the two words before the group's first
+		TreeOp *before = &first[0], *last = &first[1];
 		for (uint32_t e = lo; e < hi; ++e) {
-			ops[e].next_a = e + 1 < hi ? tip(e + 1, 0) : 0;
-			ops[e].code |= (e + 1 < hi ? base(g, e + 1) : 0) << 16;
-			ops[e].after_b = e + 2 < hi ? tip(e + 2, 1) : 0;
+			TreeOp &op = ops[e];
+			last->next_a = tip(op.id[0]);
+			before->after_b = tip(op.id[1]);
+			last->code |= pick(op.code & kTreeInB, slot0 + (op.more >> 16 & 0xFFu) * pitch,
+					   entry0 + (e - lo) % kTreeRing * step)
+				      << 16;
+			before = last;
+			last = &op;
 		}
+		h.tip[0] = first[1].next_a;
+		h.tip[1] = first[0].after_b;
+		h.tip[2] = first[1].after_b;
+		h.base = first[1].code >> 16;
 		// (the last phase needs no barrier)
 		for (uint32_t ph = 0; ph + 1 < phases; ++ph) {
 			const uint32_t end = tree_ends_[ph * G + g];
@@ -920,47 +942,52 @@ bool Calculator::segs_fit(uint32_t G) const
 			: f32_ || segs_.size() <= prune4_f64_seg_words(G * C_);
 }
 
-// The phases of G groups (order_, segs_); false where they would not
+// The phases of G groups (segs_, and pos_of_ the entries above and the pieces'
+// roots); false where they would not
 // shorten the longest group's work by a fifth.
-template <typename Emit>
-bool Calculator::split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit)
+bool Calculator::split_phases(uint32_t n, uint32_t G)
 {
+	above_mark_.assign(n, 0);
+	uint32_t at = 0;
 	// split the costliest subtree until the pieces balance; what is split
 	// belongs to the entries above
 	std::vector<uint32_t> &piece = pieces_, &above = above_;
 	piece.assign(1, n - 1);
 	above.clear();
 	while (!piece.empty() && piece.size() < 4 * G) {
-		size_t top = 0;
-		for (size_t k = 1; k < piece.size(); ++k)
-			if (cost_[piece[k]] > cost_[piece[top]])
-				top = k;
+		uint64_t most = 0; // the first of the costliest
+		for (size_t k = 0; k < piece.size(); ++k)
+			most = std::max(most, (uint64_t)nodes_[piece[k]].cost << 32 | (uint32_t)~k);
+		const size_t top = (uint32_t)~(uint32_t)most;
 		const uint32_t v = piece[top];
-		if (v != n - 1 && cost_[v] * 2 * G <= cost_[n - 1])
+		if (v != n - 1 && nodes_[v].cost * 2 * G <= nodes_[n - 1].cost)
 			break;
 		above.push_back(v);
+		above_mark_[v] = 1;
 		piece[top] = piece.back();
 		piece.pop_back();
 		for (int j = 0; j < 2; ++j)
-			if (kid_[2 * v + j] != kNone)
+			if (kid_[2 * v + j] != n)
 				piece.push_back(kid_[2 * v + j]);
 	}
 	std::sort(piece.begin(), piece.end(), [&](uint32_t a, uint32_t b) {
-		return cost_[a] != cost_[b] ? cost_[a] > cost_[b] : a < b;
+		return nodes_[a].cost != nodes_[b].cost ? nodes_[a].cost > nodes_[b].cost : a < b;
 	});
 	std::sort(above.begin(), above.end()); // children first
 	// a piece goes to the least loaded group
 	uint32_t load[16] = {}, owner[80];
 	for (size_t k = 0; k < piece.size(); ++k) {
 		owner[k] = (uint32_t)(std::min_element(load, load + G) - load);
-		load[owner[k]] += cost_[piece[k]];
+		load[owner[k]] += nodes_[piece[k]].cost;
 	}
 	segs_.clear();
 	for (uint32_t w = 0; w < G; ++w) {
 		segs_.push_back(at);
 		for (size_t k = 0; k < piece.size(); ++k)
-			if (owner[k] == w)
-				emit(piece[k]);
+			if (owner[k] == w) {
+				at += nodes_[piece[k]].size;
+				pos_of_[piece[k]] = at - 1;
+			}
 	}
 	uint32_t longest = *std::max_element(load, load + G);
 	// the entries above: runs of independent entries, each dealt out in
@@ -981,13 +1008,13 @@ bool Calculator::split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit)
 			segs_.push_back(at + (len * w + G - 1) / G);
 		}
 		for (size_t k = i; k < j; ++k)
-			order_[at++] = above[k];
+			pos_of_[above[k]] = at++;
 		longest += (len + G - 1) / G * 6 + 4; // entries, and the barrier
 		++phases;
 		i = j;
 	}
 	segs_.push_back(at);
-	if (longest * 5 > cost_[n - 1] * 4 || segs_.size() > (size_t)I_ + 1) {
+	if (longest * 5 > nodes_[n - 1].cost * 4 || segs_.size() > (size_t)I_ + 1) {
 		segs_.assign({0u, n});
 		return false;
 	}
@@ -996,91 +1023,99 @@ bool Calculator::split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit)
 	return true;
 }
 
-// Orders the list (list_ops_) depth first, heavier subtree first, so that a
-// child is mostly the previous entry's output, and for several groups splits
-// it into phases (segs_): disjoint subtrees, a balanced share a group, then
+// The list's words (list_ops_), ordered depth first, heavier subtree first, so
+// that a child is mostly the previous entry's output, and for several groups
+// split into phases (segs_): disjoint subtrees, a balanced share a group, then
 // the entries above them, run by run.  Every entry's arithmetic is the same
 // in any children-first order.  order_[k] = list position of staged entry k.
 // A list that is not one tree under its last entry keeps its order (false).
-bool Calculator::order_depth_first(uint32_t n)
+bool Calculator::order_depth_first(const uint32_t *internals, const uint32_t *children,
+				   uint32_t n)
 {
-	order_.resize(n);
-	kid_.assign(2 * (size_t)n, kNone);
-	parent_.assign(n, kNone);
-	cost_.resize(n);
-	chain_.resize(n);
-	uint32_t linked = 0;
-	bool tree = true;
-	for (uint32_t i = 0; i < n; ++i)
-		slot_pos_[list_ops_[i].out] = i;
+	fit(order_, n);
+	fit(list_ops_, n);
+	fit(kid_, 2 * (size_t)n);
+	fit(pos_of_, (size_t)n + 1);
+	fit(nodes_, (size_t)n + 1);
+	// (in locals: the stores below could alias the members)
+	const uint32_t *const stamp = stamp_.data();
+	const uint8_t *const sel = selectors_.data();
+	uint32_t *const pos = pos_.data(), *const kids = kid_.data();
+	ListNode *const nodes = nodes_.data();
+	NodeOp *const words = list_ops_.data();
+	const uint32_t L = L_, epoch = stamp_epoch_;
+	// a child that is not listed is entry n, of cost and size zero
+	nodes[n] = ListNode{0, 0, 0, kNone};
+	uint32_t linked = 0, inner = 0, twice = 0;
 	for (uint32_t i = 0; i < n; ++i) {
-		const uint32_t ids[2] = {list_ops_[i].left, list_ops_[i].right};
-		uint32_t cost = 2; // an entry, and more for each internal child
-		uint32_t below = 0;
+		// an entry's cost: 2, and 3 more for each internal child
+		uint32_t cost = 2, size = 1, chain = 0, id[2], ins = 0;
 		for (int j = 0; j < 2; ++j) {
-			if (ids[j] & kTipBit)
-				continue;
-			cost += 3;
-			const uint32_t k = slot_pos_[ids[j]];
-			if (k == kNone)
-				continue;
-			tree = tree && parent_[k] == kNone;
-			parent_[k] = i;
-			kid_[2 * i + j] = k;
-			cost += cost_[k];
-			below = std::max(below, chain_[k]);
-			++linked;
+			const uint32_t v = children[2 * i + j];
+			const uint32_t in = v < L ? 0u : kNone; // masks
+			const uint32_t k = (v - L) & in;
+			id[j] = ((kTipBit | v) & ~in) | ((2 * k + (sel[k] & 1u)) & in);
+			ins += in & 1u;
+			// (validate_lists left stamp_epoch_ on every listed internal)
+			const uint32_t is = stamp[v] == epoch ? kNone : 0u;
+			const uint32_t at = n + ((pos[v] - n) & is);
+			ListNode &kid = nodes[at];
+			twice |= (kid.parent + 1u) & is;
+			kid.parent = i;
+			kids[2 * i + j] = at;
+			cost += kid.cost;
+			size += kid.size;
+			chain = std::max(chain, kid.chain);
+			linked += is & 1u;
 		}
-		chain_[i] = below + 2 + 3 * !(ids[0] & kTipBit) + 3 * !(ids[1] & kTipBit);
-		cost_[i] = cost;
+		const uint32_t v = internals[i], k = v - L;
+		words[i] = NodeOp{2 * k + (sel[k] & 1u), id[0], id[1], 0};
+		pos[v] = i;
+		inner += ins;
+		nodes[i] = ListNode{cost + 3 * ins, chain + 2 + 3 * ins, size, kNone};
 	}
-	for (uint32_t i = 0; i < n; ++i)
-		slot_pos_[list_ops_[i].out] = kNone;
+	const bool tree = twice == 0;
+	tip_children_ = 2 * n - inner;
 	order_groups_ = 1;
 	order_phases_ = 1;
 	segs_.assign({0u, n});
-	uint32_t at = 0;
-	// post-order of the subtree of r, heavier children first
-	auto emit = [&](uint32_t r) {
-		walk_stack_.assign(1, r);
-		const uint32_t begin = at;
-		while (!walk_stack_.empty()) {
-			const uint32_t v = walk_stack_.back();
-			walk_stack_.pop_back();
-			order_[at++] = v; // reversed below: parent, light, heavy
-			uint32_t a = kid_[2 * v], b = kid_[2 * v + 1];
-			if (a != kNone && b != kNone && cost_[a] < cost_[b])
-				std::swap(a, b);
-			if (a != kNone)
-				walk_stack_.push_back(a);
-			if (b != kNone)
-				walk_stack_.push_back(b);
-		}
-		std::reverse(order_.begin() + begin, order_.begin() + at);
-	};
 	if (!tree || linked + 1 != n) {
 		for (uint32_t i = 0; i < n; ++i)
 			order_[i] = i;
-	} else {
-		// at most twice the list's work over its longest chain
-		uint32_t G = pick_groups(n);
-		while (G > 1 && G * chain_[n - 1] > 2 * cost_[n - 1])
-			G = S_ == 20 ? G - 1 : G / 2;
-		bool split = G > 1 && split_phases(n, G, at, emit);
-		// a long ladder's phases may be too many: fewer groups hold more
-		while (split && !segs_fit(G)) {
-			G = S_ == 20 ? G - 1 : G / 2;
-			at = 0;
-			split = G > 1 && split_phases(n, G, at, emit);
-		}
-		if (!split) {
-			at = 0;
-			order_groups_ = order_phases_ = 1;
-			segs_.assign({0u, n});
-			emit(n - 1);
-		}
+		return false;
 	}
-	return tree && linked + 1 == n;
+	// at most twice the list's work over its longest chain
+	uint32_t G = pick_groups(n);
+	while (G > 1 && G * nodes_[n - 1].chain > 2 * nodes_[n - 1].cost)
+		G = S_ == 20 ? G - 1 : G / 2;
+	bool split = G > 1 && split_phases(n, G);
+	// a long ladder's phases may be too many: fewer groups hold more
+	while (split && !segs_fit(G)) {
+		G = S_ == 20 ? G - 1 : G / 2;
+		split = G > 1 && split_phases(n, G);
+	}
+	if (!split) {
+		order_groups_ = order_phases_ = 1;
+		segs_.assign({0u, n});
+		above_mark_.assign(n, 0);
+		pos_of_[n - 1] = n - 1;
+	}
+	// post-order from the roots' places down, the heavier child's subtree
+	// first, so that the lighter child ends just before its parent
+	uint32_t *const place = pos_of_.data(), *const order = order_.data();
+	const uint8_t *const above = above_mark_.data();
+	for (uint32_t v = n; v-- > 0;) {
+		const uint32_t at = place[v];
+		order[at] = v;
+		const uint32_t a = kids[2 * v], b = kids[2 * v + 1];
+		const uint32_t flip = (a ^ b) & (0u - (uint32_t)(nodes[a].cost < nodes[b].cost));
+		const uint32_t heavy = a ^ flip, light = b ^ flip;
+		// (the children of an entry above the pieces have their places)
+		const uint32_t set = above[v] - 1u;
+		place[n + ((light - n) & set)] = at - 1;
+		place[n + ((heavy - n) & set)] = at - 1 - nodes[light].size;
+	}
+	return true;
 }
 
 // The ordered list's schedule words (the walks but the FP32 four-state one).
@@ -1116,6 +1151,12 @@ void Calculator::stage_inputs(const double *src, uint32_t n, size_t per_entry)
 	}
 	if (S_ == 4 && f32_) { // children in the schedule's order
 		const size_t half = per_entry / 2;
+		for (uint32_t k = 0; half == 1 && k < n; ++k) { // lengths
+			dst[2 * k] = src[2 * order_[k] + tree_swap_[k]];
+			dst[2 * k + 1] = src[2 * order_[k] + (tree_swap_[k] ^ 1u)];
+		}
+		if (half == 1)
+			return;
 		for (uint32_t k = 0; k < n; ++k)
 			for (uint32_t j = 0; j < 2; ++j)
 				std::memcpy(dst + k * per_entry + j * half,

@@ -188,15 +188,17 @@ class Calculator {
 	bool tree_clean_ = false, tree_batch_ = false; // (staging for a batch)
 	std::vector<uint32_t> tree_order_, tree_ends_;
 	std::vector<uint8_t> tree_swap_; // staged entry: first child is the right one
-	std::vector<std::vector<uint8_t>> tree_pools_;
 	uint32_t order_groups_ = 1, order_phases_ = 1;
-	std::vector<uint32_t> order_, segs_, kid_, parent_, cost_, chain_, walk_stack_, pieces_,
-		above_;
-	std::vector<uint32_t> slot_pos_; // by partial slot; kNone outside the call
+	struct ListNode {
+		uint32_t cost, chain; // of the subtree's entries, of its longest path
+		uint32_t size, parent;
+	};
+	std::vector<ListNode> nodes_;
+	std::vector<uint32_t> order_, segs_, kid_, pos_of_, pieces_, above_;
+	std::vector<uint8_t> above_mark_; // entries above the pieces (split_phases)
 	std::vector<NodeOp> list_ops_;
-	bool order_depth_first(uint32_t n);
-	template <typename Emit>
-	bool split_phases(uint32_t n, uint32_t G, uint32_t &at, Emit emit);
+	bool order_depth_first(const uint32_t *internals, const uint32_t *children, uint32_t n);
+	bool split_phases(uint32_t n, uint32_t G);
 	bool segs_fit(uint32_t G) const;
 	void stage_inputs(const double *src, uint32_t n, size_t per_entry);
 	uint32_t tip_children_ = 0;      // tip children in the staged list

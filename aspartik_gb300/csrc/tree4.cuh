@@ -34,8 +34,6 @@
 // wait on fixed latencies and shared-memory reads.  16 warps an SM (four
 // groups) were no faster (91 against 88 us a call), more at fewer registers
 // spill and were slower (96 -> 113 us).
-constexpr uint32_t kTreeRing = 4 * kTreeChunk;
-
 struct __align__(16) TreeEntry {
 	float4 tab[10]; // first child's four rows and ones, second's
 	TreeOp op;
