@@ -144,9 +144,13 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	}
 	// 20-state FP32 lists on the tensor cores: B3G_TC20=1, or a launch shape
 	// of that engine fixed by one of the two switches above
+	// (B3G_TC20=0: not at all, the autotuner does not try it either)
 	use_tc20_ = f32_ && S_ == 20 && (tc20_cluster_fixed_ || tc20_groups_fixed_);
-	if (const char *env = std::getenv("B3G_TC20"))
+	bool tc20_off = false;
+	if (const char *env = std::getenv("B3G_TC20")) {
 		use_tc20_ = f32_ && S_ == 20 && std::atoi(env) != 0;
+		tc20_off = std::atoi(env) == 0;
+	}
 	// groups of the FP64 run form (B3G_F64_GROUPS: 1, 2, 4, 8 or 16 where
 	// they fit a block; default: chosen per list)
 	if (const char *env = std::getenv("B3G_F64_GROUPS")) {
@@ -250,7 +254,7 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		dev_alloc(d_block_sums_, nblocks * sizeof(double), "block sums");
 		dev_alloc(d_ticket_, sizeof(unsigned), "ticket");
 		dev_alloc(d_lnl_, sizeof(double), "lnl");
-		if (f32_ && S_ == 20) {
+		if (f32_ && S_ == 20 && !tc20_off) {
 			dev_alloc(d_tc_tab_, (size_t)I_ * 2 * C_ * 2 * 768 * sizeof(float),
 				  "tensor-core tables");
 			dev_alloc(d_status_, sizeof(unsigned), "status");
