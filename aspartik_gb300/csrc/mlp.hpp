@@ -56,7 +56,7 @@ class Mlp {
 		    float *out);
 
       private:
-	void ensure_batch(uint32_t rows);
+	void ensure_batch(uint32_t rows, bool gradient);
 	void free_batch();
 	void forward_device(uint32_t rows); // d_x_ rows -> d_z_, d_a_
 	void backward_device(uint32_t n);   // n pairs -> d_loss_, d_grad_
@@ -71,6 +71,8 @@ class Mlp {
 	uint32_t adam_t_ = 0;
 	// activations for up to cap_ rows: z (pre) and a (post) per layer
 	uint32_t cap_ = 0;
+	// rows of a gradient, and parts of a split weight gradient
+	uint32_t grads_cap_ = 0, parts_cap_ = 0;
 	unsigned char *d_batch_ = nullptr; // holds the buffers below up to d_tickets_
 	float *d_x_ = nullptr;
 	float *d_z_[kLayers - 1] = {};
