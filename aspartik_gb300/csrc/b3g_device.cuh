@@ -45,7 +45,6 @@ constexpr uint32_t kTreeCleanA = 1u, kTreeCleanB = 2u; // (more) copied to its s
 // the kinds with code of their own
 constexpr uint32_t kTreeKind = kTreeInA | kTreeInB | kTreePrev | kTreeMemA | kTreeMemB;
 constexpr uint32_t kTreeTipTip = 0u, kTreePrevTip = kTreeInA | kTreePrev;
-constexpr uint32_t kTreePrevSlot = kTreeInA | kTreePrev | kTreeInB;
 // Leaves are given as tile times their number where the tip codes are in
 // shared memory, a slot or memory child as the row behind them (else kTreeNoTip).
 constexpr uint32_t kTreeNoTip = 0xFFFFFFFFu;

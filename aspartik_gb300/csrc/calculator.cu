@@ -124,8 +124,6 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 			runs_block_ = b;
 	}
 	use_runs_ = f32_ && S_ == 4 && runs_tile_ * C_ <= 512;
-	// fused single-launch evaluation of short lists (B3G_DIRECT=0 turns
-	// it off, e.g. to time the two-kernel path)
 	// groups of 128 threads per tensor-core CTA (B3G_TC20_GROUPS = 1 or 2;
 	// default: chosen per launch from the grid size)
 	if (const char *env = std::getenv("B3G_TC20_CLUSTER")) {
@@ -163,6 +161,8 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		if (gr >= 1 && gr <= 4)
 			s20_groups_ = static_cast<uint32_t>(gr);
 	}
+	// fused single-launch evaluation of short lists (B3G_DIRECT=0 turns
+	// it off, e.g. to time the two-kernel path)
 	use_direct_ = f32_ && S_ == 4 && (C_ == 1 || C_ == 2 || C_ == 4);
 	if (const char *env = std::getenv("B3G_DIRECT"))
 		use_direct_ = use_direct_ && std::atoi(env) != 0;
@@ -1380,7 +1380,7 @@ void Calculator::launch(uint32_t n, bool matrices_mode, double clock_rate,
 void Calculator::launch20(uint32_t n, bool matrices_mode, double clock_rate,
 			  bool want_cat, TimingSlot &slot)
 {
-	poll_result_ = false; // FP32: result read back by a copy after the kernels
+	poll_result_ = false; // (the tcgen05 walk's result is read back by a copy)
 	PtabParams pt{};
 	pt.lengths = matrices_mode
 			     ? nullptr
@@ -1990,7 +1990,7 @@ uint32_t Calculator::autotune(const uint32_t *internals,
 		if (!d_tc_tab_) // built without tensor-core buffers
 			return 0;
 		// tensor cores with one and with two thread groups per CTA
-		// (unless B3G_TC20_GROUPS fixed it), then the CUDA-core walk
+		// (unless B3G_TC20_GROUPS fixed it), then the register walk
 		use_tc20_ = true;
 		float tc = INFINITY;
 		uint32_t best_groups = tc20_groups_;

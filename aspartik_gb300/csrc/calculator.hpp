@@ -176,7 +176,8 @@ class Calculator {
 	size_t off_slots_ = 0, off_tree_ = 0;
 	uint32_t assign_slots(uint32_t n, uint32_t capacity);
 	uint32_t stamp_epoch_ = 0;
-	// depth-first order of the staged list (four-state FP64, 20-state FP32)
+	// depth-first order of the staged list (all walks but the run-synchronous,
+	// the short-list, the 20-state FP64 and the tcgen05 one)
 	static constexpr uint32_t kNone = 0xFFFFFFFFu;
 	bool depth_first_ = false;
 	// the four-state FP32 form's depth-first walk of single-tree lists

@@ -11,7 +11,7 @@
 // category and walks a list depth first (heavier subtree first), so that two
 // thirds of the internal children of a random tree are the previous entry's
 // output and stay in registers; the others wait in a shared-memory slot that
-// the host assigned (Calculator::assign_tree_slots), and so do the clean
+// the host assigned (Calculator::stage_tree), and so do the clean
 // children of a list that is not the whole tree, copied there early.
 //
 // Lane l holds patterns 2l and 2l + 1: the table rows are read once for both
@@ -282,8 +282,8 @@ __device__ __forceinline__ double tree_tile(const PruneParams &prm, uint32_t t, 
 		op1 = *(const uint4 *)&next.op;
 		ca1 = codes(op.z);
 		cb = codes(op.w);
-		// the three kinds of entry of a whole tree in one straight piece of
-		// code each, anything else through memory or slots
+		// two kinds of entry of a whole tree in straight code of their own
+		// (previous x tip, cherry), anything else through slots or memory
 		const uint32_t kind = op.y & kTreeKind;
 		if (kind == kTreePrevTip) {
 			apply_rows(tab, y.v);

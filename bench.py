@@ -378,8 +378,8 @@ def protein20(device: int, steps: int, warmup: int, seed: int = 4, L: int = 128,
         precision = "f64" if form == "f64" else "f32"
         w = 8 if precision == "f64" else 4
         old_env = os.environ.get("B3G_TC20")
-        if form == "f32_cuda_cores":
-            os.environ["B3G_TC20"] = "0"
+        if form == "f32_tcgen05":
+            os.environ["B3G_TC20"] = "1"
         try:
             calc = Calculator.GB300(device, precision).make20(leaves, P, num_categories=K)
         finally:
@@ -390,8 +390,7 @@ def protein20(device: int, steps: int, warmup: int, seed: int = 4, L: int = 128,
         calc.set_weights(weights)
         calc.set_reversible(rates, pi)
         calc.set_gamma(1.0)
-        engine = ("register matrix instructions" if form == "f32_cuda_cores"
-                  else None)
+        engine = "tcgen05" if form == "f32_tcgen05" else None
         if form == "f32":
             calc.propose_lengths(*lists, 1.0)
             calc.log_likelihood()
@@ -414,9 +413,9 @@ def protein20(device: int, steps: int, warmup: int, seed: int = 4, L: int = 128,
     if "f64" in out:
         out["lnl_rel_err_f32_vs_f64"] = abs(out["f32"]["lnl"] - out["f64"]["lnl"]) / abs(
             out["f64"]["lnl"])
-    if "f32_cuda_cores" in out:
-        out["lnl_rel_diff_tensor_vs_cuda_cores"] = abs(
-            out["f32"]["lnl"] - out["f32_cuda_cores"]["lnl"]) / abs(out["f32_cuda_cores"]["lnl"])
+    if "f32_tcgen05" in out:
+        out["lnl_rel_diff_of_the_engines"] = abs(
+            out["f32"]["lnl"] - out["f32_tcgen05"]["lnl"]) / abs(out["f32_tcgen05"]["lnl"])
     return out
 
 
@@ -862,7 +861,7 @@ def run_ours(args):
     if not args.no_protein:
         prot = protein20(device, min(args.steps, 100), args.warmup)
         prot_big = protein20(device, min(args.steps, 20), args.warmup, N=50000,
-                             forms=("f32", "f32_cuda_cores"))
+                             forms=("f32", "f32_tcgen05"))
     progress("20 states")
     batch = None if args.no_batch else batched(device, min(args.steps, 200), args.warmup)
     progress("batched chains")
