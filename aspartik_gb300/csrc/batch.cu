@@ -171,8 +171,20 @@ Batch::Batch(Calculator *const *members, uint32_t count)
 		ctas_ = 2 * members_[0]->num_sms_;
 		evaluated_.assign(M, 0);
 
-		for (uint32_t form = 0; form < 4; ++form)
-			capture(form);
+		for (uint32_t form = 0; form < 4; ++form) {
+			try {
+				capture(form);
+			} catch (...) {
+				// ended here, or the thread stays in capture mode and
+				// every later launch from it is refused
+				cudaGraph_t part = nullptr;
+				cudaStreamEndCapture(stream_, &part);
+				if (part)
+					cudaGraphDestroy(part);
+				(void)cudaGetLastError();
+				throw;
+			}
+		}
 	} catch (...) {
 		release();
 		throw;
