@@ -1145,12 +1145,12 @@ cudaError_t launch_prune4_batch(const BatchParams &p, uint32_t ctas,
 			    p.smem_ops_bytes + p.smem_tips_bytes + 16 + p.smem_ptab_bytes;
 	auto kern = p.narrow ? prune4_batch_kernel<uint32_t>
 			     : prune4_batch_kernel<size_t>;
-	if (smem > 48 * 1024) {
-		static SmemOptIn opted[2];
-		const cudaError_t e = opt_in_smem(kern, opted[p.narrow ? 0 : 1]);
-		if (e != cudaSuccess)
-			return e;
-	}
+	// (with its static shared memory the kernel passes the default limit
+	// below 48 KB of dynamic already)
+	static SmemOptIn opted[2];
+	const cudaError_t e = opt_in_smem(kern, opted[p.narrow ? 0 : 1]);
+	if (e != cudaSuccess)
+		return e;
 	kern<<<ctas, 512, smem, s>>>(p);
 	return cudaGetLastError();
 }
