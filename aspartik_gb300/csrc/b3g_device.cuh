@@ -342,9 +342,9 @@ size_t soft_tab20_bytes();
 // groups, segs.
 cudaError_t launch_prune20(const PruneParams &p, cudaStream_t s);
 // Words of prm.segs that a block's shared memory holds beside the rest (kSegSmem
-// in all): the four-state FP64 walk with `warps` warps a block, the 20-state
-// FP32 walk with `groups`.
-constexpr uint32_t kSegSmem = 48u * 1024u;
+// in all, the default limit less room for a few static words): the four-state
+// FP64 walk with `warps` warps a block, the 20-state FP32 walk with `groups`.
+constexpr uint32_t kSegSmem = 48u * 1024u - 64u;
 uint32_t prune4_f64_seg_words(uint32_t warps);
 uint32_t prune20_seg_words(uint32_t groups);
 // Blocks of `groups` warps of that walk that one SM holds.

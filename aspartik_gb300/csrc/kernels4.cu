@@ -73,7 +73,9 @@ cudaError_t launch_beside(void (*kern)(P), dim3 grid, dim3 block, size_t smem, c
 	cfg.stream = s;
 	cfg.attrs = &attr;
 	cfg.numAttrs = 1;
-	return cudaLaunchKernelEx(&cfg, kern, p);
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+	(void)cudaGetLastError(); // or the next launch's check would find it again
+	return e;
 }
 
 // ---------------------------------------------------------------------------
@@ -919,7 +921,8 @@ cudaError_t launch_ptab4(const PtabParams &p, bool f32, cudaStream_t s)
 // and device (a permission, not a reservation: no call lowers another's
 // limit and later launches pay nothing).  A limit set to each launch's own
 // size would be the process's too: a second thread with a smaller list could
-// lower it between this one's call and its launch.
+// lower it between this one's call and its launch.  Not only above 48 KB of
+// dynamic shared memory: the static part counts towards the default limit.
 struct SmemOptIn {
 	std::atomic<bool> done[64] = {};
 };
@@ -960,12 +963,10 @@ static cudaError_t launch_prune4_t(const PruneParams &p, uint32_t tile,
 		!p.wide_index && narrow_index((uint64_t)p.num_leaves * 2, p.C, p.ldp);
 	auto kern = narrow ? prune4_kernel<VT, kPow2, uint32_t>
 			   : prune4_kernel<VT, kPow2, size_t>;
-	if (smem > 48 * 1024) {
-		static SmemOptIn opted[2];
-		const cudaError_t e = opt_in_smem(kern, opted[narrow ? 0 : 1]);
-		if (e != cudaSuccess)
-			return e;
-	}
+	static SmemOptIn opted[2];
+	const cudaError_t e = opt_in_smem(kern, opted[narrow ? 0 : 1]);
+	if (e != cudaSuccess)
+		return e;
 	kern<<<grid, block, smem, s>>>(p);
 	return cudaGetLastError();
 }
@@ -1057,13 +1058,11 @@ cudaError_t launch_prune4_runs(const PruneParams &p, uint32_t ctas,
 				      : prune4_runs_kernel<size_t, 1024>)
 			    : (narrow ? prune4_runs_kernel<uint32_t, 512>
 				      : prune4_runs_kernel<size_t, 512>);
-	if (smem > 48 * 1024) {
-		static SmemOptIn opted[4];
-		const cudaError_t e =
-			opt_in_smem(kern, opted[(block == 1024 ? 2 : 0) + (narrow ? 0 : 1)]);
-		if (e != cudaSuccess)
-			return e;
-	}
+	static SmemOptIn opted[4];
+	const cudaError_t e =
+		opt_in_smem(kern, opted[(block == 1024 ? 2 : 0) + (narrow ? 0 : 1)]);
+	if (e != cudaSuccess)
+		return e;
 	kern<<<ctas, threads, smem, s>>>(p);
 	return cudaGetLastError();
 }
@@ -1101,12 +1100,10 @@ cudaError_t launch_prune4_tree(const PruneParams &p, bool clean, cudaStream_t s)
 		prune4_tree_kernel<2, false, false>, prune4_tree_kernel<2, false, true>,
 		prune4_tree_kernel<2, true, false>,  prune4_tree_kernel<2, true, true>};
 	void (*const kern)(PruneParams) = kerns[v];
-	if (smem > 48 * 1024) {
-		static SmemOptIn opted[8];
-		const cudaError_t e = opt_in_smem(kern, opted[v]);
-		if (e != cudaSuccess)
-			return e;
-	}
+	static SmemOptIn opted[8];
+	const cudaError_t e = opt_in_smem(kern, opted[v]);
+	if (e != cudaSuccess)
+		return e;
 	return launch_beside(kern, dim3(p.ldp / p.tile), dim3(32 * p.C * p.groups), smem, s, p);
 }
 
@@ -1145,8 +1142,6 @@ cudaError_t launch_prune4_batch(const BatchParams &p, uint32_t ctas,
 			    p.smem_ops_bytes + p.smem_tips_bytes + 16 + p.smem_ptab_bytes;
 	auto kern = p.narrow ? prune4_batch_kernel<uint32_t>
 			     : prune4_batch_kernel<size_t>;
-	// (with its static shared memory the kernel passes the default limit
-	// below 48 KB of dynamic already)
 	static SmemOptIn opted[2];
 	const cudaError_t e = opt_in_smem(kern, opted[p.narrow ? 0 : 1]);
 	if (e != cudaSuccess)
