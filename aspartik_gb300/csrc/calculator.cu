@@ -149,6 +149,7 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 		use_tc20_ = f32_ && S_ == 20 && std::atoi(env) != 0;
 		tc20_off = std::atoi(env) == 0;
 	}
+	tc20_by_list_ = f32_ && S_ == 20 && !use_tc20_ && !tc20_off;
 	// groups of the FP64 run form (B3G_F64_GROUPS: 1, 2, 4, 8 or 16 where
 	// they fit a block; default: chosen per list)
 	if (const char *env = std::getenv("B3G_F64_GROUPS")) {
@@ -158,8 +159,10 @@ Calculator::Calculator(const b3g_config &cfg, const uint8_t *samples)
 	}
 	if (const char *env = std::getenv("B3G_S20_GROUPS")) {
 		const int gr = std::atoi(env);
-		if (gr >= 1 && gr <= 4)
+		if (gr >= 1 && gr <= 4) {
 			s20_groups_ = static_cast<uint32_t>(gr);
+			tc20_by_list_ = false;
+		}
 	}
 	// fused single-launch evaluation of short lists (B3G_DIRECT=0 turns
 	// it off, e.g. to time the two-kernel path)
@@ -566,6 +569,8 @@ void Calculator::stage_ops(const uint32_t *internals, const uint32_t *children,
 	runs[n_runs_] = n;
 	if (n_runs_)
 		max_run_ = std::max(max_run_, n - runs[n_runs_ - 1]);
+	if (tc20_by_list_)
+		use_tc20_ = tc20_list(n);
 	depth_first_ = S_ == 4 ? !f32_ : f32_ && !use_tc20_;
 	if (!depth_first_)
 		return;
@@ -1989,6 +1994,7 @@ uint32_t Calculator::autotune(const uint32_t *internals,
 	if (S_ == 20) {
 		if (!d_tc_tab_) // built without tensor-core buffers
 			return 0;
+		tc20_by_list_ = false; // one choice for every list from here
 		// tensor cores with one and with two thread groups per CTA
 		// (unless B3G_TC20_GROUPS fixed it), then the register walk
 		use_tc20_ = true;

@@ -101,6 +101,23 @@ class Calculator {
 		       uint32_t n, bool tree);
 	void stage_tree(uint32_t n);
 	void stage_order(uint32_t n);
+	// Whether the staged 20-state FP32 list takes the tcgen05 walk where neither
+	// a switch nor the autotuner has decided: long lists over few columns whose
+	// runs have entries for the 16 groups of a cluster (the register walk has
+	// four warps a tile), and few entries, mostly tips, over very many columns.
+	// Us, register walk / tcgen05, whole trees, taxa x patterns x categories:
+	// 1,000 x 40 x 1 333 / 266, 3,000 x 2,000 x 1 1,028 / 805, 3,000 x 2,000 x 2
+	// 1,149 / 1,063, but 500 x 40 x 1 180 / 179, 1,500 x 5,000 x 1 639 / 735,
+	// 3,000 x 40 x 3 1,232 / 1,206, a ladder of 700 x 300 x 4 693 / 2,149; 3 x
+	// 300,000 x 1 111 / 102, 3 x 150,000 x 4 166 / 121, 10 x 110,000 x 4 208 / 197,
+	// but 3 x 200,000 x 1 85 / 84, 40 x 150,000 x 4 801 / 790, a path of 10 x
+	// 110,000 x 4 164 / 169.
+	bool tc20_list(uint32_t n) const
+	{
+		const uint64_t cols = (uint64_t)C_ * ldp_;
+		return n >= 800 ? C_ <= 2 && cols <= 4096 && n >= 16 * n_runs_
+				: n <= 10 && tip_children_ > n && cols >= 300000;
+	}
 	// Whether a single-tree list takes the depth-first FP32 walk: where its
 	// 64-pattern tiles reach half of the SMs, or the list is small.  Us per
 	// whole tree, run walk / depth first: 256 taxa x 8,000 patterns x 4
@@ -305,6 +322,7 @@ class Calculator {
 	bool use_runs_ = false;
 	bool use_direct_ = false;
 	bool use_tc20_ = false;
+	bool tc20_by_list_ = false; // chosen list by list (tc20_list)
 	uint32_t tc20_groups_ = 0; // 0: per launch from the grid size
 	bool tc20_groups_fixed_ = false; // set by B3G_TC20_GROUPS
 	uint32_t tc20_cluster_ = 1;      // CTAs per work item when fixed
